@@ -423,6 +423,11 @@ def pair_chunks(x, excl, box, most=24_000_000):
         yield a, b, d, torch.where(other, r2, torch.ones_like(r2)), other, far, one4
 
 
+def scale14(one4, s, dtype):
+    """s on the 1-4 pairs, 1 elsewhere."""
+    return 1.0 + (s - 1.0) * one4.to(dtype)
+
+
 def switch(r, inner, cut):
     """Energy switch (1 - u^2/w^2)^2 beyond `inner`, and its derivative."""
     u = torch.clamp(r - inner, min=0.0)
@@ -448,8 +453,8 @@ def nb_exact(x, par, excl, box, p, forces):
     for a, b, d, r2, other, far, one4 in pair_chunks(x, excl, box):
         f = (far & (r2 <= C * C)).to(x.dtype)
         r = torch.sqrt(r2)
-        sv = torch.where(one4, p["Vdw14Scaling"], 1.0) * f
-        qq = q[a:b, None] * q[None, :] * ec * torch.where(one4, p["Elec14Scaling"], 1.0) * f
+        sv = scale14(one4, p["Vdw14Scaling"], x.dtype) * f
+        qq = q[a:b, None] * q[None, :] * ec * scale14(one4, p["Elec14Scaling"], x.dtype) * f
         ev, dv = lj(r2, r, R[a:b, None] + R[None, :], se[a:b, None] * se[None, :] * sv, p["VdwInnerCutoff"],
                     p["VdwCutoff"])
         if p["ForceSwitch"]:
@@ -507,10 +512,11 @@ def gb_exact(x, par, excl, p, forces, threshold=True):
         S, dS = switch(r, p["InnerCutoff"], p["Cutoff"])
         ep = pre * qq * fgb * f * on.to(x.dtype)
         vac = (far & ins).to(x.dtype)
-        ec = torch.where(on, ECONV / p["DielectricSolute"], ECONV / p["DielectricSolvent"])
-        el = ec * qq / r * torch.where(one4, p["Elec14Scaling"], 1.0) * vac
+        near = on.to(x.dtype)
+        ec = near * (ECONV / p["DielectricSolute"]) + (1.0 - near) * (ECONV / p["DielectricSolvent"])
+        el = ec * qq / r * scale14(one4, p["Elec14Scaling"], x.dtype) * vac
         ev, dv = lj(r2, r, R[a:b, None] + R[None, :],
-                    se[a:b, None] * se[None, :] * torch.where(one4, p["Vdw14Scaling"], 1.0) * vac,
+                    se[a:b, None] * se[None, :] * scale14(one4, p["Vdw14Scaling"], x.dtype) * vac,
                     p["VdwInnerCutoff"], p["VdwCutoff"])
         E = E + torch.stack([0.5 * ev.sum(), 0.5 * (el * S).sum(), (ep * S).sum()])
         if forces:
