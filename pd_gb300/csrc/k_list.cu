@@ -263,13 +263,17 @@ __global__ void k_blocks(DevView v, int* hmax) {
     }
   }
   if (lane == 0) {
-    float4 h;
-    for (int c = 0; c < 3; c++) v.center[3 * warp + c] = 0.5 * (lo[c] + hi[c]);
-    h.x = (float)(0.5 * (hi[0] - lo[0])) + 1e-4f;
-    h.y = (float)(0.5 * (hi[1] - lo[1])) + 1e-4f;
-    h.z = (float)(0.5 * (hi[2] - lo[2])) + 1e-4f;
-    h.w = 0.f;
+    // the centre is rounded to FP32 (any point near the middle serves), so that
+    // centre differences are exact in double-float arithmetic
+    float cf[3], hf[3];
+    for (int c = 0; c < 3; c++) {
+      cf[c] = (float)(0.5 * (lo[c] + hi[c]));
+      v.center[3 * warp + c] = (double)cf[c];
+      hf[c] = (float)fmax(hi[c] - (double)cf[c], (double)cf[c] - lo[c]) + 1e-4f;
+    }
+    const float4 h = make_float4(hf[0], hf[1], hf[2], 0.f);
     v.half[warp] = h;
+    v.cenf[warp] = make_float4(cf[0], cf[1], cf[2], 0.f);
     const int s3 = 3 * v.slot_sys[warp];
     atomicMax(&hmax[s3], f2ord(h.x));
     atomicMax(&hmax[s3 + 1], f2ord(h.y));

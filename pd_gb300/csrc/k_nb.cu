@@ -70,21 +70,33 @@ __device__ __forceinline__ float nb_force_f(const NBConst& k, float r2, float rs
   return g;
 }
 
+// (ENERGY) what one warp keeps in shared memory for the energies of its work
+// item: both blocks' atoms as double-floats in the i block's frame and the list
+// of the pairs inside the cutoff
+struct NBEShared {
+  float4 ih[32], il[32], ip[32];   // (x, y, z, q) high and low parts; (R, sqrt(eps)) high and low
+  float4 jh[32], jl[32], jp[32];
+  int js[32];                      // j slots
+  unsigned short pair[1024];       // i lane | j row << 5 | 1-4 << 10
+};
+
 // 32 rotation steps of one work item: lane i holds an i atom, (xj, pj) the
 // lane's j atom already in i's frame.  Tiles: j slot jb + lane, per-pair image
 // when mi.  GROUP: the j atoms of a group (slots in gent[].w, -1 = empty lane,
-// parked far away), never masked, one image.
+// parked far away), never masked, one image.  ENERGY: the pairs inside the
+// cutoff are listed in sh->pair; returns their number.
 template <int ELEC, bool MASKED, bool ENERGY, bool GROUP, bool SW>
-__device__ __forceinline__ void nb_rot(const DevView& v, const NBConst& k, const SystemInfo& S, int lane, int si,
-                                       int ai, const float4& xi, const float4& pi, float qi, unsigned ex, unsigned m14,
-                                       float4 xj, float4 pj, bool mi_tile, int jb, const float4* gent, NBAcc& I,
-                                       NBAcc& J, double& ev, double& ee, double& vir) {
+__device__ __forceinline__ int nb_rot(const DevView& v, const NBConst& k, const SystemInfo& S, int lane, int si,
+                                      const float4& xi, const float4& pi, float qi, unsigned ex, unsigned m14,
+                                      float4 xj, float4 pj, bool mi_tile, int jb, const float4* gent, NBAcc& I,
+                                      NBAcc& J, NBEShared* sh) {
   const bool mi = !GROUP && mi_tile;
   float Lx = 1.f, Ly = 1.f, Lz = 1.f;
   if (!GROUP && S.periodic) {
     Lx = (float)S.box[0]; Ly = (float)S.box[1]; Lz = (float)S.box[2];
   }
   const float iLx = 1.f / Lx, iLy = 1.f / Ly, iLz = 1.f / Lz;
+  int np = 0;
 #pragma unroll 4
   for (int kk = 0; kk < 32; kk++) {
     float dx = xj.x - xi.x, dy = xj.y - xi.y, dz = xj.z - xi.z;
@@ -97,38 +109,27 @@ __device__ __forceinline__ void nb_rot(const DevView& v, const NBConst& k, const
     bool listed = true;
     if (MASKED) listed = !((ex >> kk) & 1u);
     bool in = r2 <= k.cut2;
-    double r2d = 0.0;  // (ENERGY) the pair's FP64 squared distance
-    int sj = 0;        // (ENERGY) the j slot
-    if (ENERGY) {
-      if (listed && (!GROUP || in || r2 <= 1.01f * k.cut2)) {
-        sj = GROUP ? __float_as_int(gent[(lane + kk) & 31].w) : jb + ((lane + kk) & 31);
-        if (sj >= 0) {
-          r2d = nb_r2_fp64(v, S, si, sj);
-          in = r2d <= k.cut2_dd;
-        }
-      }
-    } else if (listed && (fabsf(r2 - k.cut2) <= 2e-6f * k.cut2 ||
-                          (!SW && fabsf(r2 - k.vdwcut2) <= 2e-6f * k.vdwcut2))) {
+    if (listed && (fabsf(r2 - k.cut2) <= 2e-6f * k.cut2 ||
+                   (!SW && fabsf(r2 - k.vdwcut2) <= 2e-6f * k.vdwcut2))) {
       // at a hard cutoff: decide, and take the distance, in FP64 (FP64 work only on this branch)
       const int sjr = GROUP ? __float_as_int(gent[(lane + kk) & 31].w) : jb + ((lane + kk) & 31);
       const double d2 = nb_r2_fp64(v, S, si, sjr);
       in = d2 <= k.cut2_dd;
       r2 = (float)d2;
     }
-    if (listed && in) {
+    const bool take = listed && in;
+    if (ENERGY) {
+      const unsigned m = __ballot_sync(0xffffffffu, take);
+      if (take)
+        sh->pair[np + __popc(m & ((1u << lane) - 1u))] =
+            (unsigned short)(lane | (((lane + kk) & 31) << 5) | (MASKED && ((m14 >> kk) & 1u) ? 1024 : 0));
+      np += __popc(m);
+    }
+    if (take) {
       const bool is14 = MASKED && ((m14 >> kk) & 1u);
       const float eps = pi.y * pj.y * (is14 ? k.vdw14 : 1.f);
       const float qq = qi * xj.w * (is14 ? k.elec14 : 1.f);
       const float fs = nb_force_f<ELEC, SW>(k, r2, pi.x + pj.x, eps, qq);
-      if (ENERGY) {
-        // energy of this pair in FP64 from FP64 positions and parameters
-        const int aj = v.sorted_atom[sj];
-        double fsd, rdd;
-        double epsd = v.sqeps[ai] * v.sqeps[aj] * (is14 ? k.vdw14_d : 1.0);
-        double qqd = v.charge[ai] * v.charge[aj] * k.econv_diel_d * (is14 ? k.elec14_d : 1.0);
-        nb_pair<double, ELEC>(k, r2d, v.radius[ai] + v.radius[aj], epsd, qqd, ev, ee, fsd, rdd);
-        vir += rdd;
-      }
       I.fx += fs * dx; I.fy += fs * dy; I.fz += fs * dz;
       J.fx -= fs * dx; J.fy -= fs * dy; J.fz -= fs * dz;
     }
@@ -144,6 +145,176 @@ __device__ __forceinline__ void nb_rot(const DevView& v, const NBConst& k, const
     J.fy = __shfl_sync(0xffffffffu, J.fy, src);
     J.fz = __shfl_sync(0xffffffffu, J.fz, src);
   }
+  return np;
+}
+
+// ---------------------------------------------------------------------------
+// Pair energies.  FP32 cannot hold them (water's electrostatics cancel ~5000
+// fold, and so do the force-switch polynomials), and the FP64 pipe is narrow:
+// they are formed in double-float arithmetic (pdgpu_df.cuh, ~45 bits) from
+// positions and parameters held as double-floats.  The rotation lists the pairs
+// inside the cutoff (about a fifth of those it visits); the list is then dealt
+// over the lanes, so the ~300 instructions of a pair's energy run on full warps.
+// FP64 pair energies on the rotation itself, bound by the FP64 pipe, had taken
+// 5.85 ms on the solvated 22,489 atoms at 15 A (force switch), 0.331 ms on 667
+// waters at 12 A; this takes 0.472 and 0.046 ms, bound by FP32 issue.  Against
+// 64-bit sums the energies are as close as before (within 2e-8 kcal/mol, one
+// fixed-point rounding per item instead of one per lane).
+// ---------------------------------------------------------------------------
+
+// remainders of the packed slots (before each energy pass)
+__global__ void k_nb_records(DevView v, const double* charge, float4* rlo, float2* plo) {
+  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= v.nslots) return;
+  const int a = v.sorted_atom[s];
+  float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
+  float2 p = make_float2(0.f, 0.f);
+  if (a >= 0) {
+    const int b = s >> 5;
+    const SystemInfo& S = v.sys[v.slot_sys[b]];
+    const float4 x = v.xq[s], q = v.par[s];
+    const float h[3] = {x.x, x.y, x.z};
+    float l[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      double d = v.pos[3 * a + c] - v.center[3 * b + c];
+      if (S.periodic) d -= S.box[c] * rint(d * S.ibox[c]);
+      l[c] = (float)(d - (double)h[c]);
+    }
+    r = make_float4(l[0], l[1], l[2], (float)(charge[a] - (double)x.w));
+    p = make_float2((float)(v.radius[a] - (double)q.x), (float)(v.sqeps[a] - (double)q.y));
+  }
+  rlo[s] = r;
+  plo[s] = p;
+}
+
+// centre of block bj seen from block bi, as double-floats, in the image the
+// FP32 offset o was taken in
+__device__ __forceinline__ void df_offset(const DevView& v, const SystemInfo& S, int bi, int bj, const float o[3],
+                                          DF O[3]) {
+  const float4 ci = v.cenf[bi], cj = v.cenf[bj];
+  const float a[3] = {ci.x, ci.y, ci.z}, b[3] = {cj.x, cj.y, cj.z};
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    O[c] = df_two_sum(b[c], -a[c]);
+    if (S.periodic) {
+      const float n = -rintf((O[c].h - o[c]) / S.boxf[c].h);
+      O[c] = df_norm(df_add(O[c], df_scale(S.boxf[c], n)));
+    }
+  }
+}
+
+struct NBESum {
+  DF vdw, elec, vir;
+};
+
+// energies of one listed pair into the sums (same law as nb_pair)
+template <int ELEC, bool SW>
+__device__ __forceinline__ void nb_energy_df(const DevView& v, const NBConst& k, const NBEConst& e,
+                                             const SystemInfo& S, bool mi, int ibase, const NBEShared* sh,
+                                             unsigned code, NBESum& sum) {
+  const int il = code & 31, jl = (code >> 5) & 31;
+  const bool is14 = code & 1024u;
+  const float4 xh = sh->ih[il], xl = sh->il[il], xp = sh->ip[il];
+  const float4 yh = sh->jh[jl], yl = sh->jl[jl], yp = sh->jp[jl];
+  DF dx = df_sub(DF{yh.x, yl.x}, DF{xh.x, xl.x});
+  DF dy = df_sub(DF{yh.y, yl.y}, DF{xh.y, xl.y});
+  DF dz = df_sub(DF{yh.z, yl.z}, DF{xh.z, xl.z});
+  if (mi) {
+    dx = df_add(dx, df_scale(S.boxf[0], -rintf(dx.h / S.boxf[0].h)));
+    dy = df_add(dy, df_scale(S.boxf[1], -rintf(dy.h / S.boxf[1].h)));
+    dz = df_add(dz, df_scale(S.boxf[2], -rintf(dz.h / S.boxf[2].h)));
+  }
+  const DF r2 = df_norm2(dx, dy, dz);
+  const DF ir = df_rsqrt(r2);
+  const DF r = df_norm(df_mul(r2, ir));
+  const DF one = DF{1.f, 0.f};
+  // LJ: energy and r dE/dr before switching
+  DF Ev = DF{0.f, 0.f}, gv = Ev;
+  DF u = df_sub(r, e.vdwcut);
+  bool vin = e.dovdw && u.h + u.l < 0.f;
+  if (e.dovdw && e.vdw_hard && fabsf(u.h) <= 2e-6f * e.vdwcut.h)   // at an unswitched end of LJ: decide in FP64
+    vin = sqrt(nb_r2_fp64(v, S, ibase + il, sh->js[jl])) < k.vdwcut_d;
+  if (vin) {
+    const DF R = df_norm(df_add(DF{xp.x, xp.z}, DF{yp.x, yp.z}));
+    const DF t = df_norm(df_mul(R, ir)), t2 = df_norm(df_mul(t, t));
+    const DF B = df_norm(df_mul(df_mul(t2, t2), t2)), A = df_mul(B, B);
+    DF eps = df_norm(df_mul(DF{xp.y, xp.w}, DF{yp.y, yp.w}));
+    if (is14) eps = df_norm(df_mul(eps, e.vdw14));
+    Ev = df_norm(df_mul(eps, df_norm(df_sub(A, df_scale2(B, 2.f)))));
+    gv = df_norm(df_scale(df_mul(eps, df_norm(df_sub(A, B))), -12.f));
+    if (!SW) {
+      DF w = df_sub(r, e.vdwinner);
+      if (w.h > 0.f) {
+        w = df_norm(w);
+        const DF wi = df_norm(df_mul(w, e.vdwinvw2));
+        const DF sw = df_norm(df_sub(one, df_mul(w, wi)));
+        const DF Sv = df_norm(df_mul(sw, sw));
+        const DF dS = df_norm(df_scale2(df_mul(df_mul(wi, sw), r), -4.f));   // r S'
+        gv = df_add(df_mul(Sv, gv), df_mul(Ev, dS));
+        Ev = df_mul(Ev, Sv);
+      }
+    }
+  }
+  // Coulomb
+  DF Ee = DF{0.f, 0.f}, ge = Ee;
+  if (ELEC != 0) {
+    DF qq = df_norm(df_mul(DF{xh.w, xl.w}, DF{yh.w, yl.w}));   // (i's charge carries the Coulomb constant)
+    if (is14) qq = df_norm(df_mul(qq, e.elec14));
+    Ee = df_norm(df_mul(qq, ir));
+    ge = df_neg(Ee);
+    if (ELEC == 3) {
+      DF w = df_sub(r, e.inner);
+      if (w.h > 0.f) {
+        w = df_norm(w);
+        const DF wi = df_norm(df_mul(w, e.invw2));
+        const DF sw = df_norm(df_sub(one, df_mul(w, wi)));
+        const DF Se = df_norm(df_mul(sw, sw));
+        const DF dS = df_norm(df_scale2(df_mul(df_mul(wi, sw), r), -4.f));
+        if (SW) {   // one switch for both terms
+          gv = df_add(df_mul(Se, gv), df_mul(Ev, dS));
+          Ev = df_mul(Ev, Se);
+        }
+        ge = df_add(df_mul(Se, ge), df_mul(Ee, dS));
+        Ee = df_mul(Ee, Se);
+      }
+    } else if (ELEC == 4) {
+      // Steinbach & Brooks force switch, nonbonded.cpp:798-819
+      if (df_sub(r, e.inner).h > 0.f) {
+        const DF c2 = df_norm(df_sub(e.cut2, r2));
+        // -qq sA / r (C^2 - r^2)^2 (C^2 - 3 I^2 + 2 r^2)
+        const DF f = df_norm(df_mul(df_mul(c2, c2), df_norm(df_add(e.fsw_k, df_scale2(r2, 2.f)))));
+        ge = df_neg(df_mul(df_norm(df_mul(e.sA, f)), Ee));
+        // -qq (sA r (sB / r^2 + sC + sD r^2 + sE r^4) - V(C))
+        DF h = df_norm(df_add(e.sD, df_mul(e.sE, r2)));
+        h = df_norm(df_add(e.sC, df_mul(h, r2)));
+        h = df_norm(df_add(df_mul(h, r), df_mul(e.sB, ir)));
+        Ee = df_neg(df_mul(qq, df_norm(df_sub(df_mul(e.sA, h), e.cutV))));
+      } else {
+        Ee = df_mul(qq, df_norm(df_sub(ir, e.eshift)));
+      }
+    }
+  }
+  df_acc(sum.vdw, df_norm(Ev));
+  df_acc(sum.elec, df_norm(Ee));
+  df_acc(sum.vir, df_norm(df_add(gv, ge)));
+}
+
+// one block's atom of this lane into the shared rows (O: frame offset)
+__device__ __forceinline__ void nb_stage(float4* h, float4* l, float4* p, int row, const DevView& v, int slot,
+                                         const DF* O, const DF* qscale) {
+  const float4 x = v.xq[slot], rl = v.rlo[slot], par = v.par[slot];
+  const float2 pl = v.plo[slot];
+  DF X = DF{x.x, rl.x}, Y = DF{x.y, rl.y}, Z = DF{x.z, rl.z}, Q = DF{x.w, rl.w};
+  if (O) {
+    X = df_norm(df_add(X, O[0]));
+    Y = df_norm(df_add(Y, O[1]));
+    Z = df_norm(df_add(Z, O[2]));
+  }
+  if (qscale) Q = df_norm(df_mul(Q, *qscale));
+  h[row] = make_float4(X.h, Y.h, Z.h, Q.h);
+  l[row] = make_float4(X.l, Y.l, Z.l, Q.l);
+  p[row] = make_float4(par.x, par.y, pl.x, pl.y);
 }
 
 // per-tile FP32 sums enter 64-bit fixed point before they are combined, so a
@@ -171,33 +342,16 @@ __device__ __forceinline__ void nb_flush(const DevView& v, int s, const NBAcc& a
   nb_flush_fix(v, s, F);
 }
 
-// per-tile FP64 energy sums in fixed point, combined per run of tiles
-struct NBEFix {
-  long long vdw, elec, vir;
-};
-
-__device__ __forceinline__ void nb_efix_in(NBEFix& F, double& ev, double& ee, double& vir) {
-  F.vdw += fix_energy_d(ev);
-  F.elec += fix_energy_d(ee);
-  F.vir += fix_energy_d(vir);
-  ev = ee = vir = 0.0;
-}
-
-__device__ __forceinline__ void nb_flush_energy(const DevView& v, int lane, int bi, NBEFix& F) {
-  long long e0 = warp_sum_ll(F.vdw), e1 = warp_sum_ll(F.elec), e2 = warp_sum_ll(F.vir);
-  if (lane == 0) {
-    long long* E = v.eacc + (size_t)v.slot_sys[bi] * E_NSLOTS;
-    atomic_add_ll(&E[E_VDW], e0);
-    atomic_add_ll(&E[E_ELEC], e1);
-    atomic_add_ll(&E[E_VIRIAL], e2);
-  }
-  F = {0, 0, 0};
-}
-
 // One warp per work item, grid-stride: the tiles left on the tile path, then the
-// j-atom groups (cull: the last list build wrote them and they fit)
+// j-atom groups (cull: the last list build wrote them and they fit).  The energy
+// kernel's CTAs hold 4 warps (each warp keeps 5 KB of shared memory).
+constexpr int kNbThreads = 256, kNbEThreads = 128;
 template <int ELEC, bool ENERGY, bool SW = false>
-__global__ void __launch_bounds__(256, ENERGY ? 0 : 4) k_nb_tiles(const __grid_constant__ DevView v, const __grid_constant__ NBConst k, int cull) {
+__global__ void __launch_bounds__(ENERGY ? kNbEThreads : kNbThreads, ENERGY ? 5 : 4)
+    k_nb_tiles(const __grid_constant__ DevView v, const __grid_constant__ NBConst k, const __grid_constant__ NBEConst e,
+               int cull) {
+  __shared__ NBEShared shared[ENERGY ? kNbEThreads / 32 : 1];
+  NBEShared* sh = ENERGY ? &shared[threadIdx.x >> 5] : nullptr;
   const int lane = threadIdx.x & 31;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   const bool grouped = cull && v.cull_n[2];
@@ -205,8 +359,9 @@ __global__ void __launch_bounds__(256, ENERGY ? 0 : 4) k_nb_tiles(const __grid_c
   const int nitem = nrest + (grouped ? v.cull_n[1] : 0);
   for (int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < nitem; w += nwarps) {
     NBAcc I = {0.f, 0.f, 0.f}, J = {0.f, 0.f, 0.f};
-    double ev = 0.0, ee = 0.0, vir = 0.0;
-    int bi, sjl;
+    int bi, sjl, np;
+    bool mi = false;
+    float o[3];
     if (w < nrest) {
       const Tile T = v.tiles[grouped ? v.cull_rest[w] : w];
       bi = T.bi;
@@ -214,7 +369,6 @@ __global__ void __launch_bounds__(256, ENERGY ? 0 : 4) k_nb_tiles(const __grid_c
       const int si = T.bi * 32 + lane;
       const float4 xi = v.xq[si], pi = v.par[si];
       const float qi = xi.w * k.econv_diel;
-      const int ai = ENERGY ? v.sorted_atom[si] : 0;
       const SystemInfo& S = v.sys[v.slot_sys[T.bi]];
       unsigned ex = 0u, m14 = 0u;
       if (T.mask >= 0) {
@@ -226,45 +380,66 @@ __global__ void __launch_bounds__(256, ENERGY ? 0 : 4) k_nb_tiles(const __grid_c
       // j positions moved into i's frame (the tile's centre offset, periodic image included)
       float4 xj = v.xq[sjl];
       const float4 pj = v.par[sjl];
+      o[0] = T.ox;
+      o[1] = T.oy;
+      o[2] = T.oz;
       xj.x += T.ox;
       xj.y += T.oy;
       xj.z += T.oz;
-      const bool mi = T.flags & 1;
+      mi = T.flags & 1;
       if (tile_masked(T))
-        nb_rot<ELEC, true, ENERGY, false, SW>(v, k, S, lane, si, ai, xi, pi, qi, ex, m14, xj, pj, mi, T.bj * 32,
-                                          nullptr, I, J, ev, ee, vir);
+        np = nb_rot<ELEC, true, ENERGY, false, SW>(v, k, S, lane, si, xi, pi, qi, ex, m14, xj, pj, mi, T.bj * 32,
+                                                   nullptr, I, J, sh);
       else
-        nb_rot<ELEC, false, ENERGY, false, SW>(v, k, S, lane, si, ai, xi, pi, qi, ex, m14, xj, pj, mi, T.bj * 32,
-                                           nullptr, I, J, ev, ee, vir);
+        np = nb_rot<ELEC, false, ENERGY, false, SW>(v, k, S, lane, si, xi, pi, qi, ex, m14, xj, pj, mi, T.bj * 32,
+                                                    nullptr, I, J, sh);
       nb_flush(v, si, I);
     } else {
       const int g = w - nrest;
       bi = v.cull_bi[g];
       const float4* gent = v.cull_ent + (size_t)g * 32;
-      const float4 e = gent[lane];
-      sjl = __float_as_int(e.w);
+      const float4 en = gent[lane];
+      sjl = __float_as_int(en.w);
+      o[0] = en.x;
+      o[1] = en.y;
+      o[2] = en.z;
       const int si = bi * 32 + lane;
       const float4 xi = v.xq[si], pi = v.par[si];
       const float qi = xi.w * k.econv_diel;
-      const int ai = ENERGY ? v.sorted_atom[si] : 0;
       const SystemInfo& S = v.sys[v.slot_sys[bi]];
       float4 xj = make_float4(1.0e15f, 1.0e15f, 1.0e15f, 0.f), pj = make_float4(0.f, 0.f, 0.f, 0.f);
       if (sjl >= 0) {
         xj = v.xq[sjl];
         pj = v.par[sjl];
-        xj.x += e.x;
-        xj.y += e.y;
-        xj.z += e.z;
+        xj.x += en.x;
+        xj.y += en.y;
+        xj.z += en.z;
       }
-      nb_rot<ELEC, false, ENERGY, true, SW>(v, k, S, lane, si, ai, xi, pi, qi, 0u, 0u, xj, pj, false, 0, gent, I, J,
-                                        ev, ee, vir);
+      np = nb_rot<ELEC, false, ENERGY, true, SW>(v, k, S, lane, si, xi, pi, qi, 0u, 0u, xj, pj, false, 0, gent, I, J,
+                                                 sh);
       nb_flush(v, si, I);
     }
     if (sjl >= 0) nb_flush(v, sjl, J);
     if (ENERGY) {
-      NBEFix EF = {0, 0, 0};
-      nb_efix_in(EF, ev, ee, vir);
-      nb_flush_energy(v, lane, bi, EF);
+      const SystemInfo& S = v.sys[v.slot_sys[bi]];
+      nb_stage(sh->ih, sh->il, sh->ip, lane, v, bi * 32 + lane, nullptr, &e.econv);
+      sh->js[lane] = sjl;
+      if (sjl >= 0) {
+        DF O[3];
+        df_offset(v, S, bi, sjl >> 5, o, O);
+        nb_stage(sh->jh, sh->jl, sh->jp, lane, v, sjl, O, nullptr);
+      }
+      __syncwarp();
+      NBESum sum = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
+      for (int p = lane; p < np; p += 32) nb_energy_df<ELEC, SW>(v, k, e, S, mi, bi * 32, sh, sh->pair[p], sum);
+      // the lanes' sums meet in double-float and enter fixed point once per item
+      const DF ev = df_warp_sum(sum.vdw), ee = df_warp_sum(sum.elec), vir = df_warp_sum(sum.vir);
+      const DF x = lane == 0 ? ev : (lane == 1 ? ee : vir);
+      if (lane < 3) {
+        long long* E = v.eacc + (size_t)v.slot_sys[bi] * E_NSLOTS;
+        atomic_add_ll(&E[lane == 0 ? E_VDW : (lane == 1 ? E_ELEC : E_VIRIAL)], fix_energy_d((double)x.h + (double)x.l));
+      }
+      __syncwarp();
     }
   }
 }
@@ -273,22 +448,30 @@ template <bool E>
 static void launch_nb_mode(Context& c, const NBConst& k, int g) {
   DevView v = c.view();
   const int cull = c.cull_built ? 1 : 0;
+  const NBEConst e = make_nbe_const(k);
+  constexpr int T = E ? kNbEThreads : kNbThreads;
+  g *= kNbThreads / T;
   switch (k.elecmode) {
-    case 0: k_nb_tiles<0, E><<<g, 256, 0, c.stream>>>(v, k, cull); break;
-    case 1: k_nb_tiles<1, E><<<g, 256, 0, c.stream>>>(v, k, cull); break;
+    case 0: k_nb_tiles<0, E><<<g, T, 0, c.stream>>>(v, k, e, cull); break;
+    case 1: k_nb_tiles<1, E><<<g, T, 0, c.stream>>>(v, k, e, cull); break;
     case 3:
-      if (k.samesw && !E) k_nb_tiles<3, false, true><<<g, 256, 0, c.stream>>>(v, k, cull);
-      else k_nb_tiles<3, E><<<g, 256, 0, c.stream>>>(v, k, cull);
+      if (k.samesw) k_nb_tiles<3, E, true><<<g, T, 0, c.stream>>>(v, k, e, cull);
+      else k_nb_tiles<3, E><<<g, T, 0, c.stream>>>(v, k, e, cull);
       break;
-    default: k_nb_tiles<4, E><<<g, 256, 0, c.stream>>>(v, k, cull); break;
+    default: k_nb_tiles<4, E><<<g, T, 0, c.stream>>>(v, k, e, cull); break;
   }
 }
 
 int launch_nb(Context& c, const NBConst& k, bool energy) {
   c.kernel_launches += 1;
   int g = tile_grid(c);
-  if (energy) launch_nb_mode<true>(c, k, g);
-  else launch_nb_mode<false>(c, k, g);
+  if (energy) {
+    c.kernel_launches += 1;
+    k_nb_records<<<(c.nslots + 255) / 256, 256, 0, c.stream>>>(c.view(), c.d_charge.p, c.d_rlo.p, c.d_plo.p);
+    launch_nb_mode<true>(c, k, g);
+  } else {
+    launch_nb_mode<false>(c, k, g);
+  }
   return cudaGetLastError() == cudaSuccess ? PDGPU_OK : PDGPU_ERR_CUDA;
 }
 

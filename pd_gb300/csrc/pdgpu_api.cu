@@ -140,6 +140,30 @@ NBConst pdgpu::make_nb_const(const pdgpu_nb_params& p) {
   return k;
 }
 
+NBEConst pdgpu::make_nbe_const(const NBConst& k) {
+  NBEConst e{};
+  e.econv = df_split(k.econv_diel_d);
+  e.vdw14 = df_split(k.vdw14_d);
+  e.elec14 = df_split(k.elec14_d);
+  e.vdwcut = df_split(k.vdwcut_d);
+  e.vdwinner = df_split(k.vdwinner_d);
+  e.vdwinvw2 = df_split(k.vdwinvw2_d);
+  e.inner = df_split(k.inner_d);
+  e.invw2 = df_split(k.invw2_d);
+  e.sA = df_split(k.sA);
+  e.sB = df_split(k.sB);
+  e.sC = df_split(k.sC);
+  e.sD = df_split(k.sD);
+  e.sE = df_split(k.sE);
+  e.cutV = df_split(k.fsw_cutV);
+  e.eshift = df_split(k.eshift);
+  e.cut2 = df_split(k.cut2_d);
+  e.fsw_k = df_split(k.cut2_d - 3.0 * k.inner2_d);
+  e.dovdw = k.dovdw;
+  e.vdw_hard = k.vdwinvw2_d == 0.0 ? 1 : 0;
+  return e;
+}
+
 GBConst pdgpu::make_gb_const(const pdgpu_gb_params& p, double listR) {
   GBConst k{};
   double C = p.Cutoff, I = p.InnerCutoff;
@@ -253,6 +277,7 @@ pdgpu_ctx* pdgpu_create(int device, const pdgpu_system_desc* d, int* status) {
     for (int k = 0; k < 3; k++) {
       S.box[k] = d->box[3 * s + k];
       S.ibox[k] = S.box[k] > 0 ? 1.0 / S.box[k] : 0.0;
+      S.boxf[k] = df_split(S.box[k]);
       if (S.box[k] > 0) per++;
     }
     if (per != 0 && per != 3) return bad(PDGPU_ERR_ARG);
@@ -447,6 +472,7 @@ pdgpu_ctx* pdgpu_create(int device, const pdgpu_system_desc* d, int* status) {
   if (e == cudaSuccess) e = c.d_slot_of.alloc(N);
   if (e == cudaSuccess) e = c.d_center.alloc(3 * (size_t)c.nblocks);
   if (e == cudaSuccess) e = c.d_half.alloc(c.nblocks);
+  if (e == cudaSuccess) e = c.d_cenf.alloc(c.nblocks);
   // (the tile arrays are sized by the first list build, from its tile count)
   if (e == cudaSuccess) e = c.d_counters.alloc(8);
   if (e == cudaSuccess) e = cudaMemset(c.d_counters.p, 0, sizeof(int) * 8);
@@ -455,6 +481,8 @@ pdgpu_ctx* pdgpu_create(int device, const pdgpu_system_desc* d, int* status) {
   if (e == cudaSuccess) e = c.d_xq.alloc(c.nslots);
   if (e == cudaSuccess) e = c.d_par.alloc(c.nslots);
   if (e == cudaSuccess) e = c.d_rel0.alloc(c.nslots);
+  if (e == cudaSuccess) e = c.d_rlo.alloc(c.nslots);
+  if (e == cudaSuccess) e = c.d_plo.alloc(c.nslots);
   if (e == cudaSuccess) e = c.d_facc.alloc(3 * (size_t)c.nslots);
   if (e == cudaSuccess) e = c.d_eacc.alloc((size_t)c.nsys * E_NSLOTS);
   if (e == cudaSuccess) e = c.d_status.alloc(1);

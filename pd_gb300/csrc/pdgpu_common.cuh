@@ -18,6 +18,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/pdgpu.h"
+#include "pdgpu_df.cuh"
 
 namespace pdgpu {
 
@@ -60,6 +61,7 @@ struct SystemInfo {
   int periodic;
   double box[3];
   double ibox[3];   // 1 / box (periodic systems)
+  DF boxf[3];       // box as double-floats
 };
 
 struct __align__(16) Tile {
@@ -98,6 +100,14 @@ struct NBConst {
   // 1: LJ and Coulomb switched over the same radii (Cutoff = VdwCutoff,
   // InnerCutoff = VdwInnerCutoff, energy switch, LJ on): one switch serves both
   int samesw;
+};
+
+// The same constants as double-floats, for the pair energies (FF_NonBonded)
+struct NBEConst {
+  DF econv, vdw14, elec14;
+  DF vdwcut, vdwinner, vdwinvw2, inner, invw2;
+  DF sA, sB, sC, sD, sE, cutV, eshift, cut2, fsw_k;   // fsw_k = cut2 - 3 inner2
+  int dovdw, vdw_hard;   // vdw_hard: LJ ends at VdwCutoff without a switch
 };
 
 // Constants for the GB fast path (FF_GeneralizedBorn_Still::calcForcesIncludingVacuo)
@@ -146,6 +156,11 @@ struct DevView {
   float4* rel0;              // rel pos at list build (displacement check)
   double* center;            // [nblocks*3]
   float4* half;              // [nblocks] half extents
+  float4* cenf;              // [nblocks] centre in FP32 (exact: centres are FP32 numbers)
+  // (FF_NonBonded energies) what FP32 rounding takes off the packed slots:
+  // (x, y, z, charge) - xq and (LJ radius, sqrt(eps)) - par, written before the energy pass
+  float4* rlo;
+  float2* plo;
   unsigned long long* band_excl;   // [natom*2]? (see below) per atom: bit d-1 => partner i+d excluded (bo<=2)
   unsigned long long* band_14;     // per atom: bit d-1 => partner i+d is a 1-4 pair
   const int* far_start;      // CSR of partners beyond the band, per atom
@@ -260,6 +275,7 @@ int launch_slot_params(Context& c);
 int launch_census(Context& c, const NBConst& nk, const GBConst& gk, bool do_nb, bool do_gb, unsigned long long* out);
 int measure_fp32_peak(int device, double* tflops_ffma, double* tflops_ffma2);
 NBConst make_nb_const(const pdgpu_nb_params& p);
+NBEConst make_nbe_const(const NBConst& k);
 GBConst make_gb_const(const pdgpu_gb_params& p, double listR);
 int launch_bonded(Context& c, bool energy);
 int launch_finalize_forces(Context& c, double* out, size_t stride_doubles, bool add, double scale);

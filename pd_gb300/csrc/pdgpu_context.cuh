@@ -106,6 +106,7 @@ struct Context {
   DBuf<int> d_slot_of;         // [natom] sorted slot of each atom
   DBuf<double> d_center;       // [nblocks*3]
   DBuf<float4> d_half;         // [nblocks]
+  DBuf<float4> d_cenf;         // [nblocks]
   DBuf<float> d_sys_hmax;      // [nsys*3] largest block half-extent (ordered ints)
   DBuf<BlockGrid> d_bgrid;     // [nsys]
   DBuf<int> d_bcell;           // [nblocks] cell of each block
@@ -122,6 +123,8 @@ struct Context {
   DBuf<unsigned> d_items;      // [tile_cap] GB work items (with GB only)
   DBuf<uint2> d_masks;         // [mask_cap*32]
   DBuf<float4> d_xq, d_par, d_rel0;  // [nslots]
+  DBuf<float4> d_rlo;                // [nslots] FP32 remainders of the slots (FF_NonBonded energies)
+  DBuf<float2> d_plo;                // [nslots]
   // NB j-atom groups (allocated with the NB parameters)
   DBuf<unsigned> d_cull_mask;        // [tile_cap] j lanes kept per tile
   DBuf<int> d_cull_rest;             // [tile_cap]
@@ -200,6 +203,9 @@ struct Context {
     v.rel0 = d_rel0.p;
     v.center = d_center.p;
     v.half = d_half.p;
+    v.cenf = d_cenf.p;
+    v.rlo = d_rlo.p;
+    v.plo = d_plo.p;
     v.band_excl = d_band_excl.p;
     v.band_14 = d_band_14.p;
     v.far_start = d_far_start.p;
