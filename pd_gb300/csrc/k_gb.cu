@@ -7,15 +7,16 @@
 // GB uses plain Euclidean distances, as PD does.
 //
 // Work decomposition: one warp per GB work item (grid-stride over the item list
-// the list build writes): a single 32x32 tile, or a tile pair (bi, bj),
-// (bi, bj + 1) of one row.  In a single tile lane l holds i atom l and the j
-// block rotates through the warp by shuffles; in a tile pair each lane holds
-// one atom of each j block and the shared bi block rotates, so one rotation
-// serves two pairs (the Born and chain bodies also run the two pairs on packed
-// f32x2 arithmetic).  Every FP32 sum is converted to 64-bit fixed point and
-// added atomically once per item (so a slot's total does not depend on the
-// order in which items run).  Tiles without bonded pairs take a path without
-// mask tests.  Registers decide the occupancy of these kernels.
+// the list build writes): a tile pair (bi, bj), (bi, bj + 1) of one row whose
+// pairs all lie inside every cutoff, or single 32x32 tiles.  In a tile pair each
+// lane holds one atom of each j block and the shared bi block rotates, so one
+// rotation serves two pairs.  A single tile (masked, diagonal, odd, or cut by a
+// cutoff) is step-packed: lane l holds i atom l and takes the j atoms l + kk and
+// l + kk + 1 of the rotating block as one FP32x2 pair, read from the warp's rows
+// in shared memory; its exclusion bits are tested per half.  Both run on packed
+// f32x2 arithmetic.  Every FP32 sum is converted to 64-bit fixed point and added
+// atomically once per tile (so a slot's total does not depend on the order in
+// which items run).  Registers decide the occupancy of these kernels.
 #include "pdgpu_tile.cuh"
 
 namespace pdgpu {
@@ -48,98 +49,7 @@ __device__ __forceinline__ bool still_in(const DevView& v, const GBConst& k, flo
 // trigonometric code is skipped, not predicated, on nearly every step.
 __device__ __forceinline__ bool gb_contact(const GBConst& k, float r2, float rs2) { return r2 <= rs2 * k.invP5; }
 
-// P4 CCF / r^4 of one pair (rs = R_i + R_j, raw type radii); any_contact: the
-// warp vote over gb_contact
-__device__ __forceinline__ float born_w(const GBConst& k, float r2, float rs, bool any_contact) {
-  const float rs2 = rs * rs;
-  float ccf = 1.f;
-  if (any_contact) {
-    if (gb_contact(k, r2, rs2)) {
-      const float h = 0.5f - 0.5f * cospif(__fdividef(r2, rs2) * k.P5);
-      ccf = h * h;
-    }
-  }
-  const float ir2 = rcp_ftz(r2);
-  return k.P4 * ccf * ir2 * ir2;
-}
-
-template <bool MASKED, bool FULL>
-__device__ __forceinline__ void born_tile(const DevView& v, const GBConst& k, const Tile& T, int lane, int si,
-                                          const float4& xi, const float4& pi, unsigned ex, float& gi, float& gj) {
-  float4 xj = j_in_i_frame(v, T, lane);
-  float4 pj = v.par[T.bj * 32 + lane];
-#pragma unroll 4
-  for (int kk = 0; kk < 32; kk++) {
-    const float dx = xj.x - xi.x, dy = xj.y - xi.y, dz = xj.z - xi.z;
-    const float r2 = dx * dx + dy * dy + dz * dz;
-    bool in = still_in<FULL>(v, k, r2, si, T.bj * 32 + ((lane + kk) & 31));
-    if (MASKED) in = in && !((ex >> kk) & 1u);
-    const float rs = pi.z + pj.z;
-    const bool anyc = __any_sync(0xffffffffu, in && gb_contact(k, r2, rs * rs));
-    if (in) {
-      const float w = born_w(k, r2, rs, anyc);
-      gi += w * pj.w;
-      gj += w * pi.w;
-    }
-    ROT(xj.x); ROT(xj.y); ROT(xj.z); ROT(pj.z); ROT(pj.w); ROT(gj);
-  }
-}
-
-// Tile pairs: two unmasked, off-diagonal tiles (bi, bj) and (bi, bj + 1) of one
-// row at once.  The shared bi block rotates through the warp and each lane keeps
-// one atom of each j block (moved into bi's frame), so one rotation of the bi
-// atom (its data and its running sums) serves two pairs instead of one.  The two
-// pairs' arithmetic runs on packed FP32x2 instructions (.x: the atom of bj,
-// .y: the atom of bj + 1), which halves the instructions issued for it.
 __device__ __forceinline__ float2 f2(float a) { return make_float2(a, a); }
-
-template <bool FULL>
-__device__ __forceinline__ void born_tile2(const DevView& v, const GBConst& k, const Tile& A, const Tile& B, int lane,
-                                           long long* gpol) {
-  const int sa = A.bj * 32 + lane, sb = B.bj * 32 + lane, r0 = A.bi * 32;
-  const float4 xa = j_in_i_frame(v, A, lane), xb = j_in_i_frame(v, B, lane);
-  const float4 pa = v.par[sa], pb = v.par[sb];
-  const float2 nx = make_float2(-xa.x, -xb.x), ny = make_float2(-xa.y, -xb.y), nz = make_float2(-xa.z, -xb.z);
-  const float2 RS = make_float2(pa.z, pb.z), P4 = f2(k.P4);
-  float4 xr = v.xq[r0 + lane], pr = v.par[r0 + lane];
-  float2 G = f2(0.f);
-  float gr = 0.f;
-#pragma unroll 4
-  for (int kk = 0; kk < 32; kk++) {
-    const int sr = r0 + ((lane + kk) & 31);
-    const float2 dx = __fadd2_rn(f2(xr.x), nx), dy = __fadd2_rn(f2(xr.y), ny), dz = __fadd2_rn(f2(xr.z), nz);
-    const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
-    const float2 rs = __fadd2_rn(RS, f2(pr.z));
-    const float2 rs2 = __fmul2_rn(rs, rs);
-    const float2 lim = __fmul2_rn(rs2, f2(k.invP5));
-    const bool ca = r2.x <= lim.x, cb = r2.y <= lim.y;
-    float2 ccf = f2(1.f);
-    if (__any_sync(0xffffffffu, ca || cb)) {
-      if (ca) {
-        const float h = 0.5f - 0.5f * cospif(__fdividef(r2.x, rs2.x) * k.P5);
-        ccf.x = h * h;
-      }
-      if (cb) {
-        const float h = 0.5f - 0.5f * cospif(__fdividef(r2.y, rs2.y) * k.P5);
-        ccf.y = h * h;
-      }
-    }
-    const float2 ir2 = make_float2(rcp_ftz(r2.x), rcp_ftz(r2.y));
-    float2 w = __fmul2_rn(__fmul2_rn(P4, ccf), __fmul2_rn(ir2, ir2));
-    if (!FULL) {
-      if (!still_in<false>(v, k, r2.x, sa, sr)) w.x = 0.f;
-      if (!still_in<false>(v, k, r2.y, sb, sr)) w.y = 0.f;
-    }
-    G = __ffma2_rn(w, f2(pr.w), G);
-    gr = fmaf(w.x, pa.w, gr);
-    gr = fmaf(w.y, pb.w, gr);
-    ROT(xr.x); ROT(xr.y); ROT(xr.z); ROT(pr.z); ROT(pr.w); ROT(gr);
-  }
-  fix_range(v.status, fabsf(G.x) + fabsf(G.y) + fabsf(gr));
-  atomic_add_ll(&gpol[sa], fx32(G.x));
-  atomic_add_ll(&gpol[sb], fx32(G.y));
-  atomic_add_ll(&gpol[r0 + lane], fx32(gr));
-}
 
 // ---------------------------------------------------------------------------
 // All-inside tile pairs (every pair inside every cutoff, no exclusions: the
@@ -152,6 +62,18 @@ __device__ __forceinline__ float warp_max(float x) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, o));
   return x;
+}
+
+// Tile pairs far from their row's block skip a branch for the whole item: every
+// pair of the item lies farther apart than sqrt(lim), lim a bound over the
+// rotating block for each of the lane's two held atoms.  The rotating block sits
+// at the origin of the item's frame, so a held atom at x keeps at least
+// |x| - rho from it, rho the block's radius at the current positions.
+__device__ __forceinline__ bool item_far(const float4& xa, const float4& xb, const float4& xr, float lima, float limb) {
+  const float rho = sqrtf(warp_max(xr.x * xr.x + xr.y * xr.y + xr.z * xr.z));
+  const float da = sqrtf(xa.x * xa.x + xa.y * xa.y + xa.z * xa.z) * 0.99999f - rho;
+  const float db = sqrtf(xb.x * xb.x + xb.y * xb.y + xb.z * xb.z) * 0.99999f - rho;
+  return __all_sync(0xffffffffu, da > 0.f && db > 0.f && da * da > lima && db * db > limb);
 }
 
 // an upper bound of (R_i + R_j)^2 / P5 over the pairs of a tile pair: held raw
@@ -182,28 +104,79 @@ __device__ __forceinline__ float born_ccf(const GBConst& k, float r2, float rs) 
 constexpr int kBornThreads = 256;
 constexpr int kBornWarps = kBornThreads / 32;
 
-__device__ __forceinline__ void born_full2(const DevView& v, const GBConst& k, const Tile& A, const Tile& B, int lane,
-                                           long long* gpol) {
-  __shared__ float4 rot_sh[kBornWarps][2][32];   // (x, x', y, y'), (z, z', P4 V, P4 V')
-  float4 (*rs)[32] = rot_sh[threadIdx.x >> 5];
-  const int sa = A.bj * 32 + lane, sb = B.bj * 32 + lane, r0 = A.bi * 32;
-  const int l1 = (lane + 1) & 31;
-  const float4 xa = j_in_i_frame(v, A, lane), xb = j_in_i_frame(v, B, lane);
-  const float4 pa = v.par[sa], pb = v.par[sb];
-  const float2 AX = f2(-xa.x), AY = f2(-xa.y), AZ = f2(-xa.z), BX = f2(-xb.x), BY = f2(-xb.y), BZ = f2(-xb.z);
-  const float2 VA = f2(k.P4 * pa.w), VB = f2(k.P4 * pb.w);
-  const float4 x0 = v.xq[r0 + lane], x1 = v.xq[r0 + l1];
-  const float4 p0 = v.par[r0 + lane], p1 = v.par[r0 + l1];
-  __syncwarp();
-  rs[0][lane] = make_float4(x0.x, x1.x, x0.y, x1.y);
-  rs[1][lane] = make_float4(x0.z, x1.z, k.P4 * p0.w, k.P4 * p1.w);
-  __syncwarp();
-  const float c2 = pair_contact2(k, make_float2(pa.z, pb.z), p0.z);
-  float2 GA = f2(0.f), GB = f2(0.f), GR = f2(0.f);
+// rows of the rotating block in the warp's shared memory, twice over, so that a
+// lane's row at step kk lies at a fixed offset from its first (no wrap-around)
+struct BornRows {
+  float4 xy[64], zv[64];   // (x, x', y, y'), (z, z', P4 V, P4 V')
+  float2 r[64];            // (R, R'), single tiles only
+};
+
+// Born sums of a single tile, step-packed (MASKED: exclusion bits and the
+// diagonal; FULL: every pair inside the Still cutoff)
+template <bool MASKED, bool FULL>
+__device__ __forceinline__ void born_tile(const DevView& v, const GBConst& k, const Tile& T, int lane, unsigned ex,
+                                          long long* gpol, BornRows& rs) {
+  const int si = T.bi * 32 + lane, j0 = T.bj * 32, l1 = (lane + 1) & 31;
+  const float4 xi = v.xq[si], pi = v.par[si];
+  {
+    const float4 x0 = j_in_i_frame(v, T, lane), p0 = v.par[j0 + lane];
+    const float v0 = k.P4 * p0.w;
+    const float x1 = __shfl_sync(0xffffffffu, x0.x, l1), y1 = __shfl_sync(0xffffffffu, x0.y, l1);
+    const float z1 = __shfl_sync(0xffffffffu, x0.z, l1), v1 = __shfl_sync(0xffffffffu, v0, l1);
+    const float r1 = __shfl_sync(0xffffffffu, p0.z, l1);
+    __syncwarp();
+    rs.xy[lane] = rs.xy[lane + 32] = make_float4(x0.x, x1, x0.y, y1);
+    rs.zv[lane] = rs.zv[lane + 32] = make_float4(x0.z, z1, v0, v1);
+    rs.r[lane] = rs.r[lane + 32] = make_float2(p0.z, r1);
+    __syncwarp();
+  }
+  const float2 AX = f2(-xi.x), AY = f2(-xi.y), AZ = f2(-xi.z), RA = f2(pi.z), VA = f2(k.P4 * pi.w);
+  float2 GA = f2(0.f), GR = f2(0.f);
 #pragma unroll 4
   for (int kk = 0; kk < 32; kk += 2) {
-    const int j = (lane + kk) & 31;
-    const float4 P = rs[0][j], Q = rs[1][j];
+    const int j = lane + kk;
+    const float4 P = rs.xy[j], Q = rs.zv[j];
+    const float2 ax = __fadd2_rn(make_float2(P.x, P.y), AX), ay = __fadd2_rn(make_float2(P.z, P.w), AY);
+    const float2 az = __fadd2_rn(make_float2(Q.x, Q.y), AZ);
+    const float2 r2 = __ffma2_rn(az, az, __ffma2_rn(ay, ay, __fmul2_rn(ax, ax)));
+    const float2 ir2 = make_float2(rcp_ftz(r2.x), rcp_ftz(r2.y));
+    float2 w = __fmul2_rn(ir2, ir2);
+    const float2 s = __fadd2_rn(rs.r[j], RA), s2 = __fmul2_rn(s, s), lim = __fmul2_rn(s2, f2(k.invP5));
+    if (__any_sync(0xffffffffu, r2.x <= lim.x || r2.y <= lim.y)) {
+      w.x *= born_ccf(k, r2.x, s.x);
+      w.y *= born_ccf(k, r2.y, s.y);
+    }
+    bool ia = still_in<FULL>(v, k, r2.x, si, j0 + (j & 31));
+    bool ib = still_in<FULL>(v, k, r2.y, si, j0 + ((j + 1) & 31));
+    if (MASKED) {
+      ia = ia && !((ex >> kk) & 1u);
+      ib = ib && !((ex >> kk) & 2u);
+    }
+    if (MASKED || !FULL) {
+      w.x = ia ? w.x : 0.f;
+      w.y = ib ? w.y : 0.f;
+    }
+    GA = __ffma2_rn(w, make_float2(Q.z, Q.w), GA);
+    GR = __ffma2_rn(w, VA, GR);
+    ROT2(GR);
+  }
+  const float gr = GR.x + __shfl_sync(0xffffffffu, GR.y, (lane + 31) & 31), ga = GA.x + GA.y;
+  fix_range(v.status, fabsf(ga) + fabsf(gr));
+  atomic_add_ll(&gpol[si], fx32(ga));
+  atomic_add_ll(&gpol[j0 + lane], fx32(gr));
+}
+
+// FAR: no pair of the item in close contact
+template <bool FAR>
+__device__ __forceinline__ void born_loop2(const DevView& v, const GBConst& k, int lane, int r0, const BornRows& rs,
+                                           const float4& xa, const float4& xb, const float4& pa, const float4& pb,
+                                           float c2, float2& GA, float2& GB, float2& GR) {
+  const float2 AX = f2(-xa.x), AY = f2(-xa.y), AZ = f2(-xa.z), BX = f2(-xb.x), BY = f2(-xb.y), BZ = f2(-xb.z);
+  const float2 VA = f2(k.P4 * pa.w), VB = f2(k.P4 * pb.w);
+  const float4 *xy = rs.xy + lane, *zv = rs.zv + lane;
+#pragma unroll 4
+  for (int kk = 0; kk < 32; kk += 2) {
+    const float4 P = xy[kk], Q = zv[kk];
     const float2 X = make_float2(P.x, P.y), Y = make_float2(P.z, P.w), Z = make_float2(Q.x, Q.y);
     const float2 VR = make_float2(Q.z, Q.w);
     const float2 ax = __fadd2_rn(X, AX), ay = __fadd2_rn(Y, AY), az = __fadd2_rn(Z, AZ);
@@ -213,13 +186,15 @@ __device__ __forceinline__ void born_full2(const DevView& v, const GBConst& k, c
     const float2 ia = make_float2(rcp_ftz(ra.x), rcp_ftz(ra.y));
     const float2 ib = make_float2(rcp_ftz(rb.x), rcp_ftz(rb.y));
     float2 wa = __fmul2_rn(ia, ia), wb = __fmul2_rn(ib, ib);
-    if (__any_sync(0xffffffffu, fminf(fminf(ra.x, ra.y), fminf(rb.x, rb.y)) <= c2)) {
-      // rare: the rotating atoms' radii are read here, not staged
-      const float R0 = v.par[r0 + j].z, R1 = v.par[r0 + ((j + 1) & 31)].z;
-      wa.x *= born_ccf(k, ra.x, pa.z + R0);
-      wa.y *= born_ccf(k, ra.y, pa.z + R1);
-      wb.x *= born_ccf(k, rb.x, pb.z + R0);
-      wb.y *= born_ccf(k, rb.y, pb.z + R1);
+    if (!FAR) {
+      if (__any_sync(0xffffffffu, fminf(fminf(ra.x, ra.y), fminf(rb.x, rb.y)) <= c2)) {
+        // rare: the rotating atoms' radii are read here, not staged
+        const float R0 = v.par[r0 + ((lane + kk) & 31)].z, R1 = v.par[r0 + ((lane + kk + 1) & 31)].z;
+        wa.x *= born_ccf(k, ra.x, pa.z + R0);
+        wa.y *= born_ccf(k, ra.y, pa.z + R1);
+        wb.x *= born_ccf(k, rb.x, pb.z + R0);
+        wb.y *= born_ccf(k, rb.y, pb.z + R1);
+      }
     }
     GA = __ffma2_rn(wa, VR, GA);
     GB = __ffma2_rn(wb, VR, GB);
@@ -227,6 +202,24 @@ __device__ __forceinline__ void born_full2(const DevView& v, const GBConst& k, c
     GR = __ffma2_rn(wb, VB, GR);
     ROT2(GR);
   }
+}
+
+__device__ __forceinline__ void born_full2(const DevView& v, const GBConst& k, const Tile& A, const Tile& B, int lane,
+                                           long long* gpol, BornRows& rs) {
+  const int sa = A.bj * 32 + lane, sb = B.bj * 32 + lane, r0 = A.bi * 32;
+  const int l1 = (lane + 1) & 31;
+  const float4 xa = j_in_i_frame(v, A, lane), xb = j_in_i_frame(v, B, lane);
+  const float4 pa = v.par[sa], pb = v.par[sb];
+  const float4 x0 = v.xq[r0 + lane], x1 = v.xq[r0 + l1];
+  const float4 p0 = v.par[r0 + lane], p1 = v.par[r0 + l1];
+  __syncwarp();
+  rs.xy[lane] = rs.xy[lane + 32] = make_float4(x0.x, x1.x, x0.y, x1.y);
+  rs.zv[lane] = rs.zv[lane + 32] = make_float4(x0.z, x1.z, k.P4 * p0.w, k.P4 * p1.w);
+  __syncwarp();
+  const float c2 = pair_contact2(k, make_float2(pa.z, pb.z), p0.z);
+  float2 GA = f2(0.f), GB = f2(0.f), GR = f2(0.f);
+  if (item_far(xa, xb, x0, c2, c2)) born_loop2<true>(v, k, lane, r0, rs, xa, xb, pa, pb, c2, GA, GB, GR);
+  else born_loop2<false>(v, k, lane, r0, rs, xa, xb, pa, pb, c2, GA, GB, GR);
   // GR.x holds the sum of the rotating atom of this lane, GR.y that of lane + 1
   const float gr = GR.x + __shfl_sync(0xffffffffu, GR.y, (lane + 31) & 31);
   const float ga = GA.x + GA.y, gb = GB.x + GB.y;
@@ -243,7 +236,25 @@ __device__ __forceinline__ int item_tile(const DevView& v, int it, bool& two) {
   return (int)(code & 0x7fffffffu);
 }
 
-__global__ void __launch_bounds__(kBornThreads) k_gb_born(const __grid_constant__ DevView v, const __grid_constant__ GBConst k, long long* gpol) {
+__device__ __forceinline__ void born_single(const DevView& v, const GBConst& k, const Tile& T, int lane,
+                                            long long* gpol, BornRows& rs) {
+  const bool full = tile_full(T);
+  if (tile_masked(T)) {
+    unsigned ex, m14;
+    tile_masks(v, T, lane, ex, m14);
+    if (T.flags & 2) ex |= diag_exclusion(lane);
+    if (full) born_tile<true, true>(v, k, T, lane, ex, gpol, rs);
+    else born_tile<true, false>(v, k, T, lane, ex, gpol, rs);
+  } else if (full) {
+    born_tile<false, true>(v, k, T, lane, 0u, gpol, rs);
+  } else {
+    born_tile<false, false>(v, k, T, lane, 0u, gpol, rs);
+  }
+}
+
+__global__ void __launch_bounds__(kBornThreads, 5) k_gb_born(const __grid_constant__ DevView v, const __grid_constant__ GBConst k, long long* gpol) {
+  __shared__ BornRows rows[kBornWarps];
+  BornRows& rs = rows[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   const int ni = *v.nitems;
@@ -251,29 +262,12 @@ __global__ void __launch_bounds__(kBornThreads) k_gb_born(const __grid_constant_
     bool two;
     const int t = item_tile(v, it, two);
     const Tile T = v.tiles[t];
-    if (two) {
-      const Tile U = v.tiles[t + 1];
-      if (tile_full(T)) born_full2(v, k, T, U, lane, gpol);
-      else born_tile2<false>(v, k, T, U, lane, gpol);
+    if (two && tile_full(T)) {
+      born_full2(v, k, T, v.tiles[t + 1], lane, gpol, rs);
       continue;
     }
-    const int si = T.bi * 32 + lane;
-    const float4 xi = v.xq[si], pi = v.par[si];
-    unsigned ex, m14;
-    tile_masks(v, T, lane, ex, m14);
-    if (T.flags & 2) ex |= diag_exclusion(lane);
-    float gi = 0.f, gj = 0.f;
-    const bool full = tile_full(T);
-    if (tile_masked(T)) {
-      if (full) born_tile<true, true>(v, k, T, lane, si, xi, pi, ex, gi, gj);
-      else born_tile<true, false>(v, k, T, lane, si, xi, pi, ex, gi, gj);
-    } else {
-      if (full) born_tile<false, true>(v, k, T, lane, si, xi, pi, ex, gi, gj);
-      else born_tile<false, false>(v, k, T, lane, si, xi, pi, ex, gi, gj);
-    }
-    fix_range(v.status, fabsf(gi) + fabsf(gj));
-    atomic_add_ll(&gpol[si], fx32(gi));
-    atomic_add_ll(&gpol[T.bj * 32 + lane], fx32(gj));
+    born_single(v, k, T, lane, gpol, rs);
+    if (two) born_single(v, k, v.tiles[t + 1], lane, gpol, rs);
   }
 }
 
@@ -303,486 +297,479 @@ __device__ __noinline__ bool gb_on_fp64(const DevView& v, int si, int sj, double
 
 // ---------------------------------------------------------------------------
 // pass 2: GB cross term fused with vacuum LJ + Coulomb, i > j pairs within Cutoff
-// (forces, dE/da and, with ENERGY, the pair energies).  With ENERGY every pair
-// closer than sqrt(GBConst::e64_r2) (4.5 A: the close contacts that carry the
-// large repulsive terms) takes its displacement from FP64 slot records (rounded
-// once to FP32 for the force) and its energies in FP64 from FP64 per-atom
-// parameters; the other pairs' energies are FP32, in partial sums moved to FP64
-// every 8 rotation steps; a work item's sums then go over the warp in FP64 and
-// enter fixed point once.  The vdW total is a small difference of large
-// repulsive and attractive sums: FP32 positions (rounded relative to their
-// block centres) on the close contacts, or FP32 sums, leave ~1e-6 of it.
-// Energy evaluations are rare (an exchange attempt, an explicit energy call),
-// so this FP64 work stays off the force-only step; the energy pass of a
-// parameter-gradient call sets e64_r2 = 0 (its energies only weight the loss).
+// (forces, dE/da and, with ENERGY, the pair energies).
 // ---------------------------------------------------------------------------
 struct PairAcc {
   float fx, fy, fz, da;
 };
 
-// FP64 records of every sorted slot for the energy pass (DevView::epos, epar)
-__global__ void k_energy_records(DevView v, double4* epos, double2* epar) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= v.nslots) return;
-  const int a = v.sorted_atom[s];
-  if (a < 0) {
-    epos[s] = make_double4(1e6, 1e6, 1e6, 0.0);
-    epar[s] = make_double2(-1.0, 0.0);
-    return;
-  }
-  epos[s] = make_double4(v.pos[3 * a], v.pos[3 * a + 1], v.pos[3 * a + 2], v.charge[a]);
-  epar[s] = make_double2(v.radius[a], v.sqeps[a]);
-}
-
-// (ENERGY) pair energies of a work item: close pairs in FP64, the others in
-// FP32 partial sums moved to FP64 every 8 rotation steps
-struct EAcc {
-  double v = 0.0, e = 0.0, p = 0.0;
-  float fv = 0.f, fe = 0.f, fp = 0.f;
-  __device__ __forceinline__ void flush() {
-    v += (double)fv;
-    e += (double)fe;
-    p += (double)fp;
-    fv = fe = fp = 0.f;
-  }
-};
-
-// 1 / sqrt(x) in FP64 from the FP32 approximation and one Newton step
-// (relative error ~1e-13), without the FP64 square-root sequence
-__device__ __forceinline__ double rsqrt_fp64(double x) {
-  const double y = (double)rsqrtf((float)x);
-  return y * fma(-0.5 * x * y, y, 1.5);
-}
-
-// u = -r^2 / (4 a_i a_j) of a pair, and whether the pair may lie above the exp
-// threshold (the FP64 tie-break band included): the warp votes on it, and the
-// GB term's code runs only when some lane needs it (in the all-pairs case most
-// warp steps have none)
-__device__ __forceinline__ float gb_u(float r2, float ai, float aj) { return -0.25f * __fdividef(r2, ai * aj); }
-__device__ __forceinline__ bool gb_maybe_on(const GBConst& k, float u) {
-  return u >= k.thresh - 4e-6f * fabsf(k.thresh);
-}
-
-// One pair of the fused law: i = (xi.w, pix, piy, ai), j = (qj, pjx, pjy, aj),
-// (dx, dy, dz) = x_j - x_i, u = gb_u.  Adds the force on i along d to I and its
-// opposite to J, dE/da to both.  si, sj:
-// slots for the FP64 threshold tie-break; any_gb: the warp's vote on
-// gb_maybe_on (warp-uniform).  (ENERGY) pe: the pair's energies for
-// add_pair_energy.
-// (ENERGY) what a pair's energies need beyond r^2: its FP32 energies (vdW,
-// Coulomb, GB cross term) and, for the FP64 path of a close pair, whether the
-// GB term is on, fgb S, the Coulomb switch S and the vdW switch (0 beyond
-// VdwCutoff)
-struct PairE {
-  float v, e, p, fgbS, S, vsw;
-  bool gbon;
-};
-
-// FP64 energies of a close pair from the slot records (the caller enters this
-// on a warp vote, so the FP64 code is not issued for warps without a close
-// pair); returned, not accumulated, so the accumulators stay in registers
-struct E3 {
-  double v, e, p;
-};
-template <bool FAST>
-__device__ __noinline__ E3 close_energy(const DevView& v, const GBConst& k, double r2d, double4 ei, double4 ej,
-                                        double2 pi_e, int sj, bool excl, bool is14, PairE pe) {
-  E3 r = {0.0, 0.0, 0.0};
-  const double qq = ei.w * ej.w, ir = rsqrt_fp64(r2d);
-  if (pe.gbon) r.p = 2.0 * k.premul_d * qq * (double)pe.fgbS;
-  else if (!FAST) r.p = 2.0 * k.premul_d * qq * ir * (double)pe.S;
-  if (FAST && !excl) {
-    r.e = (pe.gbon ? k.econv_in_d : k.econv_out_d) * (is14 ? k.elec14_d : 1.0) * qq * ir * (double)pe.S;
-    const double2 pj_e = v.epar[sj];
-    const double sd = pi_e.x + pj_e.x, t2 = sd * sd * (ir * ir), B6 = t2 * t2 * t2;
-    r.v = pi_e.y * pj_e.y * (is14 ? k.vdw14_d : 1.0) * (B6 * B6 - 2.0 * B6) * (double)pe.vsw;
-  }
-  return r;
-}
-
-// (ENERGY) a pair's energies into the item's sums: the FP64 path for a close
-// pair (warp-voted; PRECISE passes only), the FP32 sums otherwise
-template <bool FAST, bool PRECISE>
-__device__ __forceinline__ void add_pair_energy(const DevView& v, const GBConst& k, bool in, bool close, double r2d,
-                                                const double4& ei, const double4& ej, const double2& pi_e, int sj,
-                                                bool excl, bool is14, const PairE& pe, EAcc& ea) {
-  bool fp32 = in;
-  if (PRECISE && __any_sync(0xffffffffu, in && close)) {
-    if (in && close) {
-      const E3 c = close_energy<FAST>(v, k, r2d, ei, ej, pi_e, sj, excl, is14, pe);
-      ea.v += c.v;
-      ea.e += c.e;
-      ea.p += c.p;
-      fp32 = false;
-    }
-  }
-  if (fp32) {
-    ea.fv += pe.v;
-    ea.fe += pe.e;
-    ea.fp += pe.p;
-  }
-}
-
-template <bool ENERGY, bool FULL, bool FAST>
-__device__ __forceinline__ void gb_pair_one(const DevView& v, const GBConst& k, float dx, float dy, float dz,
-                                            float r2, float u, bool any_gb, float qi, float qj, float pix, float piy,
-                                            float pjx, float pjy, float ai, float aj, bool excl, bool is14, int si,
-                                            int sj, PairAcc& I, PairAcc& J, PairE& pe) {
-    const float invr = rsqrtf(r2);
-    const float r = r2 * invr;
-    const float qiqj = qi * qj;
-    const float aiaj = ai * aj;
-    bool gbon = false;
-    if (any_gb) {
-      gbon = u > k.thresh;
-      if (fabsf(u - k.thresh) <= 2e-6f * fabsf(k.thresh))
-        gbon = gb_on_fp64(v, si, sj, k.thresh_d);
-    }
-    float g = 0.f;  // scalar multiplying (xj - xi) in the force on i
-    float elec = 0.f, delec = 0.f;
-    const float s14 = is14 ? k.elec14 : 1.f;
-    // switching (FULL: the tile lies inside the inner cutoff) without a branch:
-    // below the inner cutoff w = 0 gives S = 1 and dS = 0 exactly
-    const bool sw_on = !FULL;
-    float S = 1.f, dS = 0.f;
-    if (sw_on) {
-      const float w = fmaxf(r - k.inner, 0.f);
-      const float sw = 1.f - w * w * k.invw2;
-      dS = -4.f * k.invw2 * w * sw;
-      S = sw * sw;
-    }
-    if (ENERGY) pe = PairE{0.f, 0.f, 0.f, 0.f, S, 0.f, any_gb && gbon};
-    if (any_gb && gbon) {
-      const float tg = __expf(u);
-      const float fgb = rsqrtf(r2 + tg * aiaj);
-      const float l = fgb * fgb;
-      const float ep = k.premul * qiqj * fgb;
-      float dedr = -ep * (r - 0.25f * r * tg) * l;
-      float dalpha = -ep * tg * (1.f - u) * l;
-      if (ENERGY) {
-        pe.p = 2.f * ep * S;
-        pe.fgbS = fgb * S;
-      }
-      if (FAST && !excl) {
-        elec = k.econv_in * s14 * qiqj * invr;
-        delec = -elec * invr;
-      }
-      if (sw_on) {
-        dedr = S * dedr + dS * ep;
-        dalpha *= S;
-      }
-      g += 2.f * dedr * invr;
-      I.da += dalpha * aj;
-      J.da += dalpha * ai;
-    } else if (FAST && !excl) {
-      elec = k.econv_out * s14 * qiqj * invr;
-      delec = -elec * invr;
-    } else if (!FAST) {
-      // calcBornForces below the threshold (gbff.cpp:1308-1325): premul q_i q_j / r
-      const float ep = k.premul * qiqj * invr;
-      float dedr = -ep * invr;
-      if (ENERGY) pe.p = 2.f * ep * S;
-      if (sw_on) dedr = S * dedr + dS * ep;
-      g += 2.f * dedr * invr;
-    }
-    if (FAST && !excl) {
-      if (ENERGY) pe.e = elec * S;
-      if (sw_on) delec = S * delec + elec * dS;
-      const float t = (pix + pjx) * invr;
-      float B = t * t;
-      B = B * B * B;
-      const float A = B * B;
-      const float eps = piy * pjy * (is14 ? k.vdw14 : 1.f);
-      float dvdw = -12.f * eps * invr * (A - B);
-      float Ev = (ENERGY || !FULL) ? eps * (A - 2.f * B) : 0.f;
-      float vsw = 1.f;
-      if (!FULL) {
-        const float w = fmaxf(r - k.vdwinner, 0.f);
-        const float sw = 1.f - w * w * k.vdwinvw2;
-        dvdw = sw * sw * dvdw + Ev * (-4.f * k.vdwinvw2 * w * sw);
-        const bool vin = r < k.vdwcut;
-        vsw = vin ? sw * sw : 0.f;
-        dvdw = vin ? dvdw : 0.f;
-      }
-      if (ENERGY) {
-        pe.v = Ev * vsw;
-        pe.vsw = vsw;
-      }
-      g += (dvdw + delec) * invr;
-    }
-    I.fx += g * dx; I.fy += g * dy; I.fz += g * dz;
-    J.fx -= g * dx; J.fy -= g * dy; J.fz -= g * dz;
-}
-
-// (ENERGY) for a pair closer than sqrt(k.e64_r2): the displacement x_b - x_a
-// from the FP64 slot records (rounded once to FP32 for the force) and r^2 in
-// FP64; false (nothing written) for a farther pair or a padding slot
-__device__ __forceinline__ bool disp_fp64(const DevView& v, const GBConst& k, const double4& ea_, int sb, double4& eb,
-                                          float& dx, float& dy, float& dz, float& r2, double& r2d) {
-  if (!(r2 < k.e64_r2) || ea_.x > 1e5) return false;
-  eb = v.epos[sb];
-  if (eb.x > 1e5) return false;
-  const double ex = eb.x - ea_.x, ey = eb.y - ea_.y, ez = eb.z - ea_.z;
-  dx = (float)ex;
-  dy = (float)ey;
-  dz = (float)ez;
-  r2d = ex * ex + ey * ey + ez * ez;
-  r2 = (float)r2d;
-  return true;
-}
-
-template <bool MASKED, bool ENERGY, bool FULL, bool FAST = true, bool PRECISE = true>
-__device__ __forceinline__ void gb_pair_tile(const DevView& v, const GBConst& k, const Tile& T, int lane, int si,
-                                             const float4& xi, const float4& pi, float ai, unsigned ex,
-                                             unsigned m14, unsigned dmask, const float* born, PairAcc& I, PairAcc& J,
-                                             EAcc& ea) {
-  float4 xj = j_in_i_frame(v, T, lane);
-  float4 pj = v.par[T.bj * 32 + lane];
-  float aj = born[T.bj * 32 + lane];
-  double4 e_i = make_double4(0.0, 0.0, 0.0, 0.0), e_j = e_i;
-  double2 p_i = make_double2(0.0, 0.0);
-  if (ENERGY && PRECISE) {
-    e_i = v.epos[si];
-    p_i = v.epar[si];
-  }
-#pragma unroll 2
-  for (int kk = 0; kk < 32; kk++) {
-    float dx = xj.x - xi.x, dy = xj.y - xi.y, dz = xj.z - xi.z;
-    float r2 = dx * dx + dy * dy + dz * dz;
-    double r2d = 0.0;
-    const bool close =
-        ENERGY && PRECISE && disp_fp64(v, k, e_i, T.bj * 32 + ((lane + kk) & 31), e_j, dx, dy, dz, r2, r2d);
-    bool pair = true, excl = false, is14 = false;
-    if (MASKED) {
-      pair = !((dmask >> kk) & 1u);
-      excl = (ex >> kk) & 1u;  // bond order <= 2: GB term only
-      is14 = (m14 >> kk) & 1u;
-    }
-    const bool in = (FULL || r2 <= k.cut2) && pair;
-    const float u = gb_u(r2, ai, aj);
-    const bool any_gb = __any_sync(0xffffffffu, in && gb_maybe_on(k, u));
-    PairE pe;
-    if (in)
-      gb_pair_one<ENERGY, FULL, FAST>(v, k, dx, dy, dz, r2, u, any_gb, xi.w, xj.w, pi.x, pi.y, pj.x, pj.y, ai, aj,
-                                      excl, is14, si, T.bj * 32 + ((lane + kk) & 31), I, J, pe);
-    if (ENERGY)
-      add_pair_energy<FAST, PRECISE>(v, k, in, close, r2d, e_i, e_j, p_i, T.bj * 32 + ((lane + kk) & 31), excl,
-                                     is14, pe, ea);
-    if (ENERGY && (kk & 7) == 7) ea.flush();
-    ROT(xj.x); ROT(xj.y); ROT(xj.z); ROT(xj.w); ROT(pj.x); ROT(pj.y); ROT(aj);
-    ROT(J.fx); ROT(J.fy); ROT(J.fz); ROT(J.da);
-  }
-}
-
 // per-tile FP32 sums enter 64-bit fixed point before they are combined, so a
 // slot's total does not depend on how its tiles were grouped into work items
-struct FixAcc {
-  long long fx, fy, fz, da;
-};
-
-__device__ __forceinline__ void fix_in(const DevView& v, FixAcc& F, const PairAcc& a) {
-  fix_range(v.status, fabsf(a.fx) + fabsf(a.fy) + fabsf(a.fz) + fabsf(a.da));
-  F.fx += fx32(a.fx);
-  F.fy += fx32(a.fy);
-  F.fz += fx32(a.fz);
-  F.da += fx32(a.da);
-}
-
-__device__ __forceinline__ void flush_fix(const DevView& v, long long* deda, int s, const FixAcc& F) {
-  atomic_add_ll(&v.facc[3 * s], F.fx);
-  atomic_add_ll(&v.facc[3 * s + 1], F.fy);
-  atomic_add_ll(&v.facc[3 * s + 2], F.fz);
-  if (deda) atomic_add_ll(&deda[s], F.da);
-}
-
 __device__ __forceinline__ void flush_pair(const DevView& v, long long* deda, int s, const PairAcc& a) {
-  FixAcc F = {0, 0, 0, 0};
-  fix_in(v, F, a);
-  flush_fix(v, deda, s, F);
+  fix_range(v.status, fabsf(a.fx) + fabsf(a.fy) + fabsf(a.fz) + fabsf(a.da));
+  atomic_add_ll(&v.facc[3 * s], fx32(a.fx));
+  atomic_add_ll(&v.facc[3 * s + 1], fx32(a.fy));
+  atomic_add_ll(&v.facc[3 * s + 2], fx32(a.fz));
+  if (deda) atomic_add_ll(&deda[s], fx32(a.da));
 }
 
-__device__ __forceinline__ double warp_sum_d(double x) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-  return x;
-}
-
-// (ENERGY) a work item's pair energies: summed over the warp in FP64 (a fixed
-// butterfly order), entered in fixed point once per item
-__device__ __forceinline__ void flush_gb_energy(const DevView& v, int lane, int bi, EAcc& ea) {
-  ea.flush();
-  const double e0 = warp_sum_d(ea.v), e1 = warp_sum_d(ea.e), e2 = warp_sum_d(ea.p);
-  if (lane == 0) {
-    long long* E = v.eacc + (size_t)v.slot_sys[bi] * E_NSLOTS;
-    atomic_add_ll(&E[E_VDW], fix_energy_d(e0));
-    atomic_add_ll(&E[E_ELEC], fix_energy_d(e1));
-    atomic_add_ll(&E[E_POL_CROSS], fix_energy_d(e2));
-  }
-}
-
-template <bool ENERGY, bool FULL, bool PRECISE = true>
-__device__ __forceinline__ void gb_pair_tile2(const DevView& v, const GBConst& k, const Tile& A, const Tile& B,
-                                              int lane, const float* born, long long* deda, EAcc& ea) {
-  const int sa = A.bj * 32 + lane, sb = B.bj * 32 + lane, r0 = A.bi * 32;
-  const float4 xa = j_in_i_frame(v, A, lane), xb = j_in_i_frame(v, B, lane);
-  const float4 pa = v.par[sa], pb = v.par[sb];
-  const float aa = born[sa], ab = born[sb];
-  float4 xr = v.xq[r0 + lane], pr = v.par[r0 + lane];
-  float ar = born[r0 + lane];
-  double4 e_a = make_double4(0.0, 0.0, 0.0, 0.0), e_b = e_a, e_r = e_a;
-  double2 p_a = make_double2(0.0, 0.0), p_b = p_a;
-  if (ENERGY && PRECISE) {
-    e_a = v.epos[sa];
-    e_b = v.epos[sb];
-    p_a = v.epar[sa];
-    p_b = v.epar[sb];
-  }
-  PairAcc IA = {0.f, 0.f, 0.f, 0.f}, IB = {0.f, 0.f, 0.f, 0.f}, R = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 2
-  for (int kk = 0; kk < 32; kk++) {
-    const int sr = r0 + ((lane + kk) & 31);
-    {
-      float dx = xr.x - xa.x, dy = xr.y - xa.y, dz = xr.z - xa.z;
-      float r2 = dx * dx + dy * dy + dz * dz;
-      double r2d = 0.0;
-      const bool close = ENERGY && PRECISE && disp_fp64(v, k, e_a, sr, e_r, dx, dy, dz, r2, r2d);
-      const bool in = FULL || r2 <= k.cut2;
-      const float u = gb_u(r2, aa, ar);
-      const bool any_gb = __any_sync(0xffffffffu, in && gb_maybe_on(k, u));
-      PairE pe;
-      if (in)
-        gb_pair_one<ENERGY, FULL, true>(v, k, dx, dy, dz, r2, u, any_gb, xa.w, xr.w, pa.x, pa.y, pr.x, pr.y, aa, ar,
-                                        false, false, sa, sr, IA, R, pe);
-      if (ENERGY) add_pair_energy<true, PRECISE>(v, k, in, close, r2d, e_a, e_r, p_a, sr, false, false, pe, ea);
-    }
-    {
-      float dx = xr.x - xb.x, dy = xr.y - xb.y, dz = xr.z - xb.z;
-      float r2 = dx * dx + dy * dy + dz * dz;
-      double r2d = 0.0;
-      const bool close = ENERGY && PRECISE && disp_fp64(v, k, e_b, sr, e_r, dx, dy, dz, r2, r2d);
-      const bool in = FULL || r2 <= k.cut2;
-      const float u = gb_u(r2, ab, ar);
-      const bool any_gb = __any_sync(0xffffffffu, in && gb_maybe_on(k, u));
-      PairE pe;
-      if (in)
-        gb_pair_one<ENERGY, FULL, true>(v, k, dx, dy, dz, r2, u, any_gb, xb.w, xr.w, pb.x, pb.y, pr.x, pr.y, ab, ar,
-                                        false, false, sb, sr, IB, R, pe);
-      if (ENERGY) add_pair_energy<true, PRECISE>(v, k, in, close, r2d, e_b, e_r, p_b, sr, false, false, pe, ea);
-    }
-    if (ENERGY && (kk & 7) == 7) ea.flush();
-    ROT(xr.x); ROT(xr.y); ROT(xr.z); ROT(xr.w); ROT(pr.x); ROT(pr.y); ROT(ar);
-    ROT(R.fx); ROT(R.fy); ROT(R.fz); ROT(R.da);
-  }
-  flush_pair(v, deda, sa, IA);
-  flush_pair(v, deda, sb, IB);
-  flush_pair(v, deda, r0 + lane, R);
-}
-
-// The GB cross term of an all-inside pair the threshold test may switch on:
-// the exact decision (FP64 within rounding of the threshold, as gb_pair_one)
-// and, above it, the GB term (gbff.cpp:1592-1678) with Coulomb at eps_in in
-// place of eps_out.  akh, akr: Born radii times sqrtK; e1: the pair's eps_out
-// Coulomb energy; ir = 1/r.  Returns what the pair adds to dE/dr / r and to
-// the two atoms' dE/da.  Inlined under the caller's warp vote: a call (the
-// accumulators saved around it) or outputs through references (accumulators
-// kept in local memory) both cost more than the registers it adds.
-struct GBTerm {
-  float g, dah, dar;
+// Two pairs of the fused law on packed FP32x2 arithmetic.  In: r^2, the scaled
+// products QQ = -econv_out q q, EE = -12 eps, AA = K a a, and the LJ radius sums
+// SS.  Common pair: vacuum LJ + Coulomb at eps_out, dE/dr / r = -(12 eps (A - B)
+// + E_out) / r^2, whose bracket is one FFMA.  A pair with r^2 <= AA may lie
+// above the exp threshold; when any lane of the warp has one (a vote), the GB
+// term (gbff.cpp:1592-1678) is formed for both halves, with Coulomb at eps_in in
+// place of eps_out, and zeroed where the exact decision (FP64 within rounding of
+// the threshold) says no.
+//   MASKED: pa, pb: the pair counts at all (diagonal); xa, xb: bond order <= 2
+//     (GB term only); s14: 1-4 (vdw14 / elec14 scaling)
+//   FULL: inside every cutoff and switch radius
+//   FAST: the vacuum terms are part of the law (FastMode); else the GB term
+//     alone, premul q q / r below the threshold (calcBornForces, :1308-1325)
+struct Mask2 {
+  bool pa, pb, xa, xb, ma, mb;
 };
-__device__ __forceinline__ GBTerm gb_full_term(const DevView& v, const GBConst& k, float r2, float ir, float e1,
-                                               float akh, float akr, int sh, int sr) {
-  GBTerm t = {0.f, 0.f, 0.f};
-  const float ah = akh * k.inv_sqrtK, ar = akr * k.inv_sqrtK;
-  const float aiaj = ah * ar;
-  const float u = -0.25f * __fdividef(r2, aiaj);
-  bool on = u > k.thresh;
-  if (fabsf(u - k.thresh) <= 2e-6f * fabsf(k.thresh)) on = gb_on_fp64(v, sh, sr, k.thresh_d);
-  if (!on) return t;
-  const float r = r2 * ir;
-  const float qq = e1 * r * k.inv_eout;
-  const float tg = __expf(u);
-  const float fgb = rsqrtf(fmaf(tg, aiaj, r2));
-  const float l = fgb * fgb;
-  const float ep = k.premul * qq * fgb;
-  const float dedr = -ep * (r - 0.25f * r * tg) * l;
-  const float dalpha = -ep * tg * (1.f - u) * l;
-  t.g = 2.f * dedr * ir - k.in_over_out_m1 * e1 * ir * ir;
-  t.dah = dalpha * ar;
-  t.dar = dalpha * ah;
-  return t;
+// out: g = dE/dr / r (force on the held atom along d), W = dE/da per unit of the
+// partner's radius (zero unless `any`), and with ENERGY the pairs' energies
+// (vdW, Coulomb, GB cross term)
+struct Pair2 {
+  float2 g, W, ev, ee, ep;
+  bool any;
+};
+
+template <bool MASKED, bool FULL, bool FAST, bool ENERGY>
+__device__ __forceinline__ Pair2 gb_pair2(const DevView& v, const GBConst& k, float2 r2, float2 QQ, float2 SS,
+                                          float2 EE, float2 AA, const Mask2& m, int ha, int hb, int ra, int rb) {
+  Pair2 o;
+  const float2 ir = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
+  const float2 ir2 = __fmul2_rn(ir, ir);
+  const bool ina = (FULL || r2.x <= k.cut2) && (!MASKED || m.pa);
+  const bool inb = (FULL || r2.y <= k.cut2) && (!MASKED || m.pb);
+  float2 e1 = __fmul2_rn(QQ, ir);   // -E_out
+  // switching without a branch: below the inner cutoff w = 0 gives S = 1 and dS = 0 exactly
+  float2 S = f2(1.f), dS = f2(0.f), r = f2(0.f);
+  if (!FULL) {
+    r = __fmul2_rn(r2, ir);
+    const float2 w = make_float2(fmaxf(r.x - k.inner, 0.f), fmaxf(r.y - k.inner, 0.f));
+    const float2 wi = __fmul2_rn(w, f2(-k.invw2));
+    const float2 sw = __ffma2_rn(w, wi, f2(1.f));
+    dS = __fmul2_rn(__fmul2_rn(wi, sw), f2(4.f));
+    S = __fmul2_rn(sw, sw);
+  }
+  float2 vb = f2(0.f), ev = f2(0.f);   // -12 eps (A - B), eps (A - 2B)
+  if (FAST) {
+    if (MASKED) {
+      EE = __fmul2_rn(EE, make_float2(m.ma ? k.vdw14 : 1.f, m.mb ? k.vdw14 : 1.f));
+      e1 = __fmul2_rn(e1, make_float2(m.ma ? k.elec14 : 1.f, m.mb ? k.elec14 : 1.f));
+    }
+    const float2 t2 = __fmul2_rn(__fmul2_rn(SS, SS), ir2);
+    const float2 b6 = __fmul2_rn(__fmul2_rn(t2, t2), t2);
+    const float2 amb = __ffma2_rn(b6, b6, __fmul2_rn(b6, f2(-1.f)));
+    vb = __fmul2_rn(EE, amb);
+    if (ENERGY || !FULL) ev = __fmul2_rn(__ffma2_rn(EE, __fmul2_rn(b6, f2(-1.f)), vb), f2(-1.f / 12.f));
+    if (MASKED) {
+      vb = make_float2(m.xa ? 0.f : vb.x, m.xb ? 0.f : vb.y);
+      e1 = make_float2(m.xa ? 0.f : e1.x, m.xb ? 0.f : e1.y);
+      if (ENERGY || !FULL) ev = make_float2(m.xa ? 0.f : ev.x, m.xb ? 0.f : ev.y);
+    }
+  }
+  o.W = f2(0.f);
+  if (ENERGY) o.ep = f2(0.f);
+  float2 gg = f2(0.f);
+  const bool na = ina && r2.x <= AA.x, nb = inb && r2.y <= AA.y;
+  o.any = __any_sync(0xffffffffu, na || nb);
+  bool ona = false, onb = false;
+  if (o.any) {
+    const float2 rc = make_float2(rcp_ftz(AA.x), rcp_ftz(AA.y));
+    const float2 u = __fmul2_rn(__fmul2_rn(r2, rc), f2(k.kU));
+    const float tie = 2e-6f * fabsf(k.thresh);
+    ona = na && u.x > k.thresh;
+    onb = nb && u.y > k.thresh;
+    if (na && fabsf(u.x - k.thresh) <= tie) ona = gb_on_fp64(v, ha, ra, k.thresh_d);
+    if (nb && fabsf(u.y - k.thresh) <= tie) onb = gb_on_fp64(v, hb, rb, k.thresh_d);
+    const float2 tg = make_float2(__expf(u.x), __expf(u.y));
+    const float2 D = __ffma2_rn(tg, __fmul2_rn(AA, f2(k.invK)), r2);
+    const float2 fgb = make_float2(rsqrtf(D.x), rsqrtf(D.y));
+    float2 ep = __fmul2_rn(__fmul2_rn(QQ, f2(k.gb_ep)), fgb);
+    ep = make_float2(ona ? ep.x : 0.f, onb ? ep.y : 0.f);
+    float2 w = __fmul2_rn(ep, __fmul2_rn(fgb, fgb));
+    if (!FULL) w = __fmul2_rn(w, S);
+    gg = __fmul2_rn(w, __ffma2_rn(tg, f2(0.5f), f2(-2.f)));                   // 2 dE/dr / r
+    if (!FULL) gg = __ffma2_rn(__fmul2_rn(__fmul2_rn(ep, dS), f2(2.f)), ir, gg);
+    o.W = __fmul2_rn(__fmul2_rn(w, tg), __fadd2_rn(u, f2(-1.f)));             // -ep tg (1 - u) l
+    if (ENERGY) o.ep = __fmul2_rn(__fmul2_rn(ep, f2(2.f)), S);
+    if (FAST) e1 = make_float2(ona ? e1.x * k.in_over_out : e1.x, onb ? e1.y * k.in_over_out : e1.y);
+  }
+  if (!FAST) {
+    float2 ep = __fmul2_rn(__fmul2_rn(QQ, f2(k.gb_ep)), ir);
+    ep = make_float2(ona || !ina ? 0.f : ep.x, onb || !inb ? 0.f : ep.y);
+    gg = __ffma2_rn(__fmul2_rn(__fmul2_rn(ep, S), f2(-2.f)), ir2, gg);
+    gg = __ffma2_rn(__fmul2_rn(__fmul2_rn(ep, dS), f2(2.f)), ir, gg);
+    if (ENERGY) o.ep = __ffma2_rn(__fmul2_rn(ep, f2(2.f)), S, o.ep);
+    o.g = gg;
+    if (MASKED || !FULL) o.g = make_float2(ina ? o.g.x : 0.f, inb ? o.g.y : 0.f);
+    return o;
+  }
+  if (FULL) {
+    o.g = __ffma2_rn(__fadd2_rn(vb, e1), ir2, gg);
+    if (ENERGY) {
+      o.ev = ev;
+      o.ee = __fmul2_rn(e1, f2(-1.f));
+    }
+  } else {
+    const float2 w = make_float2(fmaxf(r.x - k.vdwinner, 0.f), fmaxf(r.y - k.vdwinner, 0.f));
+    const float2 wi = __fmul2_rn(w, f2(-k.vdwinvw2));
+    const float2 sw = __ffma2_rn(w, wi, f2(1.f));
+    const bool va = r.x < k.vdwcut, vb_ = r.y < k.vdwcut;
+    float2 Sv = __fmul2_rn(sw, sw), dSv = __fmul2_rn(__fmul2_rn(wi, sw), f2(4.f));
+    Sv = make_float2(va ? Sv.x : 0.f, vb_ ? Sv.y : 0.f);
+    dSv = make_float2(va ? dSv.x : 0.f, vb_ ? dSv.y : 0.f);
+    const float2 b = __ffma2_rn(Sv, vb, __fmul2_rn(S, e1));
+    const float2 d = __ffma2_rn(ev, dSv, __fmul2_rn(__fmul2_rn(e1, f2(-1.f)), dS));
+    o.g = __ffma2_rn(b, ir2, __ffma2_rn(d, ir, gg));
+    if (ENERGY) {
+      o.ev = __fmul2_rn(ev, Sv);
+      o.ee = __fmul2_rn(__fmul2_rn(e1, f2(-1.f)), S);
+    }
+  }
+  if (MASKED || !FULL) {   // (a select, not a product: the diagonal's own pair has r = 0)
+    o.g = make_float2(ina ? o.g.x : 0.f, inb ? o.g.y : 0.f);
+    if (ENERGY) {
+      o.ev = make_float2(ina ? o.ev.x : 0.f, inb ? o.ev.y : 0.f);
+      o.ee = make_float2(ina ? o.ee.x : 0.f, inb ? o.ee.y : 0.f);
+    }
+  }
+  return o;
 }
 
-// Force-only GB fused pair of an all-inside tile pair (the dynamics step's
-// body), the two held atoms on packed FP32x2 arithmetic.  Common pair: vacuum
-// LJ + Coulomb at eps_out,  dE/dr / r = -(12 eps (A - B) + E_out) / r^2,  with
-// the held atoms' charges scaled by -sqrt(econv_out) and sqrt(eps) by
-// -sqrt(12) (the rotating atom's by the positive factors), so one FFMA forms
-// the bracket with its sign.  A pair with r^2 <= K a_i a_j may lie above the
-// exp threshold; when any lane has one, gb_full_term runs for those pairs.
-__device__ __forceinline__ void gb_pair_full2(const DevView& v, const GBConst& k, const Tile& A, const Tile& B,
-                                              int lane, const float* born, long long* deda) {
-  const int sa = A.bj * 32 + lane, sb = B.bj * 32 + lane, r0 = A.bi * 32;
-  const float4 xa = j_in_i_frame(v, A, lane), xb = j_in_i_frame(v, B, lane);
-  const float4 pa = v.par[sa], pb = v.par[sb];
+// ---------------------------------------------------------------------------
+// Pair energies (ENERGY passes).  The vdW total is a small difference of large
+// repulsive and attractive sums: FP32 positions (rounded relative to their block
+// centres) on the close contacts, or FP32 sums, leave ~1e-6 of it.  So pairs
+// closer than sqrt(GBConst::eclose2) (4.5 A: the close contacts that carry the
+// large repulsive terms) are left out of the FP32 sums and listed, and their
+// energies formed in double-float from double-float positions and parameters,
+// the list dealt over the lanes; the other pairs' energies are the FP32 terms,
+// summed over 8 rotation steps and then in double-float.  A tile's sums meet over
+// the warp in double-float and enter fixed point once.  The displacements of these
+// passes are differences of double-float positions rounded once to FP32, so their
+// forces carry no rounding of the block frames (6e-7 of them, 1.2e-6 without).
+// ---------------------------------------------------------------------------
+// the rotating block in the warp's shared memory: single tiles as step pairs
+// (x, x', y, y'), (z, z', q, q'), (LJ radius, ', sqrt(12 eps), ') and (Born radius
+// x sqrtK, '); tile pairs as (x, y, z, q) and (LJ radius, sqrt(12 eps), Born radius
+// x sqrtK, -), twice over, so that a lane's row at step kk lies at a fixed offset
+struct PairRows {
+  union {
+    struct {
+      float4 xy[32], zq[32], se[32];
+      float2 ak[32];
+    };
+    struct {
+      float4 x2[64], p2[64];
+    };
+  };
+};
+struct PairRowsE : PairRows {
+  float4 lxy[32];                  // what FP32 rounding takes off (x, x', y, y')
+  float2 lz[32];                   // and (z, z')
+  unsigned short pair[1024];       // i lane | j row << 5 | bond order <= 2 << 10 | 1-4 << 11
+};
+
+// (ENERGY) energies of one listed close pair into the sums
+struct GBESum {
+  DF v, e, p;
+};
+template <bool FAST>
+__device__ __forceinline__ void gb_close_energy(const DevView& v, const GBConst& k, const Tile& T, const DF O[3],
+                                                unsigned code, const float* born, GBESum& sum) {
+  const int si = T.bi * 32 + (code & 31), sj = T.bj * 32 + ((code >> 5) & 31);
+  const bool excl = code & 1024u, is14 = code & 2048u;
+  const float4 xh = v.xq[si], xl = v.rlo[si], yh = v.xq[sj], yl = v.rlo[sj], pi = v.par[si], pj = v.par[sj];
+  const float2 pil = v.plo[si], pjl = v.plo[sj];
+  const DF dx = df_sub(df_add(DF{yh.x, yl.x}, O[0]), DF{xh.x, xl.x});
+  const DF dy = df_sub(df_add(DF{yh.y, yl.y}, O[1]), DF{xh.y, xl.y});
+  const DF dz = df_sub(df_add(DF{yh.z, yl.z}, O[2]), DF{xh.z, xl.z});
+  const DF r2 = df_norm2(dx, dy, dz);
+  const DF ir = df_rsqrt(r2);
+  const float r = r2.h * ir.h;
+  const float ai = born[si], aj = born[sj];
+  const float u = -0.25f * __fdividef(r2.h, ai * aj);
+  bool on = u > k.thresh;
+  if (fabsf(u - k.thresh) <= 2e-6f * fabsf(k.thresh)) on = gb_on_fp64(v, si, sj, k.thresh_d);
+  const float w = fmaxf(r - k.inner, 0.f), sw = 1.f - w * w * k.invw2, S = sw * sw;
+  const DF qq = df_norm(df_mul(DF{xh.w, xl.w}, DF{yh.w, yl.w}));
+  const DF c = df_norm(df_mul(qq, ir));
+  if (on) {
+    const float fgb = rsqrtf(fmaf(__expf(u), ai * aj, r2.h));
+    df_acc(sum.p, df_norm(df_scale(df_mul(k.premul2_f, qq), fgb * S)));
+  } else if (!FAST) {
+    df_acc(sum.p, df_norm(df_scale(df_mul(k.premul2_f, c), S)));
+  }
+  if (FAST && !excl) {
+    DF E = df_norm(df_mul(on ? k.econv_in_f : k.econv_out_f, c));
+    if (is14) E = df_norm(df_mul(E, k.elec14_f));
+    df_acc(sum.e, df_norm(df_scale(E, S)));
+    const DF R = df_norm(df_add(DF{pi.x, pil.x}, DF{pj.x, pjl.x}));
+    const DF t = df_norm(df_mul(R, ir)), t2 = df_norm(df_mul(t, t));
+    const DF B = df_norm(df_mul(df_mul(t2, t2), t2));
+    DF eps = df_norm(df_mul(DF{pi.y, pil.y}, DF{pj.y, pjl.y}));
+    if (is14) eps = df_norm(df_mul(eps, k.vdw14_f));
+    const float wv = fmaxf(r - k.vdwinner, 0.f), sv = 1.f - wv * wv * k.vdwinvw2;
+    const float Sv = r < k.vdwcut ? sv * sv : 0.f;
+    df_acc(sum.v, df_norm(df_scale(df_mul(eps, df_norm(df_sub(df_mul(B, B), df_scale2(B, 2.f)))), Sv)));
+  }
+}
+
+// Pair pass of a single tile, step-packed: lane l holds i atom l (its values in
+// both halves), the j block's atoms l + kk and l + kk + 1 come from the warp's
+// rows; the rotating atoms' sums move two lanes per step.
+template <bool MASKED, bool FULL, bool FAST, bool ENERGY, bool PRECISE>
+__device__ __forceinline__ void gb_pair_tile(const DevView& v, const GBConst& k, const Tile& T, int lane,
+                                             const float* born, long long* deda, PairRows& rs, PairRowsE* re) {
+  const int si = T.bi * 32 + lane, j0 = T.bj * 32, l1 = (lane + 1) & 31;
+  const float4 xi = v.xq[si], pi = v.par[si];
+  DF O[3];                 // (PRECISE) centre of bj seen from bi
+  float2 XL, YL, ZL;       // remainders of the held atom, negated
+  unsigned ex = 0u, m14 = 0u, dm = 0u;
+  if (MASKED) {
+    tile_masks(v, T, lane, ex, m14);
+    dm = (T.flags & 2) ? diag_exclusion(lane) : 0u;
+  }
+  {
+    float4 x0 = j_in_i_frame(v, T, lane);
+    const float4 p0 = v.par[j0 + lane];
+    if (PRECISE) {
+      const float o[3] = {T.ox, T.oy, T.oz};
+      df_offset(v, v.sys[v.slot_sys[T.bi]], T.bi, T.bj, o, O);
+      const float4 h = v.xq[j0 + lane], l = v.rlo[j0 + lane], li = v.rlo[si];
+      const DF jx = df_norm(df_add(DF{h.x, l.x}, O[0])), jy = df_norm(df_add(DF{h.y, l.y}, O[1]));
+      const DF jz = df_norm(df_add(DF{h.z, l.z}, O[2]));
+      x0.x = jx.h;
+      x0.y = jy.h;
+      x0.z = jz.h;
+      const float x1 = __shfl_sync(0xffffffffu, jx.l, l1), y1 = __shfl_sync(0xffffffffu, jy.l, l1);
+      const float z1 = __shfl_sync(0xffffffffu, jz.l, l1);
+      __syncwarp();
+      re->lxy[lane] = make_float4(jx.l, x1, jy.l, y1);
+      re->lz[lane] = make_float2(jz.l, z1);
+      XL = f2(-li.x);
+      YL = f2(-li.y);
+      ZL = f2(-li.z);
+    }
+    const float q0 = k.sq_eout * x0.w, e0 = k.sqrt12 * p0.y, a0 = k.sqrtK * born[j0 + lane];
+    const float x1 = __shfl_sync(0xffffffffu, x0.x, l1), y1 = __shfl_sync(0xffffffffu, x0.y, l1);
+    const float z1 = __shfl_sync(0xffffffffu, x0.z, l1), q1 = __shfl_sync(0xffffffffu, q0, l1);
+    const float s1 = __shfl_sync(0xffffffffu, p0.x, l1), e1 = __shfl_sync(0xffffffffu, e0, l1);
+    const float a1 = __shfl_sync(0xffffffffu, a0, l1);
+    __syncwarp();
+    rs.xy[lane] = make_float4(x0.x, x1, x0.y, y1);
+    rs.zq[lane] = make_float4(x0.z, z1, q0, q1);
+    rs.se[lane] = make_float4(p0.x, s1, e0, e1);
+    rs.ak[lane] = make_float2(a0, a1);
+    __syncwarp();
+  }
+  const float2 X = f2(-xi.x), Y = f2(-xi.y), Z = f2(-xi.z), Q = f2(k.neg_sq_eout * xi.w), R = f2(pi.x);
+  const float2 E = f2(-k.sqrt12 * pi.y), AK = f2(k.sqrtK * born[si]);
+  float2 FX = f2(0.f), FY = f2(0.f), FZ = f2(0.f), DA = f2(0.f);
+  float2 RX = f2(0.f), RY = f2(0.f), RZ = f2(0.f), RA = f2(0.f);   // minus the rotating atoms' forces; their dE/da
+  float2 cv = f2(0.f), ce = f2(0.f), cp = f2(0.f);                 // (ENERGY) FP32 sums of 8 steps
+  GBESum sum = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
+  int np = 0;
+#pragma unroll 1
+  for (int kk = 0; kk < 32; kk += 2) {
+    const int j = (lane + kk) & 31;
+    const float4 P = rs.xy[j], ZQ = rs.zq[j], SE = rs.se[j];
+    const float2 ak = rs.ak[j];
+    float2 dx = __fadd2_rn(make_float2(P.x, P.y), X), dy = __fadd2_rn(make_float2(P.z, P.w), Y);
+    float2 dz = __fadd2_rn(make_float2(ZQ.x, ZQ.y), Z);
+    if (PRECISE) {
+      const float4 L = re->lxy[j];
+      dx = __fadd2_rn(dx, __fadd2_rn(make_float2(L.x, L.y), XL));
+      dy = __fadd2_rn(dy, __fadd2_rn(make_float2(L.z, L.w), YL));
+      dz = __fadd2_rn(dz, __fadd2_rn(re->lz[j], ZL));
+    }
+    const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
+    Mask2 m = {true, true, false, false, false, false};
+    if (MASKED) {
+      m.pa = !((dm >> kk) & 1u);
+      m.pb = !((dm >> kk) & 2u);
+      m.xa = (ex >> kk) & 1u;
+      m.xb = (ex >> kk) & 2u;
+      m.ma = (m14 >> kk) & 1u;
+      m.mb = (m14 >> kk) & 2u;
+    }
+    const Pair2 o = gb_pair2<MASKED, FULL, FAST, ENERGY>(
+        v, k, r2, __fmul2_rn(Q, make_float2(ZQ.z, ZQ.w)), __fadd2_rn(R, make_float2(SE.x, SE.y)),
+        __fmul2_rn(E, make_float2(SE.z, SE.w)), __fmul2_rn(AK, ak), m, si, si, j0 + j, j0 + ((j + 1) & 31));
+    FX = __ffma2_rn(o.g, dx, FX); FY = __ffma2_rn(o.g, dy, FY); FZ = __ffma2_rn(o.g, dz, FZ);
+    RX = __ffma2_rn(o.g, dx, RX); RY = __ffma2_rn(o.g, dy, RY); RZ = __ffma2_rn(o.g, dz, RZ);
+    if (o.any) {
+      DA = __ffma2_rn(o.W, ak, DA);
+      RA = __ffma2_rn(o.W, AK, RA);
+    }
+    ROT2(RX); ROT2(RY); ROT2(RZ); ROT2(RA);
+    if (ENERGY) {
+      float2 f = f2(1.f);
+      if (PRECISE) {
+        const bool ca = r2.x < k.eclose2 && (FULL || r2.x <= k.cut2) && m.pa;
+        const bool cb = r2.y < k.eclose2 && (FULL || r2.y <= k.cut2) && m.pb;
+        if (__any_sync(0xffffffffu, ca || cb)) {
+          const unsigned ma = __ballot_sync(0xffffffffu, ca), mb = __ballot_sync(0xffffffffu, cb);
+          const unsigned lt = (1u << lane) - 1u;
+          if (ca)
+            re->pair[np + __popc(ma & lt)] = (unsigned short)(lane | (j << 5) | (m.xa ? 1024 : 0) | (m.ma ? 2048 : 0));
+          np += __popc(ma);
+          if (cb)
+            re->pair[np + __popc(mb & lt)] =
+                (unsigned short)(lane | (((j + 1) & 31) << 5) | (m.xb ? 1024 : 0) | (m.mb ? 2048 : 0));
+          np += __popc(mb);
+          f = make_float2(ca ? 0.f : 1.f, cb ? 0.f : 1.f);
+        }
+      }
+      if (FAST) {
+        cv = __ffma2_rn(f, o.ev, cv);
+        ce = __ffma2_rn(f, o.ee, ce);
+      }
+      cp = __ffma2_rn(f, o.ep, cp);
+      if ((kk & 6) == 6) {
+        if (FAST) {
+          df_acc(sum.v, df_two_sum(cv.x, cv.y));
+          df_acc(sum.e, df_two_sum(ce.x, ce.y));
+        }
+        df_acc(sum.p, df_two_sum(cp.x, cp.y));
+        cv = ce = cp = f2(0.f);
+      }
+    }
+  }
+  const int lm = (lane + 31) & 31;
+  const float rx = RX.x + __shfl_sync(0xffffffffu, RX.y, lm), ry = RY.x + __shfl_sync(0xffffffffu, RY.y, lm);
+  const float rz = RZ.x + __shfl_sync(0xffffffffu, RZ.y, lm), ra = RA.x + __shfl_sync(0xffffffffu, RA.y, lm);
+  flush_pair(v, deda, si, PairAcc{FX.x + FX.y, FY.x + FY.y, FZ.x + FZ.y, (DA.x + DA.y) * k.inv_sqrtK});
+  flush_pair(v, deda, j0 + lane, PairAcc{-rx, -ry, -rz, ra * k.inv_sqrtK});
+  if (ENERGY) {
+    if (PRECISE) {
+      __syncwarp();
+      for (int p = lane; p < np; p += 32) gb_close_energy<FAST>(v, k, T, O, re->pair[p], born, sum);
+      __syncwarp();
+    }
+    const DF e0 = df_warp_sum(sum.v), e1 = df_warp_sum(sum.e), e2 = df_warp_sum(sum.p);
+    const DF x = lane == 0 ? e0 : (lane == 1 ? e1 : e2);
+    if (lane < 3) {
+      long long* En = v.eacc + (size_t)v.slot_sys[T.bi] * E_NSLOTS;
+      atomic_add_ll(&En[lane == 0 ? E_VDW : (lane == 1 ? E_ELEC : E_POL_CROSS)],
+                    fix_energy_d((double)x.h + (double)x.l));
+    }
+  }
+}
+
+// Force-only pass of an all-inside tile pair (the dynamics step's body): each
+// lane holds one atom of either j block (.x: bj, .y: bj + 1), the shared bi
+// block's atoms come from the warp's rows, their sums rotate by shuffles.  FAR:
+// no pair of the item may lie above the exp threshold (no GB term, no dE/da).
+template <bool FAR>
+__device__ __forceinline__ void gb_pair_loop2(const DevView& v, const GBConst& k, int lane, int sa, int sb, int r0,
+                                              const PairRows& rs, const float4& xa, const float4& xb,
+                                              const float4& pa, const float4& pb, float2 AK, float2& FX, float2& FY,
+                                              float2& FZ, float2& DA, PairAcc& R) {
   const float2 nx = make_float2(-xa.x, -xb.x), ny = make_float2(-xa.y, -xb.y), nz = make_float2(-xa.z, -xb.z);
-  const float2 QN = make_float2(-k.sq_eout * xa.w, -k.sq_eout * xb.w);
+  const float2 QN = make_float2(k.neg_sq_eout * xa.w, k.neg_sq_eout * xb.w);
   const float2 S = make_float2(pa.x, pb.x);
   const float2 EN = make_float2(-k.sqrt12 * pa.y, -k.sqrt12 * pb.y);
-  const float2 AK = make_float2(k.sqrtK * born[sa], k.sqrtK * born[sb]);
-  const float2 M1 = f2(-1.f);
-  float4 xr = v.xq[r0 + lane];
-  const float4 pr = v.par[r0 + lane];
-  float qr = k.sq_eout * xr.w, sgr = pr.x, er = k.sqrt12 * pr.y, akr = k.sqrtK * born[r0 + lane];
-  float2 FX = f2(0.f), FY = f2(0.f), FZ = f2(0.f), DA = f2(0.f);
-  PairAcc R = {0.f, 0.f, 0.f, 0.f};
+  const Mask2 m = {true, true, false, false, false, false};
+  const float4 *x2 = rs.x2 + lane, *p2 = rs.p2 + lane;
 #pragma unroll 2
   for (int kk = 0; kk < 32; kk++) {
+    const float4 xr = x2[kk];
+    const float4 pr = p2[kk];
     const float2 dx = __fadd2_rn(f2(xr.x), nx), dy = __fadd2_rn(f2(xr.y), ny), dz = __fadd2_rn(f2(xr.z), nz);
     const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
-    const float2 lim = __fmul2_rn(AK, f2(akr));
-    const bool na = r2.x <= lim.x, nb = r2.y <= lim.y;
-    const float2 ir = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
-    const float2 ir2 = __fmul2_rn(ir, ir);
-    const float2 e1n = __fmul2_rn(__fmul2_rn(QN, f2(qr)), ir);   // -E_out
-    const float2 s = __fadd2_rn(S, f2(sgr));
-    const float2 t2 = __fmul2_rn(__fmul2_rn(s, s), ir2);
-    const float2 b6 = __fmul2_rn(__fmul2_rn(t2, t2), t2);
-    const float2 amb = __ffma2_rn(b6, b6, __fmul2_rn(b6, M1));    // A - B
-    float2 g = __fmul2_rn(__ffma2_rn(__fmul2_rn(EN, f2(er)), amb, e1n), ir2);
-    if (__any_sync(0xffffffffu, na || nb)) {
+    const float2 QQ = __fmul2_rn(QN, f2(xr.w)), SS = __fadd2_rn(S, f2(pr.x)), EE = __fmul2_rn(EN, f2(pr.y));
+    float2 g;
+    if (FAR) {
+      const float2 ir = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
+      const float2 ir2 = __fmul2_rn(ir, ir);
+      const float2 t2 = __fmul2_rn(__fmul2_rn(SS, SS), ir2);
+      const float2 b6 = __fmul2_rn(__fmul2_rn(t2, t2), t2);
+      const float2 amb = __fmul2_rn(b6, __fadd2_rn(b6, f2(-1.f)));
+      g = __fmul2_rn(__ffma2_rn(EE, amb, __fmul2_rn(QQ, ir)), ir2);
+    } else {
       const int sr = r0 + ((lane + kk) & 31);
-      if (na) {
-        const GBTerm t = gb_full_term(v, k, r2.x, ir.x, -e1n.x, AK.x, akr, sa, sr);
-        g.x += t.g;
-        DA.x += t.dah;
-        R.da += t.dar;
-      }
-      if (nb) {
-        const GBTerm t = gb_full_term(v, k, r2.y, ir.y, -e1n.y, AK.y, akr, sb, sr);
-        g.y += t.g;
-        DA.y += t.dah;
-        R.da += t.dar;
+      const Pair2 o = gb_pair2<false, true, true, false>(v, k, r2, QQ, SS, EE, __fmul2_rn(AK, f2(pr.z)), m, sa, sb,
+                                                         sr, sr);
+      g = o.g;
+      if (o.any) {
+        DA = __ffma2_rn(o.W, f2(pr.z), DA);
+        R.da = fmaf(o.W.x, AK.x, R.da);
+        R.da = fmaf(o.W.y, AK.y, R.da);
       }
     }
     FX = __ffma2_rn(g, dx, FX);
     FY = __ffma2_rn(g, dy, FY);
     FZ = __ffma2_rn(g, dz, FZ);
-    R.fx = fmaf(-g.x, dx.x, R.fx); R.fx = fmaf(-g.y, dx.y, R.fx);
-    R.fy = fmaf(-g.x, dy.x, R.fy); R.fy = fmaf(-g.y, dy.y, R.fy);
-    R.fz = fmaf(-g.x, dz.x, R.fz); R.fz = fmaf(-g.y, dz.y, R.fz);
-    ROT(xr.x); ROT(xr.y); ROT(xr.z); ROT(qr); ROT(sgr); ROT(er); ROT(akr);
-    ROT(R.fx); ROT(R.fy); ROT(R.fz); ROT(R.da);
+    R.fx = fmaf(g.x, dx.x, R.fx); R.fx = fmaf(g.y, dx.y, R.fx);
+    R.fy = fmaf(g.x, dy.x, R.fy); R.fy = fmaf(g.y, dy.y, R.fy);
+    R.fz = fmaf(g.x, dz.x, R.fz); R.fz = fmaf(g.y, dz.y, R.fz);
+    ROT(R.fx); ROT(R.fy); ROT(R.fz);
+    if (!FAR) ROT(R.da);
   }
-  flush_pair(v, deda, sa, PairAcc{FX.x, FY.x, FZ.x, DA.x});
-  flush_pair(v, deda, sb, PairAcc{FX.y, FY.y, FZ.y, DA.y});
-  flush_pair(v, deda, r0 + lane, R);
 }
 
-// EMODE 0: forces and dE/da only; 1: with energies (close pairs in FP64);
-// 2: with energies from FP32 pair terms (a gradient call's energy pass)
-template <int EMODE>
-__device__ __forceinline__ void gb_pair_items(const DevView& v, const GBConst& k, const float* born, long long* deda) {
-  constexpr bool ENERGY = EMODE != 0, PRECISE = EMODE == 1;
+__device__ __forceinline__ void gb_pair_full2(const DevView& v, const GBConst& k, const Tile& A, const Tile& B,
+                                              int lane, const float* born, long long* deda, PairRows& rs) {
+  const int sa = A.bj * 32 + lane, sb = B.bj * 32 + lane, r0 = A.bi * 32;
+  const float4 xa = j_in_i_frame(v, A, lane), xb = j_in_i_frame(v, B, lane);
+  const float4 pa = v.par[sa], pb = v.par[sb];
+  const float2 AK = make_float2(k.sqrtK * born[sa], k.sqrtK * born[sb]);
+  float akm;
+  const float4 x0 = v.xq[r0 + lane];
+  {
+    const float4 p0 = v.par[r0 + lane];
+    const float a0 = k.sqrtK * born[r0 + lane];
+    __syncwarp();
+    rs.x2[lane] = rs.x2[lane + 32] = make_float4(x0.x, x0.y, x0.z, k.sq_eout * x0.w);
+    rs.p2[lane] = rs.p2[lane + 32] = make_float4(p0.x, k.sqrt12 * p0.y, a0, 0.f);
+    __syncwarp();
+    akm = warp_max(a0) * 1.00001f;
+  }
+  float2 FX = f2(0.f), FY = f2(0.f), FZ = f2(0.f), DA = f2(0.f);
+  PairAcc R = {0.f, 0.f, 0.f, 0.f};   // minus the rotating atom's force; its dE/da
+  if (item_far(xa, xb, x0, AK.x * akm, AK.y * akm)) {
+    gb_pair_loop2<true>(v, k, lane, sa, sb, r0, rs, xa, xb, pa, pb, AK, FX, FY, FZ, DA, R);
+    deda = nullptr;
+  } else {
+    gb_pair_loop2<false>(v, k, lane, sa, sb, r0, rs, xa, xb, pa, pb, AK, FX, FY, FZ, DA, R);
+  }
+  flush_pair(v, deda, sa, PairAcc{FX.x, FY.x, FZ.x, DA.x * k.inv_sqrtK});
+  flush_pair(v, deda, sb, PairAcc{FX.y, FY.y, FZ.y, DA.y * k.inv_sqrtK});
+  flush_pair(v, deda, r0 + lane, PairAcc{-R.fx, -R.fy, -R.fz, R.da * k.inv_sqrtK});
+}
+
+template <bool FAST, bool ENERGY, bool PRECISE>
+__device__ __forceinline__ void gb_pair_single(const DevView& v, const GBConst& k, const Tile& T, int lane,
+                                               const float* born, long long* deda, PairRows& rs,
+                                               PairRowsE* re) {
+  const bool full = tile_full(T);
+  if (!FAST || ENERGY) {   // (rarer passes: the masked bodies serve every tile)
+    if (full) gb_pair_tile<true, true, FAST, ENERGY, PRECISE>(v, k, T, lane, born, deda, rs, re);
+    else gb_pair_tile<true, false, FAST, ENERGY, PRECISE>(v, k, T, lane, born, deda, rs, re);
+  } else if (tile_masked(T)) {
+    if (full) gb_pair_tile<true, true, FAST, ENERGY, PRECISE>(v, k, T, lane, born, deda, rs, re);
+    else gb_pair_tile<true, false, FAST, ENERGY, PRECISE>(v, k, T, lane, born, deda, rs, re);
+  } else {
+    if (full) gb_pair_tile<false, true, FAST, ENERGY, PRECISE>(v, k, T, lane, born, deda, rs, re);
+    else gb_pair_tile<false, false, FAST, ENERGY, PRECISE>(v, k, T, lane, born, deda, rs, re);
+  }
+}
+
+// the force-only pass (every dynamics step) runs in CTAs of 128 threads, five
+// per SM (20 warps at 96 registers; seven at 72 spill and were 5 % slower); FAST off: calcBornForces (gbff.cpp:1189-1340),
+// LJ and Coulomb come from the NB kernel with the GB object's own settings
+constexpr int kPairThreads = 128, kPairEThreads = 128;
+template <bool FAST>
+__global__ void __launch_bounds__(kPairThreads, 5) k_gb_pair(const __grid_constant__ DevView v, const __grid_constant__ GBConst k, const float* born, long long* deda) {
+  __shared__ PairRows rows[kPairThreads / 32];
+  PairRows& rs = rows[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   const int ni = *v.nitems;
@@ -790,88 +777,27 @@ __device__ __forceinline__ void gb_pair_items(const DevView& v, const GBConst& k
     bool two;
     const int t = item_tile(v, it, two);
     const Tile T = v.tiles[t];
-    if (two) {
-      const Tile U = v.tiles[t + 1];
-      EAcc ea;
-      if (tile_full(T)) {
-        if (ENERGY) gb_pair_tile2<true, true, PRECISE>(v, k, T, U, lane, born, deda, ea);
-        else gb_pair_full2(v, k, T, U, lane, born, deda);
-      }
-      else gb_pair_tile2<ENERGY, false, PRECISE>(v, k, T, U, lane, born, deda, ea);
-      if (ENERGY) flush_gb_energy(v, lane, T.bi, ea);
+    if (FAST && two && tile_full(T)) {
+      gb_pair_full2(v, k, T, v.tiles[t + 1], lane, born, deda, rs);
       continue;
     }
-    const int si = T.bi * 32 + lane;
-    const float4 xi = v.xq[si], pi = v.par[si];
-    const float ai = born[si];
-    unsigned ex, m14;
-    tile_masks(v, T, lane, ex, m14);
-    const unsigned dmask = (T.flags & 2) ? diag_exclusion(lane) : 0u;
-    PairAcc I = {0.f, 0.f, 0.f, 0.f}, J = {0.f, 0.f, 0.f, 0.f};
-    EAcc ea;
-    const bool full = tile_full(T);
-    if (tile_masked(T)) {
-      if (full)
-        gb_pair_tile<true, ENERGY, true, true, PRECISE>(v, k, T, lane, si, xi, pi, ai, ex, m14, dmask, born, I, J,
-                                                         ea);
-      else
-        gb_pair_tile<true, ENERGY, false, true, PRECISE>(v, k, T, lane, si, xi, pi, ai, ex, m14, dmask, born, I, J,
-                                                         ea);
-    } else {
-      if (full)
-        gb_pair_tile<false, ENERGY, true, true, PRECISE>(v, k, T, lane, si, xi, pi, ai, ex, m14, dmask, born, I, J,
-                                                         ea);
-      else
-        gb_pair_tile<false, ENERGY, false, true, PRECISE>(v, k, T, lane, si, xi, pi, ai, ex, m14, dmask, born, I, J,
-                                                         ea);
-    }
-    flush_pair(v, deda, si, I);
-    flush_pair(v, deda, T.bj * 32 + lane, J);
-    if (ENERGY) flush_gb_energy(v, lane, T.bi, ea);
+    gb_pair_single<FAST, false, false>(v, k, T, lane, born, deda, rs, nullptr);
+    if (two) gb_pair_single<FAST, false, false>(v, k, v.tiles[t + 1], lane, born, deda, rs, nullptr);
   }
 }
 
-// the force-only pass (every dynamics step) runs in CTAs of 128 threads, seven
-// per SM (28 warps at 72 registers; 3 CTAs of 256 hold 24 at 80), launched as
-// twice the tile kernels' CTA count; the energy pass carries FP64 records of
-// its close pairs and gets more registers
-__global__ void __launch_bounds__(128, 7) k_gb_pair(const __grid_constant__ DevView v, const __grid_constant__ GBConst k, const float* born, long long* deda) {
-  gb_pair_items<0>(v, k, born, deda);
-}
-__global__ void __launch_bounds__(256, 2) k_gb_pair_energy(const __grid_constant__ DevView v, const __grid_constant__ GBConst k, const float* born,
-                                                           long long* deda) {
-  gb_pair_items<1>(v, k, born, deda);
-}
-__global__ void __launch_bounds__(256, 3) k_gb_pair_energy32(const __grid_constant__ DevView v, const __grid_constant__ GBConst k, const float* born,
-                                                             long long* deda) {
-  gb_pair_items<2>(v, k, born, deda);
-}
-
-// FastMode off (calcBornForces, gbff.cpp:1189-1340): the GB term of every pair
-// within Cutoff, premul q_i q_j / r below the threshold; LJ and Coulomb come from
-// the NB kernel with the GB object's own FF_NonBonded settings.  One masked body
-// serves every tile: this mode exists for parity with PD, not for speed.
-template <bool ENERGY>
-__global__ void __launch_bounds__(256) k_gb_pair_born_only(const __grid_constant__ DevView v, const __grid_constant__ GBConst k, const float* born,
-                                                           long long* deda) {
+// the pass with energies, tile by tile (PRECISE: close pairs in double-float;
+// else a gradient call's energies, FP32 pair terms)
+template <bool FAST, bool PRECISE>
+__global__ void __launch_bounds__(kPairEThreads, 4) k_gb_pair_energy(const __grid_constant__ DevView v, const __grid_constant__ GBConst k, const float* born,
+                                                                    long long* deda) {
+  __shared__ PairRowsE rows[kPairEThreads / 32];
+  PairRowsE& rs = rows[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   const int nt = *v.ntiles;
-  for (int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < nt; t += nwarps) {
-    const Tile T = v.tiles[t];
-    const int si = T.bi * 32 + lane;
-    const float4 xi = v.xq[si], pi = v.par[si];
-    const float ai = born[si];
-    unsigned ex, m14;
-    tile_masks(v, T, lane, ex, m14);
-    const unsigned dmask = (T.flags & 2) ? diag_exclusion(lane) : 0u;
-    PairAcc I = {0.f, 0.f, 0.f, 0.f}, J = {0.f, 0.f, 0.f, 0.f};
-    EAcc ea;
-    gb_pair_tile<true, ENERGY, false, false>(v, k, T, lane, si, xi, pi, ai, ex, m14, dmask, born, I, J, ea);
-    flush_pair(v, deda, si, I);
-    flush_pair(v, deda, T.bj * 32 + lane, J);
-    if (ENERGY) flush_gb_energy(v, lane, T.bi, ea);
-  }
+  for (int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < nt; t += nwarps)
+    gb_pair_single<FAST, true, PRECISE>(v, k, v.tiles[t], lane, born, deda, rs, &rs);
 }
 
 // self term, total dE/da and the chain-rule prefactor a^2/166 * dE/da * P4
@@ -902,113 +828,7 @@ __global__ void k_gb_self(DevView v, const double* charge, GBConst k, double pre
 // ---------------------------------------------------------------------------
 // pass 3: dE/da chain rule through the Born radii, both directions of a pair
 // ---------------------------------------------------------------------------
-// (c_i V_j + c_j V_i) (4 CCF - dCCF) / r^6 of one pair: the chain-rule force per unit d
-__device__ __forceinline__ float chain_w(const GBConst& k, float r2, float rs, float cv, bool any_contact) {
-  const float rs2 = rs * rs;
-  float ccf = 1.f, dccf = 0.f;
-  if (any_contact) {
-    if (gb_contact(k, r2, rs2)) {
-      float sn, cs;
-      const float x = __fdividef(r2, rs2) * k.P5;
-      sincospif(x, &sn, &cs);
-      const float h = 0.5f - 0.5f * cs;
-      ccf = h * h;
-      dccf = 2.f * h * sn * (x * 3.14159265358979f);
-    }
-  }
-  const float ir2 = rcp_ftz(r2);
-  return cv * (4.f * ccf - dccf) * ir2 * ir2 * ir2;
-}
-
-template <bool MASKED, bool FULL>
-__device__ __forceinline__ void chain_tile(const DevView& v, const GBConst& k, const Tile& T, int lane, int si,
-                                           const float4& xi, const float4& pi, float ci, unsigned ex,
-                                           const float* chain, PairAcc& I, PairAcc& J) {
-  float4 xj = j_in_i_frame(v, T, lane);
-  float4 pj = v.par[T.bj * 32 + lane];
-  float cj = chain[T.bj * 32 + lane];
-#pragma unroll 4
-  for (int kk = 0; kk < 32; kk++) {
-    const float dx = xj.x - xi.x, dy = xj.y - xi.y, dz = xj.z - xi.z;
-    const float r2 = dx * dx + dy * dy + dz * dz;
-    bool in = still_in<FULL>(v, k, r2, si, T.bj * 32 + ((lane + kk) & 31));
-    if (MASKED) in = in && !((ex >> kk) & 1u);
-    const float rs = pi.z + pj.z;
-    const bool anyc = __any_sync(0xffffffffu, in && gb_contact(k, r2, rs * rs));
-    if (in) {
-      const float w = chain_w(k, r2, rs, ci * pj.w + cj * pi.w, anyc);
-      I.fx -= w * dx; I.fy -= w * dy; I.fz -= w * dz;
-      J.fx += w * dx; J.fy += w * dy; J.fz += w * dz;
-    }
-    ROT(xj.x); ROT(xj.y); ROT(xj.z); ROT(pj.z); ROT(pj.w); ROT(cj); ROT(J.fx); ROT(J.fy); ROT(J.fz);
-  }
-}
-
-__device__ __forceinline__ void flush_force(const DevView& v, int s, const PairAcc& a) {
-  FixAcc F = {0, 0, 0, 0};
-  fix_in(v, F, a);
-  flush_fix(v, nullptr, s, F);
-}
-
-template <bool FULL>
-__device__ __forceinline__ void chain_tile2(const DevView& v, const GBConst& k, const Tile& A, const Tile& B, int lane,
-                                            const float* chain) {
-  const int sa = A.bj * 32 + lane, sb = B.bj * 32 + lane, r0 = A.bi * 32;
-  const float4 xa = j_in_i_frame(v, A, lane), xb = j_in_i_frame(v, B, lane);
-  const float4 pa = v.par[sa], pb = v.par[sb];
-  const float2 nx = make_float2(-xa.x, -xb.x), ny = make_float2(-xa.y, -xb.y), nz = make_float2(-xa.z, -xb.z);
-  const float2 RS = make_float2(pa.z, pb.z), VS = make_float2(pa.w, pb.w);
-  const float2 CS = make_float2(chain[sa], chain[sb]);
-  float4 xr = v.xq[r0 + lane], pr = v.par[r0 + lane];
-  float cr = chain[r0 + lane];
-  float2 FX = f2(0.f), FY = f2(0.f), FZ = f2(0.f);  // the two j atoms' sums
-  PairAcc FR = {0.f, 0.f, 0.f, 0.f};               // the rotating atom's sums
-#pragma unroll 4
-  for (int kk = 0; kk < 32; kk++) {
-    const int sr = r0 + ((lane + kk) & 31);
-    const float2 dx = __fadd2_rn(f2(xr.x), nx), dy = __fadd2_rn(f2(xr.y), ny), dz = __fadd2_rn(f2(xr.z), nz);
-    const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
-    const float2 rs = __fadd2_rn(RS, f2(pr.z));
-    const float2 rs2 = __fmul2_rn(rs, rs);
-    const float2 lim = __fmul2_rn(rs2, f2(k.invP5));
-    const bool ca = r2.x <= lim.x, cb = r2.y <= lim.y;
-    float2 fac = f2(4.f);  // 4 CCF - dCCF
-    if (__any_sync(0xffffffffu, ca || cb)) {
-      if (ca) {
-        float sn, cs;
-        const float x = __fdividef(r2.x, rs2.x) * k.P5;
-        sincospif(x, &sn, &cs);
-        const float h = 0.5f - 0.5f * cs;
-        fac.x = 4.f * h * h - 2.f * h * sn * (x * 3.14159265358979f);
-      }
-      if (cb) {
-        float sn, cs;
-        const float x = __fdividef(r2.y, rs2.y) * k.P5;
-        sincospif(x, &sn, &cs);
-        const float h = 0.5f - 0.5f * cs;
-        fac.y = 4.f * h * h - 2.f * h * sn * (x * 3.14159265358979f);
-      }
-    }
-    const float2 ir2 = make_float2(rcp_ftz(r2.x), rcp_ftz(r2.y));
-    const float2 cvv = __ffma2_rn(CS, f2(pr.w), __fmul2_rn(f2(cr), VS));
-    float2 w = __fmul2_rn(__fmul2_rn(cvv, fac), __fmul2_rn(__fmul2_rn(ir2, ir2), ir2));
-    if (!FULL) {
-      if (!still_in<false>(v, k, r2.x, sa, sr)) w.x = 0.f;
-      if (!still_in<false>(v, k, r2.y, sb, sr)) w.y = 0.f;
-    }
-    const float2 nw = __fmul2_rn(w, f2(-1.f));
-    FX = __ffma2_rn(nw, dx, FX);
-    FY = __ffma2_rn(nw, dy, FY);
-    FZ = __ffma2_rn(nw, dz, FZ);
-    FR.fx = fmaf(w.x, dx.x, FR.fx); FR.fx = fmaf(w.y, dx.y, FR.fx);
-    FR.fy = fmaf(w.x, dy.x, FR.fy); FR.fy = fmaf(w.y, dy.y, FR.fy);
-    FR.fz = fmaf(w.x, dz.x, FR.fz); FR.fz = fmaf(w.y, dz.y, FR.fz);
-    ROT(xr.x); ROT(xr.y); ROT(xr.z); ROT(pr.z); ROT(pr.w); ROT(cr); ROT(FR.fx); ROT(FR.fy); ROT(FR.fz);
-  }
-  flush_force(v, sa, PairAcc{FX.x, FY.x, FZ.x, 0.f});
-  flush_force(v, sb, PairAcc{FX.y, FY.y, FZ.y, 0.f});
-  flush_force(v, r0 + lane, FR);
-}
+__device__ __forceinline__ void flush_force(const DevView& v, int s, const PairAcc& a) { flush_pair(v, nullptr, s, a); }
 
 // 0.25 (4 CCF - dCCF) of a pair in close contact, 1 otherwise
 __device__ __forceinline__ float chain_fac(const GBConst& k, float r2, float rs) {
@@ -1021,45 +841,93 @@ __device__ __forceinline__ float chain_fac(const GBConst& k, float r2, float rs)
   return 0.25f * (4.f * h * h - 2.f * h * sn * (x * 3.14159265358979f));
 }
 
-// CTAs of 128 threads, seven per SM (28 warps at 72 registers)
+// CTAs of 128 threads, six per SM (24 warps at 80 registers)
 constexpr int kChainThreads = 128;
 constexpr int kChainWarps = kChainThreads / 32;
+
+// rows of the rotating block in the warp's shared memory, twice over (as BornRows)
+struct ChainRows {
+  float4 xy[64], zv[64];   // (x, x', y, y'), (z, z', V, V')
+  float2 c[64], r[64];     // (c, c'), (R, R') (R for single tiles only)
+};
+
+// Born chain rule of a single tile, step-packed (as born_tile)
+template <bool MASKED, bool FULL>
+__device__ __forceinline__ void chain_tile(const DevView& v, const GBConst& k, const Tile& T, int lane, unsigned ex,
+                                           const float* chain, ChainRows& rs) {
+  const int si = T.bi * 32 + lane, j0 = T.bj * 32, l1 = (lane + 1) & 31;
+  const float4 xi = v.xq[si], pi = v.par[si];
+  {
+    const float4 x0 = j_in_i_frame(v, T, lane), p0 = v.par[j0 + lane];
+    const float c0 = -4.f * chain[j0 + lane];
+    const float x1 = __shfl_sync(0xffffffffu, x0.x, l1), y1 = __shfl_sync(0xffffffffu, x0.y, l1);
+    const float z1 = __shfl_sync(0xffffffffu, x0.z, l1), v1 = __shfl_sync(0xffffffffu, p0.w, l1);
+    const float r1 = __shfl_sync(0xffffffffu, p0.z, l1), c1 = __shfl_sync(0xffffffffu, c0, l1);
+    __syncwarp();
+    rs.xy[lane] = rs.xy[lane + 32] = make_float4(x0.x, x1, x0.y, y1);
+    rs.zv[lane] = rs.zv[lane + 32] = make_float4(x0.z, z1, p0.w, v1);
+    rs.c[lane] = rs.c[lane + 32] = make_float2(c0, c1);
+    rs.r[lane] = rs.r[lane + 32] = make_float2(p0.z, r1);
+    __syncwarp();
+  }
+  const float2 AX = f2(-xi.x), AY = f2(-xi.y), AZ = f2(-xi.z), RA = f2(pi.z), VA = f2(pi.w);
+  const float2 CA = f2(-4.f * chain[si]);
+  float2 FX = f2(0.f), FY = f2(0.f), FZ = f2(0.f);
+  float2 FRX = f2(0.f), FRY = f2(0.f), FRZ = f2(0.f);   // minus the rotating atoms' sums
+#pragma unroll 2
+  for (int kk = 0; kk < 32; kk += 2) {
+    const int j = lane + kk;
+    const float4 P = rs.xy[j], Q = rs.zv[j];
+    const float2 ax = __fadd2_rn(make_float2(P.x, P.y), AX), ay = __fadd2_rn(make_float2(P.z, P.w), AY);
+    const float2 az = __fadd2_rn(make_float2(Q.x, Q.y), AZ);
+    const float2 r2 = __ffma2_rn(az, az, __ffma2_rn(ay, ay, __fmul2_rn(ax, ax)));
+    const float2 ir2 = make_float2(rcp_ftz(r2.x), rcp_ftz(r2.y));
+    float2 w = __fmul2_rn(__ffma2_rn(CA, make_float2(Q.z, Q.w), __fmul2_rn(rs.c[j], VA)),
+                          __fmul2_rn(__fmul2_rn(ir2, ir2), ir2));
+    const float2 s = __fadd2_rn(rs.r[j], RA), lim = __fmul2_rn(__fmul2_rn(s, s), f2(k.invP5));
+    if (__any_sync(0xffffffffu, r2.x <= lim.x || r2.y <= lim.y)) {
+      w.x *= chain_fac(k, r2.x, s.x);
+      w.y *= chain_fac(k, r2.y, s.y);
+    }
+    bool ia = still_in<FULL>(v, k, r2.x, si, j0 + (j & 31));
+    bool ib = still_in<FULL>(v, k, r2.y, si, j0 + ((j + 1) & 31));
+    if (MASKED) {
+      ia = ia && !((ex >> kk) & 1u);
+      ib = ib && !((ex >> kk) & 2u);
+    }
+    if (MASKED || !FULL) {
+      w.x = ia ? w.x : 0.f;
+      w.y = ib ? w.y : 0.f;
+    }
+    FX = __ffma2_rn(w, ax, FX); FY = __ffma2_rn(w, ay, FY); FZ = __ffma2_rn(w, az, FZ);
+    FRX = __ffma2_rn(w, ax, FRX); FRY = __ffma2_rn(w, ay, FRY); FRZ = __ffma2_rn(w, az, FRZ);
+    ROT2(FRX); ROT2(FRY); ROT2(FRZ);
+  }
+  const int lm = (lane + 31) & 31;
+  const float frx = FRX.x + __shfl_sync(0xffffffffu, FRX.y, lm);
+  const float fry = FRY.x + __shfl_sync(0xffffffffu, FRY.y, lm);
+  const float frz = FRZ.x + __shfl_sync(0xffffffffu, FRZ.y, lm);
+  flush_force(v, si, PairAcc{FX.x + FX.y, FY.x + FY.y, FZ.x + FZ.y, 0.f});
+  flush_force(v, j0 + lane, PairAcc{-frx, -fry, -frz, 0.f});
+}
 
 // Born chain rule of an all-inside tile pair, step-packed: (c_i V_j + c_j V_i)
 // (4 CCF - dCCF) / r^6 along d, with -4 folded into c (w then carries the held
 // atom's sign and the factor 4 of the no-contact case); the CCF branch on the
 // coarse-bound vote.
-__device__ __forceinline__ void chain_full2(const DevView& v, const GBConst& k, const Tile& A, const Tile& B, int lane,
-                                            const float* chain) {
-  __shared__ float4 rot_sh[kChainWarps][3][32];   // (x, x', y, y'), (z, z', V, V'), (c, c')
-  float4 (*rs)[32] = rot_sh[threadIdx.x >> 5];
-  const int sa = A.bj * 32 + lane, sb = B.bj * 32 + lane, r0 = A.bi * 32;
-  const int l1 = (lane + 1) & 31;
-  const float4 xa = j_in_i_frame(v, A, lane), xb = j_in_i_frame(v, B, lane);
-  const float4 pa = v.par[sa], pb = v.par[sb];
+// FAR: no pair of the item in close contact.
+template <bool FAR>
+__device__ __forceinline__ void chain_loop2(const DevView& v, const GBConst& k, int lane, int r0, const ChainRows& rs,
+                                            const float4& xa, const float4& xb, const float4& pa, const float4& pb,
+                                            float ca, float cb, float c2, float2 FA[3], float2 FB[3], float2 FR[3]) {
   const float2 AX = f2(-xa.x), AY = f2(-xa.y), AZ = f2(-xa.z), BX = f2(-xb.x), BY = f2(-xb.y), BZ = f2(-xb.z);
-  const float2 VA = f2(pa.w), VB = f2(pb.w), CA = f2(-4.f * chain[sa]), CB = f2(-4.f * chain[sb]);
-  float c2;
-  {
-    const float4 x0 = v.xq[r0 + lane], p0 = v.par[r0 + lane];
-    const float c0 = -4.f * chain[r0 + lane];
-    const float x1 = __shfl_sync(0xffffffffu, x0.x, l1), y1 = __shfl_sync(0xffffffffu, x0.y, l1);
-    const float z1 = __shfl_sync(0xffffffffu, x0.z, l1), v1 = __shfl_sync(0xffffffffu, p0.w, l1);
-    const float c1 = __shfl_sync(0xffffffffu, c0, l1);
-    c2 = pair_contact2(k, make_float2(pa.z, pb.z), p0.z);
-    __syncwarp();
-    rs[0][lane] = make_float4(x0.x, x1, x0.y, y1);
-    rs[1][lane] = make_float4(x0.z, z1, p0.w, v1);
-    rs[2][lane] = make_float4(c0, c1, 0.f, 0.f);
-    __syncwarp();
-  }
-  float2 FAX = f2(0.f), FAY = f2(0.f), FAZ = f2(0.f), FBX = f2(0.f), FBY = f2(0.f), FBZ = f2(0.f);
-  float2 FRX = f2(0.f), FRY = f2(0.f), FRZ = f2(0.f);   // minus the rotating atoms' sums
-#pragma unroll 1
+  const float2 VA = f2(pa.w), VB = f2(pb.w), CA = f2(ca), CB = f2(cb);
+  const float4 *xy = rs.xy + lane, *zv = rs.zv + lane;
+  const float2* cr = rs.c + lane;
+#pragma unroll 2
   for (int kk = 0; kk < 32; kk += 2) {
-    const int j = (lane + kk) & 31;
-    const float4 P = rs[0][j], Q = rs[1][j];
-    const float2 CR = *reinterpret_cast<const float2*>(&rs[2][j]);
+    const float4 P = xy[kk], Q = zv[kk];
+    const float2 CR = cr[kk];
     const float2 X = make_float2(P.x, P.y), Y = make_float2(P.z, P.w), Z = make_float2(Q.x, Q.y);
     const float2 VR = make_float2(Q.z, Q.w);
     const float2 ax = __fadd2_rn(X, AX), ay = __fadd2_rn(Y, AY), az = __fadd2_rn(Z, AZ);
@@ -1071,31 +939,82 @@ __device__ __forceinline__ void chain_full2(const DevView& v, const GBConst& k, 
     // -w of the plain law: (c_held V_rot + c_rot V_held) (-4) / r^6
     float2 wa = __fmul2_rn(__ffma2_rn(CA, VR, __fmul2_rn(CR, VA)), __fmul2_rn(__fmul2_rn(ia, ia), ia));
     float2 wb = __fmul2_rn(__ffma2_rn(CB, VR, __fmul2_rn(CR, VB)), __fmul2_rn(__fmul2_rn(ib, ib), ib));
-    if (__any_sync(0xffffffffu, fminf(fminf(ra.x, ra.y), fminf(rb.x, rb.y)) <= c2)) {
-      // rare: the rotating atoms' radii are read here, not staged
-      const float R0 = v.par[r0 + j].z, R1 = v.par[r0 + ((j + 1) & 31)].z;
-      wa.x *= chain_fac(k, ra.x, pa.z + R0);
-      wa.y *= chain_fac(k, ra.y, pa.z + R1);
-      wb.x *= chain_fac(k, rb.x, pb.z + R0);
-      wb.y *= chain_fac(k, rb.y, pb.z + R1);
+    if (!FAR) {
+      if (__any_sync(0xffffffffu, fminf(fminf(ra.x, ra.y), fminf(rb.x, rb.y)) <= c2)) {
+        // rare: the rotating atoms' radii are read here, not staged
+        const float R0 = v.par[r0 + ((lane + kk) & 31)].z, R1 = v.par[r0 + ((lane + kk + 1) & 31)].z;
+        wa.x *= chain_fac(k, ra.x, pa.z + R0);
+        wa.y *= chain_fac(k, ra.y, pa.z + R1);
+        wb.x *= chain_fac(k, rb.x, pb.z + R0);
+        wb.y *= chain_fac(k, rb.y, pb.z + R1);
+      }
     }
-    FAX = __ffma2_rn(wa, ax, FAX); FAY = __ffma2_rn(wa, ay, FAY); FAZ = __ffma2_rn(wa, az, FAZ);
-    FBX = __ffma2_rn(wb, bx, FBX); FBY = __ffma2_rn(wb, by, FBY); FBZ = __ffma2_rn(wb, bz, FBZ);
-    FRX = __ffma2_rn(wa, ax, __ffma2_rn(wb, bx, FRX));
-    FRY = __ffma2_rn(wa, ay, __ffma2_rn(wb, by, FRY));
-    FRZ = __ffma2_rn(wa, az, __ffma2_rn(wb, bz, FRZ));
-    ROT2(FRX); ROT2(FRY); ROT2(FRZ);
+    FA[0] = __ffma2_rn(wa, ax, FA[0]); FA[1] = __ffma2_rn(wa, ay, FA[1]); FA[2] = __ffma2_rn(wa, az, FA[2]);
+    FB[0] = __ffma2_rn(wb, bx, FB[0]); FB[1] = __ffma2_rn(wb, by, FB[1]); FB[2] = __ffma2_rn(wb, bz, FB[2]);
+    FR[0] = __ffma2_rn(wa, ax, __ffma2_rn(wb, bx, FR[0]));
+    FR[1] = __ffma2_rn(wa, ay, __ffma2_rn(wb, by, FR[1]));
+    FR[2] = __ffma2_rn(wa, az, __ffma2_rn(wb, bz, FR[2]));
+    ROT2(FR[0]); ROT2(FR[1]); ROT2(FR[2]);
   }
+}
+
+__device__ __forceinline__ void chain_full2(const DevView& v, const GBConst& k, const Tile& A, const Tile& B, int lane,
+                                            const float* chain, ChainRows& rs) {
+  const int sa = A.bj * 32 + lane, sb = B.bj * 32 + lane, r0 = A.bi * 32;
+  const int l1 = (lane + 1) & 31;
+  const float4 xa = j_in_i_frame(v, A, lane), xb = j_in_i_frame(v, B, lane);
+  const float4 pa = v.par[sa], pb = v.par[sb];
+  const float ca = -4.f * chain[sa], cb = -4.f * chain[sb];
+  float c2;
+  bool far;
+  {
+    const float4 x0 = v.xq[r0 + lane], p0 = v.par[r0 + lane];
+    const float c0 = -4.f * chain[r0 + lane];
+    const float x1 = __shfl_sync(0xffffffffu, x0.x, l1), y1 = __shfl_sync(0xffffffffu, x0.y, l1);
+    const float z1 = __shfl_sync(0xffffffffu, x0.z, l1), v1 = __shfl_sync(0xffffffffu, p0.w, l1);
+    const float c1 = __shfl_sync(0xffffffffu, c0, l1);
+    c2 = pair_contact2(k, make_float2(pa.z, pb.z), p0.z);
+    far = item_far(xa, xb, x0, c2, c2);
+    __syncwarp();
+    rs.xy[lane] = rs.xy[lane + 32] = make_float4(x0.x, x1, x0.y, y1);
+    rs.zv[lane] = rs.zv[lane + 32] = make_float4(x0.z, z1, p0.w, v1);
+    rs.c[lane] = rs.c[lane + 32] = make_float2(c0, c1);
+    __syncwarp();
+  }
+  // (FR: minus the rotating atoms' sums)
+  float2 FA[3], FB[3], FR[3];
+#pragma unroll
+  for (int c = 0; c < 3; c++) FA[c] = FB[c] = FR[c] = f2(0.f);
+  if (far) chain_loop2<true>(v, k, lane, r0, rs, xa, xb, pa, pb, ca, cb, c2, FA, FB, FR);
+  else chain_loop2<false>(v, k, lane, r0, rs, xa, xb, pa, pb, ca, cb, c2, FA, FB, FR);
   const int lm = (lane + 31) & 31;
-  const float frx = FRX.x + __shfl_sync(0xffffffffu, FRX.y, lm);
-  const float fry = FRY.x + __shfl_sync(0xffffffffu, FRY.y, lm);
-  const float frz = FRZ.x + __shfl_sync(0xffffffffu, FRZ.y, lm);
-  flush_force(v, sa, PairAcc{FAX.x + FAX.y, FAY.x + FAY.y, FAZ.x + FAZ.y, 0.f});
-  flush_force(v, sb, PairAcc{FBX.x + FBX.y, FBY.x + FBY.y, FBZ.x + FBZ.y, 0.f});
+  const float frx = FR[0].x + __shfl_sync(0xffffffffu, FR[0].y, lm);
+  const float fry = FR[1].x + __shfl_sync(0xffffffffu, FR[1].y, lm);
+  const float frz = FR[2].x + __shfl_sync(0xffffffffu, FR[2].y, lm);
+  flush_force(v, sa, PairAcc{FA[0].x + FA[0].y, FA[1].x + FA[1].y, FA[2].x + FA[2].y, 0.f});
+  flush_force(v, sb, PairAcc{FB[0].x + FB[0].y, FB[1].x + FB[1].y, FB[2].x + FB[2].y, 0.f});
   flush_force(v, r0 + lane, PairAcc{-frx, -fry, -frz, 0.f});
 }
 
-__global__ void __launch_bounds__(kChainThreads, 7) k_gb_chain(const __grid_constant__ DevView v, const __grid_constant__ GBConst k, const float* chain) {
+__device__ __forceinline__ void chain_single(const DevView& v, const GBConst& k, const Tile& T, int lane,
+                                             const float* chain, ChainRows& rs) {
+  const bool full = tile_full(T);
+  if (tile_masked(T)) {
+    unsigned ex, m14;
+    tile_masks(v, T, lane, ex, m14);
+    if (T.flags & 2) ex |= diag_exclusion(lane);
+    if (full) chain_tile<true, true>(v, k, T, lane, ex, chain, rs);
+    else chain_tile<true, false>(v, k, T, lane, ex, chain, rs);
+  } else if (full) {
+    chain_tile<false, true>(v, k, T, lane, 0u, chain, rs);
+  } else {
+    chain_tile<false, false>(v, k, T, lane, 0u, chain, rs);
+  }
+}
+
+__global__ void __launch_bounds__(kChainThreads, 6) k_gb_chain(const __grid_constant__ DevView v, const __grid_constant__ GBConst k, const float* chain) {
+  __shared__ ChainRows rows[kChainWarps];
+  ChainRows& rs = rows[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   const int ni = *v.nitems;
@@ -1103,29 +1022,12 @@ __global__ void __launch_bounds__(kChainThreads, 7) k_gb_chain(const __grid_cons
     bool two;
     const int t = item_tile(v, it, two);
     const Tile T = v.tiles[t];
-    if (two) {
-      const Tile U = v.tiles[t + 1];
-      if (tile_full(T)) chain_full2(v, k, T, U, lane, chain);
-      else chain_tile2<false>(v, k, T, U, lane, chain);
+    if (two && tile_full(T)) {
+      chain_full2(v, k, T, v.tiles[t + 1], lane, chain, rs);
       continue;
     }
-    const int si = T.bi * 32 + lane;
-    const float4 xi = v.xq[si], pi = v.par[si];
-    const float ci = chain[si];
-    unsigned ex, m14;
-    tile_masks(v, T, lane, ex, m14);
-    if (T.flags & 2) ex |= diag_exclusion(lane);
-    PairAcc I = {0.f, 0.f, 0.f, 0.f}, J = {0.f, 0.f, 0.f, 0.f};
-    const bool full = tile_full(T);
-    if (tile_masked(T)) {
-      if (full) chain_tile<true, true>(v, k, T, lane, si, xi, pi, ci, ex, chain, I, J);
-      else chain_tile<true, false>(v, k, T, lane, si, xi, pi, ci, ex, chain, I, J);
-    } else {
-      if (full) chain_tile<false, true>(v, k, T, lane, si, xi, pi, ci, ex, chain, I, J);
-      else chain_tile<false, false>(v, k, T, lane, si, xi, pi, ci, ex, chain, I, J);
-    }
-    flush_force(v, si, I);
-    flush_force(v, T.bj * 32 + lane, J);
+    chain_single(v, k, T, lane, chain, rs);
+    if (two) chain_single(v, k, v.tiles[t + 1], lane, chain, rs);
   }
 }
 
@@ -1147,20 +1049,21 @@ int launch_gb(Context& c, const GBConst& k, double halfeconv, double born_offset
   cudaMemsetAsync(c.d_deda.p, 0, sizeof(long long) * c.nslots, st);
   k_gb_born<<<g, kBornThreads, 0, st>>>(v, k, c.d_gpol.p);
   k_gb_radii<<<nb, 256, 0, st>>>(v, c.d_gbT.p, c.d_gpol.p, halfeconv, born_offset, c.d_born_f.p, c.d_born_d.p);
-  GBConst ke = k;
-  if (c.gb_no_chain) ke.e64_r2 = 0.f;  // a gradient call's energy pass: FP32 pair energies
-  if (energy && ke.e64_r2 > 0.f) {
+  // (a gradient call's energy pass weights a loss: FP32 pair energies)
+  const bool precise = energy && !c.gb_no_chain;
+  if (precise) {
     c.kernel_launches += 1;
-    k_energy_records<<<nb, 256, 0, st>>>(v, c.d_epos.p, c.d_epar.p);
+    launch_df_records(c);
   }
-  if (!k.fast) {
-    if (energy) k_gb_pair_born_only<true><<<g, 256, 0, st>>>(v, k, c.d_born_f.p, c.d_deda.p);
-    else k_gb_pair_born_only<false><<<g, 256, 0, st>>>(v, k, c.d_born_f.p, c.d_deda.p);
-  } else if (energy) {
-    if (ke.e64_r2 > 0.f) k_gb_pair_energy<<<g, 256, 0, st>>>(v, ke, c.d_born_f.p, c.d_deda.p);
-    else k_gb_pair_energy32<<<g, 256, 0, st>>>(v, ke, c.d_born_f.p, c.d_deda.p);
+  const int gp = g * (256 / kPairThreads), ge = g * (256 / kPairEThreads);
+  if (energy) {
+    if (!k.fast) k_gb_pair_energy<false, true><<<ge, kPairEThreads, 0, st>>>(v, k, c.d_born_f.p, c.d_deda.p);
+    else if (precise) k_gb_pair_energy<true, true><<<ge, kPairEThreads, 0, st>>>(v, k, c.d_born_f.p, c.d_deda.p);
+    else k_gb_pair_energy<true, false><<<ge, kPairEThreads, 0, st>>>(v, k, c.d_born_f.p, c.d_deda.p);
+  } else if (!k.fast) {
+    k_gb_pair<false><<<gp, kPairThreads, 0, st>>>(v, k, c.d_born_f.p, c.d_deda.p);
   } else {
-    k_gb_pair<<<2 * g, 128, 0, st>>>(v, k, c.d_born_f.p, c.d_deda.p);
+    k_gb_pair<true><<<gp, kPairThreads, 0, st>>>(v, k, c.d_born_f.p, c.d_deda.p);
   }
   k_gb_self<<<nb, 256, 0, st>>>(v, c.d_charge.p, k, premul, c.d_deda.p, c.d_born_d.p, c.d_chain_f.p,
                                 energy ? 1 : 0);
@@ -1175,7 +1078,7 @@ int launch_gb_stage(Context& c, const GBConst& k, int stage) {
   int g = tile_grid(c);
   c.kernel_launches += 1;
   if (stage == 1) k_gb_born<<<g, kBornThreads, 0, c.stream>>>(v, k, c.d_gpol.p);
-  else if (stage == 2) k_gb_pair<<<2 * g, 128, 0, c.stream>>>(v, k, c.d_born_f.p, c.d_deda.p);
+  else if (stage == 2) k_gb_pair<true><<<g * (256 / kPairThreads), kPairThreads, 0, c.stream>>>(v, k, c.d_born_f.p, c.d_deda.p);
   else k_gb_chain<<<2 * g, kChainThreads, 0, c.stream>>>(v, k, c.d_chain_f.p);
   return cudaGetLastError() == cudaSuccess ? PDGPU_OK : PDGPU_ERR_CUDA;
 }

@@ -163,7 +163,7 @@ __device__ __forceinline__ int nb_rot(const DevView& v, const NBConst& k, const 
 // ---------------------------------------------------------------------------
 
 // remainders of the packed slots (before each energy pass)
-__global__ void k_nb_records(DevView v, const double* charge, float4* rlo, float2* plo) {
+__global__ void k_df_records(DevView v, const double* charge, float4* rlo, float2* plo) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= v.nslots) return;
   const int a = v.sorted_atom[s];
@@ -186,22 +186,6 @@ __global__ void k_nb_records(DevView v, const double* charge, float4* rlo, float
   }
   rlo[s] = r;
   plo[s] = p;
-}
-
-// centre of block bj seen from block bi, as double-floats, in the image the
-// FP32 offset o was taken in
-__device__ __forceinline__ void df_offset(const DevView& v, const SystemInfo& S, int bi, int bj, const float o[3],
-                                          DF O[3]) {
-  const float4 ci = v.cenf[bi], cj = v.cenf[bj];
-  const float a[3] = {ci.x, ci.y, ci.z}, b[3] = {cj.x, cj.y, cj.z};
-#pragma unroll
-  for (int c = 0; c < 3; c++) {
-    O[c] = df_two_sum(b[c], -a[c]);
-    if (S.periodic) {
-      const float n = -rintf((O[c].h - o[c]) / S.boxf[c].h);
-      O[c] = df_norm(df_add(O[c], df_scale(S.boxf[c], n)));
-    }
-  }
 }
 
 struct NBESum {
@@ -462,12 +446,17 @@ static void launch_nb_mode(Context& c, const NBConst& k, int g) {
   }
 }
 
+int launch_df_records(Context& c) {
+  k_df_records<<<(c.nslots + 255) / 256, 256, 0, c.stream>>>(c.view(), c.d_charge.p, c.d_rlo.p, c.d_plo.p);
+  return cudaGetLastError() == cudaSuccess ? PDGPU_OK : PDGPU_ERR_CUDA;
+}
+
 int launch_nb(Context& c, const NBConst& k, bool energy) {
   c.kernel_launches += 1;
   int g = tile_grid(c);
   if (energy) {
     c.kernel_launches += 1;
-    k_nb_records<<<(c.nslots + 255) / 256, 256, 0, c.stream>>>(c.view(), c.d_charge.p, c.d_rlo.p, c.d_plo.p);
+    launch_df_records(c);
     launch_nb_mode<true>(c, k, g);
   } else {
     launch_nb_mode<false>(c, k, g);

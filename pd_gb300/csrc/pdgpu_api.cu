@@ -164,6 +164,16 @@ NBEConst pdgpu::make_nbe_const(const NBConst& k) {
   return e;
 }
 
+void pdgpu::set_gb_threshold(GBConst& k, double thresh) {
+  k.thresh = (float)thresh;
+  k.thresh_d = thresh;
+  const double K = std::min(-4.0 * (thresh - 4e-6 * std::fabs(thresh)), 4e30);
+  k.sqrtK = K > 0 ? (float)std::sqrt(K) : 0.f;
+  k.inv_sqrtK = K > 0 ? (float)(1.0 / std::sqrt(K)) : 0.f;
+  k.invK = K > 0 ? (float)(1.0 / K) : 0.f;
+  k.kU = (float)(-0.25 * K);   // u = -r^2 / (4 a a) = kU r^2 / (K a a)
+}
+
 GBConst pdgpu::make_gb_const(const pdgpu_gb_params& p, double listR) {
   GBConst k{};
   double C = p.Cutoff, I = p.InnerCutoff;
@@ -182,31 +192,27 @@ GBConst pdgpu::make_gb_const(const pdgpu_gb_params& p, double listR) {
   k.premul = (float)(-0.5 * ec * (1.0 / p.DielectricSolute - 1.0 / p.DielectricSolvent));
   k.vdw14 = (float)p.Vdw14Scaling;
   k.elec14 = (float)p.Elec14Scaling;
-  k.thresh = (float)p.ExpApproxThreshold;
   k.P4 = (float)p.P4;
   k.P5 = (float)p.P5;
   k.invP5 = (float)(1.0 / p.P5);
-  k.cut2_d = C * C;
-  k.inner_d = I;
-  k.invw2_d = w > 0 ? 1.0 / (w * w) : 0.0;
-  k.vdwcut_d = p.VdwCutoff;
-  k.vdwinner_d = p.VdwInnerCutoff;
-  k.vdwinvw2_d = vw > 0 ? 1.0 / (vw * vw) : 0.0;
   k.still2_d = still * still;
-  k.econv_in_d = ec / p.DielectricSolute;
-  k.econv_out_d = ec / p.DielectricSolvent;
-  k.premul_d = -0.5 * ec * (1.0 / p.DielectricSolute - 1.0 / p.DielectricSolvent);
-  k.vdw14_d = p.Vdw14Scaling;
-  k.elec14_d = p.Elec14Scaling;
   k.thresh_d = p.ExpApproxThreshold;
   k.fast = 1;
-  k.e64_r2 = 4.5f * 4.5f;
-  const double K = -4.0 * (p.ExpApproxThreshold - 4e-6 * std::fabs(p.ExpApproxThreshold));
-  k.sqrtK = K > 0 ? (float)std::sqrt(std::min(K, 1e36)) : 0.f;
-  k.inv_sqrtK = K > 0 ? (float)(1.0 / std::sqrt(std::min(K, 1e36))) : 0.f;
-  k.sq_eout = (float)std::sqrt(ec / p.DielectricSolvent);
-  k.inv_eout = (float)(p.DielectricSolvent / ec);
-  k.in_over_out_m1 = (float)(p.DielectricSolvent / p.DielectricSolute - 1.0);
+  k.eclose2 = 4.5f * 4.5f;
+  const double premul = -0.5 * ec * (1.0 / p.DielectricSolute - 1.0 / p.DielectricSolvent);
+  k.econv_in_f = df_split(ec / p.DielectricSolute);
+  k.econv_out_f = df_split(ec / p.DielectricSolvent);
+  k.premul2_f = df_split(2.0 * premul);
+  k.vdw14_f = df_split(p.Vdw14Scaling);
+  k.elec14_f = df_split(p.Elec14Scaling);
+  set_gb_threshold(k, p.ExpApproxThreshold);
+  // (kept off zero for an infinite solvent dielectric: the GB term divides it out again)
+  double eout = ec / p.DielectricSolvent;
+  if (!(std::fabs(eout) > 1e-12)) eout = 1e-12;
+  k.sq_eout = (float)std::sqrt(std::fabs(eout));
+  k.neg_sq_eout = eout > 0 ? -k.sq_eout : k.sq_eout;
+  k.gb_ep = (float)(-premul / eout);
+  k.in_over_out = (float)(ec / p.DielectricSolute / eout);
   k.sqrt12 = (float)std::sqrt(12.0);
   return k;
 }
@@ -492,8 +498,6 @@ pdgpu_ctx* pdgpu_create(int device, const pdgpu_system_desc* d, int* status) {
     if (e == cudaSuccess) e = c.d_born_f.alloc(c.nslots);
     if (e == cudaSuccess) e = c.d_chain_f.alloc(c.nslots);
     if (e == cudaSuccess) e = c.d_born_d.alloc(N);
-    if (e == cudaSuccess) e = c.d_epos.alloc(c.nslots);
-    if (e == cudaSuccess) e = c.d_epar.alloc(c.nslots);
   }
   if (c.has_sa) {
     if (e == cudaSuccess) e = c.d_lc_ncand.alloc(c.nslots);
@@ -972,10 +976,7 @@ int pdgpu::enqueue_forces(Context& c, unsigned what, bool energy, bool rebuild, 
     const bool pd_energies = (what & PDGPU_PD_ENERGIES) != 0;
     if (!c.gb_fast || pd_energies) {
       k.fast = 0;
-      if (pd_energies) {
-        k.thresh = -1e30f;
-        k.thresh_d = -1e300;
-      }
+      if (pd_energies) set_gb_threshold(k, -1e30);
       st = launch_nb(c, make_nb_const(gb_vacuum_params(c)), energy);
     }
     double ec = econv_kcal();

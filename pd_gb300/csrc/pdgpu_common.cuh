@@ -117,20 +117,20 @@ struct GBConst {
   float econv_in, econv_out, premul;  // kcal units
   float vdw14, elec14, thresh;
   float P4, P5, invP5;
-  // FP64 copies for the energy arithmetic
-  double cut2_d, inner_d, invw2_d, vdwcut_d, vdwinner_d, vdwinvw2_d, still2_d;
-  double econv_in_d, econv_out_d, premul_d, vdw14_d, elec14_d, thresh_d;
-  // 1: FastMode (GB fused with LJ + Coulomb, εout Coulomb below the threshold);
+  double still2_d, thresh_d;
+  // 1: FastMode (GB fused with LJ + Coulomb, eps_out Coulomb below the threshold);
   // 0: calcBornForces (GB term alone for every pair, premul q q / r below it)
   int fast;
-  // energy passes: pairs closer than sqrt(e64_r2) take their energies in FP64
-  // from FP64 positions and parameters (0: none, every pair in FP32)
-  float e64_r2;
-  // the force-only all-inside body: Born radii scaled by sqrtK, so that
+  // energy passes: pairs closer than sqrt(eclose2) take their energies in
+  // double-float from double-float positions and parameters
+  float eclose2;
+  DF econv_in_f, econv_out_f, premul2_f, vdw14_f, elec14_f;   // premul2: 2 premul
+  // the packed pair bodies: Born radii scaled by sqrtK, so that
   // a_i a_j K >= r^2 holds for every pair the threshold test may switch on
   // (K = -4 x the threshold widened by 4e-6 relative); charges scaled by
-  // sqrt(econv_out), sqrt(eps) by sqrt(12)
-  float sqrtK, inv_sqrtK, sq_eout, inv_eout, in_over_out_m1, sqrt12;
+  // sqrt(econv_out) (the held atoms' by its negative), sqrt(eps) by sqrt(12);
+  // gb_ep: premul q q fgb per scaled charges' product -econv_out q q
+  float sqrtK, inv_sqrtK, invK, kU, sq_eout, neg_sq_eout, in_over_out, sqrt12, gb_ep;
 };
 
 // Device-side view of a context, passed by value to kernels.
@@ -144,11 +144,6 @@ struct DevView {
   const double* radius;      // natom, LJ Rmin/2
   const double* sqeps;       // natom, sqrt(kcal/mol)
   const double* born;        // natom, Born radii of the last GB pass (FP64)
-  // (GB energy evaluations) FP64 records per sorted slot, written by
-  // k_energy_records before the energy pass: (x, y, z, charge) and (LJ radius,
-  // sqrt(eps kcal/mol)); padding slots: far away, radius -1
-  const double4* epos;
-  const double2* epar;
   // sorted order
   const int* sorted_atom;    // [nslots]
   float4* xq;                // rel pos + charge
@@ -157,7 +152,7 @@ struct DevView {
   double* center;            // [nblocks*3]
   float4* half;              // [nblocks] half extents
   float4* cenf;              // [nblocks] centre in FP32 (exact: centres are FP32 numbers)
-  // (FF_NonBonded energies) what FP32 rounding takes off the packed slots:
+  // (energy evaluations) what FP32 rounding takes off the packed slots:
   // (x, y, z, charge) - xq and (LJ radius, sqrt(eps)) - par, written before the energy pass
   float4* rlo;
   float2* plo;
@@ -195,22 +190,16 @@ struct DevView {
 // sum keeps only whole units, so many small partial sums of one sign (the far
 // attractive LJ tail, per lane and tile) would be lost at a coarse scale.
 __device__ __forceinline__ long long fix_energy_d(double x) { return __double2ll_rn(x * 4294967296.0); }
-// float -> 64-bit fixed point with 32 fractional bits using integer operations
-// only (|x| < 2^31; larger magnitudes saturate near 2^62 so the overflow check
-// trips).  Rounds half away from zero.  The hardware float->int64 conversion
-// runs on the FP64 pipe, which is narrow on this GPU.
+// float -> 64-bit fixed point with 32 fractional bits (|x| < 2^29; fix_range flags
+// anything from 2^28 on): x = a / 4 + rem with a the nearest integer to 4 x, both
+// exact in FP32, so x 2^32 = a 2^30 + rem 2^32 takes three 32-bit conversions.
+// Rounds to nearest even (exact ties, common where x is small, do not drift one
+// way).  The hardware float -> int64 conversion runs on the narrow FP64 pipe, and
+// shifting the mantissa by the exponent in integers takes about twenty instructions.
 __device__ __forceinline__ long long fx32(float x) {
-  const unsigned b = __float_as_uint(x);
-  const int e = (int)((b >> 23) & 0xffu);
-  const unsigned long long m = (unsigned long long)((b & 0x7fffffu) | 0x800000u);
-  const int sh = e - 118;  // x * 2^32 = m * 2^(e - 150 + 32)
-  unsigned long long r;
-  if (e == 0) r = 0ull;
-  else if (sh >= 39) r = 1ull << 62;
-  else if (sh >= 0) r = m << sh;
-  else if (sh > -25) r = (m + (1ull << (-sh - 1))) >> (-sh);
-  else r = 0ull;
-  return (b >> 31) ? -(long long)r : (long long)r;
+  const int a = __float2int_rn(x * 4.f);
+  const float rem = __fmaf_rn(-(float)a, 0.25f, x);
+  return (long long)a * 1073741824LL + (long long)__float2int_rn(rem * 4294967296.f);
 }
 
 // Range of FP32 partial sums about to enter 64-bit fixed point (2^32 per unit):
@@ -254,6 +243,8 @@ int launch_pack(Context& c, float check_disp);
 int launch_nb(Context& c, const NBConst& k, bool need_virial);
 int launch_gb(Context& c, const GBConst& k, double halfeconv, double born_offset, double premul, bool energy);
 int launch_lcpo(Context& c, long long* facc_out, long long* esurf_out, int esurf_stride);
+// FP32 remainders of the packed slots (double-float positions and parameters), before an energy pass
+int launch_df_records(Context& c);
 int launch_gb_stage(Context& c, const GBConst& k, int stage);
 // parameter gradients after an energy evaluation of NB or GB (device outputs,
 // original atom order, J per parameter unit; null pointers are skipped)
@@ -276,6 +267,7 @@ int launch_census(Context& c, const NBConst& nk, const GBConst& gk, bool do_nb, 
 int measure_fp32_peak(int device, double* tflops_ffma, double* tflops_ffma2);
 NBConst make_nb_const(const pdgpu_nb_params& p);
 NBEConst make_nbe_const(const NBConst& k);
+void set_gb_threshold(GBConst& k, double thresh);   // ExpApproxThreshold and what the bodies derive from it
 GBConst make_gb_const(const pdgpu_gb_params& p, double listR);
 int launch_bonded(Context& c, bool energy);
 int launch_finalize_forces(Context& c, double* out, size_t stride_doubles, bool add, double scale);

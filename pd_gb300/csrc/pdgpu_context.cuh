@@ -123,7 +123,7 @@ struct Context {
   DBuf<unsigned> d_items;      // [tile_cap] GB work items (with GB only)
   DBuf<uint2> d_masks;         // [mask_cap*32]
   DBuf<float4> d_xq, d_par, d_rel0;  // [nslots]
-  DBuf<float4> d_rlo;                // [nslots] FP32 remainders of the slots (FF_NonBonded energies)
+  DBuf<float4> d_rlo;                // [nslots] FP32 remainders of the slots (energy evaluations)
   DBuf<float2> d_plo;                // [nslots]
   // NB j-atom groups (allocated with the NB parameters)
   DBuf<unsigned> d_cull_mask;        // [tile_cap] j lanes kept per tile
@@ -144,8 +144,6 @@ struct Context {
   DBuf<float> d_born_f;             // [nslots]
   DBuf<float> d_chain_f;            // [nslots] a^2/166 * dE/da * P4
   DBuf<double> d_born_d;            // [natom] original order
-  DBuf<double4> d_epos;             // [nslots] FP64 position + charge per slot (energy evaluations)
-  DBuf<double2> d_epar;             // [nslots] FP64 LJ radius + sqrt(eps) per slot
   // Monte Carlo partial energy updates (allocated on first use)
   DBuf<double> d_mc_ref;            // [natom*3] positions of the reference evaluation
   DBuf<long long> d_mc_eref;        // [nsys*2] reference vdw, elec (fixed point, energy scale)
@@ -195,8 +193,6 @@ struct Context {
     v.radius = d_radius.p;
     v.sqeps = d_sqeps.p;
     v.born = d_born_d.p;
-    v.epos = d_epos.p;
-    v.epar = d_epar.p;
     v.sorted_atom = d_sorted_atom.p;
     v.xq = d_xq.p;
     v.par = d_par.p;

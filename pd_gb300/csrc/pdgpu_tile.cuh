@@ -49,6 +49,22 @@ __device__ __forceinline__ void tile_masks(const DevView& v, const Tile& T, int 
   }
 }
 
+// centre of block bj seen from block bi, as double-floats, in the image the
+// FP32 offset o was taken in
+__device__ __forceinline__ void df_offset(const DevView& v, const SystemInfo& S, int bi, int bj, const float o[3],
+                                          DF O[3]) {
+  const float4 ci = v.cenf[bi], cj = v.cenf[bj];
+  const float a[3] = {ci.x, ci.y, ci.z}, b[3] = {cj.x, cj.y, cj.z};
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    O[c] = df_two_sum(b[c], -a[c]);
+    if (S.periodic) {
+      const float n = -rintf((O[c].h - o[c]) / S.boxf[c].h);
+      O[c] = df_norm(df_add(O[c], df_scale(S.boxf[c], n)));
+    }
+  }
+}
+
 // bond order of an atom pair as PD's list stores it; 7 when not bonded
 __device__ __forceinline__ int pair_bondorder(const DevView& v, int a, int b) {
   int lo = a < b ? a : b, hi = a < b ? b : a;
