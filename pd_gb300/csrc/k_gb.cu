@@ -49,8 +49,6 @@ __device__ __forceinline__ bool still_in(const DevView& v, const GBConst& k, flo
 // trigonometric code is skipped, not predicated, on nearly every step.
 __device__ __forceinline__ bool gb_contact(const GBConst& k, float r2, float rs2) { return r2 <= rs2 * k.invP5; }
 
-__device__ __forceinline__ float2 f2(float a) { return make_float2(a, a); }
-
 // ---------------------------------------------------------------------------
 // All-inside tile pairs (every pair inside every cutoff, no exclusions: the
 // all-pairs case) take lean Born and chain-rule bodies: per-atom factors are
@@ -91,8 +89,6 @@ __device__ __forceinline__ float pair_contact2(const GBConst& k, float2 RS, floa
 // y_l, y_l+1) ..., read with one 16-byte load per four values; only its running
 // sums rotate through the warp by shuffles, two lanes per step, so that after
 // 16 rotations lane l's pair holds the sums of atoms l and l + 1.
-#define ROT2(p) p.x = __shfl_sync(0xffffffffu, p.x, (lane + 2) & 31); p.y = __shfl_sync(0xffffffffu, p.y, (lane + 2) & 31)
-
 // the CCF of one pair: 1 outside close contact
 __device__ __forceinline__ float born_ccf(const GBConst& k, float r2, float rs) {
   const float rs2 = rs * rs;

@@ -642,6 +642,7 @@ __global__ void __launch_bounds__(128) k_tile_rows(DevView v, const BlockGrid* g
 __global__ void k_tile_total(DevView v, const int* total, long long cap) {
   const long long t = *total;
   *v.ntiles = (int)(t < cap ? t : cap);
+  v.cull_n[2] = 1;   // (the groups fit until a row finds they do not)
   if (t > cap) atomicOr(v.status, (unsigned)ST_TILE_OVERFLOW);
 }
 
@@ -758,8 +759,9 @@ __global__ void k_masks(DevView v, const int* mlist, const int* nml) {
 // check2: squared skin limit (0 = no skin check); full2: squared limit that keeps
 // tiles flagged full valid (0 = none flagged), checked where the skin check is not
 // cull: the NB j-atom groups are in use (the displacement check always runs)
+// sub: also write the boxes of each 8 slots (for the groups)
 __global__ void k_pack(DevView v, const double* charge, float check2, float full2, int store_ref,
-                       long long npairs_all, int cull) {
+                       long long npairs_all, int cull, int sub) {
   int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= v.nslots) return;
   int a = v.sorted_atom[s];
@@ -793,6 +795,23 @@ __global__ void k_pack(DevView v, const double* charge, float check2, float full
     }
   }
   v.xq[s] = o;
+  if (sub) {
+    // boxes of each 8 slots (a padding slot widens its box: it never hides an atom)
+    float4 lo = o, hi = o;
+#pragma unroll
+    for (int d = 4; d > 0; d >>= 1) {
+      lo.x = fminf(lo.x, __shfl_xor_sync(0xffffffffu, lo.x, d));
+      lo.y = fminf(lo.y, __shfl_xor_sync(0xffffffffu, lo.y, d));
+      lo.z = fminf(lo.z, __shfl_xor_sync(0xffffffffu, lo.z, d));
+      hi.x = fmaxf(hi.x, __shfl_xor_sync(0xffffffffu, hi.x, d));
+      hi.y = fmaxf(hi.y, __shfl_xor_sync(0xffffffffu, hi.y, d));
+      hi.z = fmaxf(hi.z, __shfl_xor_sync(0xffffffffu, hi.z, d));
+    }
+    if ((s & 7) == 0) {
+      v.sub[s >> 2] = lo;
+      v.sub[(s >> 2) + 1] = hi;
+    }
+  }
 }
 
 // GB work items: tiles t and t + 1 go together when they share the row, sit in
@@ -831,78 +850,80 @@ __global__ void k_item_write(DevView v, long long cap, int pairs, const int* fla
 // like a tile's j block.  Valid while every atom stays within half the skin of
 // its build position (the per-step displacement check, forced on with groups):
 // a pair inside the cutoff then had its j atom within R of the i box at build.
-// row: [0, nb) kept j atoms, [nb, 2nb) first tile, [2nb, 3nb) groups,
-// [3nb, 4nb) first group (exclusive scan).
+// The j atoms within the cutoffs themselves come first, those in the skin after
+// them, so that the skin's groups, mostly out of reach, are skipped whole by the
+// force pass.  One CTA per row: its warps take consecutive runs of the row's
+// tiles (entries keep tile order, then lane order), count, take the row's groups
+// by an atomic on the total (rows in any order: every sum is in fixed point) and
+// write.  A row's groups are an even number (the force pass takes two at once).
 // ---------------------------------------------------------------------------
-// cnt: zeroed beforehand over the tile capacity (the scan runs over it)
-__global__ void k_cull_mask(DevView v, float R2, unsigned* jmask, int* cnt, int* row) {
-  const int lane = threadIdx.x & 31;
-  const int nt = *v.ntiles;
-  const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  for (int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < nt; t += nwarps) {
+constexpr int kCullWarps = 4;
+__global__ void __launch_bounds__(kCullWarps * 32) k_cull(DevView v, float R2, float Rc2, const int* row_start,
+                                                          const int* row_cnt, uint2* jmask) {
+  __shared__ int cnt[2][kCullWarps];
+  __shared__ int first;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, b = blockIdx.x;
+  const int t0 = row_start[b], n = min(row_cnt[b], *v.ntiles - t0);
+  const int per = (max(n, 0) + kCullWarps - 1) / kCullWarps;
+  const int ta = t0 + min(wid * per, max(n, 0)), tb = t0 + min((wid + 1) * per, max(n, 0));
+  const float4 h = v.half[b];
+  int nn = 0, nf = 0;
+#pragma unroll 4
+  for (int t = ta; t < tb; t++) {
     const Tile T = v.tiles[t];
     const bool plain = T.mask < 0 && !(T.flags & 3);
-    unsigned m = 0u;
-    if (plain) {
-      const int sj = T.bj * 32 + lane;
-      const float4 x = v.xq[sj];
-      const float4 h = v.half[T.bi];
-      const float gx = fmaxf(fabsf(x.x + T.ox) - h.x, 0.f);
-      const float gy = fmaxf(fabsf(x.y + T.oy) - h.y, 0.f);
-      const float gz = fmaxf(fabsf(x.z + T.oz) - h.z, 0.f);
-      m = __ballot_sync(0xffffffffu, v.sorted_atom[sj] >= 0 && gx * gx + gy * gy + gz * gz <= R2);
-    }
+    const int sj = T.bj * 32 + lane;
+    const float4 x = v.xq[sj];
+    const float gx = fmaxf(fabsf(x.x + T.ox) - h.x, 0.f);
+    const float gy = fmaxf(fabsf(x.y + T.oy) - h.y, 0.f);
+    const float gz = fmaxf(fabsf(x.z + T.oz) - h.z, 0.f);
+    const float d2 = gx * gx + gy * gy + gz * gz;
+    const bool keep = plain && v.sorted_atom[sj] >= 0 && d2 <= R2;
+    const unsigned mn = __ballot_sync(0xffffffffu, keep && d2 <= Rc2), mf = __ballot_sync(0xffffffffu, keep && d2 > Rc2);
+    nn += __popc(mn);
+    nf += __popc(mf);
     if (lane == 0) {
-      jmask[t] = m;
-      cnt[t] = __popc(m);
-      const int nb = v.nblocks;
-      if (m) atomicAdd(&row[T.bi], __popc(m));
-      atomicMin(&row[nb + T.bi], t);
+      jmask[t] = make_uint2(mn, mf);
       if (!plain) v.cull_rest[atomicAdd(&v.cull_n[0], 1)] = t;
     }
   }
-}
-
-__global__ void k_cull_groups(int nb, int* row) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b < nb) row[2 * nb + b] = (row[b] + 31) >> 5;
-}
-
-// pos: exclusive scan of the kept counts over the tile list (a row's tiles are
-// contiguous, so its entries keep tile order, then lane order)
-__global__ void k_cull_write(DevView v, const unsigned* jmask, const int* pos, const int* row) {
-  const int lane = threadIdx.x & 31;
-  const int nt = *v.ntiles;
-  const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  const int nb = v.nblocks;
-  for (int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < nt; t += nwarps) {
-    const unsigned m = jmask[t];
-    if (!((m >> lane) & 1u)) continue;
+  if (lane == 0) {
+    cnt[0][wid] = nn;
+    cnt[1][wid] = nf;
+  }
+  __syncthreads();
+  int tn = 0, tf = 0, on = 0, of = 0;   // the row's totals, and those of the warps before this one
+#pragma unroll
+  for (int w = 0; w < kCullWarps; w++) {
+    if (w == wid) {
+      on = tn;
+      of = tf;
+    }
+    tn += cnt[0][w];
+    tf += cnt[1][w];
+  }
+  const int G = (tn + tf + 63) / 64 * 2;
+  if (threadIdx.x == 0) {
+    first = atomicAdd(&v.cull_n[1], G);
+    if ((long long)(first + G) * 32 > v.cull_cap) v.cull_n[2] = 0;   // they do not fit: the tile path serves all
+  }
+  __syncthreads();
+  const long long base = (long long)first * 32;
+  if (base + (long long)G * 32 > v.cull_cap) return;
+  for (int g = threadIdx.x; g < G; g += kCullWarps * 32) v.cull_bi[first + g] = b;
+  for (int i = tn + tf + threadIdx.x; i < G * 32; i += kCullWarps * 32)
+    v.cull_ent[base + i] = make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
+  long long en = base + on, ef = base + tn + of;
+  const unsigned lt = (1u << lane) - 1u;
+#pragma unroll 4
+  for (int t = ta; t < tb; t++) {
+    const uint2 m = jmask[t];
     const Tile T = v.tiles[t];
-    const long long e = (long long)row[3 * nb + T.bi] * 32 + (pos[t] - pos[row[nb + T.bi]]) +
-                        __popc(m & ((1u << lane) - 1u));
-    if (e < v.cull_cap) v.cull_ent[e] = make_float4(T.ox, T.oy, T.oz, __int_as_float(T.bj * 32 + lane));
-  }
-}
-
-// one warp per row: group -> row, empty entries closing the row's last group,
-// and (last row) the group count and whether it fits the capacity
-__global__ void k_cull_rows(DevView v, const int* row) {
-  const int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  const int nb = v.nblocks;
-  if (b >= nb) return;
-  const int n = row[b], G = row[2 * nb + b], base = row[3 * nb + b];
-  const long long gcap = v.cull_cap / 32;
-  for (int g = lane; g < G; g += 32)
-    if (base + g < gcap) v.cull_bi[base + g] = b;
-  for (int i = n + lane; i < G * 32; i += 32) {
-    const long long e = (long long)base * 32 + i;
-    if (e < v.cull_cap) v.cull_ent[e] = make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
-  }
-  if (b == nb - 1 && lane == 0) {
-    v.cull_n[1] = base + G;
-    v.cull_n[2] = (long long)(base + G) * 32 <= v.cull_cap ? 1 : 0;
+    const float4 e = make_float4(T.ox, T.oy, T.oz, __int_as_float(T.bj * 32 + lane));
+    if ((m.x >> lane) & 1u) v.cull_ent[en + __popc(m.x & lt)] = e;
+    if ((m.y >> lane) & 1u) v.cull_ent[ef + __popc(m.y & lt)] = e;
+    en += __popc(m.x);
+    ef += __popc(m.y);
   }
 }
 
@@ -930,22 +951,10 @@ static void scan_ints(Context& c, const int* in, int* out, int* tmp, long long n
 }
 
 static void launch_cull(Context& c, float list_radius) {
-  c.kernel_launches += 4;   // and two scans
-  DevView v = c.view();
-  cudaStream_t st = c.stream;
-  const int nb = c.nblocks;
-  int* row = c.d_cull_row.p;
-  cudaMemsetAsync(row, 0, sizeof(int) * nb, st);
-  cudaMemsetAsync(row + nb, 0x7f, sizeof(int) * nb, st);
-  const float R = list_radius + 1e-3f;
-  // the kept counts and their scan reuse the tile-compaction arrays
-  cudaMemsetAsync(c.d_tile_flag.p, 0, sizeof(int) * c.tile_cap, st);
-  k_cull_mask<<<list_tile_grid(c), 256, 0, st>>>(v, R * R, c.d_cull_mask.p, c.d_tile_flag.p, row);
-  scan_ints(c, c.d_tile_flag.p, c.d_tile_pos.p, c.d_scan_tmp2.p, c.tile_cap, st);
-  k_cull_groups<<<nblk(nb, 256), 256, 0, st>>>(nb, row);
-  scan_ints(c, row + 2 * nb, row + 3 * nb, c.d_cull_scan_tmp.p, nb, st);
-  k_cull_write<<<list_tile_grid(c), 256, 0, st>>>(v, c.d_cull_mask.p, c.d_tile_pos.p, row);
-  k_cull_rows<<<nblk((long long)nb * 32, 256), 256, 0, st>>>(v, row);
+  c.kernel_launches += 1;
+  const float R = list_radius + 1e-3f, Rc = fmaxf(list_radius - (float)c.lp.Padding, 0.f);
+  k_cull<<<c.nblocks, kCullWarps * 32, 0, c.stream>>>(c.view(), R * R, Rc * Rc, c.d_row_start.p, c.d_row_cnt.p,
+                                                      c.d_cull_mask.p);
 }
 
 // rows of the tile-list build: 4 warps per CTA, a bitmap over each warp's row
@@ -1029,7 +1038,7 @@ int launch_list_build(Context& c, float list_radius, float full_radius, ListSizi
     scan_ints(c, c.d_tile_flag.p, c.d_tile_pos.p, c.d_scan_tmp2.p, c.tile_cap, st);
     k_item_write<<<nblk(c.tile_cap, 256), 256, 0, st>>>(v, c.tile_cap, pairs, c.d_tile_flag.p, c.d_tile_pos.p);
   }
-  k_pack<<<nblk(c.nslots, 256), 256, 0, st>>>(v, c.d_charge.p, 0.f, 0.f, 1, c.npairs_all, 0);
+  k_pack<<<nblk(c.nslots, 256), 256, 0, st>>>(v, c.d_charge.p, 0.f, 0.f, 1, c.npairs_all, 0, c.nb_set ? 1 : 0);
   // NB j-atom groups: only where the per-step displacement check runs
   c.cull_built = c.nb_set && c.nb_cull && c.lp.check_skin && c.cull_cap > 0;
   if (c.cull_built) launch_cull(c, list_radius);
@@ -1058,7 +1067,7 @@ int launch_pack(Context& c, float check_disp) {
     f2 = h * h;
   }
   k_pack<<<nblk(c.nslots, 256), 256, 0, c.stream>>>(v, c.d_charge.p, c2, f2, 0, c.npairs_all,
-                                                     c.cull_built ? 1 : 0);
+                                                     c.cull_built ? 1 : 0, c.cull_built ? 1 : 0);
   return cudaGetLastError() == cudaSuccess ? PDGPU_OK : PDGPU_ERR_CUDA;
 }
 

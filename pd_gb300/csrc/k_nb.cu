@@ -5,6 +5,8 @@
 //    the dispatch at nonbonded.cpp:1222-1246).
 // Every listed pair j < i inside Cutoff contributes once; bond order <= 2
 // pairs are zero, 1-4 pairs are scaled by Vdw14Scaling / Elec14Scaling.
+#include <algorithm>
+
 #include "pdgpu_tile.cuh"
 
 namespace pdgpu {
@@ -326,6 +328,13 @@ __device__ __forceinline__ void nb_flush(const DevView& v, int s, const NBAcc& a
   nb_flush_fix(v, s, F);
 }
 
+// Whether the pass walks the j-atom groups: they fit their arrays, and they
+// replace at least half of the tiles.  In a box of about twice the list radius
+// nearly every tile needs a per-pair image and stays a tile (667 waters at 12 A:
+// 45 of 2,016 tiles become 8 groups, same time either way); then the tile path
+// serves all.
+__device__ __forceinline__ bool nb_grouped(const DevView& v) { return v.cull_n[2] && 2 * v.cull_n[0] <= *v.ntiles; }
+
 // One warp per work item, grid-stride: the tiles left on the tile path, then the
 // j-atom groups (cull: the last list build wrote them and they fit).  The energy
 // kernel's CTAs hold 4 warps (each warp keeps 5 KB of shared memory).
@@ -338,7 +347,7 @@ __global__ void __launch_bounds__(ENERGY ? kNbEThreads : kNbThreads, ENERGY ? 5 
   NBEShared* sh = ENERGY ? &shared[threadIdx.x >> 5] : nullptr;
   const int lane = threadIdx.x & 31;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  const bool grouped = cull && v.cull_n[2];
+  const bool grouped = cull && nb_grouped(v);
   const int nrest = grouped ? v.cull_n[0] : *v.ntiles;
   const int nitem = nrest + (grouped ? v.cull_n[1] : 0);
   for (int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < nitem; w += nwarps) {
@@ -428,6 +437,263 @@ __global__ void __launch_bounds__(ENERGY ? kNbEThreads : kNbThreads, ENERGY ? 5 
   }
 }
 
+// ---------------------------------------------------------------------------
+// Force-only pass (every dynamics step) where the law ends smoothly: LJ and
+// Coulomb both go to zero at their cutoffs by a switch (NBConst::smooth), so a
+// pair beyond them contributes exactly 0 by clamping the switch and no pair needs
+// a decision at a cutoff.  Packed FP32x2 arithmetic throughout.
+//  * Groups, two of a row at once (.x, .y): each lane holds a j atom of either,
+//    the i block's atoms come from the warp's rows, 8 at a time (one sub-block of
+//    the sorted order): a sub-block whose box at the current positions no held
+//    atom reaches is skipped (on the solvated box 40 % of the steps: the list
+//    radius holds the skin, and a far j atom reaches part of a 32-atom block
+//    only).  The i atoms' sums rotate within 8 lanes and meet over the four
+//    8-lane groups after each sub-block.
+//  * Tiles (masked, diagonal, or with a per-pair image), step-packed: lane l
+//    holds i atom l, the j atoms l + kk and l + kk + 1 come as one pair.
+// Bound by the FMA pipe (a packed instruction holds it two cycles) and issue.
+// Solvated box, 22,489 atoms at 12 A: 88 us (scalar rotation of 32 x 32 items)
+// -> 49 us; 8 copies 607 -> 314 us, of which the steps themselves take half.
+// ---------------------------------------------------------------------------
+enum NBLaw { kLawSame = 0, kLawSplit = 1, kLawForce = 2, kLawVdw = 3 };
+
+// dE/dr / r of two pairs; QQ = -econv q q, SS the radius sums, EE = eps.
+// Switch S = s^2, s = 1 - u^2 clamped at 0, u = (r - inner) / w clamped at 0.
+template <int LAW>
+__device__ __forceinline__ float2 nb_law2(const NBConst& k, float2 r2, float2 QQ, float2 SS, float2 EE) {
+  const float2 M1 = f2(-1.f);
+  const float2 ir = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
+  const float2 ir2 = __fmul2_rn(ir, ir), r = __fmul2_rn(r2, ir);
+  const float2 t2 = __fmul2_rn(__fmul2_rn(SS, SS), ir2);
+  const float2 b6 = __fmul2_rn(__fmul2_rn(t2, t2), t2);
+  const float2 eb = __fmul2_rn(EE, b6), ea = __fmul2_rn(eb, b6);      // eps B, eps A
+  const float2 t = __ffma2_rn(eb, M1, ea), ev = __ffma2_rn(eb, M1, t);   // eps (A - B), eps (A - 2B)
+  float2 u = __ffma2_rn(r, f2(k.vdwiw_f), f2(-k.vdwinner_iw_f));
+  u = make_float2(fmaxf(u.x, 0.f), fmaxf(u.y, 0.f));
+  float2 s = __ffma2_rn(__fmul2_rn(u, u), M1, f2(1.f));
+  s = make_float2(fmaxf(s.x, 0.f), fmaxf(s.y, 0.f));
+  const float2 Sv = __fmul2_rn(__fmul2_rn(s, s), ir2);                                 // S / r^2
+  const float2 nv = __fmul2_rn(__fmul2_rn(u, s), __fmul2_rn(ir, f2(-4.f * k.vdwiw_f)));   // S' / r
+  if (LAW == kLawVdw) return __ffma2_rn(__fmul2_rn(t, f2(-12.f)), Sv, __fmul2_rn(ev, nv));
+  const float2 e1 = __fmul2_rn(QQ, ir);   // -E_coulomb
+  if (LAW == kLawSame) return __ffma2_rn(__ffma2_rn(t, f2(-12.f), e1), Sv, __fmul2_rn(__ffma2_rn(e1, M1, ev), nv));
+  const float2 gv = __ffma2_rn(__fmul2_rn(t, f2(-12.f)), Sv, __fmul2_rn(ev, nv));
+  if (LAW == kLawSplit) {
+    u = __ffma2_rn(r, f2(k.iw_f), f2(-k.inner_iw_f));
+    u = make_float2(fmaxf(u.x, 0.f), fmaxf(u.y, 0.f));
+    s = __ffma2_rn(__fmul2_rn(u, u), M1, f2(1.f));
+    s = make_float2(fmaxf(s.x, 0.f), fmaxf(s.y, 0.f));
+    const float2 Se = __fmul2_rn(__fmul2_rn(s, s), ir2);
+    const float2 ne = __fmul2_rn(__fmul2_rn(u, s), __fmul2_rn(ir, f2(4.f * k.iw_f)));
+    return __ffma2_rn(e1, Se, __ffma2_rn(e1, ne, gv));
+  }
+  // Steinbach & Brooks force switch, nonbonded.cpp:798-819
+  float2 c = __ffma2_rn(r2, M1, f2(k.cut2));
+  c = make_float2(fmaxf(c.x, 0.f), fmaxf(c.y, 0.f));
+  const float2 f = __fmul2_rn(__fmul2_rn(__fmul2_rn(c, c), __ffma2_rn(r2, f2(2.f), f2(k.fsw_k))), f2(k.sA_f));
+  const float2 m = make_float2(r.x > k.inner_f ? f.x : 1.f, r.y > k.inner_f ? f.y : 1.f);
+  return __ffma2_rn(__fmul2_rn(e1, ir2), m, gv);
+}
+
+struct NBRows {
+  union {
+    struct {
+      float4 xy[64], zq[64], se[64];   // tiles: step pairs of the j block, twice over
+    };
+    struct {
+      float4 x[64];                    // groups: (x, y, z, q) of the i block, each sub-block twice over
+      float2 p[64];                    // (LJ radius, sqrt(eps))
+    };
+  };
+};
+
+template <int LAW, bool MASKED, bool MI>
+__device__ __forceinline__ void nb_tile2(const DevView& v, const NBConst& k, const Tile& T, int lane, NBRows& rs) {
+  const int si = T.bi * 32 + lane, sj = T.bj * 32 + lane, l1 = (lane + 1) & 31;
+  const float4 xi = v.xq[si], pi = v.par[si];
+  const SystemInfo& S = v.sys[v.slot_sys[T.bi]];
+  unsigned ex = 0u, m14 = 0u;
+  if (MASKED) {
+    tile_masks(v, T, lane, ex, m14);
+    if (T.flags & 2) ex |= diag_exclusion(lane);
+  }
+  {
+    const float4 x0 = j_in_i_frame(v, T, lane), p0 = v.par[sj];
+    const float e0 = p0.y;
+    const float x1 = __shfl_sync(0xffffffffu, x0.x, l1), y1 = __shfl_sync(0xffffffffu, x0.y, l1);
+    const float z1 = __shfl_sync(0xffffffffu, x0.z, l1), q1 = __shfl_sync(0xffffffffu, x0.w, l1);
+    const float s1 = __shfl_sync(0xffffffffu, p0.x, l1), e1 = __shfl_sync(0xffffffffu, e0, l1);
+    __syncwarp();
+    rs.xy[lane] = rs.xy[lane + 32] = make_float4(x0.x, x1, x0.y, y1);
+    rs.zq[lane] = rs.zq[lane + 32] = make_float4(x0.z, z1, x0.w, q1);
+    rs.se[lane] = rs.se[lane + 32] = make_float4(p0.x, s1, e0, e1);
+    __syncwarp();
+  }
+  const float2 X = f2(-xi.x), Y = f2(-xi.y), Z = f2(-xi.z), Q = f2(-k.econv_diel * xi.w), R = f2(pi.x);
+  const float2 E = f2(pi.y);
+  float Lx = 0.f, Ly = 0.f, Lz = 0.f, iLx = 0.f, iLy = 0.f, iLz = 0.f;
+  if (MI) {
+    Lx = S.boxf[0].h; Ly = S.boxf[1].h; Lz = S.boxf[2].h;
+    iLx = 1.f / Lx; iLy = 1.f / Ly; iLz = 1.f / Lz;
+  }
+  constexpr float kRint = 12582912.f;   // 1.5 2^23: adding and taking it off rounds to an integer
+  float2 FX = f2(0.f), FY = f2(0.f), FZ = f2(0.f), JX = f2(0.f), JY = f2(0.f), JZ = f2(0.f);   // J: minus the sums
+  const float4 *xy = rs.xy + lane, *zq = rs.zq + lane, *se = rs.se + lane;
+#pragma unroll 2
+  for (int kk = 0; kk < 32; kk += 2) {
+    const float4 P = xy[kk], ZQ = zq[kk], SE = se[kk];
+    float2 dx = __fadd2_rn(make_float2(P.x, P.y), X), dy = __fadd2_rn(make_float2(P.z, P.w), Y);
+    float2 dz = __fadd2_rn(make_float2(ZQ.x, ZQ.y), Z);
+    if (MI) {
+      const float2 nx = __fadd2_rn(__ffma2_rn(dx, f2(iLx), f2(kRint)), f2(-kRint));
+      const float2 ny = __fadd2_rn(__ffma2_rn(dy, f2(iLy), f2(kRint)), f2(-kRint));
+      const float2 nz = __fadd2_rn(__ffma2_rn(dz, f2(iLz), f2(kRint)), f2(-kRint));
+      dx = __ffma2_rn(nx, f2(-Lx), dx);
+      dy = __ffma2_rn(ny, f2(-Ly), dy);
+      dz = __ffma2_rn(nz, f2(-Lz), dz);
+    }
+    const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
+    float2 QQ = __fmul2_rn(Q, make_float2(ZQ.z, ZQ.w)), EE = __fmul2_rn(E, make_float2(SE.z, SE.w));
+    if (MASKED) {
+      const bool ma = (m14 >> kk) & 1u, mb = (m14 >> kk) & 2u;
+      QQ = __fmul2_rn(QQ, make_float2(ma ? k.elec14 : 1.f, mb ? k.elec14 : 1.f));
+      EE = __fmul2_rn(EE, make_float2(ma ? k.vdw14 : 1.f, mb ? k.vdw14 : 1.f));
+    }
+    float2 g = nb_law2<LAW>(k, r2, QQ, __fadd2_rn(R, make_float2(SE.x, SE.y)), EE);
+    if (MASKED) g = make_float2((ex >> kk) & 1u ? 0.f : g.x, (ex >> kk) & 2u ? 0.f : g.y);
+    FX = __ffma2_rn(g, dx, FX); FY = __ffma2_rn(g, dy, FY); FZ = __ffma2_rn(g, dz, FZ);
+    JX = __ffma2_rn(g, dx, JX); JY = __ffma2_rn(g, dy, JY); JZ = __ffma2_rn(g, dz, JZ);
+    ROT2(JX); ROT2(JY); ROT2(JZ);
+  }
+  const int lm = (lane + 31) & 31;
+  const float jx = JX.x + __shfl_sync(0xffffffffu, JX.y, lm), jy = JY.x + __shfl_sync(0xffffffffu, JY.y, lm);
+  const float jz = JZ.x + __shfl_sync(0xffffffffu, JZ.y, lm);
+  nb_flush(v, si, NBAcc{FX.x + FX.y, FY.x + FY.y, FZ.x + FZ.y});
+  nb_flush(v, sj, NBAcc{-jx, -jy, -jz});
+}
+
+// lower bound of the squared distance from a point to a box
+__device__ __forceinline__ float box_dist2(const float4& x, const float4& lo, const float4& hi) {
+  const float gx = fmaxf(fmaxf(lo.x - x.x, x.x - hi.x), 0.f), gy = fmaxf(fmaxf(lo.y - x.y, x.y - hi.y), 0.f);
+  const float gz = fmaxf(fmaxf(lo.z - x.z, x.z - hi.z), 0.f);
+  return gx * gx + gy * gy + gz * gz;
+}
+
+// one pair of groups of row bi (entries en[0..63])
+template <int LAW>
+__device__ __forceinline__ void nb_groups2(const DevView& v, const NBConst& k, int bi, const float4* en, int lane,
+                                           NBRows& rs) {
+  const int si = bi * 32 + lane, row = (lane >> 3) * 16 + (lane & 7);
+  const float4 xi = v.xq[si], pi = v.par[si];
+  // the lane's two j atoms in i's frame (empty lanes parked far away)
+  const float4 ea = en[lane], eb = en[32 + lane];
+  const int sa = __float_as_int(ea.w), sb = __float_as_int(eb.w);
+  float4 xa = make_float4(1.0e15f, 1.0e15f, 1.0e15f, 0.f), xb = xa, pa = make_float4(0.f, 0.f, 0.f, 0.f), pb = pa;
+  if (sa >= 0) {
+    xa = v.xq[sa];
+    pa = v.par[sa];
+    xa.x += ea.x; xa.y += ea.y; xa.z += ea.z;
+  }
+  if (sb >= 0) {
+    xb = v.xq[sb];
+    pb = v.par[sb];
+    xb.x += eb.x; xb.y += eb.y; xb.z += eb.z;
+  }
+  __syncwarp();
+  rs.x[row] = rs.x[row + 8] = make_float4(xi.x, xi.y, xi.z, k.econv_diel * xi.w);
+  rs.p[row] = rs.p[row + 8] = make_float2(pi.x, pi.y);
+  __syncwarp();
+  const float2 nx = make_float2(-xa.x, -xb.x), ny = make_float2(-xa.y, -xb.y), nz = make_float2(-xa.z, -xb.z);
+  const float2 QN = make_float2(-xa.w, -xb.w), RS = make_float2(pa.x, pb.x);
+  const float2 EN = make_float2(pa.y, pb.y);
+  float2 FX = f2(0.f), FY = f2(0.f), FZ = f2(0.f);   // force on the held atoms along d = x_i - x_j
+  float ix = 0.f, iy = 0.f, iz = 0.f;                // minus the sums of i atom `lane`
+  const float reach2 = k.cut2 * 1.00001f;
+  const int src = (lane & 24) | ((lane + 1) & 7);
+#pragma unroll 1
+  for (int s = 0; s < 4; s++) {
+    const float4 lo = v.sub[8 * bi + 2 * s], hi = v.sub[8 * bi + 2 * s + 1];
+    if (!__any_sync(0xffffffffu, fminf(box_dist2(xa, lo, hi), box_dist2(xb, lo, hi)) <= reach2)) continue;
+    const float4* xr = rs.x + s * 16 + (lane & 7);
+    const float2* pr = rs.p + s * 16 + (lane & 7);
+    float rx = 0.f, ry = 0.f, rz = 0.f;
+#pragma unroll 4
+    for (int kk = 0; kk < 8; kk++) {
+      const float4 x = xr[kk];
+      const float2 p = pr[kk];
+      const float2 dx = __fadd2_rn(f2(x.x), nx), dy = __fadd2_rn(f2(x.y), ny), dz = __fadd2_rn(f2(x.z), nz);
+      const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
+      const float2 g = nb_law2<LAW>(k, r2, __fmul2_rn(QN, f2(x.w)), __fadd2_rn(RS, f2(p.x)), __fmul2_rn(EN, f2(p.y)));
+      FX = __ffma2_rn(g, dx, FX); FY = __ffma2_rn(g, dy, FY); FZ = __ffma2_rn(g, dz, FZ);
+      rx = fmaf(g.x, dx.x, rx); rx = fmaf(g.y, dx.y, rx);
+      ry = fmaf(g.x, dy.x, ry); ry = fmaf(g.y, dy.y, ry);
+      rz = fmaf(g.x, dz.x, rz); rz = fmaf(g.y, dz.y, rz);
+      rx = __shfl_sync(0xffffffffu, rx, src);
+      ry = __shfl_sync(0xffffffffu, ry, src);
+      rz = __shfl_sync(0xffffffffu, rz, src);
+    }
+    // lane holds the sum of sub-block atom lane & 7 over its 8-lane group's j atoms
+#pragma unroll
+    for (int o = 8; o < 32; o <<= 1) {
+      rx += __shfl_xor_sync(0xffffffffu, rx, o);
+      ry += __shfl_xor_sync(0xffffffffu, ry, o);
+      rz += __shfl_xor_sync(0xffffffffu, rz, o);
+    }
+    if ((lane >> 3) == s) {
+      ix = rx;
+      iy = ry;
+      iz = rz;
+    }
+  }
+  nb_flush(v, si, NBAcc{-ix, -iy, -iz});
+  if (sa >= 0) nb_flush(v, sa, NBAcc{FX.x, FY.x, FZ.x});
+  if (sb >= 0) nb_flush(v, sb, NBAcc{FX.y, FY.y, FZ.y});
+}
+
+constexpr int kNbFThreads = 128;
+template <int LAW>
+__global__ void __launch_bounds__(kNbFThreads, 6)
+    k_nb_force(const __grid_constant__ DevView v, const __grid_constant__ NBConst k, int cull) {
+  __shared__ NBRows rows[kNbFThreads / 32];
+  NBRows& rs = rows[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31;
+  const int nwarps = (gridDim.x * blockDim.x) >> 5;
+  const bool grouped = cull && nb_grouped(v);
+  const int nrest = grouped ? v.cull_n[0] : *v.ntiles;
+  const int nitem = nrest + (grouped ? v.cull_n[1] / 2 : 0);
+  for (int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < nitem; w += nwarps) {
+    if (w < nrest) {
+      const Tile T = v.tiles[grouped ? v.cull_rest[w] : w];
+      const bool mi = T.flags & 1;
+      if (tile_masked(T)) {
+        if (mi) nb_tile2<LAW, true, true>(v, k, T, lane, rs);
+        else nb_tile2<LAW, true, false>(v, k, T, lane, rs);
+      } else {
+        if (mi) nb_tile2<LAW, false, true>(v, k, T, lane, rs);
+        else nb_tile2<LAW, false, false>(v, k, T, lane, rs);
+      }
+    } else {
+      const int g = 2 * (w - nrest);
+      nb_groups2<LAW>(v, k, v.cull_bi[g], v.cull_ent + (size_t)g * 32, lane, rs);
+    }
+  }
+}
+
+static void launch_nb_force(Context& c, const NBConst& k, int g) {
+  DevView v = c.view();
+  const int cull = c.cull_built ? 1 : 0;
+  constexpr int T = kNbFThreads;
+  // four times the other tile kernels' warps (no more than items): the items
+  // take unequal numbers of steps, and CTAs that end early make room for the next
+  // (8 copies of the solvated box: 336 -> 314 us; one copy 51 -> 49)
+  const long long want = (c.tile_cap + c.cull_cap / 64 + 3) / 4;
+  g = (int)std::min<long long>(4LL * g * (256 / T), want > 0 ? want : 1);
+  if (k.elecmode == 0) k_nb_force<kLawVdw><<<g, T, 0, c.stream>>>(v, k, cull);
+  else if (k.elecmode == 4) k_nb_force<kLawForce><<<g, T, 0, c.stream>>>(v, k, cull);
+  else if (k.samesw) k_nb_force<kLawSame><<<g, T, 0, c.stream>>>(v, k, cull);
+  else k_nb_force<kLawSplit><<<g, T, 0, c.stream>>>(v, k, cull);
+}
+
 template <bool E>
 static void launch_nb_mode(Context& c, const NBConst& k, int g) {
   DevView v = c.view();
@@ -439,7 +705,7 @@ static void launch_nb_mode(Context& c, const NBConst& k, int g) {
     case 0: k_nb_tiles<0, E><<<g, T, 0, c.stream>>>(v, k, e, cull); break;
     case 1: k_nb_tiles<1, E><<<g, T, 0, c.stream>>>(v, k, e, cull); break;
     case 3:
-      if (k.samesw) k_nb_tiles<3, E, true><<<g, T, 0, c.stream>>>(v, k, e, cull);
+      if (E && k.samesw) k_nb_tiles<3, true, true><<<g, T, 0, c.stream>>>(v, k, e, cull);
       else k_nb_tiles<3, E><<<g, T, 0, c.stream>>>(v, k, e, cull);
       break;
     default: k_nb_tiles<4, E><<<g, T, 0, c.stream>>>(v, k, e, cull); break;
@@ -458,6 +724,8 @@ int launch_nb(Context& c, const NBConst& k, bool energy) {
     c.kernel_launches += 1;
     launch_df_records(c);
     launch_nb_mode<true>(c, k, g);
+  } else if (k.smooth) {
+    launch_nb_force(c, k, g);
   } else {
     launch_nb_mode<false>(c, k, g);
   }

@@ -137,6 +137,11 @@ NBConst pdgpu::make_nb_const(const pdgpu_nb_params& p) {
   if (!p.DoElec) k.elecmode = 0;
   k.dovdw = p.DoVdw ? 1 : 0;
   k.samesw = (k.elecmode == 3 && k.dovdw && p.VdwCutoff == p.Cutoff && p.VdwInnerCutoff == p.InnerCutoff) ? 1 : 0;
+  k.smooth = k.dovdw && vw > 0 && p.VdwCutoff <= p.Cutoff && (k.elecmode == 0 || (k.elecmode >= 3 && w > 0)) ? 1 : 0;
+  k.vdwiw_f = vw > 0 ? (float)(1.0 / vw) : 0.f;
+  k.vdwinner_iw_f = vw > 0 ? (float)(p.VdwInnerCutoff / vw) : 0.f;
+  k.iw_f = w > 0 ? (float)(1.0 / w) : 0.f;
+  k.inner_iw_f = w > 0 ? (float)(I / w) : 0.f;
   return k;
 }
 
@@ -479,6 +484,7 @@ pdgpu_ctx* pdgpu_create(int device, const pdgpu_system_desc* d, int* status) {
   if (e == cudaSuccess) e = c.d_center.alloc(3 * (size_t)c.nblocks);
   if (e == cudaSuccess) e = c.d_half.alloc(c.nblocks);
   if (e == cudaSuccess) e = c.d_cenf.alloc(c.nblocks);
+  if (e == cudaSuccess) e = c.d_sub.alloc(8 * (size_t)c.nblocks);
   // (the tile arrays are sized by the first list build, from its tile count)
   if (e == cudaSuccess) e = c.d_counters.alloc(8);
   if (e == cudaSuccess) e = cudaMemset(c.d_counters.p, 0, sizeof(int) * 8);
@@ -553,28 +559,25 @@ static int size_list(Context& c) {
   return rebuild_list_impl(c);
 }
 
-// NB j-atom group buffers: the per-row arrays with the NB parameters (never
-// inside a stream capture), the per-tile ones with the tile arrays
+// NB j-atom group buffers: wanted from the NB parameters on (never allocated
+// inside a stream capture), sized with the tile arrays
 static int alloc_cull(Context& c) {
-  if (c.d_cull_row.p) return PDGPU_OK;
+  if (c.cull_want) return PDGPU_OK;
   cudaError_t e = cudaSetDevice(c.device);
-  if (e == cudaSuccess) e = c.d_cull_row.alloc(4 * (size_t)c.nblocks);
-  if (e == cudaSuccess) e = c.d_cull_scan_tmp.alloc((c.nblocks + 1023) / 1024 + 1);
-  if (e != cudaSuccess) {
-    c.d_cull_row.release();
-    c.d_cull_scan_tmp.release();
-    cudaGetLastError();
-    return PDGPU_ERR_CUDA;
-  }
-  return c.tile_cap > 0 ? alloc_cull_tiles(c) : PDGPU_OK;
+  if (e != cudaSuccess) return PDGPU_ERR_CUDA;
+  c.cull_want = true;
+  if (c.tile_cap == 0) return PDGPU_OK;
+  const int st = alloc_cull_tiles(c);
+  if (st != PDGPU_OK) c.cull_want = false;
+  return st;
 }
 
-// at most 32 entries per tile plus one open group per row, held to 8192
+// at most 32 entries per tile plus two open groups per row, held to 8192
 // entries per row (a list that needs more keeps the tile path)
 int pdgpu::alloc_cull_tiles(Context& c) {
   c.cull_cap = 0;
-  if (!c.d_cull_row.p || c.tile_cap == 0) return PDGPU_OK;
-  const long long cap = std::min(32LL * c.tile_cap + 32LL * c.nblocks, 8192LL * c.nblocks);
+  if (!c.cull_want || c.tile_cap == 0) return PDGPU_OK;
+  const long long cap = std::min(32LL * c.tile_cap + 64LL * c.nblocks, 8192LL * c.nblocks);
   cudaError_t e = c.d_cull_mask.alloc(c.tile_cap);
   if (e == cudaSuccess) e = c.d_cull_rest.alloc(c.tile_cap);
   if (e == cudaSuccess) e = c.d_cull_ent.alloc(cap);
@@ -1118,7 +1121,7 @@ int pdgpu_list_tiles(pdgpu_ctx* h, int* tiles, long long cap, long long* ntiles,
     // the arrays whose size follows the list
     *list_bytes = (long long)(c.d_tiles.n * sizeof(Tile) + c.d_items.n * 4 + c.d_tile_flag.n * 4 +
                               c.d_tile_pos.n * 4 + c.d_scan_tmp2.n * 4 + c.d_tile_need.n * 4 + c.d_mlist.n * 4 +
-                              c.d_masks.n * sizeof(uint2) + c.d_cull_mask.n * 4 + c.d_cull_rest.n * 4 +
+                              c.d_masks.n * sizeof(uint2) + c.d_cull_mask.n * sizeof(uint2) + c.d_cull_rest.n * 4 +
                               c.d_cull_ent.n * sizeof(float4) + c.d_cull_bi.n * 4);
   }
   return PDGPU_OK;

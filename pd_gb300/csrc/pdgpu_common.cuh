@@ -100,6 +100,10 @@ struct NBConst {
   // 1: LJ and Coulomb switched over the same radii (Cutoff = VdwCutoff,
   // InnerCutoff = VdwInnerCutoff, energy switch, LJ on): one switch serves both
   int samesw;
+  // 1: LJ and Coulomb (if any) both end by a switch, LJ not beyond Cutoff, so the
+  // law is continuous at every cutoff (the packed force pass)
+  int smooth;
+  float vdwiw_f, vdwinner_iw_f, iw_f, inner_iw_f;   // 1 / switch width, inner radius / width
 };
 
 // The same constants as double-floats, for the pair energies (FF_NonBonded)
@@ -151,6 +155,7 @@ struct DevView {
   float4* rel0;              // rel pos at list build (displacement check)
   double* center;            // [nblocks*3]
   float4* half;              // [nblocks] half extents
+  float4* sub;               // [nblocks*8] box (lo, hi) of each 8 slots at the packed positions, in the block's frame
   float4* cenf;              // [nblocks] centre in FP32 (exact: centres are FP32 numbers)
   // (energy evaluations) what FP32 rounding takes off the packed slots:
   // (x, y, z, charge) - xq and (LJ radius, sqrt(eps)) - par, written before the energy pass
@@ -174,7 +179,7 @@ struct DevView {
   // single-image tiles that lie within the list radius of the i block's box,
   // packed 32 to a group; the other tiles stay on the tile path (cull_rest)
   float4* cull_ent;          // [cull_cap] j offset into the i block's frame (x, y, z), j slot (int bits; -1 empty)
-  int* cull_bi;              // [cull_cap / 32] i block of each group
+  int* cull_bi;              // [cull_cap / 32] i block of each group (a row's groups: an even number)
   int* cull_rest;            // [tile capacity] tiles left on the tile path (any order)
   int* cull_n;               // [0] rest tiles, [1] groups, [2] 1 when the groups fit the capacity
   long long cull_cap;        // entries

@@ -107,6 +107,7 @@ struct Context {
   DBuf<double> d_center;       // [nblocks*3]
   DBuf<float4> d_half;         // [nblocks]
   DBuf<float4> d_cenf;         // [nblocks]
+  DBuf<float4> d_sub;          // [nblocks*8]
   DBuf<float> d_sys_hmax;      // [nsys*3] largest block half-extent (ordered ints)
   DBuf<BlockGrid> d_bgrid;     // [nsys]
   DBuf<int> d_bcell;           // [nblocks] cell of each block
@@ -126,10 +127,9 @@ struct Context {
   DBuf<float4> d_rlo;                // [nslots] FP32 remainders of the slots (energy evaluations)
   DBuf<float2> d_plo;                // [nslots]
   // NB j-atom groups (allocated with the NB parameters)
-  DBuf<unsigned> d_cull_mask;        // [tile_cap] j lanes kept per tile
+  bool cull_want = false;            // the NB parameters were set
+  DBuf<uint2> d_cull_mask;           // [tile_cap] j lanes kept per tile: near (within the cutoffs), skin
   DBuf<int> d_cull_rest;             // [tile_cap]
-  DBuf<int> d_cull_row;              // [4*nblocks] per row: kept j atoms, first tile, groups, first group
-  DBuf<int> d_cull_scan_tmp;
   DBuf<float4> d_cull_ent;           // [cull_cap]
   DBuf<int> d_cull_bi;               // [cull_cap / 32]
   long long cull_cap = 0;
@@ -200,6 +200,7 @@ struct Context {
     v.center = d_center.p;
     v.half = d_half.p;
     v.cenf = d_cenf.p;
+    v.sub = d_sub.p;
     v.rlo = d_rlo.p;
     v.plo = d_plo.p;
     v.band_excl = d_band_excl.p;

@@ -11,6 +11,10 @@ __device__ __forceinline__ unsigned diag_exclusion(int lane) {
 }
 
 #define ROT(x) x = __shfl_sync(0xffffffffu, x, (lane + 1) & 31)
+// an FP32x2 pair of a step-packed body, two lanes down
+#define ROT2(p) p.x = __shfl_sync(0xffffffffu, p.x, (lane + 2) & 31); p.y = __shfl_sync(0xffffffffu, p.y, (lane + 2) & 31)
+
+__device__ __forceinline__ float2 f2(float a) { return make_float2(a, a); }
 
 // FP64 squared distance of two sorted slots from the original positions
 static __device__ __noinline__ double r2_slots_fp64(const DevView& v, int sa, int sb) {
