@@ -225,13 +225,6 @@ __device__ __forceinline__ void born_full2(const DevView& v, const GBConst& k, c
   atomic_add_ll(&gpol[r0 + lane], fx32(gr));
 }
 
-// the warp's next work item: a tile (t) or a tile pair (t, t + 1)
-__device__ __forceinline__ int item_tile(const DevView& v, int it, bool& two) {
-  const unsigned code = v.items[it];
-  two = (code >> 31) != 0u;
-  return (int)(code & 0x7fffffffu);
-}
-
 __device__ __forceinline__ void born_single(const DevView& v, const GBConst& k, const Tile& T, int lane,
                                             long long* gpol, BornRows& rs) {
   const bool full = tile_full(T);
@@ -255,15 +248,9 @@ __global__ void __launch_bounds__(kBornThreads, 5) k_gb_born(const __grid_consta
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   const int ni = *v.nitems;
   for (int it = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; it < ni; it += nwarps) {
-    bool two;
-    const int t = item_tile(v, it, two);
-    const Tile T = v.tiles[t];
-    if (two && tile_full(T)) {
-      born_full2(v, k, T, v.tiles[t + 1], lane, gpol, rs);
-      continue;
-    }
-    born_single(v, k, T, lane, gpol, rs);
-    if (two) born_single(v, k, v.tiles[t + 1], lane, gpol, rs);
+    const int2 t = v.items[it];
+    if (t.y >= 0) born_full2(v, k, v.tiles[t.x], v.tiles[t.y], lane, gpol, rs);
+    else born_single(v, k, v.tiles[t.x], lane, gpol, rs);
   }
 }
 
@@ -770,15 +757,13 @@ __global__ void __launch_bounds__(kPairThreads, 5) k_gb_pair(const __grid_consta
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   const int ni = *v.nitems;
   for (int it = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; it < ni; it += nwarps) {
-    bool two;
-    const int t = item_tile(v, it, two);
-    const Tile T = v.tiles[t];
-    if (FAST && two && tile_full(T)) {
-      gb_pair_full2(v, k, T, v.tiles[t + 1], lane, born, deda, rs);
+    const int2 t = v.items[it];
+    if (FAST && t.y >= 0) {
+      gb_pair_full2(v, k, v.tiles[t.x], v.tiles[t.y], lane, born, deda, rs);
       continue;
     }
-    gb_pair_single<FAST, false, false>(v, k, T, lane, born, deda, rs, nullptr);
-    if (two) gb_pair_single<FAST, false, false>(v, k, v.tiles[t + 1], lane, born, deda, rs, nullptr);
+    gb_pair_single<FAST, false, false>(v, k, v.tiles[t.x], lane, born, deda, rs, nullptr);
+    if (!FAST && t.y >= 0) gb_pair_single<FAST, false, false>(v, k, v.tiles[t.y], lane, born, deda, rs, nullptr);
   }
 }
 
@@ -1015,15 +1000,9 @@ __global__ void __launch_bounds__(kChainThreads, 6) k_gb_chain(const __grid_cons
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   const int ni = *v.nitems;
   for (int it = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; it < ni; it += nwarps) {
-    bool two;
-    const int t = item_tile(v, it, two);
-    const Tile T = v.tiles[t];
-    if (two && tile_full(T)) {
-      chain_full2(v, k, T, v.tiles[t + 1], lane, chain, rs);
-      continue;
-    }
-    chain_single(v, k, T, lane, chain, rs);
-    if (two) chain_single(v, k, v.tiles[t + 1], lane, chain, rs);
+    const int2 t = v.items[it];
+    if (t.y >= 0) chain_full2(v, k, v.tiles[t.x], v.tiles[t.y], lane, chain, rs);
+    else chain_single(v, k, v.tiles[t.x], lane, chain, rs);
   }
 }
 

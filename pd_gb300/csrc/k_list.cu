@@ -8,7 +8,7 @@
 // count).  The bond order PD packs into
 // each list entry (neighbourlist.cpp:398-422, 179-220) becomes a per-tile
 // exclusion / 1-4 bit mask.
-#include <cstdio>
+#include <algorithm>
 
 #include "pdgpu_tile.cuh"
 
@@ -47,6 +47,9 @@ __device__ __forceinline__ int hilbert3(unsigned x0, unsigned x1, unsigned x2) {
   return h;
 }
 
+// rows of systems of up to this many blocks (32,768 atoms) test every column
+constexpr int kDirectBlocks = 1024;
+
 // order-preserving float <-> int for atomic min / max
 __device__ __forceinline__ int f2ord(float f) {
   int i = __float_as_int(f);
@@ -54,13 +57,22 @@ __device__ __forceinline__ int f2ord(float f) {
 }
 __device__ __forceinline__ float ord2f(int i) { return __int_as_float(i >= 0 ? i : i ^ 0x7fffffff); }
 
-__global__ void k_bbox_init(int* lo, int* hi, int* hmax, int n) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) {
-    lo[i] = f2ord(3.0e38f);
-    hi[i] = f2ord(-3.0e38f);
-    hmax[i] = f2ord(0.f);
+// everything a build counts into, cleared in one launch
+struct ListInit {
+  int *count, *cursor, *sorted_atom, *bcell_count, *bcell_cursor, *lo, *hi, *hmax, *counters;
+  int ncells, nslots, nbcells, nsys3;
+};
+__global__ void k_list_init(ListInit I) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, n = gridDim.x * blockDim.x;
+  for (int i = t; i < I.ncells; i += n) I.count[i] = I.cursor[i] = 0;
+  for (int i = t; i < I.nslots; i += n) I.sorted_atom[i] = -1;
+  for (int i = t; i < I.nbcells; i += n) I.bcell_count[i] = I.bcell_cursor[i] = 0;
+  for (int i = t; i < I.nsys3; i += n) {
+    I.lo[i] = f2ord(3.0e38f);
+    I.hi[i] = f2ord(-3.0e38f);
+    I.hmax[i] = f2ord(0.f);
   }
+  if (t < 8) I.counters[t] = t == 5 ? 1 : 0;   // [5]: the NB groups fit until a row finds they do not
 }
 
 // bounding box of each open-space system (periodic systems key on the box);
@@ -98,8 +110,42 @@ __global__ void k_bbox(DevView v, const int* atom_sys, int* lo, int* hi) {
 
 __device__ __forceinline__ double wrap_coord(double x, double L, double iL) { return x - L * floor(x * iL); }
 
-__global__ void k_keys(DevView v, const int* atom_sys, const int* lo, const int* hi, int* bucket, int* count) {
+// the grid of one system's block centres for this build
+__device__ __forceinline__ void grid_setup(const SystemInfo& S, int s, const int* lo, const int* hi, BlockGrid* grid) {
+  BlockGrid G;
+  double ext[3];
+  for (int c = 0; c < 3; c++) {
+    if (S.periodic) {
+      G.origin[c] = 0.0;
+      ext[c] = S.box[c];
+    } else {
+      const double l = ord2f(lo[3 * s + c]), h = ord2f(hi[3 * s + c]);
+      G.origin[c] = l;
+      ext[c] = fmax(h - l, 1e-3);
+    }
+  }
+  // cells of about equal edge, at most grid_cells of them
+  const double edge = cbrt(ext[0] * ext[1] * ext[2] / (double)S.grid_cells);
+  for (int c = 0; c < 3; c++) G.dims[c] = (int)fmax(1.0, fmin(floor(ext[c] / edge), 4096.0));
+  while ((long long)G.dims[0] * G.dims[1] * G.dims[2] > S.grid_cells) {
+    const int m = G.dims[0] >= G.dims[1] ? (G.dims[0] >= G.dims[2] ? 0 : 2) : (G.dims[1] >= G.dims[2] ? 1 : 2);
+    G.dims[m]--;
+  }
+  for (int c = 0; c < 3; c++) G.cell[c] = ext[c] / G.dims[c];
+  G.start = S.grid_start;
+  grid[s] = G;
+}
+
+// (the last CTA, launched past the atoms where some system uses a block grid,
+// sets those grids up)
+__global__ void k_keys(DevView v, const int* atom_sys, const int* lo, const int* hi, int* bucket, int* count,
+                       BlockGrid* grid) {
   int a = blockIdx.x * blockDim.x + threadIdx.x;
+  if (grid && blockIdx.x == gridDim.x - 1) {
+    for (int s = threadIdx.x; s < v.nsys; s += blockDim.x)
+      if (v.sys[s].nblocks > kDirectBlocks) grid_setup(v.sys[s], s, lo, hi, grid);
+    return;
+  }
   if (a >= v.natom) return;
   int s = atom_sys[a];
   const SystemInfo& S = v.sys[s];
@@ -177,21 +223,22 @@ __global__ void __launch_bounds__(1024) k_scan_sums(int* sums, int nb) {
   }
 }
 
-// one CTA for n <= kScanOne: 8 consecutive elements per thread
-constexpr int kScanOne = 8192;
+// one CTA for n <= kScanOne (one system's cells): PER consecutive elements per thread
+constexpr int kScanOne = 32768;
+template <int PER>
 __global__ void __launch_bounds__(1024) k_scan_one(const int* in, int* out, int n) {
   __shared__ int wsum[33];
-  const int base = threadIdx.x * 8;
-  int x[8], s = 0;
+  const int base = threadIdx.x * PER;
+  int x[PER], s = 0;
 #pragma unroll
-  for (int k = 0; k < 8; k++) {
+  for (int k = 0; k < PER; k++) {
     x[k] = base + k < n ? in[base + k] : 0;
     s += x[k];
   }
   int total;
   int run = cta_exclusive_scan(s, wsum, &total);
 #pragma unroll
-  for (int k = 0; k < 8; k++) {
+  for (int k = 0; k < PER; k++) {
     if (base + k < n) out[base + k] = run;
     run += x[k];
   }
@@ -209,13 +256,16 @@ __global__ void k_scatter(int natom, const int* bucket, const int* offset, int* 
   tmp[offset[b] + atomicAdd(&cursor[b], 1)] = a;
 }
 
-// insertion sort inside each non-empty cell so the order is deterministic
-__global__ void k_cell_sort(int ncells, const int* offset, const int* count, int* tmp) {
+// insertion sort inside each non-empty cell so the order is deterministic, then
+// the cell's atoms into their slots
+__global__ void k_cell_sort(DevView v, int ncells, const int* offset, const int* count, int* tmp, int* sorted_atom,
+                            int* slot_of) {
   int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= ncells) return;
   int n = count[b];
-  if (n < 2) return;
-  int* p = tmp + offset[b];
+  if (n < 1) return;
+  const int o = offset[b];
+  int* p = tmp + o;
   for (int i = 1; i < n; i++) {
     int x = p[i];
     int j = i - 1;
@@ -225,28 +275,92 @@ __global__ void k_cell_sort(int ncells, const int* offset, const int* count, int
     }
     p[j + 1] = x;
   }
+  const SystemInfo& S = v.sys[b / kCellsPerSystem];
+  const int slot = S.pad_start + (o - S.atom_start);
+  for (int i = 0; i < n; i++) {
+    const int a = p[i];
+    sorted_atom[slot + i] = a;
+    slot_of[a] = slot + i;
+  }
 }
 
-__global__ void k_to_slots(DevView v, const int* atom_sys, const int* tmp, int* sorted_atom, int* slot_of) {
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= v.natom) return;
-  int a = tmp[k];
-  int s = atom_sys[a];
-  const SystemInfo& S = v.sys[s];
-  int slot = S.pad_start + (k - S.atom_start);
-  sorted_atom[slot] = a;
-  slot_of[a] = slot;
+// boxes of each 8 slots at the packed positions (a padding slot widens its box:
+// it never hides an atom); every lane of the warp calls this
+__device__ __forceinline__ void write_sub(const DevView& v, int s, const float4& o) {
+  float4 lo = o, hi = o;
+#pragma unroll
+  for (int d = 4; d > 0; d >>= 1) {
+    lo.x = fminf(lo.x, __shfl_xor_sync(0xffffffffu, lo.x, d));
+    lo.y = fminf(lo.y, __shfl_xor_sync(0xffffffffu, lo.y, d));
+    lo.z = fminf(lo.z, __shfl_xor_sync(0xffffffffu, lo.z, d));
+    hi.x = fmaxf(hi.x, __shfl_xor_sync(0xffffffffu, hi.x, d));
+    hi.y = fmaxf(hi.y, __shfl_xor_sync(0xffffffffu, hi.y, d));
+    hi.z = fmaxf(hi.z, __shfl_xor_sync(0xffffffffu, hi.z, d));
+  }
+  if ((s & 7) == 0) {
+    v.sub[s >> 2] = lo;
+    v.sub[(s >> 2) + 1] = hi;
+  }
 }
 
-// block bounding boxes, and each system's largest half-extent; one warp per block
-__global__ void k_blocks(DevView v, int* hmax) {
-  int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  int lane = threadIdx.x & 31;
-  if (warp >= v.nblocks) return;
-  int slot = warp * 32 + lane;
-  int a = v.sorted_atom[slot];
-  const SystemInfo& S = v.sys[v.slot_sys[warp]];
-  double lo[3], hi[3];
+// slot s of atom a (-1: padding): FP64 position -> FP32 offset from the block centre
+__device__ __forceinline__ float4 packed_slot(const DevView& v, const SystemInfo& S, const double* charge, int s, int a,
+                                              const double c[3]) {
+  // padding slot: zero parameters, parked far away from everything and each other
+  if (a < 0) return make_float4(1.0e6f * (float)(1 + (s & 31)), 1.0e6f * (float)(1 + (s >> 5)), -1.0e6f, 0.f);
+  double r[3];
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    double d = v.pos[3 * a + k] - c[k];
+    if (S.periodic) d -= S.box[k] * rint(d * S.ibox[k]);
+    r[k] = d;
+  }
+  return make_float4((float)r[0], (float)r[1], (float)r[2], (float)charge[a]);
+}
+
+// cell coordinate of x along axis c (clamped into the grid)
+__device__ __forceinline__ int grid_axis(const BlockGrid& G, int c, double x) {
+  const double q = floor((x - G.origin[c]) / G.cell[c]);
+  return (int)fmin(fmax(q, 0.0), (double)(G.dims[c] - 1));
+}
+
+// One warp per block: its box (centre and half-extents), its slots' parameters and
+// packed positions, and its cell where the system's rows use the block grid.  FP32
+// box arithmetic with the half-extents on the safe side; the centre is an FP32
+// number, so that centre differences are exact in double-float arithmetic.
+struct SlotParams {
+  const double *radius, *sqeps, *gbR, *gbVj, *lcR, *charge;
+  const int* lcUse;
+  float4* lc_par;
+};
+__device__ __forceinline__ void slot_params(const DevView& v, const SlotParams& P, int s, int a) {
+  float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 l = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (a >= 0) {
+    p.x = (float)P.radius[a];
+    p.y = (float)P.sqeps[a];
+    if (P.gbR) {
+      p.z = (float)P.gbR[a];
+      p.w = (float)P.gbVj[a];
+    }
+    if (P.lcR) {
+      l.x = (float)P.lcR[a];
+      l.y = P.lcUse[a] ? 1.f : 0.f;
+    }
+  }
+  v.par[s] = p;
+  if (P.lc_par) P.lc_par[s] = l;
+}
+
+__global__ void __launch_bounds__(128) k_blocks(DevView v, SlotParams P, const BlockGrid* grid, int* hmax, int* bcell,
+                                                int* bcount, int sub) {
+  const int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (b >= v.nblocks) return;
+  const int slot = b * 32 + lane;
+  const int a = v.sorted_atom[slot];
+  const int sys = v.slot_sys[b];
+  const SystemInfo& S = v.sys[sys];
+  float lo[3], hi[3];
 #pragma unroll
   for (int c = 0; c < 3; c++) {
     double x = 0;
@@ -254,70 +368,66 @@ __global__ void k_blocks(DevView v, int* hmax) {
       x = v.pos[3 * a + c];
       if (S.periodic) x = wrap_coord(x, S.box[c], S.ibox[c]);
     }
-    lo[c] = a >= 0 ? x : 1e300;
-    hi[c] = a >= 0 ? x : -1e300;
+    lo[c] = a >= 0 ? (float)x : 3.0e38f;
+    hi[c] = a >= 0 ? (float)x : -3.0e38f;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-      lo[c] = fmin(lo[c], __shfl_xor_sync(0xffffffffu, lo[c], o));
-      hi[c] = fmax(hi[c], __shfl_xor_sync(0xffffffffu, hi[c], o));
+      lo[c] = fminf(lo[c], __shfl_xor_sync(0xffffffffu, lo[c], o));
+      hi[c] = fmaxf(hi[c], __shfl_xor_sync(0xffffffffu, hi[c], o));
     }
   }
+  slot_params(v, P, slot, a);
+  float cf[3], hf[3];
+  double cd[3];
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    cf[c] = 0.5f * lo[c] + 0.5f * hi[c];
+    cd[c] = (double)cf[c];
+    hf[c] = fmaxf(hi[c] - cf[c], cf[c] - lo[c]) + 1e-4f + 2.4e-7f * fmaxf(fabsf(lo[c]), fabsf(hi[c]));
+  }
+  const float4 o = packed_slot(v, S, P.charge, slot, a, cd);
+  v.xq[slot] = o;
+  v.rel0[slot] = o;
+  if (sub) write_sub(v, slot, o);
   if (lane == 0) {
-    // the centre is rounded to FP32 (any point near the middle serves), so that
-    // centre differences are exact in double-float arithmetic
-    float cf[3], hf[3];
-    for (int c = 0; c < 3; c++) {
-      cf[c] = (float)(0.5 * (lo[c] + hi[c]));
-      v.center[3 * warp + c] = (double)cf[c];
-      hf[c] = (float)fmax(hi[c] - (double)cf[c], (double)cf[c] - lo[c]) + 1e-4f;
+    v.half[b] = make_float4(hf[0], hf[1], hf[2], 0.f);
+    v.cenf[b] = make_float4(cf[0], cf[1], cf[2], 0.f);
+#pragma unroll
+    for (int c = 0; c < 3; c++) v.center[3 * b + c] = cd[c];
+    if (S.nblocks > kDirectBlocks) {
+      const BlockGrid& G = grid[sys];
+      const int cell = G.start + (grid_axis(G, 2, cd[2]) * G.dims[1] + grid_axis(G, 1, cd[1])) * G.dims[0] +
+                       grid_axis(G, 0, cd[0]);
+      bcell[b] = cell;
+      atomicAdd(&bcount[cell], 1);
+#pragma unroll
+      for (int c = 0; c < 3; c++) atomicMax(&hmax[3 * sys + c], f2ord(hf[c]));
     }
-    const float4 h = make_float4(hf[0], hf[1], hf[2], 0.f);
-    v.half[warp] = h;
-    v.cenf[warp] = make_float4(cf[0], cf[1], cf[2], 0.f);
-    const int s3 = 3 * v.slot_sys[warp];
-    atomicMax(&hmax[s3], f2ord(h.x));
-    atomicMax(&hmax[s3 + 1], f2ord(h.y));
-    atomicMax(&hmax[s3 + 2], f2ord(h.z));
   }
 }
-
-// static per-slot parameters (LJ radius, sqrt eps, GB radius, Vj)
-__global__ void k_slot_params(DevView v, const double* radius, const double* sqeps, const double* gbR,
-                              const double* gbVj, const double* lcR, const int* lcUse, float4* lc_par) {
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= v.nslots) return;
-  int a = v.sorted_atom[s];
-  float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
-  float4 l = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (a >= 0) {
-    p.x = (float)radius[a];
-    p.y = (float)sqeps[a];
-    if (gbR) {
-      p.z = (float)gbR[a];
-      p.w = (float)gbVj[a];
-    }
-    if (lcR) {
-      l.x = (float)lcR[a];
-      l.y = lcUse[a] ? 1.f : 0.f;
-    }
-  }
-  v.par[s] = p;
-  if (lc_par) lc_par[s] = l;
+// static per-slot parameters (LJ radius, sqrt eps, GB radius, Vj) after a parameter update
+__global__ void k_slot_params(DevView v, SlotParams P) {
+  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s < v.nslots) slot_params(v, P, s, v.sorted_atom[s]);
 }
 
 // ---------------------------------------------------------------------------
 // Tile list.  Block pair (bi, bj), bi <= bj of one system, is a tile when the
 // two blocks' bounding boxes come within R (periodic: at the minimum image of
-// their centres).  Each build bins every system's block centres on a grid of
-// at most one cell per block; row bi visits only the cells within
-// R + h_i + hmax of its centre along each axis (h: half-extents, hmax the
-// system's largest), marks its hits in a per-warp bitmap over its columns
-// bj >= bi, takes its place in the list with one atomic on the tile total and
-// writes its tiles there in ascending bj.  Rows land in any order, each
-// contiguous with ascending columns (what the binary searches, the GB tile
-// pairs and the NB groups rely on); every sum over tiles is in fixed point,
-// so the results do not depend on the rows' order.  A row whose cell range
-// spans the whole grid (all pairs within reach) walks its columns directly.
+// their centres).  One CTA per row bi finds the row's hits in a bitmap over its
+// columns bj >= bi, takes its place in the list with one atomic on the tile total
+// and writes its tiles there in ascending bj.  Rows land in any order, each
+// contiguous with ascending columns (what the work items and the NB groups rely
+// on); every sum over tiles is in fixed point, so the results do not depend on the
+// rows' order.
+//  * Systems of up to kDirectBlocks blocks test every column (32 per warp step).
+//  * Larger ones bin their block centres on a grid of at most one cell per block;
+//    a row visits only the cells within R + h_i + hmax of its centre along each
+//    axis (h: half-extents, hmax the system's largest), so the work follows the
+//    tiles, not the square of the block count.
+// The tiles that need exclusion bits (diagonal, a system's padded last block, a
+// bonded pair) are marked in a second bitmap from the row's atoms' partners and go
+// to a list as they are written.
 // ---------------------------------------------------------------------------
 // box test of one block pair; flags as Tile::flags.  FP32 geometry (the FP64
 // pipe is narrow on this GPU), every decision taken 1e-3 A on the safe side:
@@ -326,15 +436,17 @@ __device__ __forceinline__ bool tile_test(const DevView& v, const SystemInfo& S,
                                           float margin, float full_R, float full_margin, int& flags) {
   const float4 hi4 = v.half[gi], hj4 = v.half[gj];
   const float hs[3] = {hi4.x + hj4.x, hi4.y + hj4.y, hi4.z + hj4.z};
+  const float4 ci4 = v.cenf[gi], cj4 = v.cenf[gj];
+  const float ci[3] = {ci4.x, ci4.y, ci4.z}, cj[3] = {cj4.x, cj4.y, cj4.z};
   constexpr float kSafe = 1e-3f;
   float dist2 = 0.f, dmax2 = 0.f;
   bool need_mi = false;
 #pragma unroll
   for (int c = 0; c < 3; c++) {
-    float d = (float)(v.center[3 * gj + c] - v.center[3 * gi + c]);
+    float d = cj[c] - ci[c];
     if (S.periodic) {
-      const float L = (float)S.box[c];
-      d -= L * rintf(d * (float)S.ibox[c]);
+      const float L = S.boxf[c].h;
+      d -= L * rintf(d / L);
       // a pair of the two blocks inside the cutoff in some other image would
       // sit at least L - R apart along this axis in the tile's image: below
       // that every pair inside the cutoff takes the tile's image, and pairs
@@ -376,59 +488,11 @@ __device__ __forceinline__ void write_tile(const DevView& v, const SystemInfo& S
   v.tiles[t] = T;
 }
 
-// one thread per system: the grid of its block centres for this build
-__global__ void k_grid_setup(DevView v, const int* lo, const int* hi, const int* hmax, BlockGrid* grid) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= v.nsys) return;
-  const SystemInfo& S = v.sys[s];
-  BlockGrid G;
-  double ext[3];
-  for (int c = 0; c < 3; c++) {
-    if (S.periodic) {
-      G.origin[c] = 0.0;
-      ext[c] = S.box[c];
-    } else {
-      const double l = ord2f(lo[3 * s + c]), h = ord2f(hi[3 * s + c]);
-      G.origin[c] = l;
-      ext[c] = fmax(h - l, 1e-3);
-    }
-    G.hmax[c] = ord2f(hmax[3 * s + c]);
-  }
-  // cells of about equal edge, at most grid_cells of them
-  const double edge = cbrt(ext[0] * ext[1] * ext[2] / (double)S.grid_cells);
-  for (int c = 0; c < 3; c++) G.dims[c] = (int)fmax(1.0, fmin(floor(ext[c] / edge), 4096.0));
-  while ((long long)G.dims[0] * G.dims[1] * G.dims[2] > S.grid_cells) {
-    const int m = G.dims[0] >= G.dims[1] ? (G.dims[0] >= G.dims[2] ? 0 : 2) : (G.dims[1] >= G.dims[2] ? 1 : 2);
-    G.dims[m]--;
-  }
-  for (int c = 0; c < 3; c++) G.cell[c] = ext[c] / G.dims[c];
-  G.start = S.grid_start;
-  G.pad = 0.f;
-  grid[s] = G;
-}
-
-// cell coordinate of x along axis c (clamped into the grid)
-__device__ __forceinline__ int grid_axis(const BlockGrid& G, int c, double x) {
-  const double q = floor((x - G.origin[c]) / G.cell[c]);
-  return (int)fmin(fmax(q, 0.0), (double)(G.dims[c] - 1));
-}
-
-__global__ void k_bgrid_count(DevView v, const BlockGrid* grid, int* bcell, int* count) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= v.nblocks) return;
-  const BlockGrid& G = grid[v.slot_sys[b]];
-  const double* x = v.center + 3 * b;
-  const int cell = G.start + (grid_axis(G, 2, x[2]) * G.dims[1] + grid_axis(G, 1, x[1])) * G.dims[0] +
-                   grid_axis(G, 0, x[0]);
-  bcell[b] = cell;
-  atomicAdd(&count[cell], 1);
-}
-
 // blocks in cell order (the order inside a cell does not matter: rows collect
 // their hits in a bitmap)
-__global__ void k_bgrid_scatter(int nblocks, const int* bcell, const int* offset, int* cursor, int* blocks) {
+__global__ void k_bgrid_scatter(DevView v, const int* bcell, const int* offset, int* cursor, int* blocks) {
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= nblocks) return;
+  if (b >= v.nblocks || v.sys[v.slot_sys[b]].nblocks <= kDirectBlocks) return;
   const int cell = bcell[b];
   blocks[offset[cell] + atomicAdd(&cursor[cell], 1)] = b;
 }
@@ -448,101 +512,85 @@ __device__ __forceinline__ int nth_set_bit(unsigned m, int n) {
   return pos;
 }
 
-// the tiles that get an exclusion mask whatever their pairs hold (diagonal, and
-// those with a system's padded last block) and the ones k_mask_mark finds with
-// a bonded pair: each tile once (need: one bit per tile), in the mask list
-__device__ __forceinline__ void mask_list_add(unsigned* need, int* mlist, int* nml, int mask_cap, int t) {
-  const unsigned bit = 1u << (t & 31);
-  // (a plain read first: most marks repeat a tile already in the list)
-  if ((need[t >> 5] & bit) || (atomicOr(&need[t >> 5], bit) & bit)) return;
-  const int k = atomicAdd(nml, 1);
-  if (k < mask_cap) mlist[k] = t;
+constexpr int kRowWarps = 4;
+// marks the row's tiles that hold a bonded pair: each atom of block bi, its
+// partners of either side (band words, far list); the warps take one kind each
+__device__ __forceinline__ void mark_partner(const int* slot_of, int bi, int nw, const unsigned* bits, unsigned* mbits,
+                                             int b) {
+  const int o = (slot_of[b] >> 5) - bi;
+  if (o <= 0 || (o >> 5) >= nw) return;   // (the diagonal is marked anyway; lower rows mark their own)
+  if ((bits[o >> 5] >> (o & 31)) & 1u) atomicOr(&mbits[o >> 5], 1u << (o & 31));
 }
 
-// one warp per row bi, 4 warps per CTA, `words` bitmap words per warp in
-// dynamic shared memory: the row's tiles are found (hits marked in the bitmap),
-// counted, given a place in the list by an atomic on the tile total (rows land
-// in any order, each contiguous with ascending columns) and written there;
-// positions past `cap` are dropped (k_tile_total flags the overflow)
-__global__ void __launch_bounds__(128) k_tile_rows(DevView v, const BlockGrid* grid, const int* cell_off,
-                                                   const int* cell_count, const int* cell_blocks, float R,
-                                                   float margin, float full_R, float full_margin, int* row_cnt,
-                                                   int* row_start, long long cap, int words, int* total,
-                                                   unsigned* need, int* mlist, int* nml) {
+// `words` words of either bitmap in dynamic shared memory; positions past `cap`
+// are dropped (k_masks flags the overflow)
+__global__ void __launch_bounds__(kRowWarps * 32) k_tile_rows(DevView v, const BlockGrid* grid, const int* hmax,
+                                                              const int* cell_off, const int* cell_count,
+                                                              const int* cell_blocks, const int* slot_of, float R,
+                                                              float margin, float full_R, float full_margin,
+                                                              int* row_cnt, int* row_start, long long cap, int words,
+                                                              int* total, int* mlist, int* nml) {
   extern __shared__ unsigned s_bits[];
-  const int lane = threadIdx.x & 31;
-  const int bi = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (bi >= v.nblocks) return;
-  unsigned* bits = s_bits + (threadIdx.x >> 5) * words;
-  const SystemInfo& S = v.sys[v.slot_sys[bi]];
-  const BlockGrid& G = grid[v.slot_sys[bi]];
+  __shared__ int s_cnt[kRowWarps], s_base;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, bi = blockIdx.x;
+  unsigned *bits = s_bits, *mbits = s_bits + words;
+  const int sys = v.slot_sys[bi];
+  const SystemInfo& S = v.sys[sys];
   const int end = S.block_start + S.nblocks;
-  const float4 h4 = v.half[bi];
-  const float h[3] = {h4.x, h4.y, h4.z};
-  int lo[3], hi[3];
-  bool all = true;
-#pragma unroll
-  for (int c = 0; c < 3; c++) {
-    const double x = v.center[3 * bi + c] - G.origin[c];
-    // reach along the axis: list radius, both half-extents, and a slack far
-    // above the rounding of the centres and cell edges
-    const double r = (double)R + (double)h[c] + (double)G.hmax[c] + 0.01;
-    const int D = G.dims[c];
-    int a = (int)fmax(floor((x - r) / G.cell[c]), -1.0e9);
-    int b = (int)fmin(floor((x + r) / G.cell[c]), 1.0e9);
-    if (S.periodic) {
-      if (b - a + 1 >= D) {
-        a = 0;
-        b = D - 1;
-      } else {
-        all = false;
+  const int nw = (end - bi + 31) >> 5;
+  if (S.nblocks <= kDirectBlocks) {
+    for (int w = wid; w < nw; w += kRowWarps) {
+      const int bj = bi + 32 * w + lane;
+      int fl = 0;
+      const unsigned m = __ballot_sync(0xffffffffu, bj < end && tile_test(v, S, bi, bj, R, margin, 0.f, 0.f, fl));
+      if (lane == 0) {
+        bits[w] = m;
+        mbits[w] = w == 0 ? 1u : 0u;   // the diagonal
       }
-    } else {
-      a = max(a, 0);
-      b = min(b, D - 1);
-      if (a > 0 || b < D - 1) all = false;
     }
-    lo[c] = a;
-    hi[c] = b;
-  }
-  const unsigned lt = (1u << lane) - 1u;
-  long long n = 0;   // tiles of the row
-  long long base = 0;
-  if (all) {
-    // count, take the row's place, then write (the test is cheap: no cell walk)
-#pragma unroll 2
-    for (int j0 = bi; j0 < end; j0 += 32) {
-      const int bj = j0 + lane;
-      int fl = 0;
-      n += __popc(__ballot_sync(0xffffffffu, bj < end && tile_test(v, S, bi, bj, R, margin, 0.f, 0.f, fl)));
-    }
-    if (lane == 0) base = atomicAdd(total, (int)n);
-    base = __shfl_sync(0xffffffffu, base, 0);
-    long long w = 0;
-#pragma unroll 2
-    for (int j0 = bi; j0 < end; j0 += 32) {
-      const int bj = j0 + lane;
-      int fl = 0;
-      const bool hit = bj < end && tile_test(v, S, bi, bj, R, margin, full_R, full_margin, fl);
-      const unsigned m = __ballot_sync(0xffffffffu, hit);
-      if (hit) write_tile(v, S, bi, bj, fl, base + w + __popc(m & lt), cap);
-      w += __popc(m);
-    }
+    __syncthreads();
   } else {
-    const int nw = (end - bi + 31) >> 5;
-    for (int w = lane; w < nw; w += 32) bits[w] = 0u;
-    __syncwarp();
+    const BlockGrid& G = grid[sys];
+    const float4 h4 = v.half[bi];
+    const float h[3] = {h4.x, h4.y, h4.z};
+    for (int w = threadIdx.x; w < nw; w += kRowWarps * 32) {
+      bits[w] = 0u;
+      mbits[w] = w == 0 ? 1u : 0u;
+    }
+    __syncthreads();
+    int lo[3], hi[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      const double x = v.center[3 * bi + c] - G.origin[c];
+      // reach along the axis: list radius, both half-extents, and a slack far
+      // above the rounding of the centres and cell edges
+      const double r = (double)R + (double)h[c] + (double)ord2f(hmax[3 * sys + c]) + 0.01;
+      const int D = G.dims[c];
+      int a = (int)fmax(floor((x - r) / G.cell[c]), -1.0e9);
+      int b = (int)fmin(floor((x + r) / G.cell[c]), 1.0e9);
+      if (S.periodic) {
+        if (b - a + 1 >= D) {
+          a = 0;
+          b = D - 1;
+        }
+      } else {
+        a = max(a, 0);
+        b = min(b, D - 1);
+      }
+      lo[c] = a;
+      hi[c] = b;
+    }
     // the cell runs to visit: one per (y, z) cell row of the range, two where
-    // a periodic x range wraps.  Each lane reads one run's block range, then
-    // the warp deals the runs' blocks over its lanes (the reads of a row are
-    // independent of one another, not a chain of dependent loads)
+    // a periodic x range wraps, dealt over the warps.  Each lane reads one run's
+    // block range, then the warp deals the runs' blocks over its lanes (the reads
+    // of a row are independent of one another, not a chain of dependent loads)
     const int Dx = G.dims[0], Dy = G.dims[1], Dz = G.dims[2];
     const int nyr = hi[1] - lo[1] + 1, nzr = hi[2] - lo[2] + 1;
     const bool wrapx = lo[0] < 0 || hi[0] >= Dx;
     const int nxr = wrapx ? 2 : 1;
     const int nrun = nyr * nzr * nxr;
-    for (int q0 = 0; q0 < nrun; q0 += 32) {
-      const int q = q0 + lane;
+    for (int q0 = 0; q0 < nrun; q0 += 32 * kRowWarps) {
+      const int q = q0 + lane * kRowWarps + wid;
       int p0 = 0, len = 0;
       if (q < nrun) {
         const int xr = q % nxr, yz = q / nxr;
@@ -559,12 +607,7 @@ __global__ void __launch_bounds__(128) k_tile_rows(DevView v, const BlockGrid* g
         p0 = cell_off[row0 + c0];
         len = cell_off[row0 + c1] + cell_count[row0 + c1] - p0;
       }
-      int inc = len;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= o) inc += t;
-      }
+      const int inc = warp_inclusive_scan(len, lane);
       const int cnt = __shfl_sync(0xffffffffu, inc, 31);
       const int excl = inc - len;
       for (int t0 = 0; t0 < cnt; t0 += 32) {
@@ -583,113 +626,89 @@ __global__ void __launch_bounds__(128) k_tile_rows(DevView v, const BlockGrid* g
         }
       }
     }
-    __syncwarp();
-    int k = 0;
-    for (int w = lane; w < nw; w += 32) k += __popc(bits[w]);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) k += __shfl_xor_sync(0xffffffffu, k, o);
-    n = k;
-    if (lane == 0) base = atomicAdd(total, (int)n);
-    base = __shfl_sync(0xffffffffu, base, 0);
-    long long done = 0;
-    for (int w0 = 0; w0 < nw; w0 += 32) {
-      const int w = w0 + lane;
-      const unsigned word = w < nw ? bits[w] : 0u;
-      const int kw = __popc(word);
-      int inc = kw;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= o) inc += t;
-      }
-      const int tot = __shfl_sync(0xffffffffu, inc, 31);
-      // the hits of these 32 words dealt over the lanes, in column order
-      const int excl = inc - kw;
-      for (int t0 = 0; t0 < tot; t0 += 32) {
-        const int t = t0 + lane;
-        int L = 0;
-#pragma unroll
-        for (int b = 16; b > 0; b >>= 1)
-          if (__shfl_sync(0xffffffffu, excl, L + b) <= t) L += b;
-        const unsigned wl = __shfl_sync(0xffffffffu, word, L);
-        const int nth = t - __shfl_sync(0xffffffffu, excl, L);
-        if (t < tot) {
-          const int bj = bi + 32 * (w0 + L) + nth_set_bit(wl, nth);
-          int fl = 0;
-          tile_test(v, S, bi, bj, R, margin, full_R, full_margin, fl);
-          write_tile(v, S, bi, bj, fl, base + done + t, cap);
-        }
-      }
-      done += tot;
+    __syncthreads();
+  }
+  // tiles that get an exclusion mask
+  const int a = v.sorted_atom[bi * 32 + lane];
+  if (a >= 0) {
+    if (wid == 0) {
+      for (unsigned long long m = v.band_excl[a] | v.band_14[a]; m; m &= m - 1)
+        mark_partner(slot_of, bi, nw, bits, mbits, a + __ffsll((long long)m));
+    } else if (wid == 1) {
+      for (unsigned long long m = v.band_down[a]; m; m &= m - 1)
+        mark_partner(slot_of, bi, nw, bits, mbits, a - __ffsll((long long)m));
+    } else if (wid == 2) {
+      for (int q = v.far_both_start[a]; q < v.far_both_start[a + 1]; q++)
+        mark_partner(slot_of, bi, nw, bits, mbits, v.far_both_idx[q]);
     }
   }
-  if (lane == 0) {
-    row_start[bi] = (int)base;
-    row_cnt[bi] = (int)n;
-    // the diagonal tile is the row's first; a tile with the system's padded
-    // last block, its last
-    if (base < cap) mask_list_add(need, mlist, nml, v.mask_cap, (int)base);
-    const int last = end - 1;
-    int fl;
-    if (S.natom != S.npad && bi != last && n > 1 && base + n - 1 < cap &&
-        tile_test(v, S, bi, last, R, margin, 0.f, 0.f, fl))
-      mask_list_add(need, mlist, nml, v.mask_cap, (int)(base + n - 1));
+  if (threadIdx.x == kRowWarps * 32 - 1 && S.natom != S.npad) {   // the system's padded last block
+    const int o = end - 1 - bi;
+    if ((bits[o >> 5] >> (o & 31)) & 1u) atomicOr(&mbits[o >> 5], 1u << (o & 31));
   }
-}
-
-// the tile count from the rows' total, clamped to the capacity (an overflow
-// leaves a short list and is flagged)
-__global__ void k_tile_total(DevView v, const int* total, long long cap) {
-  const long long t = *total;
-  *v.ntiles = (int)(t < cap ? t : cap);
-  v.cull_n[2] = 1;   // (the groups fit until a row finds they do not)
-  if (t > cap) atomicOr(v.status, (unsigned)ST_TILE_OVERFLOW);
-}
-
-// index of tile (bi, bj) in the list (rows contiguous, ascending columns), -1 if absent
-__device__ __forceinline__ int tile_index(const DevView& v, const int* row_start, const int* row_cnt, int bi, int bj) {
-  const int nt = *v.ntiles;
-  int lo = row_start[bi], hi = min(lo + row_cnt[bi], nt) - 1;
-  while (lo <= hi) {
-    const int mid = (lo + hi) >> 1;
-    const int c = v.tiles[mid].bj;
-    if (c == bj) return mid;
-    if (c < bj) lo = mid + 1;
-    else hi = mid - 1;
+  // each warp writes a run of the words; the row's place by one atomic
+  const int per = (nw + kRowWarps - 1) / kRowWarps;
+  const int wa = min(wid * per, nw), wb = min(wa + per, nw);
+  int k = 0;
+  for (int w = wa + lane; w < wb; w += 32) k += __popc(bits[w]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) k += __shfl_xor_sync(0xffffffffu, k, o);
+  if (lane == 0) s_cnt[wid] = k;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int n = 0;
+    for (int w = 0; w < kRowWarps; w++) n += s_cnt[w];
+    s_base = atomicAdd(total, n);
+    row_start[bi] = s_base;
+    row_cnt[bi] = n;
   }
-  return -1;
-}
-
-// exclusion masks in rotation order (bit k <-> j slot (lane+k)&31); one warp per tile
-// tiles holding a bonded pair (bond order <= 3: excluded or 1-4), found from
-// each atom's partners (band words, far list) and added to the mask list
-__global__ void k_mask_mark(DevView v, const int* slot_of, const int* row_start, const int* row_cnt,
-                            unsigned* need, int* mlist, int* nml) {
-  const int a = blockIdx.x * blockDim.x + threadIdx.x;
-  if (a >= v.natom) return;
-  const unsigned long long w = v.band_excl[a] | v.band_14[a];
-  const int fs = v.far_start[a], fe = v.far_start[a + 1];
-  if (!w && fs == fe) return;
-  const int ga = slot_of[a] >> 5;
-  int last = ga;
-  auto mark = [&](int b) {
-    const int gb = slot_of[b] >> 5;
-    // (diagonal tiles are in the list already; partners of one block come in runs)
-    if (gb == last || gb == ga) return;
-    last = gb;
-    const int t = tile_index(v, row_start, row_cnt, ga < gb ? ga : gb, ga < gb ? gb : ga);
-    if (t >= 0) mask_list_add(need, mlist, nml, v.mask_cap, t);
-  };
-  for (unsigned long long m = w; m; m &= m - 1) mark(a + __ffsll((long long)m));
-  for (int q = fs; q < fe; q++)
-    if (v.far_bo[q] <= 3) mark(v.far_idx[q]);
+  __syncthreads();
+  long long base = s_base;
+  for (int w = 0; w < wid; w++) base += s_cnt[w];
+  for (int w0 = wa; w0 < wb; w0 += 32) {
+    const int w = w0 + lane;
+    const unsigned word = w < wb ? bits[w] : 0u;
+    const int kw = __popc(word);
+    const int inc = warp_inclusive_scan(kw, lane);
+    const int tot = __shfl_sync(0xffffffffu, inc, 31);
+    // the hits of these 32 words dealt over the lanes, in column order
+    const int excl = inc - kw;
+    for (int t0 = 0; t0 < tot; t0 += 32) {
+      const int t = t0 + lane;
+      int L = 0;
+#pragma unroll
+      for (int b = 16; b > 0; b >>= 1)
+        if (__shfl_sync(0xffffffffu, excl, L + b) <= t) L += b;
+      const unsigned wl = __shfl_sync(0xffffffffu, word, L);
+      const int nth = t - __shfl_sync(0xffffffffu, excl, L);
+      if (t < tot) {
+        const int bit = nth_set_bit(wl, nth);
+        const int bj = bi + 32 * (w0 + L) + bit;
+        int fl = 0;
+        tile_test(v, S, bi, bj, R, margin, full_R, full_margin, fl);
+        write_tile(v, S, bi, bj, fl, base + t, cap);
+        if (base + t < cap && ((mbits[w0 + L] >> bit) & 1u)) {
+          const int q = atomicAdd(nml, 1);
+          if (q < v.mask_cap) mlist[q] = (int)(base + t);
+        }
+      }
+    }
+    base += tot;
+  }
 }
 
 // one warp per tile of the mask list (grid-stride): the tile's exclusion and
 // 1-4 bits, a mask table entry when any is set
-__global__ void k_masks(DevView v, const int* mlist, const int* nml) {
+// (also the tile count from the rows' total, clamped to the capacity: an overflow
+// leaves a short list and is flagged)
+__global__ void k_masks(DevView v, const int* mlist, const int* nml, const int* total, long long cap) {
   const int lane = threadIdx.x & 31;
   const int n = min(*nml, v.mask_cap);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    const long long t = *total;
+    *v.ntiles = (int)(t < cap ? t : cap);
+    if (t > cap) atomicOr(v.status, (unsigned)ST_TILE_OVERFLOW);
+  }
   if (*nml > v.mask_cap && blockIdx.x == 0 && threadIdx.x == 0) atomicOr(v.status, (unsigned)ST_TILE_OVERFLOW);
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   for (int e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; e < n; e += nwarps) {
@@ -755,90 +774,71 @@ __global__ void k_masks(DevView v, const int* mlist, const int* nml) {
   }
 }
 
-// per-evaluation pack: FP64 positions -> float offsets from the block centre
+// per-evaluation pack (between list builds): the slots at the current positions
 // check2: squared skin limit (0 = no skin check); full2: squared limit that keeps
 // tiles flagged full valid (0 = none flagged), checked where the skin check is not
 // cull: the NB j-atom groups are in use (the displacement check always runs)
-// sub: also write the boxes of each 8 slots (for the groups)
-__global__ void k_pack(DevView v, const double* charge, float check2, float full2, int store_ref,
-                       long long npairs_all, int cull, int sub) {
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= v.nslots) return;
-  int a = v.sorted_atom[s];
-  int b = s >> 5;
-  float4 o;
-  if (a < 0) {
-    // padding slot: zero parameters, parked far away from everything and each other
-    o = make_float4(1.0e6f * (float)(1 + (s & 31)), 1.0e6f * (float)(1 + (s >> 5)), -1.0e6f, 0.f);
-  } else {
-    const SystemInfo& S = v.sys[v.slot_sys[b]];
-    double r[3];
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-      double d = v.pos[3 * a + c] - v.center[3 * b + c];
-      if (S.periodic) d -= S.box[c] * rint(d * S.ibox[c]);
-      r[c] = d;
-    }
-    o = make_float4((float)r[0], (float)r[1], (float)r[2], (float)charge[a]);
-    if (store_ref) {
-      v.rel0[s] = o;
-    } else {
-      // (in open space, when every block pair of every system is a tile, no pair
-      // can leave the list; in a periodic box the tile images still depend on it)
-      const bool skin = check2 > 0.f && (S.periodic || (long long)*v.ntiles < npairs_all || cull);
-      const float lim = skin ? check2 : full2;
-      if (lim > 0.f) {
-        float4 q = v.rel0[s];
-        float dx = o.x - q.x, dy = o.y - q.y, dz = o.z - q.z;
-        if (dx * dx + dy * dy + dz * dz > lim) atomicOr(v.status, (unsigned)ST_STALE_LIST);
-      }
+__global__ void k_pack(DevView v, const double* charge, float check2, float full2, long long npairs_all, int cull) {
+  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= v.nslots) return;   // (whole warps)
+  const int a = v.sorted_atom[s], b = s >> 5;
+  const SystemInfo& S = v.sys[v.slot_sys[b]];
+  const double c[3] = {v.center[3 * b], v.center[3 * b + 1], v.center[3 * b + 2]};
+  const float4 o = packed_slot(v, S, charge, s, a, c);
+  if (a >= 0) {
+    // (in open space, when every block pair of every system is a tile, no pair
+    // can leave the list; in a periodic box the tile images still depend on it)
+    const bool skin = check2 > 0.f && (S.periodic || (long long)*v.ntiles < npairs_all || cull);
+    const float lim = skin ? check2 : full2;
+    if (lim > 0.f) {
+      float4 q = v.rel0[s];
+      float dx = o.x - q.x, dy = o.y - q.y, dz = o.z - q.z;
+      if (dx * dx + dy * dy + dz * dz > lim) atomicOr(v.status, (unsigned)ST_STALE_LIST);
     }
   }
   v.xq[s] = o;
-  if (sub) {
-    // boxes of each 8 slots (a padding slot widens its box: it never hides an atom)
-    float4 lo = o, hi = o;
-#pragma unroll
-    for (int d = 4; d > 0; d >>= 1) {
-      lo.x = fminf(lo.x, __shfl_xor_sync(0xffffffffu, lo.x, d));
-      lo.y = fminf(lo.y, __shfl_xor_sync(0xffffffffu, lo.y, d));
-      lo.z = fminf(lo.z, __shfl_xor_sync(0xffffffffu, lo.z, d));
-      hi.x = fmaxf(hi.x, __shfl_xor_sync(0xffffffffu, hi.x, d));
-      hi.y = fmaxf(hi.y, __shfl_xor_sync(0xffffffffu, hi.y, d));
-      hi.z = fmaxf(hi.z, __shfl_xor_sync(0xffffffffu, hi.z, d));
+  if (cull) write_sub(v, s, o);
+}
+
+// GB work items, one warp per row: the row's all-inside tiles without exclusion
+// mask go together two by two in column order (a pairing that does not depend on
+// the other systems of a batch), every other tile is an item of its own; the row's
+// items take their place by an atomic on the total (any order: every sum is in
+// fixed point).  pairs: 0 makes every item a single tile
+__global__ void __launch_bounds__(128) k_items(DevView v, int pairs, const int* row_start, const int* row_cnt) {
+  const int lane = threadIdx.x & 31, b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (b >= v.nblocks) return;
+  const int t0 = row_start[b], n = max(min(row_cnt[b], *v.ntiles - t0), 0);
+  int np = 0;
+  for (int i = 0; i < n; i += 32) {
+    bool p = false;
+    if (pairs && i + lane < n) {
+      const Tile T = v.tiles[t0 + i + lane];
+      p = tile_full(T) && !tile_masked(T) && !(T.flags & 1);
     }
-    if ((s & 7) == 0) {
-      v.sub[s >> 2] = lo;
-      v.sub[(s >> 2) + 1] = hi;
-    }
+    np += __popc(__ballot_sync(0xffffffffu, p));
   }
-}
-
-// GB work items: tiles t and t + 1 go together when they share the row, sit in
-// adjacent columns with bj - bi odd for the first (a fixed pairing that does not
-// depend on the other systems of a batch), are both unmasked and off-diagonal,
-// need no per-pair image and agree on the all-inside flag
-__device__ __forceinline__ bool tile_pairable(const DevView& v, int t, int nt) {
-  if (t < 0 || t + 1 >= nt) return false;
-  const Tile A = v.tiles[t], B = v.tiles[t + 1];
-  return A.bi == B.bi && B.bj == A.bj + 1 && ((A.bj - A.bi) & 1) && !tile_masked(A) && !tile_masked(B) &&
-         tile_full(A) == tile_full(B) && !((A.flags | B.flags) & 1);
-}
-
-// pairs: 0 makes every item a single tile
-__global__ void k_item_flags(DevView v, long long cap, int pairs, int* flag) {
-  long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= cap) return;
-  const int nt = *v.ntiles;
-  flag[t] = (t < nt && !(pairs && tile_pairable(v, (int)t - 1, nt))) ? 1 : 0;
-}
-
-__global__ void k_item_write(DevView v, long long cap, int pairs, const int* flag, const int* pos) {
-  long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= cap) return;
-  if (t == cap - 1) *v.nitems = pos[t] + flag[t];
-  if (!flag[t]) return;
-  v.items[pos[t]] = (unsigned)t | ((pairs && tile_pairable(v, (int)t, *v.ntiles)) ? 0x80000000u : 0u);
+  int base = 0;
+  if (lane == 0) base = atomicAdd(v.nitems, (np + 1) / 2 + n - np);
+  base = __shfl_sync(0xffffffffu, base, 0);
+  if (lane == 0 && (np & 1)) v.items[base + np / 2].y = -1;   // the last one stays alone
+  int* two = reinterpret_cast<int*>(v.items + base);
+  int2* one = v.items + base + (np + 1) / 2;
+  int rp = 0, rs = 0;
+  const unsigned lt = (1u << lane) - 1u;
+  for (int i = 0; i < n; i += 32) {
+    const bool in = i + lane < n;
+    bool p = false;
+    if (pairs && in) {
+      const Tile T = v.tiles[t0 + i + lane];
+      p = tile_full(T) && !tile_masked(T) && !(T.flags & 1);
+    }
+    const unsigned mp = __ballot_sync(0xffffffffu, p), ms = __ballot_sync(0xffffffffu, in && !p);
+    if (p) two[rp + __popc(mp & lt)] = t0 + i + lane;
+    else if (in) one[rs + __popc(ms & lt)] = make_int2(t0 + i + lane, -1);
+    rp += __popc(mp);
+    rs += __popc(ms);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -857,7 +857,7 @@ __global__ void k_item_write(DevView v, long long cap, int pairs, const int* fla
 // by an atomic on the total (rows in any order: every sum is in fixed point) and
 // write.  A row's groups are an even number (the force pass takes two at once).
 // ---------------------------------------------------------------------------
-constexpr int kCullWarps = 4;
+constexpr int kCullWarps = 8;
 __global__ void __launch_bounds__(kCullWarps * 32) k_cull(DevView v, float R2, float Rc2, const int* row_start,
                                                           const int* row_cnt, uint2* jmask) {
   __shared__ int cnt[2][kCullWarps];
@@ -941,7 +941,8 @@ static int list_tile_grid(const Context& c) {
 static void scan_ints(Context& c, const int* in, int* out, int* tmp, long long n, cudaStream_t st) {
   c.kernel_launches += n <= kScanOne ? 1 : 3;
   if (n <= kScanOne) {
-    k_scan_one<<<1, 1024, 0, st>>>(in, out, (int)n);
+    if (n <= 8192) k_scan_one<8><<<1, 1024, 0, st>>>(in, out, (int)n);
+    else k_scan_one<32><<<1, 1024, 0, st>>>(in, out, (int)n);
     return;
   }
   const int nb = nblk(n, 1024);
@@ -957,103 +958,132 @@ static void launch_cull(Context& c, float list_radius) {
                                                       c.d_cull_mask.p);
 }
 
-// rows of the tile-list build: 4 warps per CTA, a bitmap over each warp's row
-// (the row total, the mask list and the need bits zeroed beforehand)
-static void launch_rows(Context& c, float R, float full_radius) {
-  const int words = (c.max_sys_blocks + 31) / 32 + 1;
-  const size_t smem = (size_t)4 * words * sizeof(unsigned);
-  DevView v = c.view();
-  const int g = nblk((long long)c.nblocks * 32, 128);
-  int* cnt = c.d_counters.p;
-  cudaMemsetAsync(cnt + 6, 0, 2 * sizeof(int), c.stream);
-  cudaMemsetAsync(c.d_tile_need.p, 0, sizeof(unsigned) * c.d_tile_need.n, c.stream);
-  k_tile_rows<<<g, 128, smem, c.stream>>>(v, c.d_bgrid.p, c.d_bcell_off.p, c.d_bcell_count.p, c.d_bcell_blocks.p, R,
-                                          (float)c.lp.Padding, full_radius, c.full_margin(), c.d_row_cnt.p,
-                                          c.d_row_start.p, c.tile_cap, words, cnt + 6, c.d_tile_need.p,
-                                          c.d_mlist.p, cnt + 7);
+// the overflow flag of a build about to be repeated into grown arrays
+__global__ void k_clear_status(unsigned* status, unsigned bits) { atomicAnd(status, ~bits); }
+static int clear_tile_overflow(Context& c) {
+  c.kernel_launches += 1;
+  k_clear_status<<<1, 1, 0, c.stream>>>(c.d_status.p, (unsigned)ST_TILE_OVERFLOW);
+  return cudaGetLastError() == cudaSuccess ? PDGPU_OK : PDGPU_ERR_CUDA;
 }
 
-int launch_list_build(Context& c, float list_radius, float full_radius, ListSizing sizing) {
-  c.kernel_launches += 16;   // and two scans
-  DevView v = c.view();
+static void launch_rows(Context& c, float R, float full_radius) {
+  const int words = (c.max_sys_blocks + 31) / 32 + 1;
+  const size_t smem = (size_t)2 * words * sizeof(unsigned);
+  int* cnt = c.d_counters.p;
+  k_tile_rows<<<c.nblocks, kRowWarps * 32, smem, c.stream>>>(
+      c.view(), c.d_bgrid.p, reinterpret_cast<int*>(c.d_sys_hmax.p), c.d_bcell_off.p, c.d_bcell_count.p,
+      c.d_bcell_blocks.p, c.d_slot_of.p, R, (float)c.lp.Padding, full_radius, c.full_margin(), c.d_row_cnt.p,
+      c.d_row_start.p, c.tile_cap, words, cnt + 6, c.d_mlist.p, cnt + 7);
+}
+
+static SlotParams slot_param_view(const Context& c) {
+  SlotParams P;
+  P.radius = c.d_radius.p;
+  P.sqeps = c.d_sqeps.p;
+  P.gbR = c.has_gb ? c.d_gbR.p : nullptr;
+  P.gbVj = c.has_gb ? c.d_gbVj.p : nullptr;
+  P.lcR = c.has_sa ? c.d_lcpoR.p : nullptr;
+  P.lcUse = c.has_sa ? c.d_lcpoUse.p : nullptr;
+  P.lc_par = c.has_sa ? c.d_lc_par.p : nullptr;
+  P.charge = c.d_charge.p;
+  return P;
+}
+
+// the part of a build after its rows: masks, GB work items, NB groups
+static void launch_list_tail(Context& c, float list_radius) {
   cudaStream_t st = c.stream;
-  int ncells = c.nsys * kCellsPerSystem;
-  int* lo = reinterpret_cast<int*>(c.d_sys_lo.p);
-  int* hi = reinterpret_cast<int*>(c.d_sys_hi.p);
-  int* hmax = reinterpret_cast<int*>(c.d_sys_hmax.p);
-  k_bbox_init<<<nblk(3 * c.nsys, 128), 128, 0, st>>>(lo, hi, hmax, 3 * c.nsys);
-  k_bbox<<<nblk(c.natom, 256), 256, 0, st>>>(v, c.d_atom_sys.p, lo, hi);
-  cudaMemsetAsync(c.d_count.p, 0, sizeof(int) * ncells, st);
-  cudaMemsetAsync(c.d_cursor.p, 0, sizeof(int) * ncells, st);
-  k_keys<<<nblk(c.natom, 256), 256, 0, st>>>(v, c.d_atom_sys.p, lo, hi, c.d_bucket.p, c.d_count.p);
-  scan_ints(c, c.d_count.p, c.d_offset.p, c.d_scan_tmp.p, ncells, st);
-  k_scatter<<<nblk(c.natom, 256), 256, 0, st>>>(c.natom, c.d_bucket.p, c.d_offset.p, c.d_cursor.p,
-                                                 c.d_tmp_sorted.p);
-  k_cell_sort<<<nblk(ncells, 256), 256, 0, st>>>(ncells, c.d_offset.p, c.d_count.p, c.d_tmp_sorted.p);
-  cudaMemsetAsync(c.d_sorted_atom.p, 0xff, sizeof(int) * c.nslots, st);
-  k_to_slots<<<nblk(c.natom, 256), 256, 0, st>>>(v, c.d_atom_sys.p, c.d_tmp_sorted.p, c.d_sorted_atom.p,
-                                                  c.d_slot_of.p);
-  k_blocks<<<nblk((long long)c.nblocks * 32, 256), 256, 0, st>>>(v, hmax);
-  k_slot_params<<<nblk(c.nslots, 256), 256, 0, st>>>(v, c.d_radius.p, c.d_sqeps.p, c.has_gb ? c.d_gbR.p : nullptr,
-                                                      c.has_gb ? c.d_gbVj.p : nullptr,
-                                                      c.has_sa ? c.d_lcpoR.p : nullptr,
-                                                      c.has_sa ? c.d_lcpoUse.p : nullptr,
-                                                      c.has_sa ? c.d_lc_par.p : nullptr);
-  // block grid and the row counts of the tile list
-  k_grid_setup<<<nblk(c.nsys, 64), 64, 0, st>>>(v, lo, hi, hmax, c.d_bgrid.p);
-  cudaMemsetAsync(c.d_bcell_count.p, 0, sizeof(int) * c.nblocks, st);
-  cudaMemsetAsync(c.d_bcell_cursor.p, 0, sizeof(int) * c.nblocks, st);
-  k_bgrid_count<<<nblk(c.nblocks, 256), 256, 0, st>>>(v, c.d_bgrid.p, c.d_bcell.p, c.d_bcell_count.p);
-  scan_ints(c, c.d_bcell_count.p, c.d_bcell_off.p, c.d_bcell_scan_tmp.p, c.nblocks, st);
-  k_bgrid_scatter<<<nblk(c.nblocks, 256), 256, 0, st>>>(c.nblocks, c.d_bcell.p, c.d_bcell_off.p,
-                                                         c.d_bcell_cursor.p, c.d_bcell_blocks.p);
-  launch_rows(c, list_radius, full_radius);
-  if (sizing != kListDevice) {
-    // the tile count against the capacity: a list that outgrew the arrays is
-    // rebuilt into grown ones
-    int total = 0;
-    if (cudaMemcpyAsync(&total, c.d_counters.p + 6, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-        cudaStreamSynchronize(st) != cudaSuccess)
-      return PDGPU_ERR_CUDA;
-    if (total > c.tile_cap) {
-      if (sizing == kListCheck) return PDGPU_ERR_CAPACITY;
-      const int e = alloc_tiles(c, total);
-      if (e != PDGPU_OK) return e;
-      v = c.view();
-      c.kernel_launches += 1;
-      launch_rows(c, list_radius, full_radius);
-    }
-  }
-  cudaMemsetAsync(c.d_counters.p, 0, sizeof(int) * 6, st);
-  k_tile_total<<<1, 1, 0, st>>>(v, c.d_counters.p + 6, c.tile_cap);
-  k_mask_mark<<<nblk(c.natom, 256), 256, 0, st>>>(v, c.d_slot_of.p, c.d_row_start.p, c.d_row_cnt.p,
-                                                   c.d_tile_need.p, c.d_mlist.p, c.d_counters.p + 7);
-  k_masks<<<nblk((long long)c.mask_cap * 32, 256) < list_tile_grid(c) ? nblk((long long)c.mask_cap * 32, 256)
-                                                                       : list_tile_grid(c),
-            256, 0, st>>>(v, c.d_mlist.p, c.d_counters.p + 7);
+  int* cnt = c.d_counters.p;
+  c.kernel_launches += 1;
+  const int gm = nblk((long long)c.mask_cap * 32, 256), gt = list_tile_grid(c);
+  k_masks<<<gm < gt ? gm : gt, 256, 0, st>>>(c.view(), c.d_mlist.p, cnt + 7, cnt + 6, c.tile_cap);
   if (c.has_gb) {
-    c.kernel_launches += 2;   // and a scan
-    const int pairs = c.gb_item_tiles == 2 ? 1 : 0;
-    k_item_flags<<<nblk(c.tile_cap, 256), 256, 0, st>>>(v, c.tile_cap, pairs, c.d_tile_flag.p);
-    scan_ints(c, c.d_tile_flag.p, c.d_tile_pos.p, c.d_scan_tmp2.p, c.tile_cap, st);
-    k_item_write<<<nblk(c.tile_cap, 256), 256, 0, st>>>(v, c.tile_cap, pairs, c.d_tile_flag.p, c.d_tile_pos.p);
+    c.kernel_launches += 1;
+    k_items<<<nblk(c.nblocks, 4), 128, 0, st>>>(c.view(), c.gb_item_tiles == 2 ? 1 : 0, c.d_row_start.p,
+                                                c.d_row_cnt.p);
   }
-  k_pack<<<nblk(c.nslots, 256), 256, 0, st>>>(v, c.d_charge.p, 0.f, 0.f, 1, c.npairs_all, 0, c.nb_set ? 1 : 0);
   // NB j-atom groups: only where the per-step displacement check runs
   c.cull_built = c.nb_set && c.nb_cull && c.lp.check_skin && c.cull_cap > 0;
   if (c.cull_built) launch_cull(c, list_radius);
+}
+
+int launch_list_build(Context& c, float list_radius, float full_radius, ListSizing sizing) {
+  c.kernel_launches += 6;   // and a scan
+  DevView v = c.view();
+  cudaStream_t st = c.stream;
+  const int ncells = c.nsys * kCellsPerSystem;
+  int* lo = reinterpret_cast<int*>(c.d_sys_lo.p);
+  int* hi = reinterpret_cast<int*>(c.d_sys_hi.p);
+  int* hmax = reinterpret_cast<int*>(c.d_sys_hmax.p);
+  const bool grid = c.max_sys_blocks > kDirectBlocks;
+  ListInit I;
+  I.count = c.d_count.p;
+  I.cursor = c.d_cursor.p;
+  I.sorted_atom = c.d_sorted_atom.p;
+  I.bcell_count = c.d_bcell_count.p;
+  I.bcell_cursor = c.d_bcell_cursor.p;
+  I.lo = lo;
+  I.hi = hi;
+  I.hmax = hmax;
+  I.counters = c.d_counters.p;
+  I.ncells = ncells;
+  I.nslots = c.nslots;
+  I.nbcells = grid ? c.nblocks : 0;
+  I.nsys3 = 3 * c.nsys;
+  k_list_init<<<std::min(nblk(std::max(ncells, c.nslots), 256), 1216), 256, 0, st>>>(I);
+  if (!c.all_periodic) {
+    c.kernel_launches += 1;
+    k_bbox<<<nblk(c.natom, 256), 256, 0, st>>>(v, c.d_atom_sys.p, lo, hi);
+  }
+  k_keys<<<nblk(c.natom, 256) + (grid ? 1 : 0), 256, 0, st>>>(v, c.d_atom_sys.p, lo, hi, c.d_bucket.p, c.d_count.p,
+                                                              grid ? c.d_bgrid.p : nullptr);
+  scan_ints(c, c.d_count.p, c.d_offset.p, c.d_scan_tmp.p, ncells, st);
+  k_scatter<<<nblk(c.natom, 256), 256, 0, st>>>(c.natom, c.d_bucket.p, c.d_offset.p, c.d_cursor.p,
+                                                 c.d_tmp_sorted.p);
+  k_cell_sort<<<nblk(ncells, 256), 256, 0, st>>>(v, ncells, c.d_offset.p, c.d_count.p, c.d_tmp_sorted.p,
+                                                 c.d_sorted_atom.p, c.d_slot_of.p);
+  k_blocks<<<nblk((long long)c.nblocks * 32, 128), 128, 0, st>>>(v, slot_param_view(c), c.d_bgrid.p, hmax, c.d_bcell.p,
+                                                                 c.d_bcell_count.p, c.nb_set ? 1 : 0);
+  if (grid) {
+    c.kernel_launches += 1;   // and a scan
+    scan_ints(c, c.d_bcell_count.p, c.d_bcell_off.p, c.d_bcell_scan_tmp.p, c.nblocks, st);
+    k_bgrid_scatter<<<nblk(c.nblocks, 256), 256, 0, st>>>(v, c.d_bcell.p, c.d_bcell_off.p, c.d_bcell_cursor.p,
+                                                           c.d_bcell_blocks.p);
+  }
+  launch_rows(c, list_radius, full_radius);
+  if (sizing != kListDevice) {
+    // the tile count against the capacity: a list that outgrew the arrays is
+    // rebuilt into grown ones.  The rest of the build is queued behind the copy of
+    // the count, so the GPU works on while the host waits for it (a list that did
+    // not fit is cut to the capacity, and the rest runs again after the growth)
+    if (cudaMemcpyAsync(c.h_total, c.d_counters.p + 6, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+        cudaEventRecord(c.ev_total, st) != cudaSuccess)
+      return PDGPU_ERR_CUDA;
+    if (c.tile_cap > 0) launch_list_tail(c, list_radius);
+    if (cudaEventSynchronize(c.ev_total) != cudaSuccess) return PDGPU_ERR_CUDA;
+    const int total = *c.h_total;
+    if (total > c.tile_cap) {
+      // (the overflow of the arrays just outgrown is no error of this build)
+      if (clear_tile_overflow(c) != PDGPU_OK) return PDGPU_ERR_CUDA;
+      if (sizing == kListCheck) return PDGPU_ERR_CAPACITY;
+      if (cudaStreamSynchronize(st) != cudaSuccess) return PDGPU_ERR_CUDA;
+      const int e = alloc_tiles(c, total);
+      if (e != PDGPU_OK) return e;
+      c.kernel_launches += 1;
+      ListInit J{};
+      J.counters = c.d_counters.p;
+      k_list_init<<<1, 32, 0, st>>>(J);
+      launch_rows(c, list_radius, full_radius);
+      launch_list_tail(c, list_radius);
+    }
+  } else {
+    launch_list_tail(c, list_radius);
+  }
   return cudaGetLastError() == cudaSuccess ? PDGPU_OK : PDGPU_ERR_CUDA;
 }
 
 int launch_slot_params(Context& c) {
   c.kernel_launches += 1;
-  DevView v = c.view();
-  k_slot_params<<<nblk(c.nslots, 256), 256, 0, c.stream>>>(v, c.d_radius.p, c.d_sqeps.p,
-                                                            c.has_gb ? c.d_gbR.p : nullptr,
-                                                            c.has_gb ? c.d_gbVj.p : nullptr,
-                                                            c.has_sa ? c.d_lcpoR.p : nullptr,
-                                                            c.has_sa ? c.d_lcpoUse.p : nullptr,
-                                                            c.has_sa ? c.d_lc_par.p : nullptr);
+  k_slot_params<<<nblk(c.nslots, 256), 256, 0, c.stream>>>(c.view(), slot_param_view(c));
   return cudaGetLastError() == cudaSuccess ? PDGPU_OK : PDGPU_ERR_CUDA;
 }
 
@@ -1066,8 +1096,7 @@ int launch_pack(Context& c, float check_disp) {
     const float h = 0.5f * c.full_margin();
     f2 = h * h;
   }
-  k_pack<<<nblk(c.nslots, 256), 256, 0, c.stream>>>(v, c.d_charge.p, c2, f2, 0, c.npairs_all,
-                                                     c.cull_built ? 1 : 0, c.cull_built ? 1 : 0);
+  k_pack<<<nblk(c.nslots, 256), 256, 0, c.stream>>>(v, c.d_charge.p, c2, f2, c.npairs_all, c.cull_built ? 1 : 0);
   return cudaGetLastError() == cudaSuccess ? PDGPU_OK : PDGPU_ERR_CUDA;
 }
 

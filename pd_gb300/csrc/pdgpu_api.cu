@@ -263,7 +263,9 @@ pdgpu_ctx* pdgpu_create(int device, const pdgpu_system_desc* d, int* status) {
   if (cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaStreamCreateWithFlags(&c.side, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreateWithFlags(&c.ev_fork, cudaEventDisableTiming) != cudaSuccess ||
-      cudaEventCreateWithFlags(&c.ev_join, cudaEventDisableTiming) != cudaSuccess)
+      cudaEventCreateWithFlags(&c.ev_join, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&c.ev_total, cudaEventDisableTiming) != cudaSuccess ||
+      cudaHostAlloc((void**)&c.h_total, sizeof(int), cudaHostAllocDefault) != cudaSuccess)
     return bad(PDGPU_ERR_CUDA);
 
   // systems and padded layout
@@ -346,6 +348,30 @@ pdgpu_ctx* pdgpu_create(int device, const pdgpu_system_desc* d, int* status) {
       fbo.push_back(p.second);
     }
   }
+  // the same partners seen from the other side (the list build marks a row's
+  // bonded tiles from the row's own atoms)
+  std::vector<unsigned long long> down(N, 0ull);
+  std::vector<int> bstart(N + 1, 0), bidx;
+  {
+    for (int a = 0; a < N; a++)
+      for (unsigned long long m = bex[a] | b14[a]; m; m &= m - 1) {
+        const int d = __builtin_ctzll(m) + 1;
+        down[a + d] |= 1ull << (d - 1);
+      }
+    for (int a = 0; a < N; a++)
+      for (auto& p : far[a]) {
+        bstart[a + 1]++;
+        bstart[p.first + 1]++;
+      }
+    for (int a = 0; a < N; a++) bstart[a + 1] += bstart[a];
+    bidx.resize(std::max(bstart[N], 1), -1);
+    std::vector<int> at(bstart.begin(), bstart.end() - 1);
+    for (int a = 0; a < N; a++)
+      for (auto& p : far[a]) {
+        bidx[at[a]++] = p.first;
+        bidx[at[p.first]++] = a;
+      }
+  }
   // exclusion-mask table: a tile gets a mask only when it is diagonal, holds a
   // padding slot (the last block of a system) or a bonded pair, so this bounds
   // the masks of any list
@@ -373,6 +399,9 @@ pdgpu_ctx* pdgpu_create(int device, const pdgpu_system_desc* d, int* status) {
   UP(c.d_sqeps, sqeps.data(), (size_t)N);
   UP(c.d_band_excl, bex.data(), (size_t)N);
   UP(c.d_band_14, b14.data(), (size_t)N);
+  UP(c.d_band_down, down.data(), (size_t)N);
+  UP(c.d_far_both_start, bstart.data(), bstart.size());
+  UP(c.d_far_both_idx, bidx.data(), bidx.size());
   UP(c.d_far_start, fstart.data(), fstart.size());
   UP(c.d_far_idx, fidx.data(), fidx.size());
   UP(c.d_far_bo, fbo.data(), fbo.size());
@@ -538,12 +567,15 @@ int pdgpu_destroy(pdgpu_ctx* h) {
   destroy_md(h->c);
   // the streams and events outlive the context's device buffers
   cudaStream_t st = h->c.stream, side = h->c.side;
-  cudaEvent_t a = h->c.ev_fork, b = h->c.ev_join;
+  cudaEvent_t a = h->c.ev_fork, b = h->c.ev_join, t = h->c.ev_total;
+  int* total = h->c.h_total;
   h->c.stream = h->c.side = nullptr;
-  h->c.ev_fork = h->c.ev_join = nullptr;
+  h->c.ev_fork = h->c.ev_join = h->c.ev_total = nullptr;
   delete h;
   if (a) cudaEventDestroy(a);
   if (b) cudaEventDestroy(b);
+  if (t) cudaEventDestroy(t);
+  if (total) cudaFreeHost(total);
   if (side) cudaStreamDestroy(side);
   if (st) cudaStreamDestroy(st);
   return PDGPU_OK;
@@ -604,10 +636,6 @@ int pdgpu::alloc_tiles(Context& c, long long tiles) {
   c.cull_cap = 0;
   cudaError_t e = c.d_tiles.alloc(cap);
   if (e == cudaSuccess && c.has_gb) e = c.d_items.alloc(cap);
-  if (e == cudaSuccess) e = c.d_tile_flag.alloc(cap);
-  if (e == cudaSuccess) e = c.d_tile_pos.alloc(cap);
-  if (e == cudaSuccess) e = c.d_tile_need.alloc(cap / 32 + 1);
-  if (e == cudaSuccess) e = c.d_scan_tmp2.alloc((cap + 1023) / 1024 + 1);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return PDGPU_ERR_CUDA;
@@ -935,6 +963,10 @@ int pdgpu_rebuild_list(pdgpu_ctx* h) {
 void pdgpu::release_streams(Context& c) {
   if (c.ev_fork) cudaEventDestroy(c.ev_fork);
   if (c.ev_join) cudaEventDestroy(c.ev_join);
+  if (c.ev_total) cudaEventDestroy(c.ev_total);
+  if (c.h_total) cudaFreeHost(c.h_total);
+  c.ev_total = nullptr;
+  c.h_total = nullptr;
   if (c.side) cudaStreamDestroy(c.side);
   if (c.stream) cudaStreamDestroy(c.stream);
   c.ev_fork = c.ev_join = nullptr;
@@ -1119,8 +1151,7 @@ int pdgpu_list_tiles(pdgpu_ctx* h, int* tiles, long long cap, long long* ntiles,
   if (tile_cap) *tile_cap = c.tile_cap;
   if (list_bytes) {
     // the arrays whose size follows the list
-    *list_bytes = (long long)(c.d_tiles.n * sizeof(Tile) + c.d_items.n * 4 + c.d_tile_flag.n * 4 +
-                              c.d_tile_pos.n * 4 + c.d_scan_tmp2.n * 4 + c.d_tile_need.n * 4 + c.d_mlist.n * 4 +
+    *list_bytes = (long long)(c.d_tiles.n * sizeof(Tile) + c.d_items.n * sizeof(int2) + c.d_mlist.n * 4 +
                               c.d_masks.n * sizeof(uint2) + c.d_cull_mask.n * sizeof(uint2) + c.d_cull_rest.n * 4 +
                               c.d_cull_ent.n * sizeof(float4) + c.d_cull_bi.n * 4);
   }

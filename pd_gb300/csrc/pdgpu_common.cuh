@@ -83,8 +83,6 @@ struct BlockGrid {
   double cell[3];   // cell edges
   int dims[3];
   int start;        // first cell in the context's cell arrays
-  float hmax[3];    // largest block half-extent of the system per axis
-  float pad;
 };
 
 // Pair-law constants for the LJ + Coulomb kernel (FF_NonBonded)
@@ -163,14 +161,17 @@ struct DevView {
   float2* plo;
   unsigned long long* band_excl;   // [natom*2]? (see below) per atom: bit d-1 => partner i+d excluded (bo<=2)
   unsigned long long* band_14;     // per atom: bit d-1 => partner i+d is a 1-4 pair
+  const unsigned long long* band_down;   // per atom: bit d-1 => partner i-d bonded (excluded or 1-4)
+  const int* far_both_start; // CSR of the bonded partners beyond the band, of either side
+  const int* far_both_idx;
   const int* far_start;      // CSR of partners beyond the band, per atom
   const int* far_idx;
   const int* far_bo;
   Tile* tiles;
   int* ntiles;
-  // GB work items over the tile list: tile index, bit 31 set when the item is the
-  // tile pair (t, t + 1) (same row, adjacent columns, both unmasked off-diagonal)
-  unsigned* items;
+  // GB work items over the tile list: a pair of all-inside tiles of one row
+  // (x, y), or a single tile (x, -1)
+  int2* items;
   int* nitems;
   uint2* masks;              // [mask_cap*32] per lane: (excluded bits, 1-4 bits) in rotation order
   int* nmasks;

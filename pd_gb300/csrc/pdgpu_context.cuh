@@ -48,6 +48,8 @@ struct Context {
   // `side` beside the pair kernels, forked from and joined back to `stream`
   cudaStream_t side = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  cudaEvent_t ev_total = nullptr;   // a list build's tile count has reached h_total
+  int* h_total = nullptr;           // (page-locked)
   int nsys = 0, natom = 0, nslots = 0, nblocks = 0;
   long long npairs_all = 0;    // block pairs bi <= bj of every system (every pair a tile)
   long long tile_cap = 0;      // tile list capacity: sized from the count of a build, with headroom
@@ -90,6 +92,8 @@ struct Context {
   DBuf<int> d_lcpoUse;
   DBuf<unsigned long long> d_band_excl, d_band_14;
   DBuf<int> d_far_start, d_far_idx, d_far_bo;
+  DBuf<unsigned long long> d_band_down;        // bonded partners of lower index (list build)
+  DBuf<int> d_far_both_start, d_far_both_idx;  // far partners of either side (list build)
   DBuf<double> d_mass;                         // kg
 
   // dynamic state
@@ -115,13 +119,11 @@ struct Context {
   DBuf<int> d_bcell_blocks;    // [nblocks] blocks in cell order
   DBuf<int> d_row_cnt, d_row_start;  // [nblocks] tiles per row, first tile of each row
   DBuf<Tile> d_tiles;          // [tile_cap] rows contiguous (any order), ascending columns
-  DBuf<int> d_tile_flag, d_tile_pos, d_scan_tmp2;  // [tile_cap] compaction scratch (GB items, NB groups)
-  DBuf<unsigned> d_tile_need;  // [tile_cap/32 + 1] one bit per tile: in the mask list
   DBuf<int> d_mlist;           // [mask_cap] tiles that get their exclusion bits (diagonal, padded, bonded)
   // [0] ntiles, [1] nmasks, [2] nitems, [3..5] NB groups (rest tiles, groups, fit),
   // [6] tiles the rows found (before the capacity clamp), [7] mask-list length
   DBuf<int> d_counters;
-  DBuf<unsigned> d_items;      // [tile_cap] GB work items (with GB only)
+  DBuf<int2> d_items;          // [tile_cap] GB work items (with GB only)
   DBuf<uint2> d_masks;         // [mask_cap*32]
   DBuf<float4> d_xq, d_par, d_rel0;  // [nslots]
   DBuf<float4> d_rlo;                // [nslots] FP32 remainders of the slots (energy evaluations)
@@ -205,6 +207,9 @@ struct Context {
     v.plo = d_plo.p;
     v.band_excl = d_band_excl.p;
     v.band_14 = d_band_14.p;
+    v.band_down = d_band_down.p;
+    v.far_both_start = d_far_both_start.p;
+    v.far_both_idx = d_far_both_idx.p;
     v.far_start = d_far_start.p;
     v.far_idx = d_far_idx.p;
     v.far_bo = d_far_bo.p;
