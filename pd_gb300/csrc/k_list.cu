@@ -47,8 +47,11 @@ __device__ __forceinline__ int hilbert3(unsigned x0, unsigned x1, unsigned x2) {
   return h;
 }
 
-// rows of systems of up to this many blocks (32,768 atoms) test every column
-constexpr int kDirectBlocks = 1024;
+// rows of systems of up to this many blocks (262,144 atoms) test every column: at
+// 5,623 blocks a build takes 334 us so, 430 us through the block grid (703 blocks:
+// 122 and 152 us); the tests grow with the square of the blocks, so larger systems
+// take the grid
+constexpr int kDirectBlocks = 8192;
 
 // order-preserving float <-> int for atomic min / max
 __device__ __forceinline__ int f2ord(float f) {
@@ -197,7 +200,7 @@ __device__ __forceinline__ int cta_exclusive_scan(int x, int* wsum, int* total) 
   return wsum[wid] + inc - x;
 }
 
-// three-phase scan, 1024 elements per CTA
+// two-phase scan, 1024 elements per CTA
 __global__ void __launch_bounds__(1024) k_scan_block(const int* in, int* out, int* block_sums, int n) {
   __shared__ int wsum[33];
   const int i = blockIdx.x * 1024 + threadIdx.x;
@@ -208,45 +211,35 @@ __global__ void __launch_bounds__(1024) k_scan_block(const int* in, int* out, in
   if (threadIdx.x == 0) block_sums[blockIdx.x] = total;
 }
 
-__global__ void __launch_bounds__(1024) k_scan_sums(int* sums, int nb) {
-  // single CTA: 1024-element chunks in order, carrying the running total
+// each CTA sums the totals before its own and adds them
+__global__ void __launch_bounds__(1024) k_scan_add(int* out, const int* sums, int n) {
   __shared__ int wsum[33];
-  int carry = 0;
-  for (int base = 0; base < nb; base += 1024) {
-    const int i = base + threadIdx.x;
-    const int x = i < nb ? sums[i] : 0;
-    int total;
-    const int e = cta_exclusive_scan(x, wsum, &total);
-    if (i < nb) sums[i] = e + carry;
-    carry += total;
-    __syncthreads();
-  }
+  int before = 0;
+  for (int i = threadIdx.x; i < blockIdx.x; i += 1024) before += sums[i];
+  int total;
+  cta_exclusive_scan(before, wsum, &total);
+  const int i = blockIdx.x * 1024 + threadIdx.x;
+  if (i < n) out[i] += total;
 }
 
-// one CTA for n <= kScanOne (one system's cells): PER consecutive elements per thread
-constexpr int kScanOne = 32768;
-template <int PER>
+// one CTA for n <= kScanOne: 8 consecutive elements per thread
+constexpr int kScanOne = 8192;
 __global__ void __launch_bounds__(1024) k_scan_one(const int* in, int* out, int n) {
   __shared__ int wsum[33];
-  const int base = threadIdx.x * PER;
-  int x[PER], s = 0;
+  const int base = threadIdx.x * 8;
+  int x[8], s = 0;
 #pragma unroll
-  for (int k = 0; k < PER; k++) {
+  for (int k = 0; k < 8; k++) {
     x[k] = base + k < n ? in[base + k] : 0;
     s += x[k];
   }
   int total;
   int run = cta_exclusive_scan(s, wsum, &total);
 #pragma unroll
-  for (int k = 0; k < PER; k++) {
+  for (int k = 0; k < 8; k++) {
     if (base + k < n) out[base + k] = run;
     run += x[k];
   }
-}
-
-__global__ void k_scan_add(int* out, const int* sums, int n) {
-  int i = blockIdx.x * 1024 + threadIdx.x;
-  if (i < n) out[i] += sums[blockIdx.x];
 }
 
 __global__ void k_scatter(int natom, const int* bucket, const int* offset, int* cursor, int* tmp) {
@@ -635,7 +628,7 @@ __global__ void __launch_bounds__(kRowWarps * 32) k_tile_rows(DevView v, const B
       for (unsigned long long m = v.band_excl[a] | v.band_14[a]; m; m &= m - 1)
         mark_partner(slot_of, bi, nw, bits, mbits, a + __ffsll((long long)m));
     } else if (wid == 1) {
-      for (unsigned long long m = v.band_down[a]; m; m &= m - 1)
+      for (unsigned long long m = v.band_dn_excl[a] | v.band_dn_14[a]; m; m &= m - 1)
         mark_partner(slot_of, bi, nw, bits, mbits, a - __ffsll((long long)m));
     } else if (wid == 2) {
       for (int q = v.far_both_start[a]; q < v.far_both_start[a + 1]; q++)
@@ -716,48 +709,36 @@ __global__ void k_masks(DevView v, const int* mlist, const int* nml, const int* 
     Tile T = v.tiles[warp];
     int ai = v.sorted_atom[T.bi * 32 + lane];
     int aj0 = v.sorted_atom[T.bj * 32 + lane];
-    // each atom's band words and far-partner range, loaded once per lane (the
-    // lower index of a pair holds them, as in pair_bondorder); j's are shuffled in
-    unsigned long long exi = 0ull, b14i = 0ull, exj0 = 0ull, b14j0 = 0ull;
-    int fsi = 0, fei = 0, fsj0 = 0, fej0 = 0;
+    // the i atom's own partners of either side: band words and far list
+    unsigned long long exu = 0ull, u14 = 0ull, exd = 0ull, d14 = 0ull;
+    int fs = 0, fe = 0;
     if (ai >= 0) {
-      exi = v.band_excl[ai];
-      b14i = v.band_14[ai];
-      fsi = v.far_start[ai];
-      fei = v.far_start[ai + 1];
-    }
-    if (aj0 >= 0) {
-      exj0 = v.band_excl[aj0];
-      b14j0 = v.band_14[aj0];
-      fsj0 = v.far_start[aj0];
-      fej0 = v.far_start[aj0 + 1];
+      exu = v.band_excl[ai];
+      u14 = v.band_14[ai];
+      exd = v.band_dn_excl[ai];
+      d14 = v.band_dn_14[ai];
+      fs = v.far_both_start[ai];
+      fe = v.far_both_start[ai + 1];
     }
     unsigned ex = 0, m14 = 0;
+#pragma unroll 4
     for (int k = 0; k < 32; k++) {
-      const int src = (lane + k) & 31;
-      const int aj = __shfl_sync(0xffffffffu, aj0, src);
-      const unsigned long long exj = __shfl_sync(0xffffffffu, exj0, src);
-      const unsigned long long b14j = __shfl_sync(0xffffffffu, b14j0, src);
-      const int fsj = __shfl_sync(0xffffffffu, fsj0, src);
-      const int fej = __shfl_sync(0xffffffffu, fej0, src);
-      if (ai < 0 || aj < 0 || ai == aj) {
+      const int aj = __shfl_sync(0xffffffffu, aj0, (lane + k) & 31);
+      const int d = aj - ai;
+      if (ai < 0 || aj < 0 || d == 0) {
         ex |= 1u << k;
-        continue;
-      }
-      const bool lo_i = ai < aj;
-      const int hi = lo_i ? aj : ai;
-      const int d = lo_i ? aj - ai : ai - aj;
-      int bo = 7;
-      if (d <= kBandWidth) {
-        const unsigned long long bit = 1ull << (d - 1);
-        if ((lo_i ? exi : exj) & bit) bo = 2;
-        else if ((lo_i ? b14i : b14j) & bit) bo = 3;
+      } else if (d >= -kBandWidth && d <= kBandWidth) {
+        const int sh = (d > 0 ? d : -d) - 1;
+        const unsigned e = (unsigned)((d > 0 ? exu : exd) >> sh) & 1u, f = (unsigned)((d > 0 ? u14 : d14) >> sh) & 1u;
+        ex |= e << k;
+        m14 |= (f & ~e) << k;
       } else {
-        for (int q = lo_i ? fsi : fsj, e = lo_i ? fei : fej; q < e; q++)
-          if (v.far_idx[q] == hi && v.far_bo[q] < bo) bo = v.far_bo[q];
+        int bo = 7;
+        for (int q = fs; q < fe; q++)
+          if (v.far_both_idx[q] == aj && v.far_both_bo[q] < bo) bo = v.far_both_bo[q];
+        if (bo <= 2) ex |= 1u << k;
+        else if (bo == 3) m14 |= 1u << k;
       }
-      if (bo <= 2) ex |= 1u << k;
-      else if (bo == 3) m14 |= 1u << k;
     }
     bool any = __any_sync(0xffffffffu, (ex | m14) != 0);
     if (!any) continue;
@@ -937,17 +918,15 @@ static int list_tile_grid(const Context& c) {
   return (int)(want < g ? (want > 0 ? want : 1) : g);
 }
 
-// exclusive scan of n ints (n <= 2^20): one CTA up to kScanOne, else three phases
+// exclusive scan of n ints (n <= 2^20): one CTA up to kScanOne, else two phases
 static void scan_ints(Context& c, const int* in, int* out, int* tmp, long long n, cudaStream_t st) {
-  c.kernel_launches += n <= kScanOne ? 1 : 3;
+  c.kernel_launches += n <= kScanOne ? 1 : 2;
   if (n <= kScanOne) {
-    if (n <= 8192) k_scan_one<8><<<1, 1024, 0, st>>>(in, out, (int)n);
-    else k_scan_one<32><<<1, 1024, 0, st>>>(in, out, (int)n);
+    k_scan_one<<<1, 1024, 0, st>>>(in, out, (int)n);
     return;
   }
   const int nb = nblk(n, 1024);
   k_scan_block<<<nb, 1024, 0, st>>>(in, out, tmp, (int)n);
-  k_scan_sums<<<1, 1024, 0, st>>>(tmp, nb);
   k_scan_add<<<nb, 1024, 0, st>>>(out, tmp, (int)n);
 }
 

@@ -350,14 +350,18 @@ pdgpu_ctx* pdgpu_create(int device, const pdgpu_system_desc* d, int* status) {
   }
   // the same partners seen from the other side (the list build marks a row's
   // bonded tiles from the row's own atoms)
-  std::vector<unsigned long long> down(N, 0ull);
-  std::vector<int> bstart(N + 1, 0), bidx;
+  std::vector<unsigned long long> dex(N, 0ull), d14(N, 0ull);
+  std::vector<int> bstart(N + 1, 0), bidx, bbo;
   {
-    for (int a = 0; a < N; a++)
-      for (unsigned long long m = bex[a] | b14[a]; m; m &= m - 1) {
-        const int d = __builtin_ctzll(m) + 1;
-        down[a + d] |= 1ull << (d - 1);
-      }
+    auto mirror = [N](const std::vector<unsigned long long>& up, std::vector<unsigned long long>& dn) {
+      for (int a = 0; a < N; a++)
+        for (unsigned long long m = up[a]; m; m &= m - 1) {
+          const int d = __builtin_ctzll(m) + 1;
+          dn[a + d] |= 1ull << (d - 1);
+        }
+    };
+    mirror(bex, dex);
+    mirror(b14, d14);
     for (int a = 0; a < N; a++)
       for (auto& p : far[a]) {
         bstart[a + 1]++;
@@ -365,9 +369,11 @@ pdgpu_ctx* pdgpu_create(int device, const pdgpu_system_desc* d, int* status) {
       }
     for (int a = 0; a < N; a++) bstart[a + 1] += bstart[a];
     bidx.resize(std::max(bstart[N], 1), -1);
+    bbo.resize(bidx.size(), 7);
     std::vector<int> at(bstart.begin(), bstart.end() - 1);
     for (int a = 0; a < N; a++)
       for (auto& p : far[a]) {
+        bbo[at[a]] = bbo[at[p.first]] = p.second;
         bidx[at[a]++] = p.first;
         bidx[at[p.first]++] = a;
       }
@@ -399,7 +405,9 @@ pdgpu_ctx* pdgpu_create(int device, const pdgpu_system_desc* d, int* status) {
   UP(c.d_sqeps, sqeps.data(), (size_t)N);
   UP(c.d_band_excl, bex.data(), (size_t)N);
   UP(c.d_band_14, b14.data(), (size_t)N);
-  UP(c.d_band_down, down.data(), (size_t)N);
+  UP(c.d_band_dn_excl, dex.data(), (size_t)N);
+  UP(c.d_band_dn_14, d14.data(), (size_t)N);
+  UP(c.d_far_both_bo, bbo.data(), bbo.size());
   UP(c.d_far_both_start, bstart.data(), bstart.size());
   UP(c.d_far_both_idx, bidx.data(), bidx.size());
   UP(c.d_far_start, fstart.data(), fstart.size());

@@ -159,11 +159,13 @@ struct DevView {
   // (x, y, z, charge) - xq and (LJ radius, sqrt(eps)) - par, written before the energy pass
   float4* rlo;
   float2* plo;
-  unsigned long long* band_excl;   // [natom*2]? (see below) per atom: bit d-1 => partner i+d excluded (bo<=2)
+  unsigned long long* band_excl;   // per atom: bit d-1 => partner i+d excluded (bo<=2)
   unsigned long long* band_14;     // per atom: bit d-1 => partner i+d is a 1-4 pair
-  const unsigned long long* band_down;   // per atom: bit d-1 => partner i-d bonded (excluded or 1-4)
+  const unsigned long long* band_dn_excl;   // the same for partners of lower index: bit d-1 => i-d
+  const unsigned long long* band_dn_14;
   const int* far_both_start; // CSR of the bonded partners beyond the band, of either side
   const int* far_both_idx;
+  const int* far_both_bo;
   const int* far_start;      // CSR of partners beyond the band, per atom
   const int* far_idx;
   const int* far_bo;

@@ -92,8 +92,8 @@ struct Context {
   DBuf<int> d_lcpoUse;
   DBuf<unsigned long long> d_band_excl, d_band_14;
   DBuf<int> d_far_start, d_far_idx, d_far_bo;
-  DBuf<unsigned long long> d_band_down;        // bonded partners of lower index (list build)
-  DBuf<int> d_far_both_start, d_far_both_idx;  // far partners of either side (list build)
+  DBuf<unsigned long long> d_band_dn_excl, d_band_dn_14;      // bonded partners of lower index (list build)
+  DBuf<int> d_far_both_start, d_far_both_idx, d_far_both_bo;  // far partners of either side (list build)
   DBuf<double> d_mass;                         // kg
 
   // dynamic state
@@ -207,7 +207,9 @@ struct Context {
     v.plo = d_plo.p;
     v.band_excl = d_band_excl.p;
     v.band_14 = d_band_14.p;
-    v.band_down = d_band_down.p;
+    v.band_dn_excl = d_band_dn_excl.p;
+    v.band_dn_14 = d_band_dn_14.p;
+    v.far_both_bo = d_far_both_bo.p;
     v.far_both_start = d_far_both_start.p;
     v.far_both_idx = d_far_both_idx.p;
     v.far_start = d_far_start.p;
