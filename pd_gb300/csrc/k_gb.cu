@@ -242,6 +242,7 @@ __device__ __forceinline__ void born_single(const DevView& v, const GBConst& k, 
 }
 
 __global__ void __launch_bounds__(kBornThreads, 5) k_gb_born(const __grid_constant__ DevView v, const __grid_constant__ GBConst k, long long* gpol) {
+  pdl_sync();
   __shared__ BornRows rows[kBornWarps];
   BornRows& rs = rows[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
@@ -257,6 +258,7 @@ __global__ void __launch_bounds__(kBornThreads, 5) k_gb_born(const __grid_consta
 // Born radii a = -halfeconv / (terms123 + sum) + BornRadiusOffset  (FP64)
 __global__ void k_gb_radii(DevView v, const double* terms123, const long long* gpol, double halfeconv,
                            double offset, float* born_f, double* born_d) {
+  pdl_sync();
   int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= v.nslots) return;
   int a = v.sorted_atom[s];
@@ -751,6 +753,7 @@ __device__ __forceinline__ void gb_pair_single(const DevView& v, const GBConst& 
 constexpr int kPairThreads = 128, kPairEThreads = 128;
 template <bool FAST>
 __global__ void __launch_bounds__(kPairThreads, 5) k_gb_pair(const __grid_constant__ DevView v, const __grid_constant__ GBConst k, const float* born, long long* deda) {
+  pdl_sync();
   __shared__ PairRows rows[kPairThreads / 32];
   PairRows& rs = rows[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
@@ -772,6 +775,7 @@ __global__ void __launch_bounds__(kPairThreads, 5) k_gb_pair(const __grid_consta
 template <bool FAST, bool PRECISE>
 __global__ void __launch_bounds__(kPairEThreads, 4) k_gb_pair_energy(const __grid_constant__ DevView v, const __grid_constant__ GBConst k, const float* born,
                                                                     long long* deda) {
+  pdl_sync();
   __shared__ PairRowsE rows[kPairEThreads / 32];
   PairRowsE& rs = rows[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
@@ -784,6 +788,7 @@ __global__ void __launch_bounds__(kPairEThreads, 4) k_gb_pair_energy(const __gri
 // self term, total dE/da and the chain-rule prefactor a^2/166 * dE/da * P4
 __global__ void k_gb_self(DevView v, const double* charge, GBConst k, double premul, const long long* deda,
                           const double* born_d, float* chain, int energy) {
+  pdl_sync();
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   long long e = 0;
   if (s < v.nslots) {  // nslots is a multiple of 32: warps are whole
@@ -994,6 +999,7 @@ __device__ __forceinline__ void chain_single(const DevView& v, const GBConst& k,
 }
 
 __global__ void __launch_bounds__(kChainThreads, 6) k_gb_chain(const __grid_constant__ DevView v, const __grid_constant__ GBConst k, const float* chain) {
+  pdl_sync();
   __shared__ ChainRows rows[kChainWarps];
   ChainRows& rs = rows[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
@@ -1020,10 +1026,8 @@ int launch_gb(Context& c, const GBConst& k, double halfeconv, double born_offset
   cudaStream_t st = c.stream;
   int g = tile_grid(c);
   int nb = (c.nslots + 255) / 256;
-  cudaMemsetAsync(c.d_gpol.p, 0, sizeof(long long) * c.nslots, st);
-  cudaMemsetAsync(c.d_deda.p, 0, sizeof(long long) * c.nslots, st);
-  k_gb_born<<<g, kBornThreads, 0, st>>>(v, k, c.d_gpol.p);
-  k_gb_radii<<<nb, 256, 0, st>>>(v, c.d_gbT.p, c.d_gpol.p, halfeconv, born_offset, c.d_born_f.p, c.d_born_d.p);
+  launch_pdl(st, g, kBornThreads, 0, k_gb_born, v, k, c.d_gpol.p);
+  launch_pdl(st, nb, 256, 0, k_gb_radii, v, c.d_gbT.p, c.d_gpol.p, halfeconv, born_offset, c.d_born_f.p, c.d_born_d.p);
   // (a gradient call's energy pass weights a loss: FP32 pair energies)
   const bool precise = energy && !c.gb_no_chain;
   if (precise) {
@@ -1032,18 +1036,18 @@ int launch_gb(Context& c, const GBConst& k, double halfeconv, double born_offset
   }
   const int gp = g * (256 / kPairThreads), ge = g * (256 / kPairEThreads);
   if (energy) {
-    if (!k.fast) k_gb_pair_energy<false, true><<<ge, kPairEThreads, 0, st>>>(v, k, c.d_born_f.p, c.d_deda.p);
-    else if (precise) k_gb_pair_energy<true, true><<<ge, kPairEThreads, 0, st>>>(v, k, c.d_born_f.p, c.d_deda.p);
-    else k_gb_pair_energy<true, false><<<ge, kPairEThreads, 0, st>>>(v, k, c.d_born_f.p, c.d_deda.p);
+    if (!k.fast) launch_pdl(st, ge, kPairEThreads, 0, k_gb_pair_energy<false, true>, v, k, c.d_born_f.p, c.d_deda.p);
+    else if (precise) launch_pdl(st, ge, kPairEThreads, 0, k_gb_pair_energy<true, true>, v, k, c.d_born_f.p, c.d_deda.p);
+    else launch_pdl(st, ge, kPairEThreads, 0, k_gb_pair_energy<true, false>, v, k, c.d_born_f.p, c.d_deda.p);
   } else if (!k.fast) {
-    k_gb_pair<false><<<gp, kPairThreads, 0, st>>>(v, k, c.d_born_f.p, c.d_deda.p);
+    launch_pdl(st, gp, kPairThreads, 0, k_gb_pair<false>, v, k, c.d_born_f.p, c.d_deda.p);
   } else {
-    k_gb_pair<true><<<gp, kPairThreads, 0, st>>>(v, k, c.d_born_f.p, c.d_deda.p);
+    launch_pdl(st, gp, kPairThreads, 0, k_gb_pair<true>, v, k, c.d_born_f.p, c.d_deda.p);
   }
-  k_gb_self<<<nb, 256, 0, st>>>(v, c.d_charge.p, k, premul, c.d_deda.p, c.d_born_d.p, c.d_chain_f.p,
+  launch_pdl(st, nb, 256, 0, k_gb_self, v, c.d_charge.p, k, premul, c.d_deda.p, c.d_born_d.p, c.d_chain_f.p,
                                 energy ? 1 : 0);
   if (c.gb_no_chain) c.kernel_launches -= 1;
-  else k_gb_chain<<<2 * g, kChainThreads, 0, st>>>(v, k, c.d_chain_f.p);
+  else launch_pdl(st, 2 * g, kChainThreads, 0, k_gb_chain, v, k, c.d_chain_f.p);
   return cudaGetLastError() == cudaSuccess ? PDGPU_OK : PDGPU_ERR_CUDA;
 }
 
@@ -1052,9 +1056,9 @@ int launch_gb_stage(Context& c, const GBConst& k, int stage) {
   DevView v = c.view();
   int g = tile_grid(c);
   c.kernel_launches += 1;
-  if (stage == 1) k_gb_born<<<g, kBornThreads, 0, c.stream>>>(v, k, c.d_gpol.p);
-  else if (stage == 2) k_gb_pair<true><<<g * (256 / kPairThreads), kPairThreads, 0, c.stream>>>(v, k, c.d_born_f.p, c.d_deda.p);
-  else k_gb_chain<<<2 * g, kChainThreads, 0, c.stream>>>(v, k, c.d_chain_f.p);
+  if (stage == 1) launch_pdl(c.stream, g, kBornThreads, 0, k_gb_born, v, k, c.d_gpol.p);
+  else if (stage == 2) launch_pdl(c.stream, g * (256 / kPairThreads), kPairThreads, 0, k_gb_pair<true>, v, k, c.d_born_f.p, c.d_deda.p);
+  else launch_pdl(c.stream, 2 * g, kChainThreads, 0, k_gb_chain, v, k, c.d_chain_f.p);
   return cudaGetLastError() == cudaSuccess ? PDGPU_OK : PDGPU_ERR_CUDA;
 }
 

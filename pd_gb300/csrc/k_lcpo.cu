@@ -16,7 +16,7 @@ namespace pdgpu {
 //  * box: the block's bounding box over its LCPO atoms in the block frame of xq,
 //    lo.w = their largest LCPO radius, or -1 when the block holds none
 __global__ void __launch_bounds__(256) k_lcpo_prep(DevView v, const float4* lc, const double* P, const double* sigma,
-                                                   float4* lpos, float4* psig, float4* box) {
+                                                   float4* lpos, float4* psig, float4* box, int* ncand) {
   const int lane = threadIdx.x & 31;
   const int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (b >= v.nblocks) return;  // whole warps
@@ -33,6 +33,7 @@ __global__ void __launch_bounds__(256) k_lcpo_prep(DevView v, const float4* lc, 
   }
   lpos[s] = p;
   psig[s] = q;
+  ncand[s] = 0;
   const bool use = a >= 0 && l.y > 0.f;
   const float4 x = v.xq[s];
   float lo0 = use ? x.x : INFINITY, lo1 = use ? x.y : INFINITY, lo2 = use ? x.z : INFINITY;
@@ -331,9 +332,8 @@ int launch_lcpo(Context& c, long long* facc_out, long long* esurf_out, int esurf
   cudaStream_t st = c.stream;
   int g = tile_grid(c);
   c.kernel_launches += 4;
-  cudaMemsetAsync(c.d_lc_ncand.p, 0, sizeof(int) * c.nslots, st);
   k_lcpo_prep<<<(int)(((long long)c.nblocks * 32 + 255) / 256), 256, 0, st>>>(
-      v, c.d_lc_par.p, c.d_lcpoP.p, c.d_lcpoSig.p, c.d_lc_pos.p, c.d_lc_psig.p, c.d_lc_box.p);
+      v, c.d_lc_par.p, c.d_lcpoP.p, c.d_lcpoSig.p, c.d_lc_pos.p, c.d_lc_psig.p, c.d_lc_box.p, c.d_lc_ncand.p);
   k_lcpo_cand<<<g, 256, 0, st>>>(v, c.d_lc_par.p, c.d_lc_box.p, c.d_lc_ncand.p, c.d_lc_cand.p);
   int nw = (int)(((long long)c.nslots * 32 + 255) / 256);
   k_lcpo_sort<<<nw, 256, 0, st>>>(v, c.d_lc_par.p, c.d_lc_pos.p, c.d_lc_ncand.p, c.d_lc_cand.p, c.d_lc_n.p,

@@ -66,6 +66,7 @@ struct ListInit {
   int ncells, nslots, nbcells, nsys3;
 };
 __global__ void k_list_init(ListInit I) {
+  pdl_sync();
   const int t = blockIdx.x * blockDim.x + threadIdx.x, n = gridDim.x * blockDim.x;
   for (int i = t; i < I.ncells; i += n) I.count[i] = I.cursor[i] = 0;
   for (int i = t; i < I.nslots; i += n) I.sorted_atom[i] = -1;
@@ -82,6 +83,7 @@ __global__ void k_list_init(ListInit I) {
 // a warp whose atoms share one system reduces first and adds one atomic per
 // coordinate (a whole system's atoms otherwise meet on the same six words)
 __global__ void k_bbox(DevView v, const int* atom_sys, int* lo, int* hi) {
+  pdl_sync();
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31;
   const int s = a < v.natom ? atom_sys[a] : -1;
@@ -143,6 +145,7 @@ __device__ __forceinline__ void grid_setup(const SystemInfo& S, int s, const int
 // sets those grids up)
 __global__ void k_keys(DevView v, const int* atom_sys, const int* lo, const int* hi, int* bucket, int* count,
                        BlockGrid* grid) {
+  pdl_sync();
   int a = blockIdx.x * blockDim.x + threadIdx.x;
   if (grid && blockIdx.x == gridDim.x - 1) {
     for (int s = threadIdx.x; s < v.nsys; s += blockDim.x)
@@ -202,6 +205,7 @@ __device__ __forceinline__ int cta_exclusive_scan(int x, int* wsum, int* total) 
 
 // two-phase scan, 1024 elements per CTA
 __global__ void __launch_bounds__(1024) k_scan_block(const int* in, int* out, int* block_sums, int n) {
+  pdl_sync();
   __shared__ int wsum[33];
   const int i = blockIdx.x * 1024 + threadIdx.x;
   const int x = i < n ? in[i] : 0;
@@ -213,6 +217,7 @@ __global__ void __launch_bounds__(1024) k_scan_block(const int* in, int* out, in
 
 // each CTA sums the totals before its own and adds them
 __global__ void __launch_bounds__(1024) k_scan_add(int* out, const int* sums, int n) {
+  pdl_sync();
   __shared__ int wsum[33];
   int before = 0;
   for (int i = threadIdx.x; i < blockIdx.x; i += 1024) before += sums[i];
@@ -225,6 +230,7 @@ __global__ void __launch_bounds__(1024) k_scan_add(int* out, const int* sums, in
 // one CTA for n <= kScanOne: 8 consecutive elements per thread
 constexpr int kScanOne = 8192;
 __global__ void __launch_bounds__(1024) k_scan_one(const int* in, int* out, int n) {
+  pdl_sync();
   __shared__ int wsum[33];
   const int base = threadIdx.x * 8;
   int x[8], s = 0;
@@ -243,6 +249,7 @@ __global__ void __launch_bounds__(1024) k_scan_one(const int* in, int* out, int 
 }
 
 __global__ void k_scatter(int natom, const int* bucket, const int* offset, int* cursor, int* tmp) {
+  pdl_sync();
   int a = blockIdx.x * blockDim.x + threadIdx.x;
   if (a >= natom) return;
   int b = bucket[a];
@@ -253,6 +260,7 @@ __global__ void k_scatter(int natom, const int* bucket, const int* offset, int* 
 // the cell's atoms into their slots
 __global__ void k_cell_sort(DevView v, int ncells, const int* offset, const int* count, int* tmp, int* sorted_atom,
                             int* slot_of) {
+  pdl_sync();
   int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= ncells) return;
   int n = count[b];
@@ -345,8 +353,9 @@ __device__ __forceinline__ void slot_params(const DevView& v, const SlotParams& 
   if (P.lc_par) P.lc_par[s] = l;
 }
 
-__global__ void __launch_bounds__(128) k_blocks(DevView v, SlotParams P, const BlockGrid* grid, int* hmax, int* bcell,
-                                                int* bcount, int sub) {
+__global__ void __launch_bounds__(128) k_blocks(DevView v, SlotParams P, StepClear C, const BlockGrid* grid, int* hmax,
+                                                int* bcell, int* bcount, int sub) {
+  pdl_sync();
   const int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (b >= v.nblocks) return;
   const int slot = b * 32 + lane;
@@ -370,6 +379,7 @@ __global__ void __launch_bounds__(128) k_blocks(DevView v, SlotParams P, const B
     }
   }
   slot_params(v, P, slot, a);
+  step_clear(C, v, slot);
   float cf[3], hf[3];
   double cd[3];
 #pragma unroll
@@ -484,6 +494,7 @@ __device__ __forceinline__ void write_tile(const DevView& v, const SystemInfo& S
 // blocks in cell order (the order inside a cell does not matter: rows collect
 // their hits in a bitmap)
 __global__ void k_bgrid_scatter(DevView v, const int* bcell, const int* offset, int* cursor, int* blocks) {
+  pdl_sync();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= v.nblocks || v.sys[v.slot_sys[b]].nblocks <= kDirectBlocks) return;
   const int cell = bcell[b];
@@ -523,6 +534,7 @@ __global__ void __launch_bounds__(kRowWarps * 32) k_tile_rows(DevView v, const B
                                                               float margin, float full_R, float full_margin,
                                                               int* row_cnt, int* row_start, long long cap, int words,
                                                               int* total, int* mlist, int* nml) {
+  pdl_sync();
   extern __shared__ unsigned s_bits[];
   __shared__ int s_cnt[kRowWarps], s_base;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, bi = blockIdx.x;
@@ -695,6 +707,7 @@ __global__ void __launch_bounds__(kRowWarps * 32) k_tile_rows(DevView v, const B
 // (also the tile count from the rows' total, clamped to the capacity: an overflow
 // leaves a short list and is flagged)
 __global__ void k_masks(DevView v, const int* mlist, const int* nml, const int* total, long long cap) {
+  pdl_sync();
   const int lane = threadIdx.x & 31;
   const int n = min(*nml, v.mask_cap);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -759,7 +772,9 @@ __global__ void k_masks(DevView v, const int* mlist, const int* nml, const int* 
 // check2: squared skin limit (0 = no skin check); full2: squared limit that keeps
 // tiles flagged full valid (0 = none flagged), checked where the skin check is not
 // cull: the NB j-atom groups are in use (the displacement check always runs)
-__global__ void k_pack(DevView v, const double* charge, float check2, float full2, long long npairs_all, int cull) {
+__global__ void k_pack(DevView v, const double* charge, StepClear C, float check2, float full2, long long npairs_all,
+                       int cull) {
+  pdl_sync();
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= v.nslots) return;   // (whole warps)
   const int a = v.sorted_atom[s], b = s >> 5;
@@ -779,6 +794,7 @@ __global__ void k_pack(DevView v, const double* charge, float check2, float full
   }
   v.xq[s] = o;
   if (cull) write_sub(v, s, o);
+  step_clear(C, v, s);
 }
 
 // GB work items, one warp per row: the row's all-inside tiles without exclusion
@@ -787,6 +803,7 @@ __global__ void k_pack(DevView v, const double* charge, float check2, float full
 // items take their place by an atomic on the total (any order: every sum is in
 // fixed point).  pairs: 0 makes every item a single tile
 __global__ void __launch_bounds__(128) k_items(DevView v, int pairs, const int* row_start, const int* row_cnt) {
+  pdl_sync();
   const int lane = threadIdx.x & 31, b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (b >= v.nblocks) return;
   const int t0 = row_start[b], n = max(min(row_cnt[b], *v.ntiles - t0), 0);
@@ -841,6 +858,7 @@ __global__ void __launch_bounds__(128) k_items(DevView v, int pairs, const int* 
 constexpr int kCullWarps = 8;
 __global__ void __launch_bounds__(kCullWarps * 32) k_cull(DevView v, float R2, float Rc2, const int* row_start,
                                                           const int* row_cnt, uint2* jmask) {
+  pdl_sync();
   __shared__ int cnt[2][kCullWarps];
   __shared__ int first;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, b = blockIdx.x;
@@ -922,18 +940,18 @@ static int list_tile_grid(const Context& c) {
 static void scan_ints(Context& c, const int* in, int* out, int* tmp, long long n, cudaStream_t st) {
   c.kernel_launches += n <= kScanOne ? 1 : 2;
   if (n <= kScanOne) {
-    k_scan_one<<<1, 1024, 0, st>>>(in, out, (int)n);
+    launch_pdl(st, 1, 1024, 0, k_scan_one, in, out, (int)n);
     return;
   }
   const int nb = nblk(n, 1024);
-  k_scan_block<<<nb, 1024, 0, st>>>(in, out, tmp, (int)n);
-  k_scan_add<<<nb, 1024, 0, st>>>(out, tmp, (int)n);
+  launch_pdl(st, nb, 1024, 0, k_scan_block, in, out, tmp, (int)n);
+  launch_pdl(st, nb, 1024, 0, k_scan_add, out, tmp, (int)n);
 }
 
 static void launch_cull(Context& c, float list_radius) {
   c.kernel_launches += 1;
   const float R = list_radius + 1e-3f, Rc = fmaxf(list_radius - (float)c.lp.Padding, 0.f);
-  k_cull<<<c.nblocks, kCullWarps * 32, 0, c.stream>>>(c.view(), R * R, Rc * Rc, c.d_row_start.p, c.d_row_cnt.p,
+  launch_pdl(c.stream, c.nblocks, kCullWarps * 32, 0, k_cull, c.view(), R * R, Rc * Rc, c.d_row_start.p, c.d_row_cnt.p,
                                                       c.d_cull_mask.p);
 }
 
@@ -949,8 +967,7 @@ static void launch_rows(Context& c, float R, float full_radius) {
   const int words = (c.max_sys_blocks + 31) / 32 + 1;
   const size_t smem = (size_t)2 * words * sizeof(unsigned);
   int* cnt = c.d_counters.p;
-  k_tile_rows<<<c.nblocks, kRowWarps * 32, smem, c.stream>>>(
-      c.view(), c.d_bgrid.p, reinterpret_cast<int*>(c.d_sys_hmax.p), c.d_bcell_off.p, c.d_bcell_count.p,
+  launch_pdl(c.stream, c.nblocks, kRowWarps * 32, smem, k_tile_rows, c.view(), c.d_bgrid.p, reinterpret_cast<int*>(c.d_sys_hmax.p), c.d_bcell_off.p, c.d_bcell_count.p,
       c.d_bcell_blocks.p, c.d_slot_of.p, R, (float)c.lp.Padding, full_radius, c.full_margin(), c.d_row_cnt.p,
       c.d_row_start.p, c.tile_cap, words, cnt + 6, c.d_mlist.p, cnt + 7);
 }
@@ -974,10 +991,10 @@ static void launch_list_tail(Context& c, float list_radius) {
   int* cnt = c.d_counters.p;
   c.kernel_launches += 1;
   const int gm = nblk((long long)c.mask_cap * 32, 256), gt = list_tile_grid(c);
-  k_masks<<<gm < gt ? gm : gt, 256, 0, st>>>(c.view(), c.d_mlist.p, cnt + 7, cnt + 6, c.tile_cap);
+  launch_pdl(st, gm < gt ? gm : gt, 256, 0, k_masks, c.view(), c.d_mlist.p, cnt + 7, cnt + 6, c.tile_cap);
   if (c.has_gb) {
     c.kernel_launches += 1;
-    k_items<<<nblk(c.nblocks, 4), 128, 0, st>>>(c.view(), c.gb_item_tiles == 2 ? 1 : 0, c.d_row_start.p,
+    launch_pdl(st, nblk(c.nblocks, 4), 128, 0, k_items, c.view(), c.gb_item_tiles == 2 ? 1 : 0, c.d_row_start.p,
                                                 c.d_row_cnt.p);
   }
   // NB j-atom groups: only where the per-step displacement check runs
@@ -1008,24 +1025,24 @@ int launch_list_build(Context& c, float list_radius, float full_radius, ListSizi
   I.nslots = c.nslots;
   I.nbcells = grid ? c.nblocks : 0;
   I.nsys3 = 3 * c.nsys;
-  k_list_init<<<std::min(nblk(std::max(ncells, c.nslots), 256), 1216), 256, 0, st>>>(I);
+  launch_pdl(st, std::min(nblk(std::max(ncells, c.nslots), 256), 1216), 256, 0, k_list_init, I);
   if (!c.all_periodic) {
     c.kernel_launches += 1;
-    k_bbox<<<nblk(c.natom, 256), 256, 0, st>>>(v, c.d_atom_sys.p, lo, hi);
+    launch_pdl(st, nblk(c.natom, 256), 256, 0, k_bbox, v, c.d_atom_sys.p, lo, hi);
   }
-  k_keys<<<nblk(c.natom, 256) + (grid ? 1 : 0), 256, 0, st>>>(v, c.d_atom_sys.p, lo, hi, c.d_bucket.p, c.d_count.p,
+  launch_pdl(st, nblk(c.natom, 256) + (grid ? 1 : 0), 256, 0, k_keys, v, c.d_atom_sys.p, lo, hi, c.d_bucket.p, c.d_count.p,
                                                               grid ? c.d_bgrid.p : nullptr);
   scan_ints(c, c.d_count.p, c.d_offset.p, c.d_scan_tmp.p, ncells, st);
-  k_scatter<<<nblk(c.natom, 256), 256, 0, st>>>(c.natom, c.d_bucket.p, c.d_offset.p, c.d_cursor.p,
+  launch_pdl(st, nblk(c.natom, 256), 256, 0, k_scatter, c.natom, c.d_bucket.p, c.d_offset.p, c.d_cursor.p,
                                                  c.d_tmp_sorted.p);
-  k_cell_sort<<<nblk(ncells, 256), 256, 0, st>>>(v, ncells, c.d_offset.p, c.d_count.p, c.d_tmp_sorted.p,
+  launch_pdl(st, nblk(ncells, 256), 256, 0, k_cell_sort, v, ncells, c.d_offset.p, c.d_count.p, c.d_tmp_sorted.p,
                                                  c.d_sorted_atom.p, c.d_slot_of.p);
-  k_blocks<<<nblk((long long)c.nblocks * 32, 128), 128, 0, st>>>(v, slot_param_view(c), c.d_bgrid.p, hmax, c.d_bcell.p,
+  launch_pdl(st, nblk((long long)c.nblocks * 32, 128), 128, 0, k_blocks, v, slot_param_view(c), c.clear, c.d_bgrid.p, hmax, c.d_bcell.p,
                                                                  c.d_bcell_count.p, c.nb_set ? 1 : 0);
   if (grid) {
     c.kernel_launches += 1;   // and a scan
     scan_ints(c, c.d_bcell_count.p, c.d_bcell_off.p, c.d_bcell_scan_tmp.p, c.nblocks, st);
-    k_bgrid_scatter<<<nblk(c.nblocks, 256), 256, 0, st>>>(v, c.d_bcell.p, c.d_bcell_off.p, c.d_bcell_cursor.p,
+    launch_pdl(st, nblk(c.nblocks, 256), 256, 0, k_bgrid_scatter, v, c.d_bcell.p, c.d_bcell_off.p, c.d_bcell_cursor.p,
                                                            c.d_bcell_blocks.p);
   }
   launch_rows(c, list_radius, full_radius);
@@ -1050,7 +1067,7 @@ int launch_list_build(Context& c, float list_radius, float full_radius, ListSizi
       c.kernel_launches += 1;
       ListInit J{};
       J.counters = c.d_counters.p;
-      k_list_init<<<1, 32, 0, st>>>(J);
+      launch_pdl(st, 1, 32, 0, k_list_init, J);
       launch_rows(c, list_radius, full_radius);
       launch_list_tail(c, list_radius);
     }
@@ -1075,7 +1092,7 @@ int launch_pack(Context& c, float check_disp) {
     const float h = 0.5f * c.full_margin();
     f2 = h * h;
   }
-  k_pack<<<nblk(c.nslots, 256), 256, 0, c.stream>>>(v, c.d_charge.p, c2, f2, c.npairs_all, c.cull_built ? 1 : 0);
+  launch_pdl(c.stream, nblk(c.nslots, 256), 256, 0, k_pack, v, c.d_charge.p, c.clear, c2, f2, c.npairs_all, c.cull_built ? 1 : 0);
   return cudaGetLastError() == cudaSuccess ? PDGPU_OK : PDGPU_ERR_CUDA;
 }
 

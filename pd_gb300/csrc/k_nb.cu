@@ -166,6 +166,7 @@ __device__ __forceinline__ int nb_rot(const DevView& v, const NBConst& k, const 
 
 // remainders of the packed slots (before each energy pass)
 __global__ void k_df_records(DevView v, const double* charge, float4* rlo, float2* plo) {
+  pdl_sync();
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= v.nslots) return;
   const int a = v.sorted_atom[s];
@@ -343,6 +344,7 @@ template <int ELEC, bool ENERGY, bool SW = false>
 __global__ void __launch_bounds__(ENERGY ? kNbEThreads : kNbThreads, ENERGY ? 5 : 4)
     k_nb_tiles(const __grid_constant__ DevView v, const __grid_constant__ NBConst k, const __grid_constant__ NBEConst e,
                int cull) {
+  pdl_sync();
   __shared__ NBEShared shared[ENERGY ? kNbEThreads / 32 : 1];
   NBEShared* sh = ENERGY ? &shared[threadIdx.x >> 5] : nullptr;
   const int lane = threadIdx.x & 31;
@@ -654,6 +656,7 @@ constexpr int kNbFThreads = 128;
 template <int LAW>
 __global__ void __launch_bounds__(kNbFThreads, 6)
     k_nb_force(const __grid_constant__ DevView v, const __grid_constant__ NBConst k, int cull) {
+  pdl_sync();
   __shared__ NBRows rows[kNbFThreads / 32];
   NBRows& rs = rows[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
@@ -688,10 +691,10 @@ static void launch_nb_force(Context& c, const NBConst& k, int g) {
   // (8 copies of the solvated box: 336 -> 314 us; one copy 51 -> 49)
   const long long want = (c.tile_cap + c.cull_cap / 64 + 3) / 4;
   g = (int)std::min<long long>(4LL * g * (256 / T), want > 0 ? want : 1);
-  if (k.elecmode == 0) k_nb_force<kLawVdw><<<g, T, 0, c.stream>>>(v, k, cull);
-  else if (k.elecmode == 4) k_nb_force<kLawForce><<<g, T, 0, c.stream>>>(v, k, cull);
-  else if (k.samesw) k_nb_force<kLawSame><<<g, T, 0, c.stream>>>(v, k, cull);
-  else k_nb_force<kLawSplit><<<g, T, 0, c.stream>>>(v, k, cull);
+  if (k.elecmode == 0) launch_pdl(c.stream, g, T, 0, k_nb_force<kLawVdw>, v, k, cull);
+  else if (k.elecmode == 4) launch_pdl(c.stream, g, T, 0, k_nb_force<kLawForce>, v, k, cull);
+  else if (k.samesw) launch_pdl(c.stream, g, T, 0, k_nb_force<kLawSame>, v, k, cull);
+  else launch_pdl(c.stream, g, T, 0, k_nb_force<kLawSplit>, v, k, cull);
 }
 
 template <bool E>
@@ -702,18 +705,18 @@ static void launch_nb_mode(Context& c, const NBConst& k, int g) {
   constexpr int T = E ? kNbEThreads : kNbThreads;
   g *= kNbThreads / T;
   switch (k.elecmode) {
-    case 0: k_nb_tiles<0, E><<<g, T, 0, c.stream>>>(v, k, e, cull); break;
-    case 1: k_nb_tiles<1, E><<<g, T, 0, c.stream>>>(v, k, e, cull); break;
+    case 0: launch_pdl(c.stream, g, T, 0, k_nb_tiles<0, E>, v, k, e, cull); break;
+    case 1: launch_pdl(c.stream, g, T, 0, k_nb_tiles<1, E>, v, k, e, cull); break;
     case 3:
-      if (E && k.samesw) k_nb_tiles<3, true, true><<<g, T, 0, c.stream>>>(v, k, e, cull);
-      else k_nb_tiles<3, E><<<g, T, 0, c.stream>>>(v, k, e, cull);
+      if (E && k.samesw) launch_pdl(c.stream, g, T, 0, k_nb_tiles<3, true, true>, v, k, e, cull);
+      else launch_pdl(c.stream, g, T, 0, k_nb_tiles<3, E>, v, k, e, cull);
       break;
-    default: k_nb_tiles<4, E><<<g, T, 0, c.stream>>>(v, k, e, cull); break;
+    default: launch_pdl(c.stream, g, T, 0, k_nb_tiles<4, E>, v, k, e, cull); break;
   }
 }
 
 int launch_df_records(Context& c) {
-  k_df_records<<<(c.nslots + 255) / 256, 256, 0, c.stream>>>(c.view(), c.d_charge.p, c.d_rlo.p, c.d_plo.p);
+  launch_pdl(c.stream, (c.nslots + 255) / 256, 256, 0, k_df_records, c.view(), c.d_charge.p, c.d_rlo.p, c.d_plo.p);
   return cudaGetLastError() == cudaSuccess ? PDGPU_OK : PDGPU_ERR_CUDA;
 }
 

@@ -983,16 +983,14 @@ void pdgpu::release_streams(Context& c) {
 
 int pdgpu::enqueue_forces(Context& c, unsigned what, bool energy, bool rebuild, long long* lcpo_f,
                           long long* lcpo_e, int lcpo_e_stride, bool run_lcpo) {
-  if (rebuild || !c.list_built) {
-    int st = rebuild_list_impl(c);
-    if (st != PDGPU_OK) return st;
-  } else {
-    int st = launch_pack(c, c.lp.check_skin ? (float)(0.5 * c.lp.Padding) : 0.f);
-    if (st != PDGPU_OK) return st;
-  }
-  CK(cudaMemsetAsync(c.d_facc.p, 0, sizeof(long long) * 3 * c.nslots, c.stream));
-  if (energy) CK(cudaMemsetAsync(c.d_eacc.p, 0, sizeof(long long) * E_NSLOTS * c.nsys, c.stream));
-  int st = PDGPU_OK;
+  c.clear.facc = c.d_facc.p;
+  c.clear.gpol = (what & PDGPU_GB) ? c.d_gpol.p : nullptr;
+  c.clear.deda = (what & PDGPU_GB) ? c.d_deda.p : nullptr;
+  c.clear.eacc = energy ? c.d_eacc.p : nullptr;
+  int st = rebuild || !c.list_built ? rebuild_list_impl(c)
+                                    : launch_pack(c, c.lp.check_skin ? (float)(0.5 * c.lp.Padding) : 0.f);
+  c.clear = StepClear{};
+  if (st != PDGPU_OK) return st;
   // the LCPO recalculation (positions, packed slots and tile list) and the bonded
   // terms (positions) need nothing from the pair kernels: they run on the side
   // stream beside them, adding into the same fixed-point accumulators (integer

@@ -191,6 +191,53 @@ struct DevView {
   unsigned* status;
 };
 
+// What an evaluation clears before it accumulates: the pass that packs the
+// positions does it (null pointers are skipped), so a step launches no memsets
+struct StepClear {
+  long long *facc, *gpol, *deda;     // per slot (facc: 3)
+  long long *facc2;                  // per slot, 3: the cached LCPO forces before their recalculation
+  long long *eacc, *surf, *ke;       // per system (eacc: E_NSLOTS)
+};
+__device__ __forceinline__ void step_clear(const StepClear& C, const DevView& v, int s) {
+  if (C.facc) C.facc[3 * s] = C.facc[3 * s + 1] = C.facc[3 * s + 2] = 0;
+  if (C.gpol) C.gpol[s] = 0;
+  if (C.deda) C.deda[s] = 0;
+  if (C.facc2) C.facc2[3 * s] = C.facc2[3 * s + 1] = C.facc2[3 * s + 2] = 0;
+  if (C.eacc)   // (no fewer slots than 32 per system: every entry of a system's has a slot)
+    if ((s & 31) < E_NSLOTS && s == 32 * v.sys[v.slot_sys[s >> 5]].block_start + (s & 31))
+      C.eacc[(size_t)v.slot_sys[s >> 5] * E_NSLOTS + (s & 31)] = 0;
+  if ((C.surf || C.ke) && s == 32 * v.sys[v.slot_sys[s >> 5]].block_start) {
+    if (C.surf) C.surf[v.slot_sys[s >> 5]] = 0;
+    if (C.ke) C.ke[v.slot_sys[s >> 5]] = 0;
+  }
+}
+
+// Programmatic dependent launch.  A kernel launched with launch_pdl may be put on
+// the SMs as soon as every CTA of its predecessor in the stream has started;
+// pdl_sync, the first thing it does, lets its own successor do the same and then
+// waits until the predecessor has finished and its writes are visible.  Every
+// kernel of the evaluation's main chain does both, so the order of the chain
+// holds across any number of kernels, and the launch latency between two of them
+// (~2 us, ten of them in a small system's step) is hidden.
+__device__ __forceinline__ void pdl_sync() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <typename... P, typename... A>
+inline cudaError_t launch_pdl(cudaStream_t st, unsigned grid, unsigned block, size_t smem, void (*kernel)(P...), A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // ---------------------------------------------------------------------------
 // fixed point helpers
 // ---------------------------------------------------------------------------

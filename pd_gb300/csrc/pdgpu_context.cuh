@@ -136,6 +136,8 @@ struct Context {
   DBuf<int> d_cull_bi;               // [cull_cap / 32]
   long long cull_cap = 0;
 
+  StepClear clear{};           // what the next pack or list build clears (set by enqueue_forces)
+
   // accumulators
   DBuf<long long> d_facc;      // [nslots*3]
   DBuf<long long> d_eacc;      // [nsys*E_NSLOTS]

@@ -70,9 +70,10 @@ __global__ void k_add_surf(long long* eacc, const long long* cache, int nsys) {
 int enqueue_step(Context& c, MDState& md, int flags, bool first) {
   const bool rebuild = flags & 1, sasa = flags & 2, energy = flags & 4;
   const bool has_sa = md.p.what & PDGPU_SA;
+  c.clear.ke = md.d_ke.p;
   if (has_sa && sasa) {
-    CK(cudaMemsetAsync(md.d_facc_sa.p, 0, sizeof(long long) * 3 * c.nslots, c.stream));
-    CK(cudaMemsetAsync(md.d_surf_cache.p, 0, sizeof(long long) * c.nsys, c.stream));
+    c.clear.facc2 = md.d_facc_sa.p;
+    c.clear.surf = md.d_surf_cache.p;
   }
   int st = enqueue_forces(c, md.p.what, energy, rebuild, md.d_facc_sa.p, md.d_surf_cache.p, 1, sasa);
   if (st != PDGPU_OK) return st;
@@ -309,6 +310,7 @@ int pdgpu_time_kernel(pdgpu_ctx* h, int kernel, int reps, int flush_l2, double* 
   int st = PDGPU_OK;
   for (int r = 0; r < reps && st == PDGPU_OK; r++) {
     if (flush_l2) CK(cudaMemsetAsync(scratch.p, r & 0xff, flush_bytes, c.stream));
+    if (kernel == 5) CK(cudaMemsetAsync(c.md->d_ke.p, 0, sizeof(long long) * c.nsys, c.stream));
     CK(cudaEventRecord(e0, c.stream));
     switch (kernel) {
       case 0: st = launch_nb(c, make_nb_const(c.nb), false); break;
