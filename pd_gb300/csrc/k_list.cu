@@ -1051,12 +1051,12 @@ int launch_list_build(Context& c, float list_radius, float full_radius, ListSizi
     // rebuilt into grown ones.  The rest of the build is queued behind the copy of
     // the count, so the GPU works on while the host waits for it (a list that did
     // not fit is cut to the capacity, and the rest runs again after the growth)
-    if (cudaMemcpyAsync(c.h_total, c.d_counters.p + 6, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+    if (cudaMemcpyAsync(c.h_total.p, c.d_counters.p + 6, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
         cudaEventRecord(c.ev_total, st) != cudaSuccess)
       return PDGPU_ERR_CUDA;
     if (c.tile_cap > 0) launch_list_tail(c, list_radius);
     if (cudaEventSynchronize(c.ev_total) != cudaSuccess) return PDGPU_ERR_CUDA;
-    const int total = *c.h_total;
+    const int total = *c.h_total.p;
     if (total > c.tile_cap) {
       // (the overflow of the arrays just outgrown is no error of this build)
       if (clear_tile_overflow(c) != PDGPU_OK) return PDGPU_ERR_CUDA;

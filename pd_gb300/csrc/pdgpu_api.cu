@@ -79,16 +79,17 @@ double full_radius(const Context& c) {
   return r;
 }
 
+// Positions of up to this many bytes (5,461 atoms) go through a page-locked copy,
+// so that pdgpu_set_positions need not wait for the device; a larger host copy
+// takes longer than the wait (131 kB: 8 us against 12 us)
+constexpr size_t kStagedPositions = 131072;
+
+// the device status, with whatever was queued to the host before it
 int read_status(Context& c) {
-  unsigned st = 0;
-  cudaError_t e = cudaMemcpyAsync(&st, c.d_status.p, sizeof(unsigned), cudaMemcpyDeviceToHost, c.stream);
+  cudaError_t e = cudaMemcpyAsync(c.h_status.p, c.d_status.p, sizeof(unsigned), cudaMemcpyDeviceToHost, c.stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c.stream);
   if (e != cudaSuccess) return cuda_status(e, &c, "status");
-  if (st & ST_NAN) return PDGPU_ERR_NAN;
-  if (st & ST_FIXED_OVERFLOW) return PDGPU_ERR_FIXED_OVERFLOW;
-  if (st & (ST_LCPO_OVERFLOW | ST_TILE_OVERFLOW)) return PDGPU_ERR_LIST_OVERFLOW;
-  if (st & ST_STALE_LIST) return PDGPU_ERR_STALE_LIST;
-  return PDGPU_OK;
+  return status_code(*c.h_status.p);
 }
 
 }  // namespace
@@ -265,7 +266,7 @@ pdgpu_ctx* pdgpu_create(int device, const pdgpu_system_desc* d, int* status) {
       cudaEventCreateWithFlags(&c.ev_fork, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&c.ev_join, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&c.ev_total, cudaEventDisableTiming) != cudaSuccess ||
-      cudaHostAlloc((void**)&c.h_total, sizeof(int), cudaHostAllocDefault) != cudaSuccess)
+      cudaEventCreateWithFlags(&c.ev_pos, cudaEventDisableTiming) != cudaSuccess)
     return bad(PDGPU_ERR_CUDA);
 
   // systems and padded layout
@@ -556,7 +557,11 @@ pdgpu_ctx* pdgpu_create(int device, const pdgpu_system_desc* d, int* status) {
   }
   if (e == cudaSuccess) e = cudaMemset(c.d_status.p, 0, sizeof(unsigned));
   if (e != cudaSuccess) return bad(PDGPU_ERR_CUDA);
-  c.h_eacc.resize((size_t)c.nsys * E_NSLOTS);
+  e = c.h_eacc.alloc((size_t)c.nsys * E_NSLOTS);
+  if (e == cudaSuccess) e = c.h_status.alloc(1);
+  if (e == cudaSuccess) e = c.h_total.alloc(1);
+  if (e == cudaSuccess && 24 * (size_t)N <= kStagedPositions) e = c.h_pos.alloc(3 * (size_t)N);
+  if (e != cudaSuccess) return bad(PDGPU_ERR_CUDA);
 
   // PD defaults: FF_NonBonded::settodefault (nonbonded.cpp:985-1021),
   // FF_GeneralizedBorn_Still constructor (gbff.cpp:33-55), NeighbourList Padding 0.5
@@ -575,15 +580,14 @@ int pdgpu_destroy(pdgpu_ctx* h) {
   destroy_md(h->c);
   // the streams and events outlive the context's device buffers
   cudaStream_t st = h->c.stream, side = h->c.side;
-  cudaEvent_t a = h->c.ev_fork, b = h->c.ev_join, t = h->c.ev_total;
-  int* total = h->c.h_total;
+  cudaEvent_t a = h->c.ev_fork, b = h->c.ev_join, t = h->c.ev_total, q = h->c.ev_pos;
   h->c.stream = h->c.side = nullptr;
-  h->c.ev_fork = h->c.ev_join = h->c.ev_total = nullptr;
+  h->c.ev_fork = h->c.ev_join = h->c.ev_total = h->c.ev_pos = nullptr;
   delete h;
   if (a) cudaEventDestroy(a);
   if (b) cudaEventDestroy(b);
   if (t) cudaEventDestroy(t);
-  if (total) cudaFreeHost(total);
+  if (q) cudaEventDestroy(q);
   if (side) cudaStreamDestroy(side);
   if (st) cudaStreamDestroy(st);
   return PDGPU_OK;
@@ -888,8 +892,21 @@ int pdgpu_set_positions(pdgpu_ctx* h, const double* xyz, size_t stride) {
   if (!h || !xyz || stride < 24 || stride % 8) return PDGPU_ERR_ARG;
   Context& c = h->c;
   CK(cudaSetDevice(c.device));
-  CK(copy_xyz_rows(c.d_pos.p, 24, xyz, stride, c.natom, cudaMemcpyHostToDevice, c.stream));
-  CK(cudaStreamSynchronize(c.stream));
+  if (c.h_pos.p) {
+    CK(cudaEventSynchronize(c.ev_pos));   // (the previous copy out of the buffer)
+    if (stride == 24) {
+      std::memcpy(c.h_pos.p, xyz, 24 * (size_t)c.natom);
+    } else {
+      const size_t sd = stride / 8;
+      for (size_t a = 0; a < (size_t)c.natom; a++)
+        for (int k = 0; k < 3; k++) c.h_pos.p[3 * a + k] = xyz[a * sd + k];
+    }
+    CK(cudaMemcpyAsync(c.d_pos.p, c.h_pos.p, 24 * (size_t)c.natom, cudaMemcpyHostToDevice, c.stream));
+    CK(cudaEventRecord(c.ev_pos, c.stream));
+  } else {
+    CK(copy_xyz_rows(c.d_pos.p, 24, xyz, stride, c.natom, cudaMemcpyHostToDevice, c.stream));
+    CK(cudaStreamSynchronize(c.stream));
+  }
   c.positions_set = true;
   return size_list(c);
 }
@@ -972,9 +989,8 @@ void pdgpu::release_streams(Context& c) {
   if (c.ev_fork) cudaEventDestroy(c.ev_fork);
   if (c.ev_join) cudaEventDestroy(c.ev_join);
   if (c.ev_total) cudaEventDestroy(c.ev_total);
-  if (c.h_total) cudaFreeHost(c.h_total);
-  c.ev_total = nullptr;
-  c.h_total = nullptr;
+  if (c.ev_pos) cudaEventDestroy(c.ev_pos);
+  c.ev_total = c.ev_pos = nullptr;
   if (c.side) cudaStreamDestroy(c.side);
   if (c.stream) cudaStreamDestroy(c.stream);
   c.ev_fork = c.ev_join = nullptr;
@@ -1040,15 +1056,15 @@ static int enqueue_compute(Context& c, unsigned what, bool energy) {
   return enqueue_forces(c, what, energy, false, c.d_facc.p, energy ? c.d_eacc.p + E_SURF : nullptr, E_NSLOTS, true);
 }
 
-int pdgpu_get_energies(pdgpu_ctx* h, pdgpu_energies* out) {
-  if (!h || !out) return PDGPU_ERR_ARG;
-  Context& c = h->c;
-  CK(cudaSetDevice(c.device));
-  CK(cudaMemcpyAsync(c.h_eacc.data(), c.d_eacc.p, sizeof(long long) * E_NSLOTS * c.nsys, cudaMemcpyDeviceToHost,
+// queue the energy sums into h_eacc; decode them once they have arrived
+static int queue_energies(Context& c) {
+  CK(cudaMemcpyAsync(c.h_eacc.p, c.d_eacc.p, sizeof(long long) * E_NSLOTS * c.nsys, cudaMemcpyDeviceToHost,
                      c.stream));
-  CK(cudaStreamSynchronize(c.stream));
+  return PDGPU_OK;
+}
+static void decode_energies(const Context& c, pdgpu_energies* out) {
   for (int s = 0; s < c.nsys; s++) {
-    const long long* E = &c.h_eacc[(size_t)s * E_NSLOTS];
+    const long long* E = c.h_eacc.p + (size_t)s * E_NSLOTS;
     auto J = [&](int k) { return (double)E[k] / kEnergyScale * kKcalMolToJ; };
     pdgpu_energies& o = out[s];
     o.vdw = J(E_VDW);
@@ -1064,6 +1080,16 @@ int pdgpu_get_energies(pdgpu_ctx* h, pdgpu_energies* out) {
     o.improper = J(E_IMPR);
     o.epot = o.vdw + o.elec + o.pol + o.surf + o.bond + o.angle + o.torsion + o.improper;
   }
+}
+
+int pdgpu_get_energies(pdgpu_ctx* h, pdgpu_energies* out) {
+  if (!h || !out) return PDGPU_ERR_ARG;
+  Context& c = h->c;
+  CK(cudaSetDevice(c.device));
+  const int st = queue_energies(c);
+  if (st != PDGPU_OK) return st;
+  CK(cudaStreamSynchronize(c.stream));
+  decode_energies(c, out);
   return PDGPU_OK;
 }
 
@@ -1073,20 +1099,30 @@ int pdgpu_compute(pdgpu_ctx* h, unsigned what, pdgpu_energies* out, double* f, s
   CK(cudaSetDevice(c.device));
   int st = enqueue_compute(c, what, out != nullptr);
   if (st != PDGPU_OK) return st;
+  // forces, energies and status are queued together: one wait for all three
   if (f) {
     st = launch_finalize_forces(c, c.d_fout.p, 3, false, kForceToN);
     if (st != PDGPU_OK) return st;
-    c.h_stage.resize(3 * (size_t)c.natom);
-    CK(cudaMemcpyAsync(c.h_stage.data(), c.d_fout.p, 24 * (size_t)c.natom, cudaMemcpyDeviceToHost, c.stream));
+    if (!c.h_stage.p) CK(c.h_stage.alloc(3 * (size_t)c.natom));
+    CK(cudaMemcpyAsync(c.h_stage.p, c.d_fout.p, 24 * (size_t)c.natom, cudaMemcpyDeviceToHost, c.stream));
+  }
+  if (out) {
+    st = queue_energies(c);
+    if (st != PDGPU_OK) return st;
   }
   st = read_status(c);
   if (st != PDGPU_OK) return st;
   if (f) {
-    const size_t sd = stride / 8;
-    for (int a = 0; a < c.natom; a++)
-      for (int k = 0; k < 3; k++) f[a * sd + k] += c.h_stage[3 * (size_t)a + k];
+    const double* src = c.h_stage.p;
+    const size_t sd = stride / 8, N = c.natom;
+    if (sd == 3) {
+      for (size_t i = 0; i < 3 * N; i++) f[i] += src[i];
+    } else {
+      for (size_t a = 0; a < N; a++)
+        for (int k = 0; k < 3; k++) f[a * sd + k] += src[3 * a + k];
+    }
   }
-  if (out) return pdgpu_get_energies(h, out);
+  if (out) decode_energies(c, out);
   return PDGPU_OK;
 }
 

@@ -257,6 +257,15 @@ __device__ __forceinline__ long long fx32(float x) {
   return (long long)a * 1073741824LL + (long long)__float2int_rn(rem * 4294967296.f);
 }
 
+// the status code of a set of status bits
+inline int status_code(unsigned st) {
+  if (st & ST_NAN) return PDGPU_ERR_NAN;
+  if (st & ST_FIXED_OVERFLOW) return PDGPU_ERR_FIXED_OVERFLOW;
+  if (st & (ST_LCPO_OVERFLOW | ST_TILE_OVERFLOW)) return PDGPU_ERR_LIST_OVERFLOW;
+  if (st & ST_STALE_LIST) return PDGPU_ERR_STALE_LIST;
+  return PDGPU_OK;
+}
+
 // Range of FP32 partial sums about to enter 64-bit fixed point (2^32 per unit):
 // m is the sum of their magnitudes.  NaN or infinity sets ST_NAN; 2^28 or more
 // sets ST_FIXED_OVERFLOW.  One conversion holds up to 2^30 and a slot's total

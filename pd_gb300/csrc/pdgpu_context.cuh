@@ -41,6 +41,27 @@ struct DBuf {
   ~DBuf() { release(); }
 };
 
+// page-locked host memory (a copy to or from it is one DMA, with no staging
+// through the driver's own buffers)
+template <typename T>
+struct HBuf {
+  T* p = nullptr;
+  size_t n = 0;
+  cudaError_t alloc(size_t count) {
+    release();
+    cudaError_t e = cudaHostAlloc(reinterpret_cast<void**>(&p), count * sizeof(T), cudaHostAllocDefault);
+    if (e == cudaSuccess) n = count;
+    else p = nullptr;
+    return e;
+  }
+  void release() {
+    if (p) cudaFreeHost(p);
+    p = nullptr;
+    n = 0;
+  }
+  ~HBuf() { release(); }
+};
+
 struct Context {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -49,7 +70,7 @@ struct Context {
   cudaStream_t side = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   cudaEvent_t ev_total = nullptr;   // a list build's tile count has reached h_total
-  int* h_total = nullptr;           // (page-locked)
+  cudaEvent_t ev_pos = nullptr;     // the copy out of h_pos is done
   int nsys = 0, natom = 0, nslots = 0, nblocks = 0;
   long long npairs_all = 0;    // block pairs bi <= bj of every system (every pair a tile)
   long long tile_cap = 0;      // tile list capacity: sized from the count of a build, with headroom
@@ -178,9 +199,12 @@ struct Context {
   // dynamics state (pdgpu_md_setup), owned by the context
   MDState* md = nullptr;
 
-  // host staging
-  std::vector<long long> h_eacc;
-  std::vector<double> h_stage;
+  // host staging (page-locked)
+  HBuf<long long> h_eacc;           // [nsys*E_NSLOTS]
+  HBuf<double> h_stage;             // [natom*3] forces (allocated on first use)
+  HBuf<double> h_pos;               // [natom*3] positions of small contexts
+  HBuf<unsigned> h_status;          // [1]
+  HBuf<int> h_total;                // [1] a list build's tile count
   int last_error = 0;
   std::string last_msg;
 

@@ -152,14 +152,9 @@ LangevinCoeffs coeffs(double gamma, double t) {
 }
 
 int read_status_md(Context& c) {
-  unsigned st = 0;
-  CK(cudaMemcpyAsync(&st, c.d_status.p, sizeof(unsigned), cudaMemcpyDeviceToHost, c.stream));
+  CK(cudaMemcpyAsync(c.h_status.p, c.d_status.p, sizeof(unsigned), cudaMemcpyDeviceToHost, c.stream));
   CK(cudaStreamSynchronize(c.stream));
-  if (st & ST_NAN) return PDGPU_ERR_NAN;
-  if (st & ST_FIXED_OVERFLOW) return PDGPU_ERR_FIXED_OVERFLOW;
-  if (st & (ST_LCPO_OVERFLOW | ST_TILE_OVERFLOW)) return PDGPU_ERR_LIST_OVERFLOW;
-  if (st & ST_STALE_LIST) return PDGPU_ERR_STALE_LIST;
-  return PDGPU_OK;
+  return status_code(*c.h_status.p);
 }
 
 int md_enqueue_impl(Context& c, MDState& md, int nsteps, bool energy_on_last) {

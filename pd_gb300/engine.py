@@ -67,6 +67,7 @@ class DeviceContext:
         self.h = ctypes.c_void_p(h)
         self.natom = im.natom
         self.nsystems = im.nsystems
+        self.settings = 0      # counts the calls that set parameters
 
     def close(self):
         if getattr(self, "h", None):
@@ -81,20 +82,24 @@ class DeviceContext:
 
     # -- parameters --------------------------------------------------------
     def set_nb(self, **kw):
+        self.settings += 1
         p = ffi.NBParams(**kw)
         ffi.check(self.lib.pdgpu_set_nb_params(self.h, ctypes.byref(p)), "pdgpu_set_nb_params")
 
     def set_gb(self, **kw):
+        self.settings += 1
         p = ffi.GBParams(**kw)
         ffi.check(self.lib.pdgpu_set_gb_params(self.h, ctypes.byref(p)), "pdgpu_set_gb_params")
 
     def set_gb_mode(self, fast_mode, **vacuum):
         """FastMode of the GB component; vacuum: the GB object's FF_NonBonded settings (PD names)."""
+        self.settings += 1
         p = ffi.NBParams(**vacuum) if vacuum else None
         ffi.check(self.lib.pdgpu_set_gb_mode(self.h, int(bool(fast_mode)), ctypes.byref(p) if p else None),
                   "pdgpu_set_gb_mode")
 
     def set_list(self, padding, check_skin=True):
+        self.settings += 1
         p = ffi.ListParams(float(padding), int(check_skin))
         ffi.check(self.lib.pdgpu_set_list_params(self.h, ctypes.byref(p)), "pdgpu_set_list_params")
 

@@ -30,17 +30,20 @@ class ForcefieldBase:
         return self.wspace
 
     def calcCheckSum(self):
+        """Changes with any setting; results (the epot fields, totalSASA) do not count."""
         return hash(tuple(sorted((k, v) for k, v in vars(self).items()
-                                 if isinstance(v, (int, float, bool, str)) and k not in ("epot", "needsetup"))))
+                                 if isinstance(v, (int, float, bool, str)) and
+                                 not k.startswith(("epot", "_")) and k not in ("needsetup", "totalSASA"))))
 
     def setup(self):
         self.needsetup = False
 
     def ensuresetup(self):
-        cs = self.calcCheckSum()
-        if self.needsetup or cs != getattr(self, "_checksum", None):
+        im = self.wspace.image
+        tables = (tuple(im.scaling14), tuple(im.gb_P))   # what setup() takes from the parameter set
+        if self.needsetup or (self.calcCheckSum(), tables) != getattr(self, "_checksum", None):
             self.setup()
-            self._checksum = cs
+            self._checksum = (self.calcCheckSum(), tables)   # (setup may settle some of the settings)
             self.wspace._ctx_params = None
 
     def configure(self, ctx):
@@ -307,8 +310,8 @@ class Forcefield:
         ws = self.wspace
         self.ensuresetup()
         ctx = ws.context()
-        key = tuple((type(c).__name__, c.calcCheckSum()) for c in self.components) + (ws.Padding,)
-        if ws._ctx_params != key:
+        key = tuple((type(c).__name__, c._checksum) for c in self.components) + (ws.Padding,)
+        if ws._ctx_params != (key, ctx.settings):
             for c in self.components:
                 c.configure(ctx)
             ctx.set_list(ws.Padding)
@@ -324,8 +327,30 @@ class Forcefield:
                     for c in self.components:
                         c.configure(ctx)
                     ctx.set_list(ws.Padding)
-            ws._ctx_params = key
+            ws._ctx_params = (key, ctx.settings)
         return ctx
+
+    def _evaluate(self, ctx, call):
+        """call() with the list kept from earlier calls, rebuilt where the atoms have
+        left its skin: PD's callers may move atoms at will between two calls.  A list
+        that proves stale (a non-finite or overflowing result may come of one as well)
+        is rebuilt and the call repeated; while every call comes with new coordinates
+        like that, the list is rebuilt before the call instead."""
+        ws = self.wspace
+        if ws._moved_from is not None:
+            if 2.0 * np.abs(ws.cur.p - ws._moved_from).max() > ws.Padding:
+                ctx.rebuild_list()
+                ws._moved_from = ws.cur.p.copy()
+            else:
+                ws._moved_from = None
+        try:
+            return call()
+        except ffi.PDGPUError as e:
+            if e.status not in (ffi.ERR_STALE_LIST, -4, -5):
+                raise
+        ctx.rebuild_list()
+        ws._moved_from = ws.cur.p.copy()
+        return call()
 
     def calcForces(self, zero=True, energies_only=False):
         """Forcefield::calcForces: zero, evaluate every component, apply max_force, NaN check.
@@ -342,7 +367,7 @@ class Forcefield:
         ctx.set_positions(ws.cur.p)
         if energies_only and (what & ffi.GB):
             what |= ffi.PD_ENERGIES
-        energies = ctx.compute(what, None if energies_only else ws.cur.f)
+        energies = self._evaluate(ctx, lambda: ctx.compute(what, None if energies_only else ws.cur.f))
         ws.per_system_energies = energies
         tot = {k: sum(e[k] for e in energies) for k in energies[0]}
         for c in self.components:
@@ -365,10 +390,11 @@ class Forcefield:
             ws = self.wspace
             ctx = self._prepare()
             ctx.set_positions(ws.cur.p)
-            key = ws._ctx_params
-            if getattr(self, "_mc_key", None) != key:
-                energies = ctx.nb_energy_full()
-                self._mc_key = key
+            # (the reference belongs to the settings it was taken with, whichever container took it)
+            if ws._mc_key != ws._ctx_params:
+                ws._mc_key = None
+                energies = self._evaluate(ctx, ctx.nb_energy_full)
+                ws._mc_key = ws._ctx_params
             else:
                 energies, _ = ctx.nb_energy_update()
             ws.zeroForces()
