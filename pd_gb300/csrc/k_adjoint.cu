@@ -21,9 +21,8 @@
 // kernels therefore sum per tile in compensated FP32 (value plus running
 // rounding error, about 48 significant bits, on the FP32 pipe: GB300's FP64 rate
 // is a small fraction of its FP32 rate), fed by plain FP32 sums over 8 rotation
-// steps; the NB kernel sums in FP64.  Per-tile sums
-// enter 64-bit fixed point (2^32 per kcal/mol per parameter unit), so the result
-// does not depend on scheduling.
+// steps; the NB kernel sums in FP64.  Per-tile sums enter 64-bit fixed point (2^32
+// per kcal/mol per parameter unit), so the result does not depend on scheduling.
 #include "pdgpu_tile.cuh"
 
 namespace pdgpu {
@@ -51,39 +50,9 @@ __device__ __forceinline__ void csum_add(CSum& c, float x) {
   c.hi = s;
 }
 
-__device__ __forceinline__ double csum_value(const CSum& c) { return (double)c.hi + (double)c.lo; }
-
 struct CAcc3 {
   CSum a, b, c;
 };
-
-__device__ __forceinline__ Acc3 cacc_value(const CAcc3& x) {
-  return Acc3{csum_value(x.a), csum_value(x.b), csum_value(x.c)};
-}
-
-#define ROT_CSUM(x) \
-  ROT(x.hi);        \
-  ROT(x.lo)
-
-// plain FP32 sums over 8 rotation steps, entered into the compensated sums at
-// the end of each run of 8 (a short FP32 run adds only a few roundings of its
-// own terms; the compensated sum then carries the long total)
-struct Chunk3 {
-  float a, b, c;
-};
-
-__device__ __forceinline__ void chunk_into(CAcc3& A, Chunk3& C) {
-  csum_add(A.a, C.a);
-  csum_add(A.b, C.b);
-  csum_add(A.c, C.c);
-  C.a = C.b = C.c = 0.f;
-}
-
-__device__ __forceinline__ void chunk_into2(CAcc3& A, Chunk3& C) {  // components a and b only
-  csum_add(A.a, C.a);
-  csum_add(A.b, C.b);
-  C.a = C.b = 0.f;
-}
 
 __device__ __forceinline__ void acc_flush(const DevView& v, long long* g0, long long* g1, long long* g2, int s,
                                           const Acc3& x) {
@@ -92,6 +61,20 @@ __device__ __forceinline__ void acc_flush(const DevView& v, long long* g0, long 
   if (g0) atomic_add_ll(&g0[s], fix_sum_d(x.a));
   if (g1) atomic_add_ll(&g1[s], fix_sum_d(x.b));
   if (g2) atomic_add_ll(&g2[s], fix_sum_d(x.c));
+}
+
+// compensated sums into fixed point without FP64 work (fx32 holds below 2^29)
+__device__ __forceinline__ void acc_flush(const DevView& v, long long* g0, long long* g1, long long* g2, int s,
+                                          const CAcc3& x) {
+  const float m = fabsf(x.a.hi) + fabsf(x.b.hi) + fabsf(x.c.hi);
+  if (!(m < 2.6e8f)) {
+    acc_flush(v, g0, g1, g2, s, Acc3{(double)x.a.hi + (double)x.a.lo, (double)x.b.hi + (double)x.b.lo,
+                                     (double)x.c.hi + (double)x.c.lo});
+    return;
+  }
+  if (g0) atomic_add_ll(&g0[s], fx32(x.a.hi) + fx32(x.a.lo));
+  if (g1) atomic_add_ll(&g1[s], fx32(x.b.hi) + fx32(x.b.lo));
+  if (g2) atomic_add_ll(&g2[s], fx32(x.c.hi) + fx32(x.c.lo));
 }
 
 // dE/dRmin of the LJ term eps (A - 2B) S(r), A = (R/r)^12, B = (R/r)^6, written
@@ -105,182 +88,319 @@ __device__ __forceinline__ float lj_dR(float R, float invr) {
 }
 
 // ---------------------------------------------------------------------------
-// GB + vacuum pair terms: dE/dq, dE/dRmin, dE/dsqrt(eps) (Born radii held fixed;
-// their dependence on the GB parameters goes through dE/da in k_adj_born)
+// GB + vacuum pair terms in one pass over the tiles: energies, dE/da, dE/dq,
+// dE/dRmin and dE/dsqrt(eps) (Born radii held fixed; their dependence on the GB
+// parameters goes through dE/da in k_adj_born).  Step-packed as the GB force
+// bodies (k_gb.cu): lane l holds i atom l, the j atoms l + kk and l + kk + 1 of
+// the tile come as one FP32x2 pair from the warp's rows.  The gradient sums run
+// over 8 rotation steps in FP32 (4 terms per half) and enter the compensated
+// sums of the lane the atom lives in, so those never rotate.  Bound by FP32
+// issue; 16 frames of 4,235 atoms: energies and gradients took 635 + 566 us in
+// two passes of scalar bodies, 468 us in this one.
 // ---------------------------------------------------------------------------
-template <bool MASKED>
-__device__ __forceinline__ void adj_gb_tile(const DevView& v, const GBConst& k, const Tile& T, int lane, int si,
+struct AdjRows {
+  float4 xy[64], zq[64], se[64];   // step pairs (x, y), (z, q), (LJ radius, sqrt(eps)), twice over
+  float2 a[64];                    // Born radii (pair pass), or w = dE/dGpol (Born pass)
+};
+
+// the sums of 8 steps: held atoms' into the lane's own, rotating atoms' into
+// their home lane's (s: rotation steps made so far)
+__device__ __forceinline__ void chunk_held(CSum& A, float2& c) {
+  csum_add(A, c.x);
+  csum_add(A, c.y);
+  c = f2(0.f);
+}
+__device__ __forceinline__ void chunk_home(CSum& A, float2& c, int lane, int s) {
+  csum_add(A, __shfl_sync(0xffffffffu, c.x, (lane - s) & 31));
+  csum_add(A, __shfl_sync(0xffffffffu, c.y, (lane - s - 1) & 31));
+  c = f2(0.f);
+}
+
+template <bool MASKED, bool FULL>
+__device__ __forceinline__ void adj_gb_tile(const DevView& v, const GBConst& k, const Tile& T, int lane,
                                             const float4& xi, const float4& pi, float ai, unsigned ex, unsigned m14,
-                                            unsigned dmask, const float* born, CAcc3& I, CAcc3& J) {
-  float4 xj = j_in_i_frame(v, T, lane);
-  float4 pj = v.par[T.bj * 32 + lane];
-  float aj = born[T.bj * 32 + lane];
-  Chunk3 IC = {0.f, 0.f, 0.f}, JC = {0.f, 0.f, 0.f};  // JC rotates with its j atom
-#pragma unroll 2
-  for (int kk = 0; kk < 32; kk++) {
-    const float dx = xj.x - xi.x, dy = xj.y - xi.y, dz = xj.z - xi.z;
-    const float r2 = dx * dx + dy * dy + dz * dz;
-    bool pair = true, excl = false, is14 = false;
+                                            unsigned dm, long long* deda, long long* gq, long long* gr, long long* ge,
+                                            const AdjRows& rs) {
+  const int si = T.bi * 32 + lane, j0 = T.bj * 32;
+  const float2 X = f2(-xi.x), Y = f2(-xi.y), Z = f2(-xi.z), Q = f2(xi.w), R = f2(pi.x), E = f2(pi.y), AI = f2(ai);
+  const float4 *xy = rs.xy + lane, *zq = rs.zq + lane, *se = rs.se + lane;
+  const float2* aj = rs.a + lane;
+  CAcc3 I = {}, J = {};
+  float2 iq = f2(0.f), ir_ = f2(0.f), ie = f2(0.f), jq = f2(0.f), jr = f2(0.f), je = f2(0.f);
+  float2 DA = f2(0.f), RA = f2(0.f), cv = f2(0.f), ce = f2(0.f), cp = f2(0.f);
+  CSum ev = {0.f, 0.f}, ee = ev, ep_ = ev;
+#pragma unroll 1
+  for (int kk = 0; kk < 32; kk += 2) {
+    const float4 P = xy[kk], ZQ = zq[kk], SE = se[kk];
+    const float2 AJ = aj[kk];
+    const float2 dx = __fadd2_rn(make_float2(P.x, P.y), X), dy = __fadd2_rn(make_float2(P.z, P.w), Y);
+    const float2 dz = __fadd2_rn(make_float2(ZQ.x, ZQ.y), Z);
+    const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
+    const float2 ir = make_float2(rsqrtf(r2.x), rsqrtf(r2.y)), ir2 = __fmul2_rn(ir, ir);
+    bool ina = FULL || r2.x <= k.cut2, inb = FULL || r2.y <= k.cut2, xa = false, xb = false, ma = false, mb = false;
     if (MASKED) {
-      pair = !((dmask >> kk) & 1u);
-      excl = (ex >> kk) & 1u;
-      is14 = (m14 >> kk) & 1u;
+      ina = ina && !((dm >> kk) & 1u);
+      inb = inb && !((dm >> kk) & 2u);
+      xa = (ex >> kk) & 1u;
+      xb = (ex >> kk) & 2u;
+      ma = (m14 >> kk) & 1u;
+      mb = (m14 >> kk) & 2u;
     }
-    // the GB term's code runs only when some lane may lie above the exp
-    // threshold (warp vote, FP64 tie-break band included)
-    const bool in = r2 <= k.cut2 && pair;
-    const float u = -0.25f * __fdividef(r2, ai * aj);
-    const bool any_gb = __any_sync(0xffffffffu, in && u >= k.thresh - 4e-6f * fabsf(k.thresh));
-    if (in) {
-      const float invr = rsqrtf(r2);
-      const float r = r2 * invr;
-      bool gbon = false;
-      if (any_gb) {
-        gbon = u > k.thresh;
-        if (fabsf(u - k.thresh) <= 2e-6f * fabsf(k.thresh)) {
-          const int a = v.sorted_atom[si], b = v.sorted_atom[T.bj * 32 + ((lane + kk) & 31)];
-          gbon = a >= 0 && b >= 0 && -0.25 * r2_slots_fp64(v, si, T.bj * 32 + ((lane + kk) & 31)) /
-                                             (v.born[a] * v.born[b]) > k.thresh_d;
-        }
-      }
-      float S = 1.f;
-      if (r >= k.inner) {
-        const float w = r - k.inner;
-        const float sw = 1.f - w * w * k.invw2;
-        S = sw * sw;
-      }
-      const float s14 = is14 ? k.elec14 : 1.f;
-      float phi = 0.f;  // energy per unit q_i q_j
-      if (any_gb && gbon) {
-        const float fgb = rsqrtf(r2 + __expf(u) * ai * aj);
-        phi = 2.f * k.premul * fgb * S;
-        if (!excl) phi += k.econv_in * s14 * invr * S;
-      } else if (!excl) {
-        phi = k.econv_out * s14 * invr * S;
-      }
-      IC.a += phi * xj.w;
-      JC.a += phi * xi.w;
-      if (!excl && r < k.vdwcut) {
-        const float R = pi.x + pj.x;
-        const float t = R * invr;
-        float B = t * t;
-        B = B * B * B;
-        float Sv = is14 ? k.vdw14 : 1.f;
-        if (r > k.vdwinner) {
-          const float w = r - k.vdwinner;
-          const float sw = 1.f - w * w * k.vdwinvw2;
-          Sv *= sw * sw;
-        }
-        const float e1 = (B * B - 2.f * B) * Sv;  // energy per unit sqrt(eps_i) sqrt(eps_j)
-        const float dR = lj_dR(R, invr) * Sv * pi.y * pj.y;
-        IC.b += dR;
-        JC.b += dR;
-        IC.c += e1 * pj.y;
-        JC.c += e1 * pi.y;
-      }
+    float2 S = f2(1.f), Sv = f2(1.f);
+    if (!FULL) {
+      const float2 r = __fmul2_rn(r2, ir);
+      const float2 w = make_float2(fmaxf(r.x - k.inner, 0.f), fmaxf(r.y - k.inner, 0.f));
+      const float2 sw = __ffma2_rn(__fmul2_rn(w, w), f2(-k.invw2), f2(1.f));
+      S = __fmul2_rn(sw, sw);
+      const float2 wv = make_float2(fmaxf(r.x - k.vdwinner, 0.f), fmaxf(r.y - k.vdwinner, 0.f));
+      const float2 sv = __ffma2_rn(__fmul2_rn(wv, wv), f2(-k.vdwinvw2), f2(1.f));
+      Sv = __fmul2_rn(sv, sv);
+      Sv = make_float2(r.x < k.vdwcut ? Sv.x : 0.f, r.y < k.vdwcut ? Sv.y : 0.f);
     }
-    if ((kk & 7) == 7) {
-      chunk_into(I, IC);
-      chunk_into(J, JC);
+    // (selects, not products, below: the diagonal's own pair has r = 0)
+    float2 el = __fmul2_rn(ir, S);   // Coulomb energy per unit q q, without its constant ec
+    float2 ec = f2(k.econv_out);
+    if (MASKED) el = __fmul2_rn(el, make_float2(ma ? k.elec14 : 1.f, mb ? k.elec14 : 1.f));
+    // the GB term's code runs only when some lane may lie above the exp threshold
+    // (warp vote, FP64 tie-break band included)
+    const float2 aa = __fmul2_rn(AI, AJ);
+    const float2 u = __fmul2_rn(__fmul2_rn(r2, f2(-0.25f)), make_float2(rcp_ftz(aa.x), rcp_ftz(aa.y)));
+    const float lim = k.thresh - 4e-6f * fabsf(k.thresh);
+    const bool na = ina && u.x >= lim, nb = inb && u.y >= lim;
+    float2 po = f2(0.f);   // GB energy per unit q q
+    float2 QQ = __fmul2_rn(Q, make_float2(ZQ.z, ZQ.w));
+    if (__any_sync(0xffffffffu, na || nb)) {
+      const float tie = 2e-6f * fabsf(k.thresh);
+      bool ona = na && u.x > k.thresh, onb = nb && u.y > k.thresh;
+      if (na && fabsf(u.x - k.thresh) <= tie) ona = gb_on_fp64(v, si, j0 + ((lane + kk) & 31), k.thresh_d);
+      if (nb && fabsf(u.y - k.thresh) <= tie) onb = gb_on_fp64(v, si, j0 + ((lane + kk + 1) & 31), k.thresh_d);
+      const float2 tg = make_float2(__expf(u.x), __expf(u.y));
+      const float2 D = __ffma2_rn(tg, aa, r2);
+      const float2 fgb = make_float2(rsqrtf(D.x), rsqrtf(D.y));
+      float2 e = __fmul2_rn(__fmul2_rn(f2(k.premul), fgb), S);
+      e = make_float2(ona ? e.x : 0.f, onb ? e.y : 0.f);
+      po = __fadd2_rn(e, e);
+      const float2 W = __fmul2_rn(__fmul2_rn(__fmul2_rn(__fmul2_rn(e, QQ), __fmul2_rn(fgb, fgb)), tg),
+                                  __fadd2_rn(u, f2(-1.f)));
+      DA = __ffma2_rn(W, AJ, DA);
+      RA = __ffma2_rn(W, AI, RA);
+      ec = make_float2(ona ? k.econv_in : k.econv_out, onb ? k.econv_in : k.econv_out);
     }
-    ROT(xj.x); ROT(xj.y); ROT(xj.z); ROT(xj.w); ROT(pj.x); ROT(pj.y); ROT(aj);
-    ROT_CSUM(J.a); ROT_CSUM(J.b); ROT_CSUM(J.c);
-    ROT(JC.a); ROT(JC.b); ROT(JC.c);
+    el = __fmul2_rn(el, ec);
+    if (MASKED || !FULL) el = make_float2(ina && !xa ? el.x : 0.f, inb && !xb ? el.y : 0.f);
+    const float2 phi = __fadd2_rn(po, el);
+    iq = __ffma2_rn(phi, make_float2(ZQ.z, ZQ.w), iq);
+    jq = __ffma2_rn(phi, Q, jq);
+    cp = __ffma2_rn(po, QQ, cp);
+    ce = __ffma2_rn(el, QQ, ce);
+    // LJ: e1 = A - 2B per unit sqrt(eps) sqrt(eps), and its derivative in R
+    // (written without dividing by R: two zero-radius hydrogens give 0, not 0/0)
+    const float2 RR = __fadd2_rn(R, make_float2(SE.x, SE.y)), R2 = __fmul2_rn(RR, RR);
+    const float2 b5 = __fmul2_rn(__fmul2_rn(__fmul2_rn(R2, R2), RR), __fmul2_rn(__fmul2_rn(ir2, ir2), ir2));   // B / R
+    const float2 B = __fmul2_rn(b5, RR);
+    if (MASKED) Sv = __fmul2_rn(Sv, make_float2(ma ? k.vdw14 : 1.f, mb ? k.vdw14 : 1.f));
+    float2 e1 = __fmul2_rn(__fmul2_rn(B, __fadd2_rn(B, f2(-2.f))), Sv);
+    const float2 ee2 = __fmul2_rn(E, make_float2(SE.z, SE.w));
+    float2 dR = __fmul2_rn(__fmul2_rn(__fmul2_rn(b5, __fadd2_rn(B, f2(-1.f))), f2(12.f)), __fmul2_rn(Sv, ee2));
+    if (MASKED || !FULL) {
+      e1 = make_float2(ina && !xa ? e1.x : 0.f, inb && !xb ? e1.y : 0.f);
+      dR = make_float2(ina && !xa ? dR.x : 0.f, inb && !xb ? dR.y : 0.f);
+    }
+    ir_ = __fadd2_rn(ir_, dR);
+    jr = __fadd2_rn(jr, dR);
+    ie = __ffma2_rn(e1, make_float2(SE.z, SE.w), ie);
+    je = __ffma2_rn(e1, E, je);
+    cv = __ffma2_rn(e1, ee2, cv);
+    ROT2(jq); ROT2(jr); ROT2(je); ROT2(RA);
+    if ((kk & 6) == 6) {
+      chunk_held(I.a, iq);
+      chunk_held(I.b, ir_);
+      chunk_held(I.c, ie);
+      chunk_home(J.a, jq, lane, kk + 2);
+      chunk_home(J.b, jr, lane, kk + 2);
+      chunk_home(J.c, je, lane, kk + 2);
+      chunk_held(ev, cv);
+      chunk_held(ee, ce);
+      chunk_held(ep_, cp);
+    }
+  }
+  const float ra = RA.x + __shfl_sync(0xffffffffu, RA.y, (lane + 31) & 31), da = DA.x + DA.y;
+  fix_range(v.status, fabsf(da) + fabsf(ra));
+  atomic_add_ll(&deda[si], fx32(da));
+  atomic_add_ll(&deda[j0 + lane], fx32(ra));
+  acc_flush(v, gq, gr, ge, si, I);
+  acc_flush(v, gq, gr, ge, j0 + lane, J);
+  // the tile's energies meet over the warp in double-float and enter fixed point once
+  const DF e0 = df_warp_sum(DF{ev.hi, ev.lo}), e1 = df_warp_sum(DF{ee.hi, ee.lo}), e2 = df_warp_sum(DF{ep_.hi, ep_.lo});
+  const DF x = lane == 0 ? e0 : (lane == 1 ? e1 : e2);
+  if (lane < 3) {
+    long long* En = v.eacc + (size_t)v.slot_sys[T.bi] * E_NSLOTS;
+    atomic_add_ll(&En[lane == 0 ? E_VDW : (lane == 1 ? E_ELEC : E_POL_CROSS)], fix_energy_d((double)x.h + (double)x.l));
   }
 }
 
-__global__ void __launch_bounds__(256) k_adj_gb_pair(const __grid_constant__ DevView v, const __grid_constant__ GBConst k, const float* born, long long* gq,
+// the j block of a tile into the warp's rows (a0: the lane's value for rs.a)
+__device__ __forceinline__ void adj_stage(const DevView& v, int lane, const float4& x0, const float4& p0, float s0,
+                                          float e0, float a0, AdjRows& rs) {
+  const int l1 = (lane + 1) & 31;
+  const float x1 = __shfl_sync(0xffffffffu, x0.x, l1), y1 = __shfl_sync(0xffffffffu, x0.y, l1);
+  const float z1 = __shfl_sync(0xffffffffu, x0.z, l1), q1 = __shfl_sync(0xffffffffu, x0.w, l1);
+  const float s1 = __shfl_sync(0xffffffffu, s0, l1), e1 = __shfl_sync(0xffffffffu, e0, l1);
+  const float a1 = __shfl_sync(0xffffffffu, a0, l1);
+  __syncwarp();
+  rs.xy[lane] = rs.xy[lane + 32] = make_float4(x0.x, x1, x0.y, y1);
+  rs.zq[lane] = rs.zq[lane + 32] = make_float4(x0.z, z1, x0.w, q1);
+  rs.se[lane] = rs.se[lane + 32] = make_float4(s0, s1, e0, e1);
+  rs.a[lane] = rs.a[lane + 32] = make_float2(a0, a1);
+  __syncwarp();
+}
+
+constexpr int kAdjThreads = 128;
+__global__ void __launch_bounds__(kAdjThreads, 4) k_adj_gb_pair(const __grid_constant__ DevView v, const __grid_constant__ GBConst k, const float* born, long long* deda, long long* gq,
                                                       long long* gr, long long* ge) {
+  __shared__ AdjRows rows[kAdjThreads / 32];
+  AdjRows& rs = rows[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   const int nt = *v.ntiles;
   for (int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < nt; t += nwarps) {
     const Tile T = v.tiles[t];
-    const int si = T.bi * 32 + lane;
-    const float4 xi = v.xq[si], pi = v.par[si];
+    const int si = T.bi * 32 + lane, sj = T.bj * 32 + lane;
+    const float4 xi = v.xq[si], pi = v.par[si], xj = j_in_i_frame(v, T, lane), pj = v.par[sj];
+    adj_stage(v, lane, xj, pj, pj.x, pj.y, born[sj], rs);
     const float ai = born[si];
-    unsigned ex, m14;
-    tile_masks(v, T, lane, ex, m14);
-    const unsigned dmask = (T.flags & 2) ? diag_exclusion(lane) : 0u;
-    CAcc3 I = {}, J = {};
-    if (tile_masked(T)) adj_gb_tile<true>(v, k, T, lane, si, xi, pi, ai, ex, m14, dmask, born, I, J);
-    else adj_gb_tile<false>(v, k, T, lane, si, xi, pi, ai, ex, m14, dmask, born, I, J);
-    acc_flush(v, gq, gr, ge, si, cacc_value(I));
-    acc_flush(v, gq, gr, ge, T.bj * 32 + lane, cacc_value(J));
+    const bool full = tile_full_now(k, T, xi, xj);
+    if (tile_masked(T)) {
+      unsigned ex, m14;
+      tile_masks(v, T, lane, ex, m14);
+      const unsigned dm = (T.flags & 2) ? diag_exclusion(lane) : 0u;
+      if (full) adj_gb_tile<true, true>(v, k, T, lane, xi, pi, ai, ex, m14, dm, deda, gq, gr, ge, rs);
+      else adj_gb_tile<true, false>(v, k, T, lane, xi, pi, ai, ex, m14, dm, deda, gq, gr, ge, rs);
+    } else {
+      if (full) adj_gb_tile<false, true>(v, k, T, lane, xi, pi, ai, 0u, 0u, 0u, deda, gq, gr, ge, rs);
+      else adj_gb_tile<false, false>(v, k, T, lane, xi, pi, ai, 0u, 0u, 0u, deda, gq, gr, ge, rs);
+    }
   }
+}
+
+// the energy pass of a gradient call: energies and dE/da, and with them the pair
+// terms' gradients into c.adj_g (G_NACC x nslots, cleared by the caller)
+int launch_adj_gb_pair(Context& c, const GBConst& k) {
+  const size_t ns = c.nslots;
+  long long* g = c.adj_g;
+  k_adj_gb_pair<<<2 * tile_grid(c), kAdjThreads, 0, c.stream>>>(c.view(), k, c.d_born_f.p, c.d_deda.p, g + G_Q * ns,
+                                                                g + G_R * ns, g + G_EPS * ns);
+  return cudaGetLastError() == cudaSuccess ? PDGPU_OK : PDGPU_ERR_CUDA;
 }
 
 // ---------------------------------------------------------------------------
 // Born-radius sums Gpol_i += P4 Vj CCF(r^2/(Ri+Rj)^2) / r^4 (bond order > 2,
-// r <= GbsaStillCutoff): dE/dVj and dE/dR through w = dE/dGpol per slot
+// r <= GbsaStillCutoff): dE/dVj and dE/dR through w = dE/dGpol per slot.
+// Step-packed; rows: (x, y), (z, P4 V), (R, -), w.  340 us on 16 frames of 4,235
+// atoms as a scalar rotation, 210 us so.
 // ---------------------------------------------------------------------------
-template <bool MASKED>
-__device__ __forceinline__ void adj_born_tile(const DevView& v, const GBConst& k, const Tile& T, int lane, int si,
-                                              const float4& xi, const float4& pi, float wi, unsigned ex,
-                                              const float* w, CAcc3& I, CAcc3& J) {
-  float4 xj = j_in_i_frame(v, T, lane);
-  float4 pj = v.par[T.bj * 32 + lane];
-  float wj = w[T.bj * 32 + lane];
-  Chunk3 IC = {0.f, 0.f, 0.f}, JC = {0.f, 0.f, 0.f};  // (a, b used) JC rotates with its j atom
-#pragma unroll 4
-  for (int kk = 0; kk < 32; kk++) {
-    const float dx = xj.x - xi.x, dy = xj.y - xi.y, dz = xj.z - xi.z;
-    const float r2 = dx * dx + dy * dy + dz * dz;
-    bool in = r2 <= k.still2;
-    if (fabsf(r2 - k.still2) <= 2e-6f * k.still2)
-      in = r2_slots_fp64(v, si, T.bj * 32 + ((lane + kk) & 31)) <= k.still2_d;
-    if (MASKED) in = in && !((ex >> kk) & 1u);
-    // close contact (r^2 <= rs^2 / P5, where the CCF switches on) is rare: its
-    // branch runs on a warp vote
-    const float rs = pi.z + pj.z, rs2 = rs * rs;
-    const bool anyc = __any_sync(0xffffffffu, in && r2 <= rs2 * k.invP5);
-    if (in) {
-      float ccf = 1.f, gx = 0.f;  // CCF, and dCCF/dx * dx/dR (0 outside contact)
-      if (anyc) {
-        if (r2 <= rs2 * k.invP5) {
-          const float x = __fdividef(r2, rs2);
-          float sn, cs;
-          sincospif(x * k.P5, &sn, &cs);
-          const float h = 0.5f - 0.5f * cs;
-          ccf = h * h;
-          gx = h * sn * (k.P5 * 3.14159265358979f) * (-2.f * __fdividef(x, rs));
-        }
-      }
-      const float ir2 = __fdividef(1.f, r2);
-      const float h4 = k.P4 * ir2 * ir2;
-      IC.b += wj * h4 * ccf;  // dE/dV_i from Gpol_j
-      JC.b += wi * h4 * ccf;  // dE/dV_j from Gpol_i
-      const float gR = (wi * pj.w + wj * pi.w) * h4 * gx;
-      IC.a += gR;
-      JC.a += gR;
-    }
-    if ((kk & 7) == 7) {
-      chunk_into2(I, IC);
-      chunk_into2(J, JC);
-    }
-    ROT(xj.x); ROT(xj.y); ROT(xj.z); ROT(pj.z); ROT(pj.w); ROT(wj); ROT_CSUM(J.a); ROT_CSUM(J.b);
-    ROT(JC.a); ROT(JC.b);
-  }
+// CCF, and dCCF/dx * dx/dR, of a pair (1 and 0 outside close contact)
+__device__ __forceinline__ float2 ccf_grad(const GBConst& k, float r2, float rs) {
+  const float rs2 = rs * rs;
+  if (r2 > rs2 * k.invP5) return make_float2(1.f, 0.f);
+  const float x = __fdividef(r2, rs2);
+  float sn, cs;
+  sincospif(x * k.P5, &sn, &cs);
+  const float h = 0.5f - 0.5f * cs;
+  return make_float2(h * h, h * sn * (k.P5 * 3.14159265358979f) * (-2.f * __fdividef(x, rs)));
 }
 
-__global__ void __launch_bounds__(256) k_adj_born(const __grid_constant__ DevView v, const __grid_constant__ GBConst k, const float* w, long long* gR,
+template <bool MASKED, bool FULL>
+__device__ __forceinline__ void adj_born_tile(const DevView& v, const GBConst& k, const Tile& T, int lane,
+                                              const float4& xi, const float4& pi, float wi, unsigned ex,
+                                              long long* gR, long long* gV, const AdjRows& rs) {
+  const int si = T.bi * 32 + lane, j0 = T.bj * 32;
+  const float2 X = f2(-xi.x), Y = f2(-xi.y), Z = f2(-xi.z), R = f2(pi.z), V = f2(pi.w), WI = f2(wi);
+  const float4 *xy = rs.xy + lane, *zv = rs.zq + lane, *se = rs.se + lane;
+  const float2* wj = rs.a + lane;
+  CSum IV = {0.f, 0.f}, JV = IV, IR = IV, JR = IV;
+  float2 iv = f2(0.f), jv = f2(0.f), irr = f2(0.f), jrr = f2(0.f);
+  bool contact = false;   // some pair so far was in close contact (else the R sums stay zero)
+#pragma unroll 1
+  for (int kk = 0; kk < 32; kk += 2) {
+    const float4 P = xy[kk], Q = zv[kk], SR = se[kk];
+    const float2 WJ = wj[kk];
+    const float2 dx = __fadd2_rn(make_float2(P.x, P.y), X), dy = __fadd2_rn(make_float2(P.z, P.w), Y);
+    const float2 dz = __fadd2_rn(make_float2(Q.x, Q.y), Z);
+    const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
+    bool ina = true, inb = true;
+    if (!FULL) {
+      ina = r2.x <= k.still2;
+      inb = r2.y <= k.still2;
+      if (fabsf(r2.x - k.still2) <= 2e-6f * k.still2)
+        ina = r2_slots_fp64(v, si, j0 + ((lane + kk) & 31)) <= k.still2_d;
+      if (fabsf(r2.y - k.still2) <= 2e-6f * k.still2)
+        inb = r2_slots_fp64(v, si, j0 + ((lane + kk + 1) & 31)) <= k.still2_d;
+    }
+    if (MASKED) {
+      ina = ina && !((ex >> kk) & 1u);
+      inb = inb && !((ex >> kk) & 2u);
+    }
+    const float2 i2 = make_float2(rcp_ftz(r2.x), rcp_ftz(r2.y));
+    float2 h4 = __fmul2_rn(__fmul2_rn(i2, i2), f2(k.P4));
+    if (MASKED || !FULL) h4 = make_float2(ina ? h4.x : 0.f, inb ? h4.y : 0.f);
+    const float2 s = __fadd2_rn(R, make_float2(SR.x, SR.y));
+    const float2 lim = __fmul2_rn(__fmul2_rn(s, s), f2(k.invP5));
+    // close contact (r^2 <= rs^2 / P5, where the CCF switches on) is rare: its
+    // branch runs on a warp vote
+    if (__any_sync(0xffffffffu, (ina && r2.x <= lim.x) || (inb && r2.y <= lim.y))) {
+      contact = true;
+      const float2 ca = ccf_grad(k, r2.x, s.x), cb = ccf_grad(k, r2.y, s.y);
+      const float2 gx = make_float2(ina ? ca.y : 0.f, inb ? cb.y : 0.f);
+      const float2 gr = __fmul2_rn(__fmul2_rn(__ffma2_rn(WI, make_float2(Q.z, Q.w), __fmul2_rn(WJ, V)), h4), gx);
+      irr = __fadd2_rn(irr, gr);
+      jrr = __fadd2_rn(jrr, gr);
+      h4 = __fmul2_rn(h4, make_float2(ina ? ca.x : 1.f, inb ? cb.x : 1.f));
+    }
+    iv = __ffma2_rn(WJ, h4, iv);   // dE/dV_i from Gpol_j
+    jv = __ffma2_rn(WI, h4, jv);   // dE/dV_j from Gpol_i
+    ROT2(jv);
+    if (contact) { ROT2(jrr); }
+    if ((kk & 6) == 6) {
+      chunk_held(IV, iv);
+      chunk_home(JV, jv, lane, kk + 2);
+      if (contact) {
+        chunk_held(IR, irr);
+        chunk_home(JR, jrr, lane, kk + 2);
+        contact = false;
+      }
+    }
+  }
+  acc_flush(v, gR, gV, nullptr, si, CAcc3{IR, IV, {0.f, 0.f}});
+  acc_flush(v, gR, gV, nullptr, j0 + lane, CAcc3{JR, JV, {0.f, 0.f}});
+}
+
+__global__ void __launch_bounds__(kAdjThreads, 6) k_adj_born(const __grid_constant__ DevView v, const __grid_constant__ GBConst k, const float* w, long long* gR,
                                                    long long* gV) {
+  __shared__ AdjRows rows[kAdjThreads / 32];
+  AdjRows& rs = rows[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   const int nt = *v.ntiles;
   for (int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < nt; t += nwarps) {
     const Tile T = v.tiles[t];
-    const int si = T.bi * 32 + lane;
-    const float4 xi = v.xq[si], pi = v.par[si];
+    const int si = T.bi * 32 + lane, sj = T.bj * 32 + lane;
+    const float4 xi = v.xq[si], pi = v.par[si], pj = v.par[sj];
+    float4 xj = j_in_i_frame(v, T, lane);
+    const bool full = tile_full_now(k, T, xi, xj);
+    xj.w = pj.w;
+    adj_stage(v, lane, xj, pj, pj.z, 0.f, w[sj], rs);
     const float wi = w[si];
-    unsigned ex, m14;
-    tile_masks(v, T, lane, ex, m14);
-    if (T.flags & 2) ex |= diag_exclusion(lane);
-    CAcc3 I = {}, J = {};
-    if (tile_masked(T)) adj_born_tile<true>(v, k, T, lane, si, xi, pi, wi, ex, w, I, J);
-    else adj_born_tile<false>(v, k, T, lane, si, xi, pi, wi, ex, w, I, J);
-    acc_flush(v, gR, gV, nullptr, si, cacc_value(I));
-    acc_flush(v, gR, gV, nullptr, T.bj * 32 + lane, cacc_value(J));
+    if (tile_masked(T)) {
+      unsigned ex, m14;
+      tile_masks(v, T, lane, ex, m14);
+      if (T.flags & 2) ex |= diag_exclusion(lane);
+      if (full) adj_born_tile<true, true>(v, k, T, lane, xi, pi, wi, ex, gR, gV, rs);
+      else adj_born_tile<true, false>(v, k, T, lane, xi, pi, wi, ex, gR, gV, rs);
+    } else {
+      if (full) adj_born_tile<false, true>(v, k, T, lane, xi, pi, wi, 0u, gR, gV, rs);
+      else adj_born_tile<false, false>(v, k, T, lane, xi, pi, wi, 0u, gR, gV, rs);
+    }
   }
 }
 
@@ -420,11 +540,12 @@ __global__ void k_adj_out(DevView v, const long long* g, int nslots, bool gb, co
 }
 
 
-// Runs after an energy evaluation of the same component (its Born radii, Gpol
-// sums and dE/da are read from the context).  g: G_NACC * nslots fixed-point
-// accumulators (cleared here), w: nslots floats (written in full here).
-static int launch_adjoint_into(Context& c, unsigned what, long long* g, float* w, double* d_q, double* d_r,
-                               double* d_e, double* d_R, double* d_V, double* d_T) {
+// Runs after the energy pass of the same component (its Born radii, Gpol sums,
+// dE/da and, for GB, the pair terms' gradients are there already).  g: G_NACC *
+// nslots fixed-point accumulators, cleared before that pass; w: nslots floats
+// (written in full here).
+int launch_adjoint(Context& c, unsigned what, const AdjScratch& a, double* d_q, double* d_r, double* d_e, double* d_R,
+                   double* d_V, double* d_T) {
   DevView v = c.view();
   cudaStream_t st = c.stream;
   const int ns = c.nslots;
@@ -433,15 +554,14 @@ static int launch_adjoint_into(Context& c, unsigned what, long long* g, float* w
   const double ec = econv_kcal();
   const double halfeconv = 0.5 * ec;
   const double premul = gb ? -0.5 * ec * (1.0 / c.gb.DielectricSolute - 1.0 / c.gb.DielectricSolvent) : 0.0;
-  if (cudaMemsetAsync(g, 0, sizeof(long long) * G_NACC * (size_t)ns, st) != cudaSuccess) return PDGPU_ERR_CUDA;
-  long long *gq = g + G_Q * (size_t)ns, *gr = g + G_R * (size_t)ns, *ge = g + G_EPS * (size_t)ns;
+  long long* g = a.g;
   if (gb) {
     GBConst k = make_gb_const(c.gb, c.list_radius_built);
-    c.kernel_launches += 3;
-    k_adj_gb_pair<<<grid, 256, 0, st>>>(v, k, c.d_born_f.p, gq, gr, ge);
-    k_adj_w<<<nb, 256, 0, st>>>(v, c.d_gbT.p, c.d_gpol.p, c.d_deda.p, premul, halfeconv, w);
-    k_adj_born<<<grid, 256, 0, st>>>(v, k, w, g + G_GBR * (size_t)ns, g + G_VJ * (size_t)ns);
+    c.kernel_launches += 2;
+    k_adj_w<<<nb, 256, 0, st>>>(v, c.d_gbT.p, c.d_gpol.p, c.d_deda.p, premul, halfeconv, a.w);
+    k_adj_born<<<2 * grid, kAdjThreads, 0, st>>>(v, k, a.w, g + G_GBR * (size_t)ns, g + G_VJ * (size_t)ns);
   } else {
+    long long *gq = g + G_Q * (size_t)ns, *gr = g + G_R * (size_t)ns, *ge = g + G_EPS * (size_t)ns;
     NBConst k = make_nb_const(c.nb);
     c.kernel_launches += 1;
     switch (k.elecmode) {
@@ -458,13 +578,20 @@ static int launch_adjoint_into(Context& c, unsigned what, long long* g, float* w
   return cudaGetLastError() == cudaSuccess ? PDGPU_OK : PDGPU_ERR_CUDA;
 }
 
-int launch_adjoint(Context& c, unsigned what, double* d_q, double* d_r, double* d_e, double* d_R, double* d_V,
-                   double* d_T) {
+int clear_adjoint(Context& c, const AdjScratch& a) {
+  return cudaMemsetAsync(a.g, 0, sizeof(long long) * G_NACC * (size_t)c.nslots, c.stream) == cudaSuccess
+             ? PDGPU_OK
+             : PDGPU_ERR_CUDA;
+}
+
+// the context's own scratch, allocated on first use
+int adjoint_scratch(Context& c, AdjScratch& a) {
   if (c.d_adj.n < (size_t)G_NACC * c.nslots) {
     if (c.d_adj.alloc((size_t)G_NACC * c.nslots) != cudaSuccess) return PDGPU_ERR_CUDA;
     if (c.d_adj_w.alloc((size_t)c.nslots) != cudaSuccess) return PDGPU_ERR_CUDA;
   }
-  return launch_adjoint_into(c, what, c.d_adj.p, c.d_adj_w.p, d_q, d_r, d_e, d_R, d_V, d_T);
+  a = AdjScratch{c.d_adj.p, c.d_adj_w.p};
+  return PDGPU_OK;
 }
 
 // ---------------------------------------------------------------------------
@@ -481,8 +608,7 @@ int launch_adjoint(Context& c, unsigned what, double* d_q, double* d_r, double* 
 static __device__ __align__(256) unsigned char g_adj_scratch[(size_t)kNoAllocMaxSlots *
                                                              (G_NACC * sizeof(long long) + sizeof(float))];
 
-int launch_adjoint_static(Context& c, unsigned what, double* d_q, double* d_r, double* d_e, double* d_R, double* d_V,
-                          double* d_T) {
+int adjoint_scratch_static(Context& c, AdjScratch& a) {
   if (c.nslots > kNoAllocMaxSlots) return PDGPU_ERR_CAPACITY;
   // The array's device address on the current device (the caller made the
   // context's device current).  In host code the array's name only stands in
@@ -493,9 +619,9 @@ int launch_adjoint_static(Context& c, unsigned what, double* d_q, double* d_r, d
   void* p = nullptr;
   if (cudaGetSymbolAddress(&p, g_adj_scratch) != cudaSuccess || !p) return PDGPU_ERR_CUDA;
   unsigned char* base = static_cast<unsigned char*>(p);
-  long long* g = reinterpret_cast<long long*>(base);
-  float* w = reinterpret_cast<float*>(base + (size_t)kNoAllocMaxSlots * G_NACC * sizeof(long long));
-  return launch_adjoint_into(c, what, g, w, d_q, d_r, d_e, d_R, d_V, d_T);
+  a.g = reinterpret_cast<long long*>(base);
+  a.w = reinterpret_cast<float*>(base + (size_t)kNoAllocMaxSlots * G_NACC * sizeof(long long));
+  return PDGPU_OK;
 }
 
 }  // namespace pdgpu

@@ -21,14 +21,6 @@
 
 namespace pdgpu {
 
-// 1 / x by the special-function unit alone (rcp.approx.ftz, ~1 ulp): the pair
-// terms' reciprocals of r^2 (no multiply by the numerator 1 as __fdividef has)
-__device__ __forceinline__ float rcp_ftz(float x) {
-  float y;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
 // ---------------------------------------------------------------------------
 // pass 1: Born-radius pair sums  Gpol_i += P4 Vj CCF / r^4  (bond order > 2)
 // ---------------------------------------------------------------------------
@@ -225,9 +217,19 @@ __device__ __forceinline__ void born_full2(const DevView& v, const GBConst& k, c
   atomic_add_ll(&gpol[r0 + lane], fx32(gr));
 }
 
+// whether both tiles of a work item are all inside, by their flags or (gradient
+// calls, whose lists carry none) at run time
+__device__ __forceinline__ bool pair_full_now(const DevView& v, const GBConst& k, const Tile& T, const Tile& U,
+                                              int lane) {
+  if (tile_full(T) && tile_full(U)) return true;
+  if (k.far_inner <= 0.f) return false;
+  const float4 x = v.xq[T.bi * 32 + lane];
+  return tile_full_now(k, T, x, j_in_i_frame(v, T, lane)) && tile_full_now(k, U, x, j_in_i_frame(v, U, lane));
+}
+
 __device__ __forceinline__ void born_single(const DevView& v, const GBConst& k, const Tile& T, int lane,
                                             long long* gpol, BornRows& rs) {
-  const bool full = tile_full(T);
+  const bool full = tile_full_now(k, T, v.xq[T.bi * 32 + lane], j_in_i_frame(v, T, lane));
   if (tile_masked(T)) {
     unsigned ex, m14;
     tile_masks(v, T, lane, ex, m14);
@@ -250,8 +252,16 @@ __global__ void __launch_bounds__(kBornThreads, 5) k_gb_born(const __grid_consta
   const int ni = *v.nitems;
   for (int it = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; it < ni; it += nwarps) {
     const int2 t = v.items[it];
-    if (t.y >= 0) born_full2(v, k, v.tiles[t.x], v.tiles[t.y], lane, gpol, rs);
-    else born_single(v, k, v.tiles[t.x], lane, gpol, rs);
+    const Tile T = v.tiles[t.x];
+    if (t.y >= 0) {
+      const Tile U = v.tiles[t.y];
+      if (pair_full_now(v, k, T, U, lane)) {
+        born_full2(v, k, T, U, lane, gpol, rs);
+        continue;
+      }
+      born_single(v, k, U, lane, gpol, rs);
+    }
+    born_single(v, k, T, lane, gpol, rs);
   }
 }
 
@@ -270,14 +280,6 @@ __global__ void k_gb_radii(DevView v, const double* terms123, const long long* g
   double r = -halfeconv / G + offset;
   born_f[s] = (float)r;
   born_d[a] = r;
-}
-
-// the exp-approximation switch is discontinuous: pairs within FP32 rounding of
-// the threshold are decided in FP64
-__device__ __noinline__ bool gb_on_fp64(const DevView& v, int si, int sj, double thresh) {
-  int a = v.sorted_atom[si], b = v.sorted_atom[sj];
-  if (a < 0 || b < 0) return false;
-  return -0.25 * r2_slots_fp64(v, si, sj) / (v.born[a] * v.born[b]) > thresh;
 }
 
 // ---------------------------------------------------------------------------
@@ -509,12 +511,12 @@ __device__ __forceinline__ void gb_close_energy(const DevView& v, const GBConst&
 // Pair pass of a single tile, step-packed: lane l holds i atom l (its values in
 // both halves), the j block's atoms l + kk and l + kk + 1 come from the warp's
 // rows; the rotating atoms' sums move two lanes per step.
-template <bool MASKED, bool FULL, bool FAST, bool ENERGY, bool PRECISE>
+template <bool MASKED, bool FULL, bool FAST, bool ENERGY>
 __device__ __forceinline__ void gb_pair_tile(const DevView& v, const GBConst& k, const Tile& T, int lane,
                                              const float* born, long long* deda, PairRows& rs, PairRowsE* re) {
   const int si = T.bi * 32 + lane, j0 = T.bj * 32, l1 = (lane + 1) & 31;
   const float4 xi = v.xq[si], pi = v.par[si];
-  DF O[3];                 // (PRECISE) centre of bj seen from bi
+  DF O[3];                 // (ENERGY) centre of bj seen from bi
   float2 XL, YL, ZL;       // remainders of the held atom, negated
   unsigned ex = 0u, m14 = 0u, dm = 0u;
   if (MASKED) {
@@ -524,7 +526,7 @@ __device__ __forceinline__ void gb_pair_tile(const DevView& v, const GBConst& k,
   {
     float4 x0 = j_in_i_frame(v, T, lane);
     const float4 p0 = v.par[j0 + lane];
-    if (PRECISE) {
+    if (ENERGY) {
       const float o[3] = {T.ox, T.oy, T.oz};
       df_offset(v, v.sys[v.slot_sys[T.bi]], T.bi, T.bj, o, O);
       const float4 h = v.xq[j0 + lane], l = v.rlo[j0 + lane], li = v.rlo[si];
@@ -568,7 +570,7 @@ __device__ __forceinline__ void gb_pair_tile(const DevView& v, const GBConst& k,
     const float2 ak = rs.ak[j];
     float2 dx = __fadd2_rn(make_float2(P.x, P.y), X), dy = __fadd2_rn(make_float2(P.z, P.w), Y);
     float2 dz = __fadd2_rn(make_float2(ZQ.x, ZQ.y), Z);
-    if (PRECISE) {
+    if (ENERGY) {
       const float4 L = re->lxy[j];
       dx = __fadd2_rn(dx, __fadd2_rn(make_float2(L.x, L.y), XL));
       dy = __fadd2_rn(dy, __fadd2_rn(make_float2(L.z, L.w), YL));
@@ -596,7 +598,7 @@ __device__ __forceinline__ void gb_pair_tile(const DevView& v, const GBConst& k,
     ROT2(RX); ROT2(RY); ROT2(RZ); ROT2(RA);
     if (ENERGY) {
       float2 f = f2(1.f);
-      if (PRECISE) {
+      {
         const bool ca = r2.x < k.eclose2 && (FULL || r2.x <= k.cut2) && m.pa;
         const bool cb = r2.y < k.eclose2 && (FULL || r2.y <= k.cut2) && m.pb;
         if (__any_sync(0xffffffffu, ca || cb)) {
@@ -633,7 +635,7 @@ __device__ __forceinline__ void gb_pair_tile(const DevView& v, const GBConst& k,
   flush_pair(v, deda, si, PairAcc{FX.x + FX.y, FY.x + FY.y, FZ.x + FZ.y, (DA.x + DA.y) * k.inv_sqrtK});
   flush_pair(v, deda, j0 + lane, PairAcc{-rx, -ry, -rz, ra * k.inv_sqrtK});
   if (ENERGY) {
-    if (PRECISE) {
+    if (ENERGY) {
       __syncwarp();
       for (int p = lane; p < np; p += 32) gb_close_energy<FAST>(v, k, T, O, re->pair[p], born, sum);
       __syncwarp();
@@ -730,20 +732,20 @@ __device__ __forceinline__ void gb_pair_full2(const DevView& v, const GBConst& k
   flush_pair(v, deda, r0 + lane, PairAcc{-R.fx, -R.fy, -R.fz, R.da * k.inv_sqrtK});
 }
 
-template <bool FAST, bool ENERGY, bool PRECISE>
+template <bool FAST, bool ENERGY>
 __device__ __forceinline__ void gb_pair_single(const DevView& v, const GBConst& k, const Tile& T, int lane,
                                                const float* born, long long* deda, PairRows& rs,
                                                PairRowsE* re) {
   const bool full = tile_full(T);
   if (!FAST || ENERGY) {   // (rarer passes: the masked bodies serve every tile)
-    if (full) gb_pair_tile<true, true, FAST, ENERGY, PRECISE>(v, k, T, lane, born, deda, rs, re);
-    else gb_pair_tile<true, false, FAST, ENERGY, PRECISE>(v, k, T, lane, born, deda, rs, re);
+    if (full) gb_pair_tile<true, true, FAST, ENERGY>(v, k, T, lane, born, deda, rs, re);
+    else gb_pair_tile<true, false, FAST, ENERGY>(v, k, T, lane, born, deda, rs, re);
   } else if (tile_masked(T)) {
-    if (full) gb_pair_tile<true, true, FAST, ENERGY, PRECISE>(v, k, T, lane, born, deda, rs, re);
-    else gb_pair_tile<true, false, FAST, ENERGY, PRECISE>(v, k, T, lane, born, deda, rs, re);
+    if (full) gb_pair_tile<true, true, FAST, ENERGY>(v, k, T, lane, born, deda, rs, re);
+    else gb_pair_tile<true, false, FAST, ENERGY>(v, k, T, lane, born, deda, rs, re);
   } else {
-    if (full) gb_pair_tile<false, true, FAST, ENERGY, PRECISE>(v, k, T, lane, born, deda, rs, re);
-    else gb_pair_tile<false, false, FAST, ENERGY, PRECISE>(v, k, T, lane, born, deda, rs, re);
+    if (full) gb_pair_tile<false, true, FAST, ENERGY>(v, k, T, lane, born, deda, rs, re);
+    else gb_pair_tile<false, false, FAST, ENERGY>(v, k, T, lane, born, deda, rs, re);
   }
 }
 
@@ -761,18 +763,21 @@ __global__ void __launch_bounds__(kPairThreads, 5) k_gb_pair(const __grid_consta
   const int ni = *v.nitems;
   for (int it = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; it < ni; it += nwarps) {
     const int2 t = v.items[it];
-    if (FAST && t.y >= 0) {
-      gb_pair_full2(v, k, v.tiles[t.x], v.tiles[t.y], lane, born, deda, rs);
-      continue;
+    const Tile T = v.tiles[t.x];
+    if (t.y >= 0) {
+      const Tile U = v.tiles[t.y];
+      if (FAST && tile_full(T) && tile_full(U)) {
+        gb_pair_full2(v, k, T, U, lane, born, deda, rs);
+        continue;
+      }
+      gb_pair_single<FAST, false>(v, k, U, lane, born, deda, rs, nullptr);
     }
-    gb_pair_single<FAST, false, false>(v, k, v.tiles[t.x], lane, born, deda, rs, nullptr);
-    if (!FAST && t.y >= 0) gb_pair_single<FAST, false, false>(v, k, v.tiles[t.y], lane, born, deda, rs, nullptr);
+    gb_pair_single<FAST, false>(v, k, T, lane, born, deda, rs, nullptr);
   }
 }
 
-// the pass with energies, tile by tile (PRECISE: close pairs in double-float;
-// else a gradient call's energies, FP32 pair terms)
-template <bool FAST, bool PRECISE>
+// the pass with energies, tile by tile
+template <bool FAST>
 __global__ void __launch_bounds__(kPairEThreads, 4) k_gb_pair_energy(const __grid_constant__ DevView v, const __grid_constant__ GBConst k, const float* born,
                                                                     long long* deda) {
   pdl_sync();
@@ -782,7 +787,7 @@ __global__ void __launch_bounds__(kPairEThreads, 4) k_gb_pair_energy(const __gri
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   const int nt = *v.ntiles;
   for (int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < nt; t += nwarps)
-    gb_pair_single<FAST, true, PRECISE>(v, k, v.tiles[t], lane, born, deda, rs, &rs);
+    gb_pair_single<FAST, true>(v, k, v.tiles[t], lane, born, deda, rs, &rs);
 }
 
 // self term, total dE/da and the chain-rule prefactor a^2/166 * dE/da * P4
@@ -1007,8 +1012,16 @@ __global__ void __launch_bounds__(kChainThreads, 6) k_gb_chain(const __grid_cons
   const int ni = *v.nitems;
   for (int it = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; it < ni; it += nwarps) {
     const int2 t = v.items[it];
-    if (t.y >= 0) chain_full2(v, k, v.tiles[t.x], v.tiles[t.y], lane, chain, rs);
-    else chain_single(v, k, v.tiles[t.x], lane, chain, rs);
+    const Tile T = v.tiles[t.x];
+    if (t.y >= 0) {
+      const Tile U = v.tiles[t.y];
+      if (tile_full(T) && tile_full(U)) {
+        chain_full2(v, k, T, U, lane, chain, rs);
+        continue;
+      }
+      chain_single(v, k, U, lane, chain, rs);
+    }
+    chain_single(v, k, T, lane, chain, rs);
   }
 }
 
@@ -1028,17 +1041,17 @@ int launch_gb(Context& c, const GBConst& k, double halfeconv, double born_offset
   int nb = (c.nslots + 255) / 256;
   launch_pdl(st, g, kBornThreads, 0, k_gb_born, v, k, c.d_gpol.p);
   launch_pdl(st, nb, 256, 0, k_gb_radii, v, c.d_gbT.p, c.d_gpol.p, halfeconv, born_offset, c.d_born_f.p, c.d_born_d.p);
-  // (a gradient call's energy pass weights a loss: FP32 pair energies)
-  const bool precise = energy && !c.gb_no_chain;
-  if (precise) {
+  const int gp = g * (256 / kPairThreads), ge = g * (256 / kPairEThreads);
+  if (c.gb_no_chain) {
+    // a gradient call: energies (FP32 pair terms: they weight a loss), dE/da and the
+    // pair terms' gradients in one pass, no forces
+    const int e = launch_adj_gb_pair(c, k);
+    if (e != PDGPU_OK) return e;
+  } else if (energy) {
     c.kernel_launches += 1;
     launch_df_records(c);
-  }
-  const int gp = g * (256 / kPairThreads), ge = g * (256 / kPairEThreads);
-  if (energy) {
-    if (!k.fast) launch_pdl(st, ge, kPairEThreads, 0, k_gb_pair_energy<false, true>, v, k, c.d_born_f.p, c.d_deda.p);
-    else if (precise) launch_pdl(st, ge, kPairEThreads, 0, k_gb_pair_energy<true, true>, v, k, c.d_born_f.p, c.d_deda.p);
-    else launch_pdl(st, ge, kPairEThreads, 0, k_gb_pair_energy<true, false>, v, k, c.d_born_f.p, c.d_deda.p);
+    if (!k.fast) launch_pdl(st, ge, kPairEThreads, 0, k_gb_pair_energy<false>, v, k, c.d_born_f.p, c.d_deda.p);
+    else launch_pdl(st, ge, kPairEThreads, 0, k_gb_pair_energy<true>, v, k, c.d_born_f.p, c.d_deda.p);
   } else if (!k.fast) {
     launch_pdl(st, gp, kPairThreads, 0, k_gb_pair<false>, v, k, c.d_born_f.p, c.d_deda.p);
   } else {

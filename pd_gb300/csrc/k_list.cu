@@ -798,11 +798,12 @@ __global__ void k_pack(DevView v, const double* charge, StepClear C, float check
 }
 
 // GB work items, one warp per row: the row's all-inside tiles without exclusion
-// mask go together two by two in column order (a pairing that does not depend on
+// mask (far: where the passes find all-inside tiles at run time, every tile
+// without one) go together two by two in column order (a pairing that does not depend on
 // the other systems of a batch), every other tile is an item of its own; the row's
 // items take their place by an atomic on the total (any order: every sum is in
 // fixed point).  pairs: 0 makes every item a single tile
-__global__ void __launch_bounds__(128) k_items(DevView v, int pairs, const int* row_start, const int* row_cnt) {
+__global__ void __launch_bounds__(128) k_items(DevView v, int pairs, int far, const int* row_start, const int* row_cnt) {
   pdl_sync();
   const int lane = threadIdx.x & 31, b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (b >= v.nblocks) return;
@@ -812,7 +813,7 @@ __global__ void __launch_bounds__(128) k_items(DevView v, int pairs, const int* 
     bool p = false;
     if (pairs && i + lane < n) {
       const Tile T = v.tiles[t0 + i + lane];
-      p = tile_full(T) && !tile_masked(T) && !(T.flags & 1);
+      p = (far || tile_full(T)) && !tile_masked(T) && !(T.flags & 1);
     }
     np += __popc(__ballot_sync(0xffffffffu, p));
   }
@@ -829,7 +830,7 @@ __global__ void __launch_bounds__(128) k_items(DevView v, int pairs, const int* 
     bool p = false;
     if (pairs && in) {
       const Tile T = v.tiles[t0 + i + lane];
-      p = tile_full(T) && !tile_masked(T) && !(T.flags & 1);
+      p = (far || tile_full(T)) && !tile_masked(T) && !(T.flags & 1);
     }
     const unsigned mp = __ballot_sync(0xffffffffu, p), ms = __ballot_sync(0xffffffffu, in && !p);
     if (p) two[rp + __popc(mp & lt)] = t0 + i + lane;
@@ -994,7 +995,8 @@ static void launch_list_tail(Context& c, float list_radius) {
   launch_pdl(st, gm < gt ? gm : gt, 256, 0, k_masks, c.view(), c.d_mlist.p, cnt + 7, cnt + 6, c.tile_cap);
   if (c.has_gb) {
     c.kernel_launches += 1;
-    launch_pdl(st, nblk(c.nblocks, 4), 128, 0, k_items, c.view(), c.gb_item_tiles == 2 ? 1 : 0, c.d_row_start.p,
+    const int far = c.gb_set && make_gb_const(c.gb, c.list_radius_built).far_inner > 0.f ? 1 : 0;
+    launch_pdl(st, nblk(c.nblocks, 4), 128, 0, k_items, c.view(), c.gb_item_tiles == 2 ? 1 : 0, far, c.d_row_start.p,
                                                 c.d_row_cnt.p);
   }
   // NB j-atom groups: only where the per-step displacement check runs

@@ -220,6 +220,8 @@ GBConst pdgpu::make_gb_const(const pdgpu_gb_params& p, double listR) {
   k.gb_ep = (float)(-premul / eout);
   k.in_over_out = (float)(ec / p.DielectricSolute / eout);
   k.sqrt12 = (float)std::sqrt(12.0);
+  const double fi = std::min(std::min(p.InnerCutoff, p.VdwInnerCutoff), still);
+  k.far_inner = fi >= 64.0 ? (float)fi : 0.f;
   return k;
 }
 
@@ -704,12 +706,16 @@ int pdgpu_set_list_params(pdgpu_ctx* h, const pdgpu_list_params* p) {
 
 static int enqueue_compute(Context& c, unsigned what, bool energy);
 
-// the energy pass a parameter gradient reads (Born radii, Gpol sums, dE/da and
-// energies); the GB chain-rule pass only forms forces and is left out
-static int enqueue_grad_energies(Context& c, unsigned what) {
+// the energy pass of a parameter gradient (Born radii, Gpol sums, dE/da, energies
+// and the GB pair terms' gradients); the passes that only form forces are left out
+static int enqueue_grad_energies(Context& c, unsigned what, const AdjScratch& a) {
+  int st = clear_adjoint(c, a);
+  if (st != PDGPU_OK) return st;
   c.gb_no_chain = true;
-  const int st = enqueue_compute(c, what & ~PDGPU_ENERGY, true);
+  c.adj_g = a.g;
+  st = enqueue_compute(c, what & ~PDGPU_ENERGY, true);
   c.gb_no_chain = false;
+  c.adj_g = nullptr;
   return st;
 }
 
@@ -846,9 +852,11 @@ int pdgpu_param_grad_device(pdgpu_ctx* h, unsigned what, const pdgpu_param_grads
   int st = param_grad_check(c, what);
   if (st != PDGPU_OK) return st;
   CK(cudaSetDevice(c.device));
-  st = enqueue_grad_energies(c, what);
+  AdjScratch a;
+  st = adjoint_scratch(c, a);
+  if (st == PDGPU_OK) st = enqueue_grad_energies(c, what, a);
   if (st != PDGPU_OK) return st;
-  return launch_adjoint(c, what, g->charge, g->radius, g->epsilon, g->gb_radius, g->gb_vj, g->gb_terms123);
+  return launch_adjoint(c, what, a, g->charge, g->radius, g->epsilon, g->gb_radius, g->gb_vj, g->gb_terms123);
 }
 
 int pdgpu_param_grad_device_noalloc(pdgpu_ctx* h, unsigned what, const pdgpu_param_grads* g) {
@@ -858,11 +866,14 @@ int pdgpu_param_grad_device_noalloc(pdgpu_ctx* h, unsigned what, const pdgpu_par
   if (st != PDGPU_OK) return st;
   if (c.nslots > kNoAllocMaxSlots) return PDGPU_ERR_CAPACITY;
   CK(cudaSetDevice(c.device));
+  AdjScratch a;
+  st = adjoint_scratch_static(c, a);
+  if (st != PDGPU_OK) return st;
   c.no_alloc = true;
-  st = enqueue_grad_energies(c, what);
+  st = enqueue_grad_energies(c, what, a);
   c.no_alloc = false;
   if (st != PDGPU_OK) return st;
-  return launch_adjoint_static(c, what, g->charge, g->radius, g->epsilon, g->gb_radius, g->gb_vj, g->gb_terms123);
+  return launch_adjoint(c, what, a, g->charge, g->radius, g->epsilon, g->gb_radius, g->gb_vj, g->gb_terms123);
 }
 
 int pdgpu_param_grad(pdgpu_ctx* h, unsigned what, pdgpu_energies* out, const pdgpu_param_grads* g) {
@@ -876,9 +887,11 @@ int pdgpu_param_grad(pdgpu_ctx* h, unsigned what, pdgpu_energies* out, const pdg
   double* host[6] = {g->charge, g->radius, g->epsilon, g->gb_radius, g->gb_vj, g->gb_terms123};
   double* dev[6];
   for (int k = 0; k < 6; k++) dev[k] = host[k] ? c.d_adj_out.p + k * N : nullptr;
-  st = enqueue_grad_energies(c, what);
+  AdjScratch a;
+  st = adjoint_scratch(c, a);
+  if (st == PDGPU_OK) st = enqueue_grad_energies(c, what, a);
   if (st != PDGPU_OK) return st;
-  st = launch_adjoint(c, what, dev[0], dev[1], dev[2], dev[3], dev[4], dev[5]);
+  st = launch_adjoint(c, what, a, dev[0], dev[1], dev[2], dev[3], dev[4], dev[5]);
   if (st != PDGPU_OK) return st;
   for (int k = 0; k < 6; k++)
     if (host[k]) CK(cudaMemcpyAsync(host[k], dev[k], N * 8, cudaMemcpyDeviceToHost, c.stream));

@@ -132,6 +132,9 @@ struct GBConst {
   // (K = -4 x the threshold widened by 4e-6 relative); charges scaled by
   // sqrt(econv_out) (the held atoms' by its negative), sqrt(eps) by sqrt(12);
   // gb_ep: premul q q fgb per scaled charges' product -econv_out q q
+  // far_inner: the smallest inner cutoff where it is 64 A or more (0 otherwise):
+  // tiles inside it are worth finding by their blocks' radii (tile_full_now)
+  float far_inner;
   float sqrtK, inv_sqrtK, invK, kU, sq_eout, neg_sq_eout, in_over_out, sqrt12, gb_ep;
 };
 
@@ -310,15 +313,22 @@ int launch_lcpo(Context& c, long long* facc_out, long long* esurf_out, int esurf
 // FP32 remainders of the packed slots (double-float positions and parameters), before an energy pass
 int launch_df_records(Context& c);
 int launch_gb_stage(Context& c, const GBConst& k, int stage);
-// parameter gradients after an energy evaluation of NB or GB (device outputs,
-// original atom order, J per parameter unit; null pointers are skipped)
-int launch_adjoint(Context& c, unsigned what, double* d_q, double* d_r, double* d_e, double* d_R, double* d_V,
-                   double* d_T);
-// the same into a static device array: no allocation during the call (at most
-// kNoAllocMaxSlots sorted slots; one scratch per device shared by all contexts)
+// parameter gradients (device outputs, original atom order, J per parameter unit;
+// null pointers are skipped): scratch, cleared, filled by the energy pass of NB or
+// GB (GB: the pair terms' gradients, launch_adj_gb_pair) and finished here
+struct AdjScratch {
+  long long* g = nullptr;   // fixed-point sums, 5 per slot
+  float* w = nullptr;       // dE/dGpol per slot
+};
+int adjoint_scratch(Context& c, AdjScratch& a);
+// a static device array: no allocation during the call (at most kNoAllocMaxSlots
+// sorted slots; one scratch per device shared by all contexts)
 constexpr int kNoAllocMaxSlots = 65536;
-int launch_adjoint_static(Context& c, unsigned what, double* d_q, double* d_r, double* d_e, double* d_R, double* d_V,
-                          double* d_T);
+int adjoint_scratch_static(Context& c, AdjScratch& a);
+int clear_adjoint(Context& c, const AdjScratch& a);
+int launch_adj_gb_pair(Context& c, const GBConst& k);
+int launch_adjoint(Context& c, unsigned what, const AdjScratch& a, double* d_q, double* d_r, double* d_e, double* d_R,
+                   double* d_V, double* d_T);
 // Monte Carlo partial NB energies: take the reference from the last energy
 // evaluation / update it by the pairs of the moved atoms
 int launch_mc_reference(Context& c);

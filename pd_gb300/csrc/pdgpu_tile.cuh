@@ -69,6 +69,38 @@ __device__ __forceinline__ void df_offset(const DevView& v, const SystemInfo& S,
   }
 }
 
+// Whether every pair of the tile lies inside every GB cutoff and switch radius at
+// the current positions: by the list's flag, or (lists without the displacement
+// check carry none) from the blocks' radii where the cutoffs are far away
+// (GBConst::far_inner).  xj: in the i block's frame; every lane calls this.
+__device__ __forceinline__ bool tile_full_now(const GBConst& k, const Tile& T, const float4& xi, const float4& xj) {
+  if (tile_full(T)) return true;
+  if (k.far_inner <= 0.f) return false;
+  float a = xi.x * xi.x + xi.y * xi.y + xi.z * xi.z, b = xj.x * xj.x + xj.y * xj.y + xj.z * xj.z;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, o));
+    b = fmaxf(b, __shfl_xor_sync(0xffffffffu, b, o));
+  }
+  return sqrtf(a) + sqrtf(b) + 1e-3f < k.far_inner;   // |x_i| + |x_j| bounds every distance
+}
+
+// the exp-approximation switch is discontinuous: pairs within FP32 rounding of
+// the threshold are decided in FP64
+static __device__ __noinline__ bool gb_on_fp64(const DevView& v, int si, int sj, double thresh) {
+  int a = v.sorted_atom[si], b = v.sorted_atom[sj];
+  if (a < 0 || b < 0) return false;
+  return -0.25 * r2_slots_fp64(v, si, sj) / (v.born[a] * v.born[b]) > thresh;
+}
+
+// 1 / x by the special-function unit alone (rcp.approx.ftz, ~1 ulp): the pair
+// terms' reciprocals of r^2 (no multiply by the numerator 1 as __fdividef has)
+__device__ __forceinline__ float rcp_ftz(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
 // bond order of an atom pair as PD's list stores it; 7 when not bonded
 __device__ __forceinline__ int pair_bondorder(const DevView& v, int a, int b) {
   int lo = a < b ? a : b, hi = a < b ? b : a;
