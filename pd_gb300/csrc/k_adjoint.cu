@@ -15,13 +15,13 @@
 //
 // Layout: the same tiles and slots as the force kernels.  Pair distances and
 // most pair terms are FP32; for FF_NonBonded the Coulomb energy per unit charge
-// product is formed in FP64 (the force-switch form cancels badly in FP32).  A
-// charge gradient is a potential: a sum of many terms of both signs, which plain
-// FP32 sums do not resolve to the 1e-4 a parameter fit checks against.  The GB
+// product is formed in double-float (the force-switch form cancels badly in FP32).
+// A charge gradient is a potential: a sum of many terms of both signs, which plain
+// FP32 sums do not resolve to the 1e-4 a parameter fit checks against.  The
 // kernels therefore sum per tile in compensated FP32 (value plus running
 // rounding error, about 48 significant bits, on the FP32 pipe: GB300's FP64 rate
 // is a small fraction of its FP32 rate), fed by plain FP32 sums over 8 rotation
-// steps; the NB kernel sums in FP64.  Per-tile sums enter 64-bit fixed point (2^32
+// steps (FF_NonBonded's charge gradients: by every term).  Per-tile sums enter 64-bit fixed point (2^32
 // per kcal/mol per parameter unit), so the result does not depend on scheduling.
 #include "pdgpu_tile.cuh"
 
@@ -422,12 +422,37 @@ __global__ void k_adj_w(DevView v, const double* terms123, const long long* gpol
 }
 
 // ---------------------------------------------------------------------------
-// NB (FF_NonBonded) pair terms: dE/dq, dE/dRmin, dE/dsqrt(eps)
+// NB (FF_NonBonded) pair terms: dE/dq, dE/dRmin, dE/dsqrt(eps).  The Coulomb
+// energy per unit charge product is formed in double-float from the FP32 distance
+// and its sums are double-float; the LJ terms are FP32, summed over 8 steps and
+// then compensated.  (In FP64, with FP64 sums on the rotation, the pass took
+// 751 us on 4 frames of 1,094 waters, bound by the FP64 pipe; 120 us so.)
 // ---------------------------------------------------------------------------
+// Coulomb energy of a pair per unit q q econv (elec14 aside): nb_pair's law
+template <int ELEC>
+__device__ __forceinline__ DF nb_phi_df(const NBEConst& e, float r2f) {
+  const DF r2 = DF{r2f, 0.f}, ir = df_rsqrt(r2);
+  if (ELEC == 1) return ir;
+  const DF r = df_norm(df_mul(r2, ir));
+  const DF w = df_norm(df_sub(r, e.inner));
+  if (ELEC == 3) {
+    if (w.h <= 0.f) return ir;
+    const DF s = df_norm(df_sub(DF{1.f, 0.f}, df_mul(w, df_norm(df_mul(w, e.invw2)))));
+    return df_norm(df_mul(ir, df_norm(df_mul(s, s))));
+  }
+  // Steinbach & Brooks force switch, nonbonded.cpp:798-819
+  if (w.h <= 0.f) return df_norm(df_sub(ir, e.eshift));
+  DF h = df_norm(df_add(e.sD, df_mul(e.sE, r2)));
+  h = df_norm(df_add(e.sC, df_mul(h, r2)));
+  h = df_norm(df_add(df_mul(h, r), df_mul(e.sB, ir)));
+  return df_norm(df_sub(e.cutV, df_mul(e.sA, h)));
+}
+
 template <int ELEC, bool MASKED>
-__device__ __forceinline__ void adj_nb_tile(const DevView& v, const NBConst& k, const Tile& T, const SystemInfo& S,
-                                            int lane, int si, const float4& xi, const float4& pi, unsigned ex,
-                                            unsigned m14, Acc3& I, Acc3& J) {
+__device__ __forceinline__ void adj_nb_tile(const DevView& v, const NBConst& k, const Tile& T, const NBEConst& e,
+                                            const SystemInfo& S, int lane, int si, const float4& xi, const float4& pi,
+                                            unsigned ex, unsigned m14, CAcc3& I, CAcc3& J) {
+  float ib = 0.f, ic = 0.f, jb = 0.f, jc = 0.f;   // LJ sums of 8 steps (the j atom's rotate with it)
   float4 xj = v.xq[T.bj * 32 + lane];
   float4 pj = v.par[T.bj * 32 + lane];
   float Lx = 1.f, Ly = 1.f, Lz = 1.f;
@@ -459,15 +484,15 @@ __device__ __forceinline__ void adj_nb_tile(const DevView& v, const NBConst& k, 
     if (listed && in) {
       const bool is14 = MASKED && ((m14 >> kk) & 1u);
       const float sv = is14 ? k.vdw14 : 1.f;
-      float ev = 0.f, ee = 0.f, fs, rd;
-      // unit sqrt(eps_i) sqrt(eps_j) and unit q_i q_j: both terms are linear in them
-      nb_pair<float, ELEC>(k, r2, pi.x + pj.x, sv, 0.f, ev, ee, fs, rd);
-      double evd = 0.0, eed = 0.0, fsd, rdd;
-      nb_pair<double, ELEC>(k, (double)r2, 0.0, 0.0, (is14 ? k.elec14_d : 1.0) * k.econv_diel_d, evd, eed, fsd, rdd);
-      I.a += eed * (double)xj.w;
-      J.a += eed * (double)xi.w;
-      I.c += (double)(ev * pj.y);
-      J.c += (double)(ev * pi.y);
+      if (ELEC != 0) {
+        DF phi = df_norm(df_mul(nb_phi_df<ELEC>(e, r2), e.econv));
+        if (is14) phi = df_norm(df_mul(phi, e.elec14));
+        const DF a = df_norm(df_scale(phi, xj.w)), b = df_norm(df_scale(phi, xi.w));
+        csum_add(I.a, a.h);
+        I.a.lo = __fadd_rn(I.a.lo, a.l);
+        csum_add(J.a, b.h);
+        J.a.lo = __fadd_rn(J.a.lo, b.l);
+      }
       const float invr = rsqrtf(r2), r = r2 * invr;
       if (k.dovdw && r < (float)k.vdwcut_d) {
         float Sv = sv;
@@ -476,18 +501,30 @@ __device__ __forceinline__ void adj_nb_tile(const DevView& v, const NBConst& k, 
           const float sw = 1.f - u * u * (float)k.vdwinvw2_d;
           Sv *= sw * sw;
         }
-        const float dR = lj_dR(pi.x + pj.x, invr) * Sv * pi.y * pj.y;
-        I.b += (double)dR;
-        J.b += (double)dR;
+        const float R = pi.x + pj.x, t2 = R * R * invr * invr, B = t2 * t2 * t2;
+        const float dR = lj_dR(R, invr) * Sv * pi.y * pj.y;
+        const float e1 = (B * B - 2.f * B) * Sv;   // energy per unit sqrt(eps_i) sqrt(eps_j)
+        ib += dR;
+        jb += dR;
+        ic += e1 * pj.y;
+        jc += e1 * pi.y;
       }
     }
     ROT(xj.x); ROT(xj.y); ROT(xj.z); ROT(xj.w); ROT(pj.x); ROT(pj.y);
-    ROT(J.a); ROT(J.b); ROT(J.c);
+    ROT(J.a.hi); ROT(J.a.lo); ROT(jb); ROT(jc);
+    if ((kk & 7) == 7) {
+      csum_add(I.b, ib);
+      csum_add(I.c, ic);
+      // the j atom now at this lane lives in lane + kk + 1: its sums go home
+      csum_add(J.b, __shfl_sync(0xffffffffu, jb, (lane - kk - 1) & 31));
+      csum_add(J.c, __shfl_sync(0xffffffffu, jc, (lane - kk - 1) & 31));
+      ib = ic = jb = jc = 0.f;
+    }
   }
 }
 
 template <int ELEC>
-__global__ void __launch_bounds__(256) k_adj_nb(const __grid_constant__ DevView v, const __grid_constant__ NBConst k, long long* gq, long long* gr, long long* ge) {
+__global__ void __launch_bounds__(256) k_adj_nb(const __grid_constant__ DevView v, const __grid_constant__ NBConst k, const __grid_constant__ NBEConst e, long long* gq, long long* gr, long long* ge) {
   const int lane = threadIdx.x & 31;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   const int nt = *v.ntiles;
@@ -503,9 +540,9 @@ __global__ void __launch_bounds__(256) k_adj_nb(const __grid_constant__ DevView 
       m14 = m.y;
     }
     if (T.flags & 2) ex |= diag_exclusion(lane);
-    Acc3 I = {0.0, 0.0, 0.0}, J = {0.0, 0.0, 0.0};
-    if (tile_masked(T)) adj_nb_tile<ELEC, true>(v, k, T, S, lane, si, xi, pi, ex, m14, I, J);
-    else adj_nb_tile<ELEC, false>(v, k, T, S, lane, si, xi, pi, ex, m14, I, J);
+    CAcc3 I = {}, J = {};
+    if (tile_masked(T)) adj_nb_tile<ELEC, true>(v, k, T, e, S, lane, si, xi, pi, ex, m14, I, J);
+    else adj_nb_tile<ELEC, false>(v, k, T, e, S, lane, si, xi, pi, ex, m14, I, J);
     acc_flush(v, gq, gr, ge, si, I);
     acc_flush(v, gq, gr, ge, T.bj * 32 + lane, J);
   }
@@ -562,13 +599,14 @@ int launch_adjoint(Context& c, unsigned what, const AdjScratch& a, double* d_q, 
     k_adj_born<<<2 * grid, kAdjThreads, 0, st>>>(v, k, a.w, g + G_GBR * (size_t)ns, g + G_VJ * (size_t)ns);
   } else {
     long long *gq = g + G_Q * (size_t)ns, *gr = g + G_R * (size_t)ns, *ge = g + G_EPS * (size_t)ns;
-    NBConst k = make_nb_const(c.nb);
+    const NBConst k = make_nb_const(c.nb);
+    const NBEConst e = make_nbe_const(k);
     c.kernel_launches += 1;
     switch (k.elecmode) {
-      case 0: k_adj_nb<0><<<grid, 256, 0, st>>>(v, k, gq, gr, ge); break;
-      case 1: k_adj_nb<1><<<grid, 256, 0, st>>>(v, k, gq, gr, ge); break;
-      case 3: k_adj_nb<3><<<grid, 256, 0, st>>>(v, k, gq, gr, ge); break;
-      default: k_adj_nb<4><<<grid, 256, 0, st>>>(v, k, gq, gr, ge); break;
+      case 0: k_adj_nb<0><<<grid, 256, 0, st>>>(v, k, e, gq, gr, ge); break;
+      case 1: k_adj_nb<1><<<grid, 256, 0, st>>>(v, k, e, gq, gr, ge); break;
+      case 3: k_adj_nb<3><<<grid, 256, 0, st>>>(v, k, e, gq, gr, ge); break;
+      default: k_adj_nb<4><<<grid, 256, 0, st>>>(v, k, e, gq, gr, ge); break;
     }
   }
   AdjOut o = {d_q, d_r, d_e, d_R, d_V, d_T};
