@@ -201,8 +201,9 @@ int launch_bonded(Context& c, bool energy) {
   b.bpar = c.d_bpar.p; b.apar = c.d_apar.p; b.tpar = c.d_tpar.p; b.ipar = c.d_ipar.p;
   int total = c.nbond + c.nangle + c.ntors + c.nimpr;
   if (total == 0) return PDGPU_OK;
-  if (energy) k_bonded<true><<<(total + 255) / 256, 256, 0, c.stream>>>(b);
-  else k_bonded<false><<<(total + 255) / 256, 256, 0, c.stream>>>(b);
+  const Spread sp = spread(total);
+  if (energy) k_bonded<true><<<sp.grid, sp.threads, 0, c.stream>>>(b);
+  else k_bonded<false><<<sp.grid, sp.threads, 0, c.stream>>>(b);
   return cudaGetLastError() == cudaSuccess ? PDGPU_OK : PDGPU_ERR_CUDA;
 }
 

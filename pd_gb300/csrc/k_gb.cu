@@ -1038,9 +1038,9 @@ int launch_gb(Context& c, const GBConst& k, double halfeconv, double born_offset
   DevView v = c.view();
   cudaStream_t st = c.stream;
   int g = tile_grid(c);
-  int nb = (c.nslots + 255) / 256;
+  const Spread sp = spread(c.nslots);
   launch_pdl(st, g, kBornThreads, 0, k_gb_born, v, k, c.d_gpol.p);
-  launch_pdl(st, nb, 256, 0, k_gb_radii, v, c.d_gbT.p, c.d_gpol.p, halfeconv, born_offset, c.d_born_f.p, c.d_born_d.p);
+  launch_pdl(st, sp.grid, sp.threads, 0, k_gb_radii, v, c.d_gbT.p, c.d_gpol.p, halfeconv, born_offset, c.d_born_f.p, c.d_born_d.p);
   const int gp = g * (256 / kPairThreads), ge = g * (256 / kPairEThreads);
   if (c.gb_no_chain) {
     // a gradient call: energies (FP32 pair terms: they weight a loss), dE/da and the
@@ -1057,7 +1057,7 @@ int launch_gb(Context& c, const GBConst& k, double halfeconv, double born_offset
   } else {
     launch_pdl(st, gp, kPairThreads, 0, k_gb_pair<true>, v, k, c.d_born_f.p, c.d_deda.p);
   }
-  launch_pdl(st, nb, 256, 0, k_gb_self, v, c.d_charge.p, k, premul, c.d_deda.p, c.d_born_d.p, c.d_chain_f.p,
+  launch_pdl(st, sp.grid, sp.threads, 0, k_gb_self, v, c.d_charge.p, k, premul, c.d_deda.p, c.d_born_d.p, c.d_chain_f.p,
                                 energy ? 1 : 0);
   if (c.gb_no_chain) c.kernel_launches -= 1;
   else launch_pdl(st, 2 * g, kChainThreads, 0, k_gb_chain, v, k, c.d_chain_f.p);

@@ -317,9 +317,9 @@ __global__ void k_zero_ll(long long* p, size_t n) {
 int launch_integrate(Context& c, MDState& md, bool first, bool last) {
   c.kernel_launches += 1;
   MDView m = md_view(c, md);
-  int nb = (c.natom + 255) / 256;
-  if (md.p.Integrator == 0) k_vv<<<nb, 256, 0, c.stream>>>(m, md.p.Timestep);
-  else k_langevin<<<nb, 256, 0, c.stream>>>(m, md.L, first ? 1 : 0, last ? 1 : 0);
+  const Spread sp = spread(c.natom);
+  if (md.p.Integrator == 0) k_vv<<<sp.grid, sp.threads, 0, c.stream>>>(m, md.p.Timestep);
+  else k_langevin<<<sp.grid, sp.threads, 0, c.stream>>>(m, md.L, first ? 1 : 0, last ? 1 : 0);
   return cudaGetLastError() == cudaSuccess ? PDGPU_OK : PDGPU_ERR_CUDA;
 }
 

@@ -716,7 +716,8 @@ static void launch_nb_mode(Context& c, const NBConst& k, int g) {
 }
 
 int launch_df_records(Context& c) {
-  launch_pdl(c.stream, (c.nslots + 255) / 256, 256, 0, k_df_records, c.view(), c.d_charge.p, c.d_rlo.p, c.d_plo.p);
+  const Spread sp = spread(c.nslots);
+  launch_pdl(c.stream, sp.grid, sp.threads, 0, k_df_records, c.view(), c.d_charge.p, c.d_rlo.p, c.d_plo.p);
   return cudaGetLastError() == cudaSuccess ? PDGPU_OK : PDGPU_ERR_CUDA;
 }
 
@@ -754,7 +755,8 @@ __global__ void k_finalize_forces(DevView v, double* out, size_t stride, int add
 int launch_finalize_forces(Context& c, double* out, size_t stride_doubles, bool add, double scale) {
   c.kernel_launches += 1;
   DevView v = c.view();
-  k_finalize_forces<<<(c.nslots + 255) / 256, 256, 0, c.stream>>>(v, out, stride_doubles, add ? 1 : 0, scale);
+  const Spread sp = spread(c.nslots);
+  k_finalize_forces<<<sp.grid, sp.threads, 0, c.stream>>>(v, out, stride_doubles, add ? 1 : 0, scale);
   return cudaGetLastError() == cudaSuccess ? PDGPU_OK : PDGPU_ERR_CUDA;
 }
 
