@@ -11,6 +11,7 @@
 #include <algorithm>
 
 #include "pdgpu_tile.cuh"
+#include "pdgpu_pack.cuh"
 
 namespace pdgpu {
 
@@ -285,40 +286,6 @@ __global__ void k_cell_sort(DevView v, int ncells, const int* offset, const int*
   }
 }
 
-// boxes of each 8 slots at the packed positions (a padding slot widens its box:
-// it never hides an atom); every lane of the warp calls this
-__device__ __forceinline__ void write_sub(const DevView& v, int s, const float4& o) {
-  float4 lo = o, hi = o;
-#pragma unroll
-  for (int d = 4; d > 0; d >>= 1) {
-    lo.x = fminf(lo.x, __shfl_xor_sync(0xffffffffu, lo.x, d));
-    lo.y = fminf(lo.y, __shfl_xor_sync(0xffffffffu, lo.y, d));
-    lo.z = fminf(lo.z, __shfl_xor_sync(0xffffffffu, lo.z, d));
-    hi.x = fmaxf(hi.x, __shfl_xor_sync(0xffffffffu, hi.x, d));
-    hi.y = fmaxf(hi.y, __shfl_xor_sync(0xffffffffu, hi.y, d));
-    hi.z = fmaxf(hi.z, __shfl_xor_sync(0xffffffffu, hi.z, d));
-  }
-  if ((s & 7) == 0) {
-    v.sub[s >> 2] = lo;
-    v.sub[(s >> 2) + 1] = hi;
-  }
-}
-
-// slot s of atom a (-1: padding): FP64 position -> FP32 offset from the block centre
-__device__ __forceinline__ float4 packed_slot(const DevView& v, const SystemInfo& S, const double* charge, int s, int a,
-                                              const double c[3]) {
-  // padding slot: zero parameters, parked far away from everything and each other
-  if (a < 0) return make_float4(1.0e6f * (float)(1 + (s & 31)), 1.0e6f * (float)(1 + (s >> 5)), -1.0e6f, 0.f);
-  double r[3];
-#pragma unroll
-  for (int k = 0; k < 3; k++) {
-    double d = v.pos[3 * a + k] - c[k];
-    if (S.periodic) d -= S.box[k] * rint(d * S.ibox[k]);
-    r[k] = d;
-  }
-  return make_float4((float)r[0], (float)r[1], (float)r[2], (float)charge[a]);
-}
-
 // cell coordinate of x along axis c (clamped into the grid)
 __device__ __forceinline__ int grid_axis(const BlockGrid& G, int c, double x) {
   const double q = floor((x - G.origin[c]) / G.cell[c]);
@@ -388,7 +355,7 @@ __global__ void __launch_bounds__(128) k_blocks(DevView v, SlotParams P, StepCle
     cd[c] = (double)cf[c];
     hf[c] = fmaxf(hi[c] - cf[c], cf[c] - lo[c]) + 1e-4f + 2.4e-7f * fmaxf(fabsf(lo[c]), fabsf(hi[c]));
   }
-  const float4 o = packed_slot(v, S, P.charge, slot, a, cd);
+  const float4 o = packed_slot(v, S, P.charge, slot, a, v.pos + 3 * (a < 0 ? 0 : a), cd);
   v.xq[slot] = o;
   v.rel0[slot] = o;
   if (sub) write_sub(v, slot, o);
@@ -769,32 +736,12 @@ __global__ void k_masks(DevView v, const int* mlist, const int* nml, const int* 
 }
 
 // per-evaluation pack (between list builds): the slots at the current positions
-// check2: squared skin limit (0 = no skin check); full2: squared limit that keeps
-// tiles flagged full valid (0 = none flagged), checked where the skin check is not
-// cull: the NB j-atom groups are in use (the displacement check always runs)
-__global__ void k_pack(DevView v, const double* charge, StepClear C, float check2, float full2, long long npairs_all,
-                       int cull) {
+__global__ void k_pack(DevView v, PackArgs P) {
   pdl_sync();
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= v.nslots) return;   // (whole warps)
-  const int a = v.sorted_atom[s], b = s >> 5;
-  const SystemInfo& S = v.sys[v.slot_sys[b]];
-  const double c[3] = {v.center[3 * b], v.center[3 * b + 1], v.center[3 * b + 2]};
-  const float4 o = packed_slot(v, S, charge, s, a, c);
-  if (a >= 0) {
-    // (in open space, when every block pair of every system is a tile, no pair
-    // can leave the list; in a periodic box the tile images still depend on it)
-    const bool skin = check2 > 0.f && (S.periodic || (long long)*v.ntiles < npairs_all || cull);
-    const float lim = skin ? check2 : full2;
-    if (lim > 0.f) {
-      float4 q = v.rel0[s];
-      float dx = o.x - q.x, dy = o.y - q.y, dz = o.z - q.z;
-      if (dx * dx + dy * dy + dz * dz > lim) atomicOr(v.status, (unsigned)ST_STALE_LIST);
-    }
-  }
-  v.xq[s] = o;
-  if (cull) write_sub(v, s, o);
-  step_clear(C, v, s);
+  const int a = v.sorted_atom[s];
+  pack_slot(v, P, s, a, v.pos + 3 * (a < 0 ? 0 : a));
 }
 
 // GB work items, one warp per row: the row's all-inside tiles without exclusion
@@ -1086,17 +1033,24 @@ int launch_slot_params(Context& c) {
   return cudaGetLastError() == cudaSuccess ? PDGPU_OK : PDGPU_ERR_CUDA;
 }
 
-int launch_pack(Context& c, float check_disp) {
-  c.kernel_launches += 1;
-  DevView v = c.view();
-  float c2 = check_disp > 0 ? check_disp * check_disp : 0.f;
-  float f2 = 0.f;
+PackArgs pack_args(const Context& c, float check_disp) {
+  PackArgs P{};
+  P.charge = c.d_charge.p;
+  P.clear = c.clear;
+  P.check2 = check_disp > 0 ? check_disp * check_disp : 0.f;
   if (c.full_radius_built > 0.f) {
     const float h = 0.5f * c.full_margin();
-    f2 = h * h;
+    P.full2 = h * h;
   }
+  P.npairs_all = c.npairs_all;
+  P.cull = c.cull_built ? 1 : 0;
+  return P;
+}
+
+int launch_pack(Context& c, float check_disp) {
+  c.kernel_launches += 1;
   const Spread sp = spread(c.nslots, 64);   // (32: 1 us a step slower at 2,001 atoms)
-  launch_pdl(c.stream, sp.grid, sp.threads, 0, k_pack, v, c.d_charge.p, c.clear, c2, f2, c.npairs_all, c.cull_built ? 1 : 0);
+  launch_pdl(c.stream, sp.grid, sp.threads, 0, k_pack, c.view(), pack_args(c, check_disp));
   return cudaGetLastError() == cudaSuccess ? PDGPU_OK : PDGPU_ERR_CUDA;
 }
 

@@ -10,6 +10,7 @@
 #include <new>
 
 #include "pdgpu_context.cuh"
+#include "pdgpu_pack.cuh"
 
 using namespace pdgpu;
 
@@ -996,7 +997,8 @@ int pdgpu_rebuild_list(pdgpu_ctx* h) {
 // One force evaluation on the context stream (no host synchronisation).
 // rebuild: rebuild the list first (else pack the positions and check the skin).
 // LCPO forces go to lcpo_f and its energy to lcpo_e (stride lcpo_e_stride) when
-// run_lcpo; dynamics points them at the cached-LCPO buffers.
+// run_lcpo; dynamics points them at the cached-LCPO buffers.  packed: the last
+// integrator packed the positions and cleared the accumulators already.
 // (set-up failure) the context's streams and events
 void pdgpu::release_streams(Context& c) {
   if (c.ev_fork) cudaEventDestroy(c.ev_fork);
@@ -1011,13 +1013,14 @@ void pdgpu::release_streams(Context& c) {
 }
 
 int pdgpu::enqueue_forces(Context& c, unsigned what, bool energy, bool rebuild, long long* lcpo_f,
-                          long long* lcpo_e, int lcpo_e_stride, bool run_lcpo) {
+                          long long* lcpo_e, int lcpo_e_stride, bool run_lcpo, bool packed) {
   c.clear.facc = c.d_facc.p;
   c.clear.gpol = (what & PDGPU_GB) ? c.d_gpol.p : nullptr;
   c.clear.deda = (what & PDGPU_GB) ? c.d_deda.p : nullptr;
   c.clear.eacc = energy ? c.d_eacc.p : nullptr;
-  int st = rebuild || !c.list_built ? rebuild_list_impl(c)
-                                    : launch_pack(c, c.lp.check_skin ? (float)(0.5 * c.lp.Padding) : 0.f);
+  int st = packed                     ? PDGPU_OK
+           : rebuild || !c.list_built ? rebuild_list_impl(c)
+                                      : launch_pack(c, skin_disp(c));
   c.clear = StepClear{};
   if (st != PDGPU_OK) return st;
   // the LCPO recalculation (positions, packed slots and tile list) and the bonded

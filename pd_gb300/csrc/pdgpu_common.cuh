@@ -349,7 +349,7 @@ int launch_finalize_forces(Context& c, double* out, size_t stride_doubles, bool 
 int rebuild_list_impl(Context& c);
 void release_streams(Context& c);
 int enqueue_forces(Context& c, unsigned what, bool energy, bool rebuild, long long* lcpo_f, long long* lcpo_e,
-                   int lcpo_e_stride, bool run_lcpo);
+                   int lcpo_e_stride, bool run_lcpo, bool packed = false);
 struct MDState;
 void destroy_md(Context& c);
 // captured step graphs hold buffer addresses: dropped when a buffer is replaced

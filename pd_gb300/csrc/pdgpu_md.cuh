@@ -44,8 +44,12 @@ struct MDState {
   int traj_slots = 0;
   long long traj_frames = 0;
   bool force_sasa = false;            // recompute LCPO at the next step
+  // captured steps: a flavour's single step, or a run of it and plain steps after it
+  // (key: flags | steps << 3)
   std::map<int, cudaGraphExec_t> graphs;
-  std::map<int, long long> graph_kernels;  // kernel nodes of each captured flavour
+  std::map<int, long long> graph_kernels;  // kernel nodes of each captured run
+  long long replayed = 0;             // steps replayed since the graphs were last dropped
+  bool runs = true;                   // capture runs of several steps (off while autotuning)
 };
 
 struct MDView {
@@ -85,6 +89,7 @@ inline MDView md_view(Context& c, MDState& md) {
 }
 
 int launch_integrate(Context& c, MDState& md, bool first, bool last);
+int launch_integrate_pack(Context& c, MDState& md);
 int launch_remd(Context& c, MDState& md, int parity, unsigned long long round);
 int launch_zero_ll(Context& c, long long* p, size_t n);
 // crash rescue: flags non-finite systems into bad_host (nsys ints, synchronous)

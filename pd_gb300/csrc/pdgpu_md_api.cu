@@ -5,7 +5,8 @@
 // components, LCPO on its UpdateSasa cadence (its forces and energy cached in
 // between, as FF_SASA_LCPO::calcForces does, lcpo.cpp:193-206), then the
 // integrator.  The step sequence of each distinct flavour (rebuild / LCPO /
-// energy) is captured once into a CUDA graph and replayed.
+// energy) is captured once into a CUDA graph and replayed; longer dynamics capture
+// runs of plain steps.
 #include <algorithm>
 #include <chrono>
 #include <cmath>
@@ -32,6 +33,7 @@ void drop_step_graphs(Context& c) {
   if (!c.md) return;
   for (auto& kv : c.md->graphs) cudaGraphExecDestroy(kv.second);
   c.md->graphs.clear();
+  c.md->replayed = 0;
 }
 
 }  // namespace pdgpu
@@ -47,6 +49,7 @@ namespace {
 void invalidate_graphs(MDState& md) {
   for (auto& kv : md.graphs) cudaGraphExecDestroy(kv.second);
   md.graphs.clear();
+  md.replayed = 0;
 }
 
 // per-atom mass terms of the integrators: 1 / m and sqrt(k_B / m) (md.cpp:951-960)
@@ -67,7 +70,8 @@ __global__ void k_add_surf(long long* eacc, const long long* cache, int nsys) {
 }
 
 // enqueue one step; flags: 1 rebuild, 2 LCPO recalculation, 4 energies
-int enqueue_step(Context& c, MDState& md, int flags, bool first) {
+// packed: the step before packed the positions; pack_next: the next step is plain
+int enqueue_step(Context& c, MDState& md, int flags, bool first, bool packed = false, bool pack_next = false) {
   const bool rebuild = flags & 1, sasa = flags & 2, energy = flags & 4;
   const bool has_sa = md.p.what & PDGPU_SA;
   c.clear.ke = md.d_ke.p;
@@ -75,25 +79,35 @@ int enqueue_step(Context& c, MDState& md, int flags, bool first) {
     c.clear.facc2 = md.d_facc_sa.p;
     c.clear.surf = md.d_surf_cache.p;
   }
-  int st = enqueue_forces(c, md.p.what, energy, rebuild, md.d_facc_sa.p, md.d_surf_cache.p, 1, sasa);
+  int st = enqueue_forces(c, md.p.what, energy, rebuild, md.d_facc_sa.p, md.d_surf_cache.p, 1, sasa, packed);
   if (st != PDGPU_OK) return st;
   if (has_sa && energy) {
     k_add_surf<<<(c.nsys + 127) / 128, 128, 0, c.stream>>>(c.d_eacc.p, md.d_surf_cache.p, c.nsys);
     c.kernel_launches += 1;
     CK(cudaGetLastError());
   }
-  return launch_integrate(c, md, first, false);
+  if (!pack_next) return launch_integrate(c, md, first, false);
+  c.clear.facc = c.d_facc.p;   // (what enqueue_forces has a plain step's pack clear)
+  c.clear.gpol = (md.p.what & PDGPU_GB) ? c.d_gpol.p : nullptr;
+  c.clear.deda = (md.p.what & PDGPU_GB) ? c.d_deda.p : nullptr;
+  st = launch_integrate_pack(c, md);
+  c.clear = StepClear{};
+  return st;
 }
 
-int run_step(Context& c, MDState& md, int flags, bool first) {
-  if (!md.p.use_graph || first) return enqueue_step(c, md, flags, first);
-  auto it = md.graphs.find(flags);
+// n steps, the first of flavour `flags`, the others plain
+int run_steps(Context& c, MDState& md, int flags, int n, bool first) {
+  if (!md.p.use_graph || first) return enqueue_step(c, md, flags, first);   // (n is 1)
+  const int key = flags | n << 3;
+  auto it = md.graphs.find(key);
   if (it == md.graphs.end()) {
     cudaGraph_t g = nullptr;
     CK(cudaStreamBeginCapture(c.stream, cudaStreamCaptureModeThreadLocal));
     const long long before = c.kernel_launches;
-    int st = enqueue_step(c, md, flags, false);
-    md.graph_kernels[flags] = c.kernel_launches - before;
+    int st = PDGPU_OK;
+    for (int i = 0; i < n && st == PDGPU_OK; i++)
+      st = enqueue_step(c, md, i ? 0 : flags, false, i > 0, i + 1 < n);
+    md.graph_kernels[key] = c.kernel_launches - before;
     c.kernel_launches = before;
     cudaError_t e = cudaStreamEndCapture(c.stream, &g);
     if (st != PDGPU_OK) {
@@ -105,11 +119,43 @@ int run_step(Context& c, MDState& md, int flags, bool first) {
     e = cudaGraphInstantiate(&ex, g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) return PDGPU_ERR_CUDA;
-    it = md.graphs.emplace(flags, ex).first;
+    it = md.graphs.emplace(key, ex).first;
   }
   CK(cudaGraphLaunch(it->second, c.stream));
-  c.kernel_launches += md.graph_kernels[flags];
+  c.kernel_launches += md.graph_kernels[key];
+  md.replayed += n;
   return PDGPU_OK;
+}
+
+int step_flags(const MDState& md, unsigned long long s) {
+  int f = s % (unsigned long long)md.p.UpdateNList == 0 ? 1 : 0;
+  if ((md.p.what & PDGPU_SA) && s % (unsigned long long)md.p.UpdateSasa == 0) f |= 2;
+  return f;
+}
+
+// How many of the next `left` steps (the first of flavour `flags`, none of the rest
+// with energies) run as one captured graph: up to the next step that is not plain,
+// the next trajectory frame or kRunMax.  Where the run ends at `left` instead, the
+// largest power of two, so that callers of any step counts meet few lengths.  A graph
+// of its own costs a step some 3 us of idle GPU and its pack a launch; a run costs
+// ~20 us a step to capture, once, so it pays after a few dozen steps: the first
+// kRunsAfter steps, and what a state with kRunGraphs graphs still meets, go singly.
+constexpr int kRunMax = 16, kRunsAfter = 64, kRunGraphs = 32;
+int run_length(const MDState& md, int flags, int left) {
+  if (!md.p.use_graph || !md.runs || md.replayed < kRunsAfter || (flags & 4)) return 1;
+  int n = 1;
+  bool whole = false;
+  for (;;) {
+    const unsigned long long s = md.step + n;   // the step after the run
+    whole = n == kRunMax || step_flags(md, s) != 0 ||
+            (md.traj_every > 0 && s % (unsigned long long)md.traj_every == 0);
+    if (whole || n >= left) break;
+    n++;
+  }
+  if (!whole)
+    while (n & (n - 1)) n &= n - 1;
+  if (n > 1 && md.graphs.size() >= kRunGraphs && !md.graphs.count(flags | n << 3)) return 1;
+  return n;
 }
 
 LangevinCoeffs coeffs(double gamma, double t) {
@@ -158,18 +204,19 @@ int read_status_md(Context& c) {
 }
 
 int md_enqueue_impl(Context& c, MDState& md, int nsteps, bool energy_on_last) {
-  for (int k = 0; k < nsteps; k++) {
-    const unsigned long long s = md.step;
-    int flags = 0;
-    if (s % (unsigned long long)md.p.UpdateNList == 0 || !c.list_built) flags |= 1;
-    if ((md.p.what & PDGPU_SA) && (s % (unsigned long long)md.p.UpdateSasa == 0 || md.force_sasa)) flags |= 2;
+  for (int k = 0; k < nsteps;) {
+    int flags = step_flags(md, md.step);
+    if (!c.list_built) flags |= 1;
+    if ((md.p.what & PDGPU_SA) && md.force_sasa) flags |= 2;
     md.force_sasa = false;
     if (energy_on_last && k == nsteps - 1) flags |= 4;
-    bool first = !md.trajectory_started;
-    int st = run_step(c, md, flags, first);
+    const bool first = !md.trajectory_started;
+    const int n = first ? 1 : run_length(md, flags, nsteps - k - (energy_on_last ? 1 : 0));
+    int st = run_steps(c, md, flags, n, first);
     if (st != PDGPU_OK) return st;
     md.trajectory_started = true;
-    md.step++;
+    md.step += n;
+    k += n;
     if (md.traj_every > 0 && md.step % (unsigned long long)md.traj_every == 0) {
       // a frame of every system's positions, queued behind the step on the context stream
       double* dst = md.traj_ring + (size_t)(md.traj_frames % md.traj_slots) * 3 * (size_t)c.natom;
@@ -517,6 +564,11 @@ int pdgpu_md_autotune(pdgpu_ctx* h, int trial_steps, int* update_nlist, int* cta
   if (!c.md || !c.md->ready) return PDGPU_ERR_STATE;
   MDState& md = *c.md;
   CK(cudaSetDevice(c.device));
+  struct SingleSteps {   // (capturing runs would fall into some trials' time)
+    MDState& md;
+    explicit SingleSteps(MDState& m) : md(m) { md.runs = false; }
+    ~SingleSteps() { md.runs = true; }
+  } single(md);
   // save the state; every trial starts from it
   const size_t N3 = 3 * (size_t)c.natom;
   DBuf<double> pos0, vel0;
