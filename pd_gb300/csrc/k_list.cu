@@ -10,6 +10,8 @@
 // exclusion / 1-4 bit mask.
 #include <algorithm>
 
+#include <cuda_fp16.h>
+
 #include "pdgpu_tile.cuh"
 #include "pdgpu_pack.cuh"
 
@@ -796,81 +798,170 @@ __global__ void __launch_bounds__(128) k_items(DevView v, int pairs, int far, co
 // like a tile's j block.  Valid while every atom stays within half the skin of
 // its build position (the per-step displacement check, forced on with groups):
 // a pair inside the cutoff then had its j atom within R of the i box at build.
-// The j atoms within the cutoffs themselves come first, those in the skin after
-// them, so that the skin's groups, mostly out of reach, are skipped whole by the
-// force pass.  One CTA per row: its warps take consecutive runs of the row's
-// tiles (entries keep tile order, then lane order), count, take the row's groups
-// by an atomic on the total (rows in any order: every sum is in fixed point) and
-// write.  A row's groups are an even number (the force pass takes two at once).
+// The row's j atoms go by class: which of the block's four 8-atom sub-blocks lie
+// within the cutoffs of the atom, in Gray-code order, so that a group's atoms reach
+// the same sub-blocks and the force pass skips the others; those in the skin alone
+// (no sub-block) come last.  Sorted this way a solvated box of 22,489 atoms at 12 A
+// computes 2.2 pairs per pair inside the cutoff instead of 3.0 (within the cutoffs
+// first, then the skin) and 4.4 (unskipped).  One CTA per row: its warps take
+// consecutive runs of the row's tiles, count, take the row's groups by an atomic on
+// the total (rows in any order: every sum is in fixed point) and write; a class keeps
+// tile order, then lane order.  A row's groups are an even number (the force pass
+// takes two at once).
 // ---------------------------------------------------------------------------
-constexpr int kCullWarps = 8;
-__global__ void __launch_bounds__(kCullWarps * 32) k_cull(DevView v, float R2, float Rc2, const int* row_start,
-                                                          const int* row_cnt, uint2* jmask) {
+constexpr int kCullClasses = 16;
+// class c holds the atoms that reach the sub-blocks of Gray code c + 1 (the last: none)
+__device__ __forceinline__ unsigned cull_code(int c) {
+  const unsigned g = (c + 1) & 15;
+  return g ^ (g >> 1);
+}
+__device__ __forceinline__ int cull_class(unsigned code) {
+  return ((code ^ (code >> 1) ^ (code >> 2) ^ (code >> 3)) + 15) & 15;
+}
+// lanes of a tile whose j atom has the given code: r[s] those that reach sub-block s,
+// of the kept ones
+__device__ __forceinline__ unsigned cull_lanes(unsigned code, const uint4& r, unsigned kept) {
+  const unsigned a = (code & 1u) - 1u, b = ((code >> 1) & 1u) - 1u, c = ((code >> 2) & 1u) - 1u, d = ((code >> 3) & 1u) - 1u;
+  return kept & (r.x ^ a) & (r.y ^ b) & (r.z ^ c) & (r.w ^ d);
+}
+
+// what pass one leaves of a tile: the lanes that reach each sub-block, the lanes kept,
+// whether the tile stays a tile
+struct __align__(16) CullTile {
+  uint4 r;
+  unsigned kept, rest, pad[2];
+};
+
+// W: warps of a row's CTA.  16 while a row's latency counts (fewer than 8 rows an SM:
+// 703 rows 37 -> 24 us), 8 above (5,623 rows: 16 warps are 14 us slower)
+template <int W>
+__global__ void __launch_bounds__(W * 32, 48 / W) k_cull(DevView v, float R2, float Rc2, const int* row_start, const int* row_cnt,
+                                                 CullTile* info) {
   pdl_sync();
-  __shared__ int cnt[2][kCullWarps];
-  __shared__ int first;
+  // the sub-blocks' boxes two by two: centres, half-extents.  FP16 is ample to sort
+  // atoms into classes (0.01 A at 16 A): the force pass tests the boxes itself.
+  __shared__ __half2 sc[2][3], sh[2][3];
+  __shared__ int cnt[W][kCullClasses + 1];   // per class; [kCullClasses]: tiles that stay tiles
+  __shared__ int first, first_rest;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, b = blockIdx.x;
   const int t0 = row_start[b], n = min(row_cnt[b], *v.ntiles - t0);
-  const int per = (max(n, 0) + kCullWarps - 1) / kCullWarps;
+  const int per = (max(n, 0) + W - 1) / W;
   const int ta = t0 + min(wid * per, max(n, 0)), tb = t0 + min((wid + 1) * per, max(n, 0));
   const float4 h = v.half[b];
-  int nn = 0, nf = 0;
-#pragma unroll 4
+  const SystemInfo& S = v.sys[v.slot_sys[b]];
+  const int last = S.block_start + S.nblocks - 1;   // the block that holds the system's padding slots
+  if (threadIdx.x < 2) {
+    const float4 l0 = v.sub[8 * b + 4 * threadIdx.x], h0 = v.sub[8 * b + 4 * threadIdx.x + 1];
+    const float4 l1 = v.sub[8 * b + 4 * threadIdx.x + 2], h1 = v.sub[8 * b + 4 * threadIdx.x + 3];
+    sc[threadIdx.x][0] = __floats2half2_rn(0.5f * (l0.x + h0.x), 0.5f * (l1.x + h1.x));
+    sc[threadIdx.x][1] = __floats2half2_rn(0.5f * (l0.y + h0.y), 0.5f * (l1.y + h1.y));
+    sc[threadIdx.x][2] = __floats2half2_rn(0.5f * (l0.z + h0.z), 0.5f * (l1.z + h1.z));
+    sh[threadIdx.x][0] = __floats2half2_rn(0.5f * (h0.x - l0.x), 0.5f * (h1.x - l1.x));
+    sh[threadIdx.x][1] = __floats2half2_rn(0.5f * (h0.y - l0.y), 0.5f * (h1.y - l1.y));
+    sh[threadIdx.x][2] = __floats2half2_rn(0.5f * (h0.z - l0.z), 0.5f * (h1.z - l1.z));
+  }
+  __syncthreads();
+  __half2 C[2][3], H[2][3];
+#pragma unroll
+  for (int q = 0; q < 2; q++)
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      C[q][k] = sc[q][k];
+      H[q][k] = sh[q][k];
+    }
+  const __half2 zero = __float2half2_rn(0.f), rc2 = __float2half2_rn(Rc2);
+  const unsigned mine = cull_code(lane & 15);   // lanes 0-15 keep the counts of a class each
+  int mycnt = 0, rest = 0;
+#pragma unroll 1
   for (int t = ta; t < tb; t++) {
     const Tile T = v.tiles[t];
     const bool plain = T.mask < 0 && !(T.flags & 3);
     const int sj = T.bj * 32 + lane;
-    const float4 x = v.xq[sj];
-    const float gx = fmaxf(fabsf(x.x + T.ox) - h.x, 0.f);
-    const float gy = fmaxf(fabsf(x.y + T.oy) - h.y, 0.f);
-    const float gz = fmaxf(fabsf(x.z + T.oz) - h.z, 0.f);
-    const float d2 = gx * gx + gy * gy + gz * gz;
-    const bool keep = plain && v.sorted_atom[sj] >= 0 && d2 <= R2;
-    const unsigned mn = __ballot_sync(0xffffffffu, keep && d2 <= Rc2), mf = __ballot_sync(0xffffffffu, keep && d2 > Rc2);
-    nn += __popc(mn);
-    nf += __popc(mf);
-    if (lane == 0) {
-      jmask[t] = make_uint2(mn, mf);
-      if (!plain) v.cull_rest[atomicAdd(&v.cull_n[0], 1)] = t;
-    }
-  }
-  if (lane == 0) {
-    cnt[0][wid] = nn;
-    cnt[1][wid] = nf;
-  }
-  __syncthreads();
-  int tn = 0, tf = 0, on = 0, of = 0;   // the row's totals, and those of the warps before this one
+    float4 x = v.xq[sj];
+    x.x += T.ox;
+    x.y += T.oy;
+    x.z += T.oz;
+    const float gx = fmaxf(fabsf(x.x) - h.x, 0.f), gy = fmaxf(fabsf(x.y) - h.y, 0.f);
+    const float gz = fmaxf(fabsf(x.z) - h.z, 0.f);
+    const bool keep = plain && gx * gx + gy * gy + gz * gz <= R2 && (T.bj != last || v.sorted_atom[sj] >= 0);
+    const unsigned kept = __ballot_sync(0xffffffffu, keep);
+    rest += plain ? 0 : 1;
+    CullTile I;
+    I.r = make_uint4(0u, 0u, 0u, 0u);
+    I.kept = kept;
+    I.rest = plain ? 0u : 1u;
+    if (kept) {
+      const __half2 X = __float2half2_rn(x.x), Y = __float2half2_rn(x.y), Z = __float2half2_rn(x.z);
+      unsigned r[4];
 #pragma unroll
-  for (int w = 0; w < kCullWarps; w++) {
-    if (w == wid) {
-      on = tn;
-      of = tf;
+      for (int q = 0; q < 2; q++) {
+        const __half2 dx = __hmax2(__hsub2(__habs2(__hsub2(X, C[q][0])), H[q][0]), zero);
+        const __half2 dy = __hmax2(__hsub2(__habs2(__hsub2(Y, C[q][1])), H[q][1]), zero);
+        const __half2 dz = __hmax2(__hsub2(__habs2(__hsub2(Z, C[q][2])), H[q][2]), zero);
+        const __half2 d2 = __hfma2(dz, dz, __hfma2(dy, dy, __hmul2(dx, dx)));
+        const unsigned le = __hle2_mask(d2, rc2);
+        r[2 * q] = __ballot_sync(0xffffffffu, keep && (le & 1u));
+        r[2 * q + 1] = __ballot_sync(0xffffffffu, keep && (le >> 31));
+      }
+      I.r = make_uint4(r[0], r[1], r[2], r[3]);
+      mycnt += __popc(cull_lanes(mine, I.r, kept));
     }
-    tn += cnt[0][w];
-    tf += cnt[1][w];
+    if (lane == 0) {
+      info[t].r = I.r;
+      *reinterpret_cast<uint2*>(&info[t].kept) = make_uint2(I.kept, I.rest);
+    }
   }
-  const int G = (tn + tf + 63) / 64 * 2;
+  if (lane < kCullClasses) cnt[wid][lane] = mycnt;
+  else if (lane == kCullClasses) cnt[wid][lane] = rest;
+  __syncthreads();
+  // lane c: entries before class c, and before this warp's of class c; lane 16: the
+  // tiles that stay tiles in the warps before
+  int mycls = 0, before = 0;
+  if (lane <= kCullClasses) {
+#pragma unroll
+    for (int w = 0; w < W; w++) {
+      const int x = cnt[w][lane];
+      mycls += x;
+      before += w < wid ? x : 0;
+    }
+  }
+  const int nrest = __shfl_sync(0xffffffffu, mycls, kCullClasses);
+  int inc = lane < kCullClasses ? mycls : 0;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += y;
+  }
+  const int total = __shfl_sync(0xffffffffu, inc, 31);
+  int off = (lane < kCullClasses ? inc - mycls : 0) + before;
+  const int G = (total + 63) / 64 * 2;
   if (threadIdx.x == 0) {
-    first = atomicAdd(&v.cull_n[1], G);
+    first_rest = nrest ? atomicAdd(&v.cull_n[0], nrest) : 0;
+    first = G ? atomicAdd(&v.cull_n[1], G) : 0;
     if ((long long)(first + G) * 32 > v.cull_cap) v.cull_n[2] = 0;   // they do not fit: the tile path serves all
   }
   __syncthreads();
   const long long base = (long long)first * 32;
   if (base + (long long)G * 32 > v.cull_cap) return;
-  for (int g = threadIdx.x; g < G; g += kCullWarps * 32) v.cull_bi[first + g] = b;
-  for (int i = tn + tf + threadIdx.x; i < G * 32; i += kCullWarps * 32)
+  for (int g = threadIdx.x; g < G; g += W * 32) v.cull_bi[first + g] = b;
+  for (int i = total + threadIdx.x; i < G * 32; i += W * 32)
     v.cull_ent[base + i] = make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
-  long long en = base + on, ef = base + tn + of;
   const unsigned lt = (1u << lane) - 1u;
-#pragma unroll 4
+  int at_rest = first_rest + __shfl_sync(0xffffffffu, off, kCullClasses);
+#pragma unroll 2
   for (int t = ta; t < tb; t++) {
-    const uint2 m = jmask[t];
+    const uint2 k = *reinterpret_cast<const uint2*>(&info[t].kept);
+    const unsigned kept = k.x;
+    if (k.y && lane == 0) v.cull_rest[at_rest] = t;
+    at_rest += k.y;
+    if (!kept) continue;
+    const uint4 r = info[t].r;
     const Tile T = v.tiles[t];
-    const float4 e = make_float4(T.ox, T.oy, T.oz, __int_as_float(T.bj * 32 + lane));
-    if ((m.x >> lane) & 1u) v.cull_ent[en + __popc(m.x & lt)] = e;
-    if ((m.y >> lane) & 1u) v.cull_ent[ef + __popc(m.y & lt)] = e;
-    en += __popc(m.x);
-    ef += __popc(m.y);
+    const unsigned code = ((r.x >> lane) & 1u) | ((r.y >> lane) & 1u) << 1 | ((r.z >> lane) & 1u) << 2 |
+                          ((r.w >> lane) & 1u) << 3;
+    const int at = __shfl_sync(0xffffffffu, off, cull_class(code)) + __popc(cull_lanes(code, r, kept) & lt);
+    if ((kept >> lane) & 1u) v.cull_ent[base + at] = make_float4(T.ox, T.oy, T.oz, __int_as_float(T.bj * 32 + lane));
+    off += lane < kCullClasses ? __popc(cull_lanes(mine, r, kept)) : 0;
   }
 }
 
@@ -899,8 +990,11 @@ static void scan_ints(Context& c, const int* in, int* out, int* tmp, long long n
 static void launch_cull(Context& c, float list_radius) {
   c.kernel_launches += 1;
   const float R = list_radius + 1e-3f, Rc = fmaxf(list_radius - (float)c.lp.Padding, 0.f);
-  launch_pdl(c.stream, c.nblocks, kCullWarps * 32, 0, k_cull, c.view(), R * R, Rc * Rc, c.d_row_start.p, c.d_row_cnt.p,
-                                                      c.d_cull_mask.p);
+  CullTile* info = reinterpret_cast<CullTile*>(c.d_cull_mask.p);
+  if (c.nblocks <= 8 * 152)
+    launch_pdl(c.stream, c.nblocks, 16 * 32, 0, k_cull<16>, c.view(), R * R, Rc * Rc, c.d_row_start.p, c.d_row_cnt.p, info);
+  else
+    launch_pdl(c.stream, c.nblocks, 8 * 32, 0, k_cull<8>, c.view(), R * R, Rc * Rc, c.d_row_start.p, c.d_row_cnt.p, info);
 }
 
 // the overflow flag of a build about to be repeated into grown arrays

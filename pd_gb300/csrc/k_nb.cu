@@ -447,15 +447,16 @@ __global__ void __launch_bounds__(ENERGY ? kNbEThreads : kNbThreads, ENERGY ? 5 
 //  * Groups, two of a row at once (.x, .y): each lane holds a j atom of either,
 //    the i block's atoms come from the warp's rows, 8 at a time (one sub-block of
 //    the sorted order): a sub-block whose box at the current positions no held
-//    atom reaches is skipped (on the solvated box 40 % of the steps: the list
-//    radius holds the skin, and a far j atom reaches part of a 32-atom block
-//    only).  The i atoms' sums rotate within 8 lanes and meet over the four
-//    8-lane groups after each sub-block.
+//    atom reaches is skipped (on the solvated box half of the steps: a far j atom
+//    reaches part of a 32-atom block only, and the list build puts j atoms that
+//    reach the same sub-blocks together).  The i atoms' sums rotate within 8 lanes
+//    and meet over the four 8-lane groups after each sub-block.
 //  * Tiles (masked, diagonal, or with a per-pair image), step-packed: lane l
 //    holds i atom l, the j atoms l + kk and l + kk + 1 come as one pair.
-// Bound by the FMA pipe (a packed instruction holds it two cycles) and issue.
-// Solvated box, 22,489 atoms at 12 A: 88 us (scalar rotation of 32 x 32 items)
-// -> 49 us; 8 copies 607 -> 314 us, of which the steps themselves take half.
+// Bound by the FMA pipe (a packed instruction holds it two cycles) in the steps and
+// by the gathers and atomics of the j atoms in an item's rest, about half each.
+// Solvated box, 22,489 atoms at 12 A: 88 us (scalar rotation of 32 x 32 items) ->
+// 49 (packed, skipping) -> 46 us (j atoms by class); 8 copies 607 -> 314 -> 275 us.
 // ---------------------------------------------------------------------------
 enum NBLaw { kLawSame = 0, kLawSplit = 1, kLawForce = 2, kLawVdw = 3 };
 
@@ -505,6 +506,7 @@ struct NBRows {
     struct {
       float4 x[64];                    // groups: (x, y, z, q) of the i block, each sub-block twice over
       float2 p[64];                    // (LJ radius, sqrt(eps))
+      float4 c[4], h[4];               // the sub-blocks' boxes: centres, half-extents
     };
   };
 };
@@ -574,13 +576,6 @@ __device__ __forceinline__ void nb_tile2(const DevView& v, const NBConst& k, con
   nb_flush(v, sj, NBAcc{-jx, -jy, -jz});
 }
 
-// lower bound of the squared distance from a point to a box
-__device__ __forceinline__ float box_dist2(const float4& x, const float4& lo, const float4& hi) {
-  const float gx = fmaxf(fmaxf(lo.x - x.x, x.x - hi.x), 0.f), gy = fmaxf(fmaxf(lo.y - x.y, x.y - hi.y), 0.f);
-  const float gz = fmaxf(fmaxf(lo.z - x.z, x.z - hi.z), 0.f);
-  return gx * gx + gy * gy + gz * gz;
-}
-
 // one pair of groups of row bi (entries en[0..63])
 template <int LAW>
 __device__ __forceinline__ void nb_groups2(const DevView& v, const NBConst& k, int bi, const float4* en, int lane,
@@ -601,7 +596,16 @@ __device__ __forceinline__ void nb_groups2(const DevView& v, const NBConst& k, i
     pb = v.par[sb];
     xb.x += eb.x; xb.y += eb.y; xb.z += eb.z;
   }
+  float4 blo = make_float4(0.f, 0.f, 0.f, 0.f), bhi = blo;
+  if (lane < 4) {
+    blo = v.sub[8 * bi + 2 * lane];
+    bhi = v.sub[8 * bi + 2 * lane + 1];
+  }
   __syncwarp();
+  if (lane < 4) {
+    rs.c[lane] = make_float4(0.5f * (blo.x + bhi.x), 0.5f * (blo.y + bhi.y), 0.5f * (blo.z + bhi.z), 0.f);
+    rs.h[lane] = make_float4(0.5f * (bhi.x - blo.x), 0.5f * (bhi.y - blo.y), 0.5f * (bhi.z - blo.z), 0.f);
+  }
   rs.x[row] = rs.x[row + 8] = make_float4(xi.x, xi.y, xi.z, k.econv_diel * xi.w);
   rs.p[row] = rs.p[row + 8] = make_float2(pi.x, pi.y);
   __syncwarp();
@@ -610,12 +614,23 @@ __device__ __forceinline__ void nb_groups2(const DevView& v, const NBConst& k, i
   const float2 EN = make_float2(pa.y, pb.y);
   float2 FX = f2(0.f), FY = f2(0.f), FZ = f2(0.f);   // force on the held atoms along d = x_i - x_j
   float ix = 0.f, iy = 0.f, iz = 0.f;                // minus the sums of i atom `lane`
+  // the sub-blocks that a held atom reaches (a hair more than the cutoff)
   const float reach2 = k.cut2 * 1.00001f;
+  unsigned todo = 0u;
+#pragma unroll
+  for (int s = 0; s < 4; s++) {
+    const float4 c = rs.c[s], h = rs.h[s];
+    float2 gx = __fadd2_rn(nx, f2(c.x)), gy = __fadd2_rn(ny, f2(c.y)), gz = __fadd2_rn(nz, f2(c.z));
+    gx = make_float2(fmaxf(fabsf(gx.x) - h.x, 0.f), fmaxf(fabsf(gx.y) - h.x, 0.f));
+    gy = make_float2(fmaxf(fabsf(gy.x) - h.y, 0.f), fmaxf(fabsf(gy.y) - h.y, 0.f));
+    gz = make_float2(fmaxf(fabsf(gz.x) - h.z, 0.f), fmaxf(fabsf(gz.y) - h.z, 0.f));
+    const float2 d2 = __ffma2_rn(gz, gz, __ffma2_rn(gy, gy, __fmul2_rn(gx, gx)));
+    todo |= __any_sync(0xffffffffu, fminf(d2.x, d2.y) <= reach2) ? 1u << s : 0u;
+  }
   const int src = (lane & 24) | ((lane + 1) & 7);
 #pragma unroll 1
-  for (int s = 0; s < 4; s++) {
-    const float4 lo = v.sub[8 * bi + 2 * s], hi = v.sub[8 * bi + 2 * s + 1];
-    if (!__any_sync(0xffffffffu, fminf(box_dist2(xa, lo, hi), box_dist2(xb, lo, hi)) <= reach2)) continue;
+  for (; todo; todo &= todo - 1u) {
+    const int s = __ffs(todo) - 1;
     const float4* xr = rs.x + s * 16 + (lane & 7);
     const float2* pr = rs.p + s * 16 + (lane & 7);
     float rx = 0.f, ry = 0.f, rz = 0.f;

@@ -625,7 +625,7 @@ int pdgpu::alloc_cull_tiles(Context& c) {
   c.cull_cap = 0;
   if (!c.cull_want || c.tile_cap == 0) return PDGPU_OK;
   const long long cap = std::min(32LL * c.tile_cap + 64LL * c.nblocks, 8192LL * c.nblocks);
-  cudaError_t e = c.d_cull_mask.alloc(c.tile_cap);
+  cudaError_t e = c.d_cull_mask.alloc(2 * (size_t)c.tile_cap);
   if (e == cudaSuccess) e = c.d_cull_rest.alloc(c.tile_cap);
   if (e == cudaSuccess) e = c.d_cull_ent.alloc(cap);
   if (e == cudaSuccess) e = c.d_cull_bi.alloc(cap / 32);
@@ -1210,7 +1210,7 @@ int pdgpu_list_tiles(pdgpu_ctx* h, int* tiles, long long cap, long long* ntiles,
   if (list_bytes) {
     // the arrays whose size follows the list
     *list_bytes = (long long)(c.d_tiles.n * sizeof(Tile) + c.d_items.n * sizeof(int2) + c.d_mlist.n * 4 +
-                              c.d_masks.n * sizeof(uint2) + c.d_cull_mask.n * sizeof(uint2) + c.d_cull_rest.n * 4 +
+                              c.d_masks.n * sizeof(uint2) + c.d_cull_mask.n * sizeof(uint4) + c.d_cull_rest.n * 4 +
                               c.d_cull_ent.n * sizeof(float4) + c.d_cull_bi.n * 4);
   }
   return PDGPU_OK;

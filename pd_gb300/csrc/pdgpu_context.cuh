@@ -152,7 +152,7 @@ struct Context {
   DBuf<float2> d_plo;                // [nslots]
   // NB j-atom groups (allocated with the NB parameters)
   bool cull_want = false;            // the NB parameters were set
-  DBuf<uint2> d_cull_mask;           // [tile_cap] j lanes kept per tile: near (within the cutoffs), skin
+  DBuf<uint4> d_cull_mask;           // [tile_cap*2] lanes of a tile's j atoms that reach each i sub-block; kept lanes
   DBuf<int> d_cull_rest;             // [tile_cap]
   DBuf<float4> d_cull_ent;           // [cull_cap]
   DBuf<int> d_cull_bi;               // [cull_cap / 32]
