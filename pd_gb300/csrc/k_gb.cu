@@ -294,9 +294,9 @@ struct PairAcc {
 // slot's total does not depend on how its tiles were grouped into work items
 __device__ __forceinline__ void flush_pair(const DevView& v, long long* deda, int s, const PairAcc& a) {
   fix_range(v.status, fabsf(a.fx) + fabsf(a.fy) + fabsf(a.fz) + fabsf(a.da));
-  atomic_add_ll(&v.facc[3 * s], fx32(a.fx));
-  atomic_add_ll(&v.facc[3 * s + 1], fx32(a.fy));
-  atomic_add_ll(&v.facc[3 * s + 2], fx32(a.fz));
+  atomic_add_ll(&v.facc[force_at(s, 0)], fx32(a.fx));
+  atomic_add_ll(&v.facc[force_at(s, 1)], fx32(a.fy));
+  atomic_add_ll(&v.facc[force_at(s, 2)], fx32(a.fz));
   if (deda) atomic_add_ll(&deda[s], fx32(a.da));
 }
 

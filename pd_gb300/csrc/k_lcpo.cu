@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(kLcpoWarps * 32, 6) k_lcpo_main(DevView v, con
     }
     sasa_out[a] = SA;
     // PD adds SASAderiv / Angstrom; the derivative terms already hold d(sigma*SA)
-    for (int c = 0; c < 3; c++) atomic_add_ll(&facc_out[3 * s + c], f[c]);
+    for (int c = 0; c < 3; c++) atomic_add_ll(&facc_out[force_at(s, c)], f[c]);
     int sys = v.slot_sys[s >> 5];
     if (esurf_out) atomic_add_ll(&esurf_out[(size_t)sys * esurf_stride], fix_energy_d(SA * sigma[a]));
   }

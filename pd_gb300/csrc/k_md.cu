@@ -46,8 +46,8 @@ __device__ __forceinline__ void box_muller(unsigned a, unsigned b, double& n1, d
 __device__ __forceinline__ void slot_force(const MDView& m, int s, double f[3]) {
 #pragma unroll
   for (int c = 0; c < 3; c++) {
-    long long q = m.facc[3 * s + c];
-    if (m.facc_sa) q += m.facc_sa[3 * s + c];
+    long long q = m.facc[force_at(s, c)];
+    if (m.facc_sa) q += m.facc_sa[force_at(s, c)];
     f[c] = (double)q * (1.0 / kForceScale) * kForceToN;
   }
 }

@@ -318,9 +318,9 @@ __device__ __forceinline__ void nb_fix_in(const DevView& v, NBFix& F, const NBAc
 }
 
 __device__ __forceinline__ void nb_flush_fix(const DevView& v, int s, const NBFix& F) {
-  atomic_add_ll(&v.facc[3 * s], F.fx);
-  atomic_add_ll(&v.facc[3 * s + 1], F.fy);
-  atomic_add_ll(&v.facc[3 * s + 2], F.fz);
+  atomic_add_ll(&v.facc[force_at(s, 0)], F.fx);
+  atomic_add_ll(&v.facc[force_at(s, 1)], F.fy);
+  atomic_add_ll(&v.facc[force_at(s, 2)], F.fz);
 }
 
 __device__ __forceinline__ void nb_flush(const DevView& v, int s, const NBAcc& a) {
@@ -759,7 +759,7 @@ __global__ void k_finalize_forces(DevView v, double* out, size_t stride, int add
   if (a < 0) return;
 #pragma unroll
   for (int c = 0; c < 3; c++) {
-    long long q = v.facc[3 * s + c];
+    long long q = v.facc[force_at(s, c)];
     if (q >= (1ll << 62) || q <= -(1ll << 62)) atomicOr(v.status, (unsigned)ST_FIXED_OVERFLOW);
     double f = (double)q * (1.0 / kForceScale) * scale;
     if (add) out[a * stride + c] += f;

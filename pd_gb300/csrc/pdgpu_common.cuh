@@ -138,6 +138,11 @@ struct GBConst {
   float sqrtK, inv_sqrtK, invK, kU, sq_eout, neg_sq_eout, in_over_out, sqrt12, gb_ep;
 };
 
+// Where component c of slot s lies in a force accumulator: a block's 32 x sums, its y
+// sums, its z sums.  A warp adds one component of consecutive slots with one
+// instruction; 8 bytes apart they fill 8 sectors, 24 bytes apart they touch 24.
+__host__ __device__ __forceinline__ size_t force_at(int s, int c) { return (size_t)(s >> 5) * 96 + 32 * c + (s & 31); }
+
 // Device-side view of a context, passed by value to kernels.
 struct DevView {
   int nsys, natom, nslots, nblocks;
@@ -189,7 +194,7 @@ struct DevView {
   int* cull_rest;            // [tile capacity] tiles left on the tile path (any order)
   int* cull_n;               // [0] rest tiles, [1] groups, [2] 1 when the groups fit the capacity
   long long cull_cap;        // entries
-  long long* facc;           // [nslots*3]
+  long long* facc;           // [nslots*3], component c of slot s at force_at(s, c)
   long long* eacc;           // [nsys*E_NSLOTS]
   unsigned* status;
 };
@@ -202,10 +207,10 @@ struct StepClear {
   long long *eacc, *surf, *ke;       // per system (eacc: E_NSLOTS)
 };
 __device__ __forceinline__ void step_clear(const StepClear& C, const DevView& v, int s) {
-  if (C.facc) C.facc[3 * s] = C.facc[3 * s + 1] = C.facc[3 * s + 2] = 0;
+  if (C.facc) C.facc[force_at(s, 0)] = C.facc[force_at(s, 1)] = C.facc[force_at(s, 2)] = 0;
   if (C.gpol) C.gpol[s] = 0;
   if (C.deda) C.deda[s] = 0;
-  if (C.facc2) C.facc2[3 * s] = C.facc2[3 * s + 1] = C.facc2[3 * s + 2] = 0;
+  if (C.facc2) C.facc2[force_at(s, 0)] = C.facc2[force_at(s, 1)] = C.facc2[force_at(s, 2)] = 0;
   if (C.eacc)   // (no fewer slots than 32 per system: every entry of a system's has a slot)
     if ((s & 31) < E_NSLOTS && s == 32 * v.sys[v.slot_sys[s >> 5]].block_start + (s & 31))
       C.eacc[(size_t)v.slot_sys[s >> 5] * E_NSLOTS + (s & 31)] = 0;
