@@ -1048,8 +1048,6 @@ int launch_gb(Context& c, const GBConst& k, double halfeconv, double born_offset
     const int e = launch_adj_gb_pair(c, k);
     if (e != PDGPU_OK) return e;
   } else if (energy) {
-    c.kernel_launches += 1;
-    launch_df_records(c);
     if (!k.fast) launch_pdl(st, ge, kPairEThreads, 0, k_gb_pair_energy<false>, v, k, c.d_born_f.p, c.d_deda.p);
     else launch_pdl(st, ge, kPairEThreads, 0, k_gb_pair_energy<true>, v, k, c.d_born_f.p, c.d_deda.p);
   } else if (!k.fast) {
@@ -1059,7 +1057,7 @@ int launch_gb(Context& c, const GBConst& k, double halfeconv, double born_offset
   }
   launch_pdl(st, sp.grid, sp.threads, 0, k_gb_self, v, c.d_charge.p, k, premul, c.d_deda.p, c.d_born_d.p, c.d_chain_f.p,
                                 energy ? 1 : 0);
-  if (c.gb_no_chain) c.kernel_launches -= 1;
+  if (c.gb_no_chain || c.no_forces) c.kernel_launches -= 1;
   else launch_pdl(st, 2 * g, kChainThreads, 0, k_gb_chain, v, k, c.d_chain_f.p);
   return cudaGetLastError() == cudaSuccess ? PDGPU_OK : PDGPU_ERR_CUDA;
 }

@@ -20,25 +20,11 @@ struct NBAcc {
   float fx, fy, fz;
 };
 
-// Force part of the pair law in FP32 (same law as nb_pair): dE/dr divided by r.
-// SW (energy switch on both terms over the same radii, the common PD setting):
-// one switch factor serves LJ and Coulomb, dE/dr / r = S^2 (gv + ge) +
-// (Ev + Ee) S' / r with S' = -4 u S / w^2.
-template <int ELEC, bool SW = false>
+// Force part of the pair law in FP32: dE/dr divided by r.
+template <int ELEC>
 __device__ __forceinline__ float nb_force_f(const NBConst& k, float r2, float rsum, float eps, float qq) {
   const float invr = rsqrtf(r2), ir2 = invr * invr;
   const float r = r2 * invr;
-  if (SW) {
-    const float t2 = rsum * rsum * ir2;
-    const float B = t2 * t2 * t2, A = B * B;
-    const bool vin = r < k.vdwcut_f;
-    const float ev = vin ? eps * (A - 2.f * B) : 0.f;
-    const float gv = vin ? -12.f * eps * ir2 * (A - B) : 0.f;
-    const float Ee = qq * invr;
-    const float u = fmaxf(r - k.inner_f, 0.f);
-    const float sw = 1.f - u * u * k.invw2_f;
-    return sw * sw * (gv - Ee * ir2) + (ev + Ee) * (-4.f * k.invw2_f * u * sw) * invr;
-  }
   float g = 0.f;
   // switching without a branch: below the inner cutoff u = 0, so sw = 1 and the
   // derivative term is exactly 0 (same value as the unswitched law); a branch
@@ -72,33 +58,21 @@ __device__ __forceinline__ float nb_force_f(const NBConst& k, float r2, float rs
   return g;
 }
 
-// (ENERGY) what one warp keeps in shared memory for the energies of its work
-// item: both blocks' atoms as double-floats in the i block's frame and the list
-// of the pairs inside the cutoff
-struct NBEShared {
-  float4 ih[32], il[32], ip[32];   // (x, y, z, q) high and low parts; (R, sqrt(eps)) high and low
-  float4 jh[32], jl[32], jp[32];
-  int js[32];                      // j slots
-  unsigned short pair[1024];       // i lane | j row << 5 | 1-4 << 10
-};
-
 // 32 rotation steps of one work item: lane i holds an i atom, (xj, pj) the
 // lane's j atom already in i's frame.  Tiles: j slot jb + lane, per-pair image
 // when mi.  GROUP: the j atoms of a group (slots in gent[].w, -1 = empty lane,
-// parked far away), never masked, one image.  ENERGY: the pairs inside the
-// cutoff are listed in sh->pair; returns their number.
-template <int ELEC, bool MASKED, bool ENERGY, bool GROUP, bool SW>
-__device__ __forceinline__ int nb_rot(const DevView& v, const NBConst& k, const SystemInfo& S, int lane, int si,
+// parked far away), never masked, one image.
+template <int ELEC, bool MASKED, bool GROUP>
+__device__ __forceinline__ void nb_rot(const DevView& v, const NBConst& k, const SystemInfo& S, int lane, int si,
                                       const float4& xi, const float4& pi, float qi, unsigned ex, unsigned m14,
                                       float4 xj, float4 pj, bool mi_tile, int jb, const float4* gent, NBAcc& I,
-                                      NBAcc& J, NBEShared* sh) {
+                                      NBAcc& J) {
   const bool mi = !GROUP && mi_tile;
   float Lx = 1.f, Ly = 1.f, Lz = 1.f;
   if (!GROUP && S.periodic) {
     Lx = (float)S.box[0]; Ly = (float)S.box[1]; Lz = (float)S.box[2];
   }
   const float iLx = 1.f / Lx, iLy = 1.f / Ly, iLz = 1.f / Lz;
-  int np = 0;
 #pragma unroll 4
   for (int kk = 0; kk < 32; kk++) {
     float dx = xj.x - xi.x, dy = xj.y - xi.y, dz = xj.z - xi.z;
@@ -112,26 +86,18 @@ __device__ __forceinline__ int nb_rot(const DevView& v, const NBConst& k, const 
     if (MASKED) listed = !((ex >> kk) & 1u);
     bool in = r2 <= k.cut2;
     if (listed && (fabsf(r2 - k.cut2) <= 2e-6f * k.cut2 ||
-                   (!SW && fabsf(r2 - k.vdwcut2) <= 2e-6f * k.vdwcut2))) {
+                   fabsf(r2 - k.vdwcut2) <= 2e-6f * k.vdwcut2)) {
       // at a hard cutoff: decide, and take the distance, in FP64 (FP64 work only on this branch)
       const int sjr = GROUP ? __float_as_int(gent[(lane + kk) & 31].w) : jb + ((lane + kk) & 31);
       const double d2 = nb_r2_fp64(v, S, si, sjr);
       in = d2 <= k.cut2_dd;
       r2 = (float)d2;
     }
-    const bool take = listed && in;
-    if (ENERGY) {
-      const unsigned m = __ballot_sync(0xffffffffu, take);
-      if (take)
-        sh->pair[np + __popc(m & ((1u << lane) - 1u))] =
-            (unsigned short)(lane | (((lane + kk) & 31) << 5) | (MASKED && ((m14 >> kk) & 1u) ? 1024 : 0));
-      np += __popc(m);
-    }
-    if (take) {
+    if (listed && in) {
       const bool is14 = MASKED && ((m14 >> kk) & 1u);
       const float eps = pi.y * pj.y * (is14 ? k.vdw14 : 1.f);
       const float qq = qi * xj.w * (is14 ? k.elec14 : 1.f);
-      const float fs = nb_force_f<ELEC, SW>(k, r2, pi.x + pj.x, eps, qq);
+      const float fs = nb_force_f<ELEC>(k, r2, pi.x + pj.x, eps, qq);
       I.fx += fs * dx; I.fy += fs * dy; I.fz += fs * dz;
       J.fx -= fs * dx; J.fy -= fs * dy; J.fz -= fs * dz;
     }
@@ -147,21 +113,24 @@ __device__ __forceinline__ int nb_rot(const DevView& v, const NBConst& k, const 
     J.fy = __shfl_sync(0xffffffffu, J.fy, src);
     J.fz = __shfl_sync(0xffffffffu, J.fz, src);
   }
-  return np;
 }
 
 // ---------------------------------------------------------------------------
 // Pair energies.  FP32 cannot hold them (water's electrostatics cancel ~5000
 // fold, and so do the force-switch polynomials), and the FP64 pipe is narrow:
 // they are formed in double-float arithmetic (pdgpu_df.cuh, ~45 bits) from
-// positions and parameters held as double-floats.  The rotation lists the pairs
-// inside the cutoff (about a fifth of those it visits); the list is then dealt
-// over the lanes, so the ~300 instructions of a pair's energy run on full warps.
-// FP64 pair energies on the rotation itself, bound by the FP64 pipe, had taken
-// 5.85 ms on the solvated 22,489 atoms at 15 A (force switch), 0.331 ms on 667
-// waters at 12 A; this takes 0.472 and 0.046 ms, bound by FP32 issue.  Against
-// 64-bit sums the energies are as close as before (within 2e-8 kcal/mol, one
-// fixed-point rounding per item instead of one per lane).
+// positions and parameters held as double-floats, in a pass of their own beside
+// the force pass.  It lists the pairs inside the cutoff, with the force pass's
+// items and skipping and nothing else in the loop, and deals the list over the
+// lanes, so the ~300 instructions of a pair's energy run on full warps; an item
+// passes its odd pairs on from one eighth to the next.  Against 64-bit sums the
+// energies are within 2e-8 kcal/mol (one fixed-point rounding per item).
+// Bound by the FMA pipe and, in small systems, by the latency of its chains: two pairs
+// a lane in packed arithmetic.  FP64 pair energies on the rotation, with the forces:
+// 5.85 ms on the solvated 22,489 atoms at 15 A (force switch), 0.331 ms on 667 waters
+// at 12 A; scalar double-float on a list kept by
+// the force rotation: 0.461, 0.046, 0.119 ms; this pass 0.334, 0.031, 0.097 ms beside
+// force passes of 0.060, 0.011 and 0.019 ms (left out of calls that read no forces).
 // ---------------------------------------------------------------------------
 
 // remainders of the packed slots (before each energy pass)
@@ -192,100 +161,149 @@ __global__ void k_df_records(DevView v, const double* charge, float4* rlo, float
 }
 
 struct NBESum {
-  DF vdw, elec, vir;
+  DF2 vdw, elec, vir;
+  float2 f;   // of the pairs' force magnitudes: range check
 };
 
-// energies of one listed pair into the sums (same law as nb_pair)
+// what an item keeps in shared memory: its atoms as double-floats in the i
+// block's frame (a tile's j block, or two groups) and the list of pairs
+constexpr int kNbList = 512 + 64;
+struct NBEShared {
+  float4 ih[32], il[32], ip[32];   // (x, y, z, q) high and low parts; (R, sqrt(eps)) high and low
+  float4 jh[64], jl[64], jp[64];
+  int js[64];                      // j slots
+  unsigned short pair[2][kNbList]; // a warp's list: i row | j row << 5 | 1-4 << 11
+  DF sum[3];                       // the second warp's sums
+};
+
+// S = (1 - w^2 / width^2)^2 and r S' of an energy switch, w = r - inner > 0 for one of
+// the two pairs at least; 1 and 0 for a pair inside
+__device__ __forceinline__ void nb_switch_df(DF2 r, DF2 w, DF invw2, DF2& S, DF2& dS) {
+  w = df_select(w.h.x > 0.f, w.h.y > 0.f, w, df2(DF{0.f, 0.f}));
+  const DF2 wi = df_mul(w, df2(invw2));
+  const DF2 sw = df_norm(df_sub(df2(DF{1.f, 0.f}), df_mul(w, wi)));
+  S = df_norm(df_sqr(sw));
+  dS = df_norm(df_scale2(df_mul(df_mul(wi, sw), r), -4.f));
+}
+
+// a per-pair-image tile's box; minus the images to take off a displacement
+struct NBEBox {
+  bool mi;
+  DF x, y, z;
+  float ix, iy, iz;
+};
+__device__ __forceinline__ float2 nb_images(float2 d, float iL) {
+  constexpr float kRint = 12582912.f;   // 1.5 2^23: adding and taking it off rounds to an integer
+  return __fadd2_rn(__ffma2_rn(d, f2(-iL), f2(kRint)), f2(-kRint));
+}
+
+// energies of two listed pairs into the sums (same law as the force bodies; pair b
+// counts only if two).  Products of products stay unnormalised where their l holds a
+// few roundings of h: what df_mul leaves out is then below 1e-13.
 template <int ELEC, bool SW>
-__device__ __forceinline__ void nb_energy_df(const DevView& v, const NBConst& k, const NBEConst& e,
-                                             const SystemInfo& S, bool mi, int ibase, const NBEShared* sh,
-                                             unsigned code, NBESum& sum) {
-  const int il = code & 31, jl = (code >> 5) & 31;
-  const bool is14 = code & 1024u;
-  const float4 xh = sh->ih[il], xl = sh->il[il], xp = sh->ip[il];
-  const float4 yh = sh->jh[jl], yl = sh->jl[jl], yp = sh->jp[jl];
-  DF dx = df_sub(DF{yh.x, yl.x}, DF{xh.x, xl.x});
-  DF dy = df_sub(DF{yh.y, yl.y}, DF{xh.y, xl.y});
-  DF dz = df_sub(DF{yh.z, yl.z}, DF{xh.z, xl.z});
-  if (mi) {
-    dx = df_add(dx, df_scale(S.boxf[0], -rintf(dx.h / S.boxf[0].h)));
-    dy = df_add(dy, df_scale(S.boxf[1], -rintf(dy.h / S.boxf[1].h)));
-    dz = df_add(dz, df_scale(S.boxf[2], -rintf(dz.h / S.boxf[2].h)));
+__device__ __forceinline__ void nb_energy_df2(const DevView& v, const NBConst& k, const NBEConst& e,
+                                              const SystemInfo& S, const NBEBox& box, int ibase, const NBEShared* sh,
+                                              unsigned ca, unsigned cb, bool two, NBESum& sum) {
+  const int ia = ca & 31, ib = cb & 31, ja = (ca >> 5) & 63, jb = (cb >> 5) & 63;
+  const float4 xha = sh->ih[ia], xhb = sh->ih[ib], xla = sh->il[ia], xlb = sh->il[ib];
+  const float4 yha = sh->jh[ja], yhb = sh->jh[jb], yla = sh->jl[ja], ylb = sh->jl[jb];
+  DF2 dx = df_sub(df2(yha.x, yla.x, yhb.x, ylb.x), df2(xha.x, xla.x, xhb.x, xlb.x));
+  DF2 dy = df_sub(df2(yha.y, yla.y, yhb.y, ylb.y), df2(xha.y, xla.y, xhb.y, xlb.y));
+  DF2 dz = df_sub(df2(yha.z, yla.z, yhb.z, ylb.z), df2(xha.z, xla.z, xhb.z, xlb.z));
+  if (box.mi) {
+    // (the image count times the box is exact in both parts)
+    auto wrap = [](DF2 d, DF L, float iL) {
+      const float2 n = nb_images(d.h, iL);
+      return df_add(d, DF2{__fmul2_rn(n, f2(L.h)), __fmul2_rn(n, f2(L.l))});
+    };
+    dx = wrap(dx, box.x, box.ix);
+    dy = wrap(dy, box.y, box.iy);
+    dz = wrap(dz, box.z, box.iz);
   }
-  const DF r2 = df_norm2(dx, dy, dz);
-  const DF ir = df_rsqrt(r2);
-  const DF r = df_norm(df_mul(r2, ir));
-  const DF one = DF{1.f, 0.f};
+  const DF2 r2 = df_norm2(dx, dy, dz);
+  const DF2 ir = df_rsqrt(r2);
+  const DF2 r = df_norm(df_mul(r2, ir));
+  const bool scaled = (ca | cb) & 2048u;   // (1-4 pairs: masked tiles only)
+  const DF2 zero = df2(DF{0.f, 0.f}), one = df2(DF{1.f, 0.f});
   // LJ: energy and r dE/dr before switching
-  DF Ev = DF{0.f, 0.f}, gv = Ev;
-  DF u = df_sub(r, e.vdwcut);
-  bool vin = e.dovdw && u.h + u.l < 0.f;
-  if (e.dovdw && e.vdw_hard && fabsf(u.h) <= 2e-6f * e.vdwcut.h)   // at an unswitched end of LJ: decide in FP64
-    vin = sqrt(nb_r2_fp64(v, S, ibase + il, sh->js[jl])) < k.vdwcut_d;
-  if (vin) {
-    const DF R = df_norm(df_add(DF{xp.x, xp.z}, DF{yp.x, yp.z}));
-    const DF t = df_norm(df_mul(R, ir)), t2 = df_norm(df_mul(t, t));
-    const DF B = df_norm(df_mul(df_mul(t2, t2), t2)), A = df_mul(B, B);
-    DF eps = df_norm(df_mul(DF{xp.y, xp.w}, DF{yp.y, yp.w}));
-    if (is14) eps = df_norm(df_mul(eps, e.vdw14));
-    Ev = df_norm(df_mul(eps, df_norm(df_sub(A, df_scale2(B, 2.f)))));
-    gv = df_norm(df_scale(df_mul(eps, df_norm(df_sub(A, B))), -12.f));
+  DF2 Ev = zero, gv = zero;
+  if (e.dovdw) {
+    const float4 pa = sh->ip[ia], pb = sh->ip[ib], qa = sh->jp[ja], qb = sh->jp[jb];
+    const DF2 R = df_norm(df_add(df2(pa.x, pa.z, pb.x, pb.z), df2(qa.x, qa.z, qb.x, qb.z)));
+    const DF2 t = df_mul(R, ir), t2 = df_norm(df_sqr(t));
+    const DF2 B = df_norm(df_mul(df_sqr(t2), t2)), A = df_sqr(B);
+    DF2 eps = df_mul(df2(pa.y, pa.w, pb.y, pb.w), df2(qa.y, qa.w, qb.y, qb.w));
+    if (scaled) eps = df_norm(df_mul(eps, df_select(ca & 2048u, cb & 2048u, df2(e.vdw14), one)));
+    const DF2 AB = df_sub(A, B);
+    Ev = df_norm(df_mul(eps, df_sub(AB, B)));
+    gv = df_norm(df_mul(df_scale(eps, -12.f), df_norm(AB)));
     if (!SW) {
-      DF w = df_sub(r, e.vdwinner);
-      if (w.h > 0.f) {
-        w = df_norm(w);
-        const DF wi = df_norm(df_mul(w, e.vdwinvw2));
-        const DF sw = df_norm(df_sub(one, df_mul(w, wi)));
-        const DF Sv = df_norm(df_mul(sw, sw));
-        const DF dS = df_norm(df_scale2(df_mul(df_mul(wi, sw), r), -4.f));   // r S'
+      const DF2 w = df_sub(r, df2(e.vdwinner));
+      if (w.h.x > 0.f || w.h.y > 0.f) {
+        DF2 Sv, dS;
+        nb_switch_df(r, w, e.vdwinvw2, Sv, dS);
         gv = df_add(df_mul(Sv, gv), df_mul(Ev, dS));
         Ev = df_mul(Ev, Sv);
       }
+      const float ua = (r.h.x - e.vdwcut.h) + (r.l.x - e.vdwcut.l), ub = (r.h.y - e.vdwcut.h) + (r.l.y - e.vdwcut.l);
+      bool va = ua < 0.f, vb = ub < 0.f;
+      if (e.vdw_hard) {   // at an unswitched end of LJ: decided in FP64
+        if (fabsf(ua) <= 2e-6f * e.vdwcut.h) va = sqrt(nb_r2_fp64(v, S, ibase + ia, sh->js[ja])) < k.vdwcut_d;
+        if (fabsf(ub) <= 2e-6f * e.vdwcut.h) vb = sqrt(nb_r2_fp64(v, S, ibase + ib, sh->js[jb])) < k.vdwcut_d;
+      }
+      gv = df_select(va, vb, gv, zero);
+      Ev = df_select(va, vb, Ev, zero);
     }
   }
-  // Coulomb
-  DF Ee = DF{0.f, 0.f}, ge = Ee;
+  // Coulomb: energy and minus r dE/dr
+  DF2 Ee = zero, fe = zero;
   if (ELEC != 0) {
-    DF qq = df_norm(df_mul(DF{xh.w, xl.w}, DF{yh.w, yl.w}));   // (i's charge carries the Coulomb constant)
-    if (is14) qq = df_norm(df_mul(qq, e.elec14));
-    Ee = df_norm(df_mul(qq, ir));
-    ge = df_neg(Ee);
+    DF2 qq = df_mul(df2(xha.w, xla.w, xhb.w, xlb.w), df2(yha.w, yla.w, yhb.w, ylb.w));   // (i's charge carries the Coulomb constant)
+    if (scaled) qq = df_mul(qq, df_select(ca & 2048u, cb & 2048u, df2(e.elec14), one));
+    Ee = fe = df_norm(df_mul(qq, ir));
     if (ELEC == 3) {
-      DF w = df_sub(r, e.inner);
-      if (w.h > 0.f) {
-        w = df_norm(w);
-        const DF wi = df_norm(df_mul(w, e.invw2));
-        const DF sw = df_norm(df_sub(one, df_mul(w, wi)));
-        const DF Se = df_norm(df_mul(sw, sw));
-        const DF dS = df_norm(df_scale2(df_mul(df_mul(wi, sw), r), -4.f));
+      const DF2 w = df_sub(r, df2(e.inner));
+      if (w.h.x > 0.f || w.h.y > 0.f) {
+        DF2 Se, dS;
+        nb_switch_df(r, w, e.invw2, Se, dS);
         if (SW) {   // one switch for both terms
           gv = df_add(df_mul(Se, gv), df_mul(Ev, dS));
           Ev = df_mul(Ev, Se);
         }
-        ge = df_add(df_mul(Se, ge), df_mul(Ee, dS));
+        fe = df_sub(df_mul(Se, Ee), df_mul(Ee, dS));
         Ee = df_mul(Ee, Se);
       }
     } else if (ELEC == 4) {
       // Steinbach & Brooks force switch, nonbonded.cpp:798-819
-      if (df_sub(r, e.inner).h > 0.f) {
-        const DF c2 = df_norm(df_sub(e.cut2, r2));
-        // -qq sA / r (C^2 - r^2)^2 (C^2 - 3 I^2 + 2 r^2)
-        const DF f = df_norm(df_mul(df_mul(c2, c2), df_norm(df_add(e.fsw_k, df_scale2(r2, 2.f)))));
-        ge = df_neg(df_mul(df_norm(df_mul(e.sA, f)), Ee));
+      const bool oa = r.h.x > e.inner.h, ob = r.h.y > e.inner.h;
+      DF2 h = df_sub(ir, df2(e.eshift));
+      if (oa || ob) {
+        const DF2 c2 = df_norm(df_sub(df2(e.cut2), r2));
+        // qq sA / r (C^2 - r^2)^2 (C^2 - 3 I^2 + 2 r^2)
+        const DF2 f = df_mul(df_sqr(c2), df_norm(df_add(df2(e.fsw_k), df_scale2(r2, 2.f))));
+        fe = df_select(oa, ob, df_mul(df_norm(df_mul(df2(e.sA), f)), fe), fe);
         // -qq (sA r (sB / r^2 + sC + sD r^2 + sE r^4) - V(C))
-        DF h = df_norm(df_add(e.sD, df_mul(e.sE, r2)));
-        h = df_norm(df_add(e.sC, df_mul(h, r2)));
-        h = df_norm(df_add(df_mul(h, r), df_mul(e.sB, ir)));
-        Ee = df_neg(df_mul(qq, df_norm(df_sub(df_mul(e.sA, h), e.cutV))));
-      } else {
-        Ee = df_mul(qq, df_norm(df_sub(ir, e.eshift)));
+        DF2 g = df_norm(df_add(df2(e.sD), df_mul(df2(e.sE), r2)));
+        g = df_norm(df_add(df2(e.sC), df_mul(g, r2)));
+        g = df_norm(df_add(df_mul(g, r), df_mul(df2(e.sB), ir)));
+        h = df_select(oa, ob, df_sub(df2(e.cutV), df_mul(df2(e.sA), g)), h);
       }
+      Ee = df_mul(qq, df_norm(h));
     }
   }
-  df_acc(sum.vdw, df_norm(Ev));
-  df_acc(sum.elec, df_norm(Ee));
-  df_acc(sum.vir, df_norm(df_add(gv, ge)));
+  DF2 vir = df_sub(gv, fe);
+  Ev = df_select(true, two, Ev, zero);
+  Ee = df_select(true, two, Ee, zero);
+  vir = df_select(true, two, vir, zero);
+  df_acc(sum.vdw, Ev);
+  df_acc(sum.elec, Ee);
+  df_acc(sum.vir, vir);
+  const float2 f = __fmul2_rn(vir.h, ir.h);
+  sum.f = __fadd2_rn(sum.f, make_float2(fabsf(f.x), fabsf(f.y)));
 }
+
+// both halves' sum
+__device__ __forceinline__ DF df_fold(DF2 x) { return df_add(DF{x.h.x, x.l.x}, DF{x.h.y, x.l.y}); }
 
 // one block's atom of this lane into the shared rows (O: frame offset)
 __device__ __forceinline__ void nb_stage(float4* h, float4* l, float4* p, int row, const DevView& v, int slot,
@@ -336,17 +354,14 @@ __device__ __forceinline__ void nb_flush(const DevView& v, int s, const NBAcc& a
 // serves all.
 __device__ __forceinline__ bool nb_grouped(const DevView& v) { return v.cull_n[2] && 2 * v.cull_n[0] <= *v.ntiles; }
 
-// One warp per work item, grid-stride: the tiles left on the tile path, then the
-// j-atom groups (cull: the last list build wrote them and they fit).  The energy
-// kernel's CTAs hold 4 warps (each warp keeps 5 KB of shared memory).
-constexpr int kNbThreads = 256, kNbEThreads = 128;
-template <int ELEC, bool ENERGY, bool SW = false>
-__global__ void __launch_bounds__(ENERGY ? kNbEThreads : kNbThreads, ENERGY ? 5 : 4)
-    k_nb_tiles(const __grid_constant__ DevView v, const __grid_constant__ NBConst k, const __grid_constant__ NBEConst e,
-               int cull) {
+// Forces where the law does not end smoothly (a hard cutoff).  One warp per work
+// item, grid-stride: the tiles left on the tile path, then the j-atom groups (cull:
+// the last list build wrote them and they fit).
+constexpr int kNbThreads = 256;
+template <int ELEC>
+__global__ void __launch_bounds__(kNbThreads, 4)
+    k_nb_tiles(const __grid_constant__ DevView v, const __grid_constant__ NBConst k, int cull) {
   pdl_sync();
-  __shared__ NBEShared shared[ENERGY ? kNbEThreads / 32 : 1];
-  NBEShared* sh = ENERGY ? &shared[threadIdx.x >> 5] : nullptr;
   const int lane = threadIdx.x & 31;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   const bool grouped = cull && nb_grouped(v);
@@ -354,51 +369,29 @@ __global__ void __launch_bounds__(ENERGY ? kNbEThreads : kNbThreads, ENERGY ? 5 
   const int nitem = nrest + (grouped ? v.cull_n[1] : 0);
   for (int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < nitem; w += nwarps) {
     NBAcc I = {0.f, 0.f, 0.f}, J = {0.f, 0.f, 0.f};
-    int bi, sjl, np;
-    bool mi = false;
-    float o[3];
+    int sjl;
     if (w < nrest) {
       const Tile T = v.tiles[grouped ? v.cull_rest[w] : w];
-      bi = T.bi;
       sjl = T.bj * 32 + lane;
       const int si = T.bi * 32 + lane;
-      const float4 xi = v.xq[si], pi = v.par[si];
+      const float4 xi = v.xq[si], pi = v.par[si], xj = j_in_i_frame(v, T, lane), pj = v.par[sjl];
       const float qi = xi.w * k.econv_diel;
       const SystemInfo& S = v.sys[v.slot_sys[T.bi]];
-      unsigned ex = 0u, m14 = 0u;
-      if (T.mask >= 0) {
-        uint2 m = v.masks[T.mask * 32 + lane];
-        ex = m.x;
-        m14 = m.y;
+      const bool mi = T.flags & 1;
+      if (tile_masked(T)) {
+        unsigned ex, m14;
+        tile_masks(v, T, lane, ex, m14);
+        if (T.flags & 2) ex |= diag_exclusion(lane);
+        nb_rot<ELEC, true, false>(v, k, S, lane, si, xi, pi, qi, ex, m14, xj, pj, mi, T.bj * 32, nullptr, I, J);
+      } else {
+        nb_rot<ELEC, false, false>(v, k, S, lane, si, xi, pi, qi, 0u, 0u, xj, pj, mi, T.bj * 32, nullptr, I, J);
       }
-      if (T.flags & 2) ex |= diag_exclusion(lane);
-      // j positions moved into i's frame (the tile's centre offset, periodic image included)
-      float4 xj = v.xq[sjl];
-      const float4 pj = v.par[sjl];
-      o[0] = T.ox;
-      o[1] = T.oy;
-      o[2] = T.oz;
-      xj.x += T.ox;
-      xj.y += T.oy;
-      xj.z += T.oz;
-      mi = T.flags & 1;
-      if (tile_masked(T))
-        np = nb_rot<ELEC, true, ENERGY, false, SW>(v, k, S, lane, si, xi, pi, qi, ex, m14, xj, pj, mi, T.bj * 32,
-                                                   nullptr, I, J, sh);
-      else
-        np = nb_rot<ELEC, false, ENERGY, false, SW>(v, k, S, lane, si, xi, pi, qi, ex, m14, xj, pj, mi, T.bj * 32,
-                                                    nullptr, I, J, sh);
       nb_flush(v, si, I);
     } else {
-      const int g = w - nrest;
-      bi = v.cull_bi[g];
+      const int g = w - nrest, bi = v.cull_bi[g], si = bi * 32 + lane;
       const float4* gent = v.cull_ent + (size_t)g * 32;
       const float4 en = gent[lane];
       sjl = __float_as_int(en.w);
-      o[0] = en.x;
-      o[1] = en.y;
-      o[2] = en.z;
-      const int si = bi * 32 + lane;
       const float4 xi = v.xq[si], pi = v.par[si];
       const float qi = xi.w * k.econv_diel;
       const SystemInfo& S = v.sys[v.slot_sys[bi]];
@@ -410,31 +403,156 @@ __global__ void __launch_bounds__(ENERGY ? kNbEThreads : kNbThreads, ENERGY ? 5 
         xj.y += en.y;
         xj.z += en.z;
       }
-      np = nb_rot<ELEC, false, ENERGY, true, SW>(v, k, S, lane, si, xi, pi, qi, 0u, 0u, xj, pj, false, 0, gent, I, J,
-                                                 sh);
+      nb_rot<ELEC, false, true>(v, k, S, lane, si, xi, pi, qi, 0u, 0u, xj, pj, false, 0, gent, I, J);
       nb_flush(v, si, I);
     }
     if (sjl >= 0) nb_flush(v, sjl, J);
-    if (ENERGY) {
-      const SystemInfo& S = v.sys[v.slot_sys[bi]];
-      nb_stage(sh->ih, sh->il, sh->ip, lane, v, bi * 32 + lane, nullptr, &e.econv);
-      sh->js[lane] = sjl;
-      if (sjl >= 0) {
+  }
+}
+
+// appends this lane's pair to the warp's list where take (every lane calls this)
+__device__ __forceinline__ void nb_list(unsigned short* list, int& np, bool take, unsigned code, unsigned lt) {
+  const unsigned m = __ballot_sync(0xffffffffu, take);
+  if (take) list[np + __popc(m & lt)] = (unsigned short)code;
+  np += __popc(m);
+}
+
+// Energies: items as k_nb_force's, a CTA of two warps each (with one, 2,016 tiles of
+// 667 waters left the chip with three warps a scheduler and a list of six rounds a warp).
+// An item goes in four parts (a quarter of a tile's rotation; one 8-atom sub-block of the
+// i block against two groups), two to a warp, so that the lists stay short.
+constexpr int kNbEThreads = 64;
+template <int ELEC, bool SW = false>
+__global__ void __launch_bounds__(kNbEThreads, 8)
+    k_nb_energy(const __grid_constant__ DevView v, const __grid_constant__ NBConst k, const __grid_constant__ NBEConst e,
+                int cull) {
+  pdl_sync();
+  __shared__ NBEShared shared;
+  NBEShared* sh = &shared;
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  const unsigned lt = (1u << lane) - 1u;
+  unsigned short* list = sh->pair[wp];
+  const bool grouped = cull && nb_grouped(v);
+  const int nrest = grouped ? v.cull_n[0] : *v.ntiles;
+  const int nitem = nrest + (grouped ? v.cull_n[1] / 2 : 0);
+  const float tol = 2e-6f * k.cut2, reach2 = k.cut2 * 1.00001f;
+  for (int w = blockIdx.x; w < nitem; w += gridDim.x) {
+    const bool tile = w < nrest;
+    int bi;
+    NBEBox box = {};
+    unsigned ex = 0u, m14 = 0u;
+    if (tile) {
+      const Tile T = v.tiles[grouped ? v.cull_rest[w] : w];
+      bi = T.bi;
+      tile_masks(v, T, lane, ex, m14);
+      if (T.flags & 2) ex |= diag_exclusion(lane);
+      if (T.flags & 1) {
+        const SystemInfo& S = v.sys[v.slot_sys[bi]];
+        box = NBEBox{true, S.boxf[0], S.boxf[1], S.boxf[2], 1.f / S.boxf[0].h, 1.f / S.boxf[1].h, 1.f / S.boxf[2].h};
+      }
+      if (wp == 1) {
+        const float o[3] = {T.ox, T.oy, T.oz};
         DF O[3];
-        df_offset(v, S, bi, sjl >> 5, o, O);
-        nb_stage(sh->jh, sh->jl, sh->jp, lane, v, sjl, O, nullptr);
+        df_offset(v, v.sys[v.slot_sys[bi]], bi, T.bj, o, O);
+        nb_stage(sh->jh, sh->jl, sh->jp, lane, v, T.bj * 32 + lane, O, nullptr);
+        sh->js[lane] = T.bj * 32 + lane;
       }
-      __syncwarp();
-      NBESum sum = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
-      for (int p = lane; p < np; p += 32) nb_energy_df<ELEC, SW>(v, k, e, S, mi, bi * 32, sh, sh->pair[p], sum);
-      // the lanes' sums meet in double-float and enter fixed point once per item
-      const DF ev = df_warp_sum(sum.vdw), ee = df_warp_sum(sum.elec), vir = df_warp_sum(sum.vir);
-      const DF x = lane == 0 ? ev : (lane == 1 ? ee : vir);
-      if (lane < 3) {
-        long long* E = v.eacc + (size_t)v.slot_sys[bi] * E_NSLOTS;
-        atomic_add_ll(&E[lane == 0 ? E_VDW : (lane == 1 ? E_ELEC : E_VIRIAL)], fix_energy_d((double)x.h + (double)x.l));
+    } else {
+      const int g = 2 * (w - nrest) + wp, row = threadIdx.x;
+      bi = v.cull_bi[g];
+      const float4 en = v.cull_ent[(size_t)g * 32 + lane];
+      const int sj = __float_as_int(en.w);
+      sh->js[row] = sj;
+      if (sj >= 0) {
+        const float o[3] = {en.x, en.y, en.z};
+        DF O[3];
+        df_offset(v, v.sys[v.slot_sys[bi]], bi, sj >> 5, o, O);
+        nb_stage(sh->jh, sh->jl, sh->jp, row, v, sj, O, nullptr);
+      } else {
+        sh->jh[row] = make_float4(1.0e15f, 1.0e15f, 1.0e15f, 0.f);   // (empty lanes: far away)
       }
+    }
+    const SystemInfo& S = v.sys[v.slot_sys[bi]];
+    if (wp == 0) nb_stage(sh->ih, sh->il, sh->ip, lane, v, bi * 32 + lane, nullptr, &e.econv);
+    __syncthreads();
+    // a tile's i atom of this lane; minus its two j atoms of a group pair
+    const float4 xi = sh->ih[lane], ja = sh->jh[lane], jb = sh->jh[tile ? lane : 32 + lane];
+    const float2 nx = make_float2(-ja.x, -jb.x), ny = make_float2(-ja.y, -jb.y), nz = make_float2(-ja.z, -jb.z);
+    const DF2 zero = df2(DF{0.f, 0.f});
+    NBESum sum = {zero, zero, zero, f2(0.f)};
+    int np = 0;
+#pragma unroll 1
+    for (int s = 2 * wp; s < 2 * wp + 2; s++) {
+      if (tile) {
+#pragma unroll 4
+        for (int kk = 8 * s; kk < 8 * s + 8; kk++) {
+          const int row = (lane + kk) & 31;
+          const float4 x = sh->jh[row];
+          float dx = x.x - xi.x, dy = x.y - xi.y, dz = x.z - xi.z;
+          if (box.mi) {
+            constexpr float kRint = 12582912.f;
+            dx = fmaf(fmaf(dx, -box.ix, kRint) - kRint, box.x.h, dx);
+            dy = fmaf(fmaf(dy, -box.iy, kRint) - kRint, box.y.h, dy);
+            dz = fmaf(fmaf(dz, -box.iz, kRint) - kRint, box.z.h, dz);
+          }
+          const float r2 = dx * dx + dy * dy + dz * dz;
+          bool in = r2 <= k.cut2;
+          const bool listed = !((ex >> kk) & 1u);
+          // at the cutoff: decided in FP64
+          if (listed && fabsf(r2 - k.cut2) <= tol) in = nb_r2_fp64(v, S, bi * 32 + lane, sh->js[row]) <= k.cut2_dd;
+          nb_list(list, np, listed && in, lane | row << 5 | (((m14 >> kk) & 1u) << 11), lt);
+        }
+      } else {
+        const float4 lo = v.sub[8 * bi + 2 * s], hi = v.sub[8 * bi + 2 * s + 1];
+        float d2 = 3.0e38f;
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+          const float4 x = q ? jb : ja;
+          const float gx = fmaxf(fmaxf(lo.x - x.x, x.x - hi.x), 0.f), gy = fmaxf(fmaxf(lo.y - x.y, x.y - hi.y), 0.f);
+          const float gz = fmaxf(fmaxf(lo.z - x.z, x.z - hi.z), 0.f);
+          d2 = fminf(d2, gx * gx + gy * gy + gz * gz);
+        }
+        if (__any_sync(0xffffffffu, d2 <= reach2)) {
+#pragma unroll 4
+          for (int kk = 0; kk < 8; kk++) {
+            const int row = 8 * s + ((lane + kk) & 7);
+            const float4 x = sh->ih[row];
+            const float2 dx = __fadd2_rn(f2(x.x), nx), dy = __fadd2_rn(f2(x.y), ny), dz = __fadd2_rn(f2(x.z), nz);
+            const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
+            bool ina = r2.x <= k.cut2, inb = r2.y <= k.cut2;
+            if (fminf(fabsf(r2.x - k.cut2), fabsf(r2.y - k.cut2)) <= tol) {
+              if (fabsf(r2.x - k.cut2) <= tol) ina = nb_r2_fp64(v, S, bi * 32 + row, sh->js[lane]) <= k.cut2_dd;
+              if (fabsf(r2.y - k.cut2) <= tol) inb = nb_r2_fp64(v, S, bi * 32 + row, sh->js[32 + lane]) <= k.cut2_dd;
+            }
+            nb_list(list, np, ina, row | lane << 5, lt);
+            nb_list(list, np, inb, row | (32 + lane) << 5, lt);
+          }
+        }
+      }
+      // full rounds of two pairs a lane now, the rest with the next part
+      const int n = s & 1 ? np : np & ~63;
       __syncwarp();
+      for (int p = lane; p < n; p += 64) {
+        const bool two = p + 32 < n;
+        nb_energy_df2<ELEC, SW>(v, k, e, S, box, bi * 32, sh, list[p], list[two ? p + 32 : p], two, sum);
+      }
+      const unsigned short keep0 = list[min(n + lane, kNbList - 1)], keep1 = list[min(n + 32 + lane, kNbList - 1)];
+      __syncwarp();
+      np -= n;
+      if (lane < np) list[lane] = keep0;
+      if (lane + 32 < np) list[lane + 32] = keep1;
+    }
+    // (as the force passes check theirs: a call may come without forces)
+    fix_range(v.status, sum.f.x + sum.f.y);
+    // the lanes' sums meet in double-float and enter fixed point once per item
+    const DF ev = df_warp_sum(df_fold(sum.vdw)), ee = df_warp_sum(df_fold(sum.elec)), vir = df_warp_sum(df_fold(sum.vir));
+    const DF x = lane == 0 ? ev : (lane == 1 ? ee : vir);
+    if (wp == 1 && lane < 3) sh->sum[lane] = x;
+    __syncthreads();
+    if (wp == 0 && lane < 3) {
+      const DF y = df_add(x, sh->sum[lane]);
+      long long* E = v.eacc + (size_t)v.slot_sys[bi] * E_NSLOTS;
+      atomic_add_ll(&E[lane == 0 ? E_VDW : (lane == 1 ? E_ELEC : E_VIRIAL)], fix_energy_d((double)y.h + (double)y.l));
     }
   }
 }
@@ -697,56 +815,72 @@ __global__ void __launch_bounds__(kNbFThreads, 6)
   }
 }
 
+// CTAs of T threads for the passes whose items take unequal times: `times` the other
+// tile kernels' warps, no more than items, so that CTAs that end early make room for
+// the next (k_nb_force, 8 copies of the solvated box: 336 -> 314 us; one copy 51 -> 49)
+// items: per CTA
+static int uneven_grid(const Context& c, int g, int T, int items, int times) {
+  const long long want = (c.tile_cap + c.cull_cap / 64 + items - 1) / items;
+  return (int)std::min<long long>((long long)times * g * (kNbThreads / T), want > 0 ? want : 1);
+}
+
 static void launch_nb_force(Context& c, const NBConst& k, int g) {
   DevView v = c.view();
   const int cull = c.cull_built ? 1 : 0;
   constexpr int T = kNbFThreads;
-  // four times the other tile kernels' warps (no more than items): the items
-  // take unequal numbers of steps, and CTAs that end early make room for the next
-  // (8 copies of the solvated box: 336 -> 314 us; one copy 51 -> 49)
-  const long long want = (c.tile_cap + c.cull_cap / 64 + 3) / 4;
-  g = (int)std::min<long long>(4LL * g * (256 / T), want > 0 ? want : 1);
+  g = uneven_grid(c, g, T, T / 32, 4);
   if (k.elecmode == 0) launch_pdl(c.stream, g, T, 0, k_nb_force<kLawVdw>, v, k, cull);
   else if (k.elecmode == 4) launch_pdl(c.stream, g, T, 0, k_nb_force<kLawForce>, v, k, cull);
   else if (k.samesw) launch_pdl(c.stream, g, T, 0, k_nb_force<kLawSame>, v, k, cull);
   else launch_pdl(c.stream, g, T, 0, k_nb_force<kLawSplit>, v, k, cull);
 }
 
-template <bool E>
-static void launch_nb_mode(Context& c, const NBConst& k, int g) {
+static void launch_nb_tiles(Context& c, const NBConst& k, int g) {
+  DevView v = c.view();
+  const int cull = c.cull_built ? 1 : 0;
+  switch (k.elecmode) {
+    case 0: launch_pdl(c.stream, g, kNbThreads, 0, k_nb_tiles<0>, v, k, cull); break;
+    case 1: launch_pdl(c.stream, g, kNbThreads, 0, k_nb_tiles<1>, v, k, cull); break;
+    case 3: launch_pdl(c.stream, g, kNbThreads, 0, k_nb_tiles<3>, v, k, cull); break;
+    default: launch_pdl(c.stream, g, kNbThreads, 0, k_nb_tiles<4>, v, k, cull); break;
+  }
+}
+
+static void launch_nb_energy(Context& c, const NBConst& k, int g) {
   DevView v = c.view();
   const int cull = c.cull_built ? 1 : 0;
   const NBEConst e = make_nbe_const(k);
-  constexpr int T = E ? kNbEThreads : kNbThreads;
-  g *= kNbThreads / T;
+  constexpr int T = kNbEThreads;
+  g = uneven_grid(c, g, T, 1, 8);
   switch (k.elecmode) {
-    case 0: launch_pdl(c.stream, g, T, 0, k_nb_tiles<0, E>, v, k, e, cull); break;
-    case 1: launch_pdl(c.stream, g, T, 0, k_nb_tiles<1, E>, v, k, e, cull); break;
+    case 0: launch_pdl(c.stream, g, T, 0, k_nb_energy<0>, v, k, e, cull); break;
+    case 1: launch_pdl(c.stream, g, T, 0, k_nb_energy<1>, v, k, e, cull); break;
     case 3:
-      if (E && k.samesw) launch_pdl(c.stream, g, T, 0, k_nb_tiles<3, true, true>, v, k, e, cull);
-      else launch_pdl(c.stream, g, T, 0, k_nb_tiles<3, E>, v, k, e, cull);
+      if (k.samesw) launch_pdl(c.stream, g, T, 0, k_nb_energy<3, true>, v, k, e, cull);
+      else launch_pdl(c.stream, g, T, 0, k_nb_energy<3>, v, k, e, cull);
       break;
-    default: launch_pdl(c.stream, g, T, 0, k_nb_tiles<4, E>, v, k, e, cull); break;
+    default: launch_pdl(c.stream, g, T, 0, k_nb_energy<4>, v, k, e, cull); break;
   }
 }
 
 int launch_df_records(Context& c) {
+  c.kernel_launches += 1;
   const Spread sp = spread(c.nslots);
   launch_pdl(c.stream, sp.grid, sp.threads, 0, k_df_records, c.view(), c.d_charge.p, c.d_rlo.p, c.d_plo.p);
   return cudaGetLastError() == cudaSuccess ? PDGPU_OK : PDGPU_ERR_CUDA;
 }
 
-int launch_nb(Context& c, const NBConst& k, bool energy) {
-  c.kernel_launches += 1;
-  int g = tile_grid(c);
+// (the energies read the records of launch_df_records)
+int launch_nb(Context& c, const NBConst& k, bool energy, bool forces) {
+  const int g = tile_grid(c);
+  if (forces) {
+    c.kernel_launches += 1;
+    if (k.smooth) launch_nb_force(c, k, g);
+    else launch_nb_tiles(c, k, g);
+  }
   if (energy) {
     c.kernel_launches += 1;
-    launch_df_records(c);
-    launch_nb_mode<true>(c, k, g);
-  } else if (k.smooth) {
-    launch_nb_force(c, k, g);
-  } else {
-    launch_nb_mode<false>(c, k, g);
+    launch_nb_energy(c, k, g);
   }
   return cudaGetLastError() == cudaSuccess ? PDGPU_OK : PDGPU_ERR_CUDA;
 }

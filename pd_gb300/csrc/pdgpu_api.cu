@@ -705,7 +705,7 @@ int pdgpu_set_list_params(pdgpu_ctx* h, const pdgpu_list_params* p) {
   return PDGPU_OK;
 }
 
-static int enqueue_compute(Context& c, unsigned what, bool energy);
+static int enqueue_compute(Context& c, unsigned what, bool energy, bool forces);
 
 // the energy pass of a parameter gradient (Born radii, Gpol sums, dE/da, energies
 // and the GB pair terms' gradients); the passes that only form forces are left out
@@ -714,7 +714,7 @@ static int enqueue_grad_energies(Context& c, unsigned what, const AdjScratch& a)
   if (st != PDGPU_OK) return st;
   c.gb_no_chain = true;
   c.adj_g = a.g;
-  st = enqueue_compute(c, what & ~PDGPU_ENERGY, true);
+  st = enqueue_compute(c, what & ~PDGPU_ENERGY, true, false);
   c.gb_no_chain = false;
   c.adj_g = nullptr;
   return st;
@@ -817,7 +817,7 @@ int pdgpu_nb_energy_full(pdgpu_ctx* h, pdgpu_energies* out) {
   CK(cudaSetDevice(c.device));
   int st = mc_alloc(c);
   if (st != PDGPU_OK) return st;
-  st = enqueue_compute(c, PDGPU_NB, true);
+  st = enqueue_compute(c, PDGPU_NB, true, false);
   if (st != PDGPU_OK) return st;
   st = launch_mc_reference(c);
   if (st != PDGPU_OK) return st;
@@ -1027,8 +1027,15 @@ int pdgpu::enqueue_forces(Context& c, unsigned what, bool energy, bool rebuild, 
   // terms (positions) need nothing from the pair kernels: they run on the side
   // stream beside them, adding into the same fixed-point accumulators (integer
   // sums: the result does not depend on how the two streams interleave)
+  // ... and so do an energy call's LJ + Coulomb forces, a pass beside that of the energies
   const bool side_sa = (what & PDGPU_SA) && run_lcpo, side_bonded = (what & PDGPU_BONDED) != 0;
-  const bool forked = side_sa || side_bonded;
+  // FastMode off, or PD's calcEnergies (gbff.cpp:178-183: calcBornEnergy, no
+  // ExpApproxThreshold): the GB part alone plus the vacuum part from the GB
+  // object's own FF_NonBonded settings
+  const bool pd_energies = (what & PDGPU_PD_ENERGIES) != 0;
+  const bool vacuum = (what & PDGPU_GB) && (!c.gb_fast || pd_energies);
+  const bool side_nb = energy && !c.no_forces && ((what & PDGPU_NB) || vacuum);
+  const bool forked = side_sa || side_bonded || side_nb;
   if (forked) {
     CK(cudaEventRecord(c.ev_fork, c.stream));
     CK(cudaStreamWaitEvent(c.side, c.ev_fork, 0));
@@ -1036,21 +1043,20 @@ int pdgpu::enqueue_forces(Context& c, unsigned what, bool energy, bool rebuild, 
     c.stream = c.side;
     if (side_sa) st = launch_lcpo(c, lcpo_f, lcpo_e, lcpo_e_stride);
     if (st == PDGPU_OK && side_bonded) st = launch_bonded(c, energy);
+    if (st == PDGPU_OK && side_nb && (what & PDGPU_NB)) st = launch_nb(c, make_nb_const(c.nb), false, true);
+    if (st == PDGPU_OK && side_nb && vacuum) st = launch_nb(c, make_nb_const(gb_vacuum_params(c)), false, true);
     c.stream = main;
     // joined back below on every path, so a stream capture always closes
     CK(cudaEventRecord(c.ev_join, c.side));
   }
-  if (st == PDGPU_OK && (what & PDGPU_NB)) st = launch_nb(c, make_nb_const(c.nb), energy);
+  if (st == PDGPU_OK && energy && ((what & PDGPU_NB) || vacuum || ((what & PDGPU_GB) && !c.gb_no_chain))) st = launch_df_records(c);
+  if (st == PDGPU_OK && (what & PDGPU_NB)) st = launch_nb(c, make_nb_const(c.nb), energy, !energy);
   if (st == PDGPU_OK && (what & PDGPU_GB)) {
     GBConst k = make_gb_const(c.gb, c.list_radius_built);
-    // FastMode off, or PD's calcEnergies (gbff.cpp:178-183: calcBornEnergy, no
-    // ExpApproxThreshold): the GB part alone plus the vacuum part from the GB
-    // object's own FF_NonBonded settings
-    const bool pd_energies = (what & PDGPU_PD_ENERGIES) != 0;
-    if (!c.gb_fast || pd_energies) {
+    if (vacuum) {
       k.fast = 0;
       if (pd_energies) set_gb_threshold(k, -1e30);
-      st = launch_nb(c, make_nb_const(gb_vacuum_params(c)), energy);
+      st = launch_nb(c, make_nb_const(gb_vacuum_params(c)), energy, !energy);
     }
     double ec = econv_kcal();
     double premul = -0.5 * ec * (1.0 / c.gb.DielectricSolute - 1.0 / c.gb.DielectricSolvent);
@@ -1062,14 +1068,18 @@ int pdgpu::enqueue_forces(Context& c, unsigned what, bool energy, bool rebuild, 
 
 extern "C" {
 
-static int enqueue_compute(Context& c, unsigned what, bool energy) {
+static int enqueue_compute(Context& c, unsigned what, bool energy, bool forces) {
   if (!c.positions_set) return PDGPU_ERR_STATE;
   if ((what & PDGPU_NB) && !c.nb_set) return PDGPU_ERR_STATE;
   if ((what & PDGPU_GB) && (!c.has_gb || !c.gb_set)) return PDGPU_ERR_STATE;
   if ((what & PDGPU_SA) && !c.has_sa) return PDGPU_ERR_STATE;
   if ((what & (PDGPU_GB | PDGPU_SA)) && c.any_periodic) return PDGPU_ERR_UNSUPPORTED;
   CK(cudaMemsetAsync(c.d_status.p, 0, sizeof(unsigned), c.stream));
-  return enqueue_forces(c, what, energy, false, c.d_facc.p, energy ? c.d_eacc.p + E_SURF : nullptr, E_NSLOTS, true);
+  c.no_forces = !forces;
+  const int st =
+      enqueue_forces(c, what, energy, false, c.d_facc.p, energy ? c.d_eacc.p + E_SURF : nullptr, E_NSLOTS, true);
+  c.no_forces = false;
+  return st;
 }
 
 // queue the energy sums into h_eacc; decode them once they have arrived
@@ -1113,7 +1123,7 @@ int pdgpu_compute(pdgpu_ctx* h, unsigned what, pdgpu_energies* out, double* f, s
   if (!h || (f && (stride < 24 || stride % 8))) return PDGPU_ERR_ARG;
   Context& c = h->c;
   CK(cudaSetDevice(c.device));
-  int st = enqueue_compute(c, what, out != nullptr);
+  int st = enqueue_compute(c, what, out != nullptr, f != nullptr);
   if (st != PDGPU_OK) return st;
   // forces, energies and status are queued together: one wait for all three
   if (f) {
@@ -1146,7 +1156,7 @@ int pdgpu_compute_device(pdgpu_ctx* h, unsigned what, double* d_f) {
   if (!h) return PDGPU_ERR_ARG;
   Context& c = h->c;
   CK(cudaSetDevice(c.device));
-  int st = enqueue_compute(c, what, (what & PDGPU_ENERGY) != 0);
+  int st = enqueue_compute(c, what, (what & PDGPU_ENERGY) != 0, d_f != nullptr);
   if (st != PDGPU_OK) return st;
   if (d_f) st = launch_finalize_forces(c, d_f, 3, false, kForceToN);
   return st;

@@ -312,7 +312,7 @@ int alloc_tiles(Context& c, long long tiles);
 // the NB j-atom group arrays for the current tile capacity
 int alloc_cull_tiles(Context& c);
 int launch_pack(Context& c, float check_disp);
-int launch_nb(Context& c, const NBConst& k, bool need_virial);
+int launch_nb(Context& c, const NBConst& k, bool energy, bool forces);
 int launch_gb(Context& c, const GBConst& k, double halfeconv, double born_offset, double premul, bool energy);
 int launch_lcpo(Context& c, long long* facc_out, long long* esurf_out, int esurf_stride);
 // FP32 remainders of the packed slots (double-float positions and parameters), before an energy pass

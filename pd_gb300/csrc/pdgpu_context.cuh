@@ -90,6 +90,7 @@ struct Context {
   bool nb_set = false, gb_set = false;
   bool gb_fast = true;             // FF_GeneralizedBorn_Still::FastMode
   bool gb_no_chain = false;        // a gradient call: no GB force passes, pair gradients with the energies
+  bool no_forces = false;          // the running call reads no forces: passes that only add to them are left out
   long long* adj_g = nullptr;      // where they go, during that call
   pdgpu_nb_params gb_vac{};        // the GB object's own FF_NonBonded settings (FastMode off, calcEnergies)
   bool gb_vac_set = false;

@@ -355,7 +355,7 @@ int pdgpu_time_kernel(pdgpu_ctx* h, int kernel, int reps, int flush_l2, double* 
     if (kernel == 5) CK(cudaMemsetAsync(c.md->d_ke.p, 0, sizeof(long long) * c.nsys, c.stream));
     CK(cudaEventRecord(e0, c.stream));
     switch (kernel) {
-      case 0: st = launch_nb(c, make_nb_const(c.nb), false); break;
+      case 0: st = launch_nb(c, make_nb_const(c.nb), false, true); break;
       case 1: case 2: case 3: st = launch_gb_stage(c, make_gb_const(c.gb, c.list_radius_built), kernel); break;
       case 4: st = launch_lcpo(c, c.d_facc.p, nullptr, 0); break;
       case 5: st = launch_integrate(c, *c.md, false, false); break;
