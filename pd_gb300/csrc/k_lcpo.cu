@@ -17,6 +17,7 @@ namespace pdgpu {
 //    lo.w = their largest LCPO radius, or -1 when the block holds none
 __global__ void __launch_bounds__(256) k_lcpo_prep(DevView v, const float4* lc, const double* P, const double* sigma,
                                                    float4* lpos, float4* psig, float4* box, int* ncand) {
+  pdl_sync();
   const int lane = threadIdx.x & 31;
   const int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (b >= v.nblocks) return;  // whole warps
@@ -61,6 +62,7 @@ __global__ void __launch_bounds__(256) k_lcpo_prep(DevView v, const float4* lc, 
 // Candidates land in any order: k_lcpo_sort orders them by atom index.
 __global__ void __launch_bounds__(256) k_lcpo_cand(DevView v, const float4* lc, const float4* box, int* ncand,
                                                    int* cand) {
+  pdl_sync();
   const int lane = threadIdx.x & 31;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   const int nt = *v.ntiles;
@@ -115,6 +117,7 @@ __global__ void __launch_bounds__(256) k_lcpo_cand(DevView v, const float4* lc, 
 // records in sequence instead of chasing slot indices
 __global__ void k_lcpo_sort(DevView v, const float4* lc, const float4* lpos, const int* ncand, const int* cand,
                             int* nl_n, int2* nl_e2, float4* nl_ent) {
+  pdl_sync();
   __shared__ int sh_key[8][kLcpoCand];
   __shared__ int sh_slot[8][kLcpoCand];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -194,6 +197,7 @@ __global__ void __launch_bounds__(kLcpoWarps * 32, 6) k_lcpo_main(DevView v, con
                                                    const float4* nl_ent, const int* ncand, const double* P,
                                                    const double* sigma, double* sasa_out, long long* facc_out,
                                                    long long* esurf_out, int esurf_stride) {
+  pdl_sync();
   __shared__ float4 tab_sh[kLcpoWarps][2][kLcpoMax];   // (d_ik, r_k), (w3, w3b, Si3ik term, atom_k)
   const int lane = threadIdx.x & 31;
   const int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -332,15 +336,14 @@ int launch_lcpo(Context& c, long long* facc_out, long long* esurf_out, int esurf
   cudaStream_t st = c.stream;
   int g = tile_grid(c);
   c.kernel_launches += 4;
-  k_lcpo_prep<<<(int)(((long long)c.nblocks * 32 + 255) / 256), 256, 0, st>>>(
-      v, c.d_lc_par.p, c.d_lcpoP.p, c.d_lcpoSig.p, c.d_lc_pos.p, c.d_lc_psig.p, c.d_lc_box.p, c.d_lc_ncand.p);
-  k_lcpo_cand<<<g, 256, 0, st>>>(v, c.d_lc_par.p, c.d_lc_box.p, c.d_lc_ncand.p, c.d_lc_cand.p);
-  int nw = (int)(((long long)c.nslots * 32 + 255) / 256);
-  k_lcpo_sort<<<nw, 256, 0, st>>>(v, c.d_lc_par.p, c.d_lc_pos.p, c.d_lc_ncand.p, c.d_lc_cand.p, c.d_lc_n.p,
-                                   c.d_lc_e2.p, c.d_lc_ent.p);
-  k_lcpo_main<<<(int)(((long long)c.nslots * 32 + kLcpoWarps * 32 - 1) / (kLcpoWarps * 32)), kLcpoWarps * 32, 0, st>>>(
-      v, c.d_lc_par.p, c.d_lc_pos.p, c.d_lc_psig.p, c.d_lc_n.p, c.d_lc_e2.p, c.d_lc_ent.p, c.d_lc_ncand.p, c.d_lcpoP.p, c.d_lcpoSig.p, c.d_sasa.p, facc_out, esurf_out,
-                                   esurf_stride);
+  launch_pdl(st, (c.nblocks + 7) / 8, 256, 0, k_lcpo_prep, v, c.d_lc_par.p, c.d_lcpoP.p, c.d_lcpoSig.p, c.d_lc_pos.p,
+             c.d_lc_psig.p, c.d_lc_box.p, c.d_lc_ncand.p);
+  launch_pdl(st, g, 256, 0, k_lcpo_cand, v, c.d_lc_par.p, c.d_lc_box.p, c.d_lc_ncand.p, c.d_lc_cand.p);
+  launch_pdl(st, (c.nslots + 7) / 8, 256, 0, k_lcpo_sort, v, c.d_lc_par.p, c.d_lc_pos.p, c.d_lc_ncand.p, c.d_lc_cand.p,
+             c.d_lc_n.p, c.d_lc_e2.p, c.d_lc_ent.p);
+  launch_pdl(st, (c.nslots + kLcpoWarps - 1) / kLcpoWarps, kLcpoWarps * 32, 0, k_lcpo_main, v, c.d_lc_par.p,
+             c.d_lc_pos.p, c.d_lc_psig.p, c.d_lc_n.p, c.d_lc_e2.p, c.d_lc_ent.p, c.d_lc_ncand.p, c.d_lcpoP.p,
+             c.d_lcpoSig.p, c.d_sasa.p, facc_out, esurf_out, esurf_stride);
   return cudaGetLastError() == cudaSuccess ? PDGPU_OK : PDGPU_ERR_CUDA;
 }
 

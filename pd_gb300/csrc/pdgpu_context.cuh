@@ -67,8 +67,8 @@ struct Context {
   cudaStream_t stream = nullptr;
   // work that reads positions only (bonded terms, the LCPO recalculation) runs on
   // `side` beside the pair kernels, forked from and joined back to `stream`
-  cudaStream_t side = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  cudaStream_t side = nullptr, side2 = nullptr;
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_join2 = nullptr;
   cudaEvent_t ev_total = nullptr;   // a list build's tile count has reached h_total
   cudaEvent_t ev_pos = nullptr;     // the copy out of h_pos is done
   int nsys = 0, natom = 0, nslots = 0, nblocks = 0;
