@@ -63,23 +63,35 @@ __device__ __forceinline__ int f2ord(float f) {
 }
 __device__ __forceinline__ float ord2f(int i) { return __int_as_float(i >= 0 ? i : i ^ 0x7fffffff); }
 
-// everything a build counts into, cleared in one launch
-struct ListInit {
-  int *count, *cursor, *sorted_atom, *bcell_count, *bcell_cursor, *lo, *hi, *hmax, *counters;
-  int ncells, nslots, nbcells, nsys3;
+// What a build starts from.  The kernels of a build put these back for the next one
+// once they are through with them (the first build finds them set by launch_list_init):
+// cells empty, boxes of open systems turned inside out, block cells empty.
+struct ListState {
+  int *count, *head;               // per cell: atoms, the last of them to arrive (-1: none)
+  int *lo, *hi, *hmax;             // per system, 3: box of an open system, largest half-extents
+  int *bcell_count, *bcell_cursor; // per block cell
+  int* counters;
+  int ncells, nbcells, nsys3;
 };
-__global__ void k_list_init(ListInit I) {
-  pdl_sync();
+__device__ __forceinline__ void reset_counter(const ListState& I, int t) {
+  if (t < 8) I.counters[t] = t == 5 ? 1 : 0;   // [5]: the NB groups fit until a row finds they do not
+}
+__global__ void k_list_init(ListState I, int* sorted_atom, int nslots) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x, n = gridDim.x * blockDim.x;
-  for (int i = t; i < I.ncells; i += n) I.count[i] = I.cursor[i] = 0;
-  for (int i = t; i < I.nslots; i += n) I.sorted_atom[i] = -1;
-  for (int i = t; i < I.nbcells; i += n) I.bcell_count[i] = I.bcell_cursor[i] = 0;
+  for (int i = t; i < I.ncells; i += n) {
+    I.count[i] = 0;
+    I.head[i] = -1;
+  }
+  for (int i = t; i < nslots; i += n) sorted_atom[i] = -1;   // (padding slots keep that)
   for (int i = t; i < I.nsys3; i += n) {
     I.lo[i] = f2ord(3.0e38f);
     I.hi[i] = f2ord(-3.0e38f);
-    I.hmax[i] = f2ord(0.f);
   }
-  if (t < 8) I.counters[t] = t == 5 ? 1 : 0;   // [5]: the NB groups fit until a row finds they do not
+}
+// (a list that outgrew its arrays: its rows run again)
+__global__ void k_reset_counters(ListState I) {
+  pdl_sync();
+  reset_counter(I, threadIdx.x);
 }
 
 // bounding box of each open-space system (periodic systems key on the box);
@@ -146,10 +158,15 @@ __device__ __forceinline__ void grid_setup(const SystemInfo& S, int s, const int
 
 // (the last CTA, launched past the atoms where some system uses a block grid,
 // sets those grids up)
-__global__ void k_keys(DevView v, const int* atom_sys, const int* lo, const int* hi, int* bucket, int* count,
-                       BlockGrid* grid) {
+__global__ void k_keys(DevView v, const int* atom_sys, ListState I, int* next, BlockGrid* grid) {
   pdl_sync();
   int a = blockIdx.x * blockDim.x + threadIdx.x;
+  const int *lo = I.lo, *hi = I.hi;
+  reset_counter(I, a);
+  for (int i = a, n = gridDim.x * blockDim.x; i < max(I.nbcells, I.nsys3); i += n) {
+    if (i < I.nsys3) I.hmax[i] = f2ord(0.f);
+    if (i < I.nbcells) I.bcell_count[i] = I.bcell_cursor[i] = 0;
+  }
   if (grid && blockIdx.x == gridDim.x - 1) {
     for (int s = threadIdx.x; s < v.nsys; s += blockDim.x)
       if (v.sys[s].nblocks > kDirectBlocks) grid_setup(v.sys[s], s, lo, hi, grid);
@@ -174,8 +191,8 @@ __global__ void k_keys(DevView v, const int* atom_sys, const int* lo, const int*
     q[c] = (unsigned)qi;
   }
   int b = s * kCellsPerSystem + hilbert3(q[0], q[1], q[2]);
-  bucket[a] = b;
-  atomicAdd(&count[b], 1);
+  next[a] = atomicExch(&I.head[b], a);
+  atomicAdd(&I.count[b], 1);
 }
 
 // --- exclusive scans --------------------------------------------------------
@@ -251,27 +268,43 @@ __global__ void __launch_bounds__(1024) k_scan_one(const int* in, int* out, int 
   }
 }
 
-__global__ void k_scatter(int natom, const int* bucket, const int* offset, int* cursor, int* tmp) {
-  pdl_sync();
-  int a = blockIdx.x * blockDim.x + threadIdx.x;
-  if (a >= natom) return;
-  int b = bucket[a];
-  tmp[offset[b] + atomicAdd(&cursor[b], 1)] = a;
+// A thread per cell: the cell's place (after the system's atoms in runs of 1024 cells
+// before, whose sums k_scan_block left with the cells' offsets within their runs), its
+// atoms from their chain, sorted by insertion so that the order is deterministic, into
+// their slots.
+constexpr int kSortThreads = 256;
+__device__ __forceinline__ int warp_sum_int(int x) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+  return x;
 }
-
-// insertion sort inside each non-empty cell so the order is deterministic, then
-// the cell's atoms into their slots
-__global__ void k_cell_sort(DevView v, int ncells, const int* offset, const int* count, int* tmp, int* sorted_atom,
-                            int* slot_of) {
+__global__ void __launch_bounds__(kSortThreads) k_cell_sort(DevView v, ListState I, const int* offset, const int* run_sums,
+                                                            const int* next, int* tmp, int* sorted_atom, int* slot_of) {
+  static_assert(kCellsPerSystem == 32 * 1024 && 1024 % kSortThreads == 0, "a warp adds a system's runs");
   pdl_sync();
-  int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= ncells) return;
-  int n = count[b];
+  __shared__ int base;
+  const int b = blockIdx.x * kSortThreads + threadIdx.x;   // (ncells is a multiple of 1024)
+  const SystemInfo& S = v.sys[b / kCellsPerSystem];
+  if (threadIdx.x < 32) {
+    const int run = b / 1024, r0 = b / kCellsPerSystem * 32;
+    const int x = warp_sum_int(r0 + (int)threadIdx.x < run ? run_sums[r0 + threadIdx.x] : 0);
+    if (threadIdx.x == 0) base = S.atom_start + x;
+  }
+  const int n = I.count[b];
+  int a = n ? I.head[b] : -1;
+  __syncthreads();
+  const int o = base + (n ? offset[b] : 0);
+  if (b < I.nsys3) {
+    I.lo[b] = f2ord(3.0e38f);
+    I.hi[b] = f2ord(-3.0e38f);
+  }
   if (n < 1) return;
-  const int o = offset[b];
+  I.count[b] = 0;
+  I.head[b] = -1;
   int* p = tmp + o;
-  for (int i = 1; i < n; i++) {
-    int x = p[i];
+  for (int i = 0; i < n; i++) {
+    const int x = a;
+    a = next[a];
     int j = i - 1;
     while (j >= 0 && p[j] > x) {
       p[j + 1] = p[j];
@@ -279,12 +312,11 @@ __global__ void k_cell_sort(DevView v, int ncells, const int* offset, const int*
     }
     p[j + 1] = x;
   }
-  const SystemInfo& S = v.sys[b / kCellsPerSystem];
   const int slot = S.pad_start + (o - S.atom_start);
   for (int i = 0; i < n; i++) {
-    const int a = p[i];
-    sorted_atom[slot + i] = a;
-    slot_of[a] = slot + i;
+    const int x = p[i];
+    sorted_atom[slot + i] = x;
+    slot_of[x] = slot + i;
   }
 }
 
@@ -1039,43 +1071,46 @@ static void launch_list_tail(Context& c, float list_radius) {
   if (c.cull_built) launch_cull(c, list_radius);
 }
 
-int launch_list_build(Context& c, float list_radius, float full_radius, ListSizing sizing) {
-  c.kernel_launches += 6;   // and a scan
-  DevView v = c.view();
-  cudaStream_t st = c.stream;
-  const int ncells = c.nsys * kCellsPerSystem;
-  int* lo = reinterpret_cast<int*>(c.d_sys_lo.p);
-  int* hi = reinterpret_cast<int*>(c.d_sys_hi.p);
-  int* hmax = reinterpret_cast<int*>(c.d_sys_hmax.p);
-  const bool grid = c.max_sys_blocks > kDirectBlocks;
-  ListInit I;
+static ListState list_state(Context& c, bool grid) {
+  ListState I;
   I.count = c.d_count.p;
-  I.cursor = c.d_cursor.p;
-  I.sorted_atom = c.d_sorted_atom.p;
+  I.head = c.d_head.p;
+  I.lo = reinterpret_cast<int*>(c.d_sys_lo.p);
+  I.hi = reinterpret_cast<int*>(c.d_sys_hi.p);
+  I.hmax = reinterpret_cast<int*>(c.d_sys_hmax.p);
   I.bcell_count = c.d_bcell_count.p;
   I.bcell_cursor = c.d_bcell_cursor.p;
-  I.lo = lo;
-  I.hi = hi;
-  I.hmax = hmax;
   I.counters = c.d_counters.p;
-  I.ncells = ncells;
-  I.nslots = c.nslots;
+  I.ncells = c.nsys * kCellsPerSystem;
   I.nbcells = grid ? c.nblocks : 0;
   I.nsys3 = 3 * c.nsys;
-  launch_pdl(st, std::min(nblk(std::max(ncells, c.nslots), 256), 1216), 256, 0, k_list_init, I);
+  return I;
+}
+
+// (once, before a context's first build)
+int launch_list_init(Context& c) {
+  k_list_init<<<std::min(nblk(std::max(c.nsys * kCellsPerSystem, c.nslots), 256), 1216), 256, 0, c.stream>>>(
+      list_state(c, false), c.d_sorted_atom.p, c.nslots);
+  return cudaGetLastError() == cudaSuccess ? PDGPU_OK : PDGPU_ERR_CUDA;
+}
+
+int launch_list_build(Context& c, float list_radius, float full_radius, ListSizing sizing) {
+  c.kernel_launches += 4;
+  DevView v = c.view();
+  cudaStream_t st = c.stream;
+  const bool grid = c.max_sys_blocks > kDirectBlocks;
+  const ListState I = list_state(c, grid);
   if (!c.all_periodic) {
     c.kernel_launches += 1;
-    launch_pdl(st, nblk(c.natom, 256), 256, 0, k_bbox, v, c.d_atom_sys.p, lo, hi);
+    launch_pdl(st, nblk(c.natom, 256), 256, 0, k_bbox, v, c.d_atom_sys.p, I.lo, I.hi);
   }
   const Spread ks = spread(c.natom, 64);
-  launch_pdl(st, ks.grid + (grid ? 1 : 0), ks.threads, 0, k_keys, v, c.d_atom_sys.p, lo, hi, c.d_bucket.p, c.d_count.p,
-                                                              grid ? c.d_bgrid.p : nullptr);
-  scan_ints(c, c.d_count.p, c.d_offset.p, c.d_scan_tmp.p, ncells, st);
-  launch_pdl(st, nblk(c.natom, 256), 256, 0, k_scatter, c.natom, c.d_bucket.p, c.d_offset.p, c.d_cursor.p,
-                                                 c.d_tmp_sorted.p);
-  launch_pdl(st, nblk(ncells, 256), 256, 0, k_cell_sort, v, ncells, c.d_offset.p, c.d_count.p, c.d_tmp_sorted.p,
-                                                 c.d_sorted_atom.p, c.d_slot_of.p);
-  launch_pdl(st, nblk((long long)c.nblocks * 32, 128), 128, 0, k_blocks, v, slot_param_view(c), c.clear, c.d_bgrid.p, hmax, c.d_bcell.p,
+  launch_pdl(st, ks.grid + (grid ? 1 : 0), ks.threads, 0, k_keys, v, c.d_atom_sys.p, I, c.d_next.p,
+             grid ? c.d_bgrid.p : nullptr);
+  launch_pdl(st, nblk(I.ncells, 1024), 1024, 0, k_scan_block, c.d_count.p, c.d_offset.p, c.d_scan_tmp.p, I.ncells);
+  launch_pdl(st, nblk(I.ncells, kSortThreads), kSortThreads, 0, k_cell_sort, v, I, c.d_offset.p, c.d_scan_tmp.p, c.d_next.p,
+             c.d_tmp_sorted.p, c.d_sorted_atom.p, c.d_slot_of.p);
+  launch_pdl(st, nblk((long long)c.nblocks * 32, 128), 128, 0, k_blocks, v, slot_param_view(c), c.clear, c.d_bgrid.p, I.hmax, c.d_bcell.p,
                                                                  c.d_bcell_count.p, c.nb_set ? 1 : 0);
   if (grid) {
     c.kernel_launches += 1;   // and a scan
@@ -1103,9 +1138,7 @@ int launch_list_build(Context& c, float list_radius, float full_radius, ListSizi
       const int e = alloc_tiles(c, total);
       if (e != PDGPU_OK) return e;
       c.kernel_launches += 1;
-      ListInit J{};
-      J.counters = c.d_counters.p;
-      launch_pdl(st, 1, 32, 0, k_list_init, J);
+      launch_pdl(st, 1, 32, 0, k_reset_counters, I);
       launch_rows(c, list_radius, full_radius);
       launch_list_tail(c, list_radius);
     }

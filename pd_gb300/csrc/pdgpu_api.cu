@@ -504,10 +504,10 @@ pdgpu_ctx* pdgpu_create(int device, const pdgpu_system_desc* d, int* status) {
   const size_t nsb = (ncells + 1023) / 1024;
   if (e == cudaSuccess) e = c.d_pos.alloc(3 * (size_t)N);
   if (e == cudaSuccess) e = c.d_fout.alloc(3 * (size_t)N);
-  if (e == cudaSuccess) e = c.d_bucket.alloc(N);
+  if (e == cudaSuccess) e = c.d_next.alloc(N);
   if (e == cudaSuccess) e = c.d_count.alloc(ncells);
   if (e == cudaSuccess) e = c.d_offset.alloc(ncells);
-  if (e == cudaSuccess) e = c.d_cursor.alloc(ncells);
+  if (e == cudaSuccess) e = c.d_head.alloc(ncells);
   if (e == cudaSuccess) e = c.d_scan_tmp.alloc(nsb + 1);
   if (e == cudaSuccess) e = c.d_tmp_sorted.alloc(N);
   if (e == cudaSuccess) e = c.d_sys_lo.alloc(3 * (size_t)c.nsys);
@@ -567,6 +567,7 @@ pdgpu_ctx* pdgpu_create(int device, const pdgpu_system_desc* d, int* status) {
   if (e == cudaSuccess) e = c.h_total.alloc(1);
   if (e == cudaSuccess && 24 * (size_t)N <= kStagedPositions) e = c.h_pos.alloc(3 * (size_t)N);
   if (e != cudaSuccess) return bad(PDGPU_ERR_CUDA);
+  if (launch_list_init(c) != PDGPU_OK) return bad(PDGPU_ERR_CUDA);
 
   // PD defaults: FF_NonBonded::settodefault (nonbonded.cpp:985-1021),
   // FF_GeneralizedBorn_Still constructor (gbff.cpp:33-55), NeighbourList Padding 0.5

@@ -311,6 +311,7 @@ int launch_list_build(Context& c, float list_radius, float full_radius, ListSizi
 int alloc_tiles(Context& c, long long tiles);
 // the NB j-atom group arrays for the current tile capacity
 int alloc_cull_tiles(Context& c);
+int launch_list_init(Context& c);
 int launch_pack(Context& c, float check_disp);
 int launch_nb(Context& c, const NBConst& k, bool energy, bool forces);
 int launch_gb(Context& c, const GBConst& k, double halfeconv, double born_offset, double premul, bool energy);

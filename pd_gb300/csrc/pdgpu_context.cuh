@@ -124,8 +124,8 @@ struct Context {
   DBuf<double> d_fout;         // [natom*3] N (device-side output buffer)
 
   // list build scratch
-  DBuf<int> d_bucket;          // [natom]
-  DBuf<int> d_count, d_offset, d_cursor;      // [nsys*kCellsPerSystem]
+  DBuf<int> d_next;            // [natom] the chain of each cell's atoms
+  DBuf<int> d_count, d_offset, d_head;        // [nsys*kCellsPerSystem]
   DBuf<int> d_scan_tmp;
   DBuf<int> d_tmp_sorted;      // [natom]
   DBuf<float> d_sys_lo, d_sys_hi;              // [nsys*3]
