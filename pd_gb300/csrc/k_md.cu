@@ -43,12 +43,15 @@ __device__ __forceinline__ void box_muller(unsigned a, unsigned b, double& n1, d
   n2 = (double)(r * s);
 }
 
-__device__ __forceinline__ void slot_force(const MDView& m, int s, double f[3]) {
+// the force on slot s times `scale`, from the fixed-point accumulators (scale takes their
+// unit with it: kForceUnit newtons)
+constexpr double kForceUnit = kForceToN / kForceScale;
+__device__ __forceinline__ void slot_force(const MDView& m, int s, double scale, double f[3]) {
 #pragma unroll
   for (int c = 0; c < 3; c++) {
     long long q = m.facc[force_at(s, c)];
     if (m.facc_sa) q += m.facc_sa[force_at(s, c)];
-    f[c] = (double)q * (1.0 / kForceScale) * kForceToN;
+    f[c] = (double)q * scale;
   }
 }
 
@@ -98,25 +101,19 @@ __device__ __forceinline__ void advance_step(const MDView& m) {
 // GB Langevin step of 4,224 75.2 -> 70.1, a solvated step of 22,489 88.6 -> 84.5.
 
 // PD velocity Verlet as written: half kick, (KE), half kick, drift t*(v+dv), kick.
-// In: v the velocity and p the position of atom a; out: v after the half kick
-__device__ __forceinline__ void vv_half(const MDView& m, double dt, int a, int s, double f[3], double v[3], double p[3],
-                                        double& tm) {
-  slot_force(m, s, f);
-  tm = 0.5 * dt * m.mterms[a].x;
+// vv_half: dv the half kick, v the velocity after the first; vv_rest: the others, p the
+// new position
+__device__ __forceinline__ void vv_half(const MDView& m, double dt, int a, int s, double dv[3], double v[3]) {
+  slot_force(m, s, 0.5 * kForceUnit * dt * m.mterms[a].x, dv);
 #pragma unroll
-  for (int c = 0; c < 3; c++) {
-    v[c] = m.vel[3 * a + c] + f[c] * tm;
-    p[c] = m.pos[3 * a + c];
-  }
+  for (int c = 0; c < 3; c++) v[c] = m.vel[3 * a + c] + dv[c];
 }
-__device__ __forceinline__ void vv_rest(const MDView& m, double dt, int a, const double f[3], double v[3], double p[3],
-                                        double tm) {
+__device__ __forceinline__ void vv_rest(const MDView& m, double dt, int a, const double dv[3], double v[3], double p[3]) {
+  const double dta = dt * (1.0 / kAngstrom);
 #pragma unroll
   for (int c = 0; c < 3; c++) {
-    double dv = f[c] * tm;
-    v[c] += dv;
-    p[c] += dt * (v[c] + dv) * (1.0 / kAngstrom);
-    v[c] += dv;
+    v[c] += dv[c] + dv[c];
+    p[c] = m.pos[3 * a + c] + dta * v[c];
     m.vel[3 * a + c] = v[c];
     m.pos[3 * a + c] = p[c];
   }
@@ -125,11 +122,10 @@ __device__ __forceinline__ void vv_rest(const MDView& m, double dt, int a, const
 __global__ void k_vv(MDView m, double dt) {
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
   const bool valid = a < m.natom;
-  double f[3] = {0.0, 0.0, 0.0}, v[3] = {0.0, 0.0, 0.0}, p[3];
-  double tm = 0.0;
-  if (valid) vv_half(m, dt, a, m.slot_of[a], f, v, p, tm);
+  double dv[3] = {0.0, 0.0, 0.0}, v[3] = {0.0, 0.0, 0.0}, p[3];
+  if (valid) vv_half(m, dt, a, m.slot_of[a], dv, v);
   add_ke(m, a, valid, v);
-  if (valid) vv_rest(m, dt, a, f, v, p, tm);
+  if (valid) vv_rest(m, dt, a, dv, v, p);
   advance_step(m);
 }
 
@@ -137,40 +133,39 @@ __global__ void k_vv_pack(MDView m, double dt, DevView d, PackArgs P) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s < d.nslots) {   // (whole warps)
     const int a = d.sorted_atom[s];
-    double f[3], v[3], p[3] = {0.0, 0.0, 0.0}, tm;
+    double dv[3], v[3], p[3] = {0.0, 0.0, 0.0};
     if (a >= 0) {
-      vv_half(m, dt, a, s, f, v, p, tm);
-      vv_rest(m, dt, a, f, v, p, tm);
+      vv_half(m, dt, a, s, dv, v);
+      vv_rest(m, dt, a, dv, v, p);
     }
     pack_slot(d, P, s, a, p);
   }
   advance_step(m);
 }
 
-// PD Langevin step (gamma*dt > 1e-5 branch) with per-system target temperature
-// Per-launch constants are folded on the host (LangevinCoeffs: kick = (1 -
-// c0/c1)/gt, drift_f = c0 c2 / c1, sv = sqrt(varv), sr = sqrt(varr)/gamma):
-// one division and one square root per atom remain on the narrow FP64 pipe.
-// langevin_kick: the velocity v with the force's kick; langevin_move: the drift and
-// the noise, which leave the new position in p and the new velocity in v
+// PD Langevin step (gamma*dt > 1e-5 branch) with per-system target temperature.  Bound
+// by the FP64 pipe (two results a cycle and SM): every product of constants is folded on
+// the host (LangevinCoeffs) or once per atom, which leaves ten FP64 operations a
+// component instead of twenty (179,912 atoms: 35.0 -> 28.3 us).
+// langevin_kick: ft the force times dt / m, v the velocity with the force's kick;
+// langevin_move: the drift and the noise, which leave the new position in p and the new
+// velocity in v
 __device__ __forceinline__ void langevin_kick(const MDView& m, const LangevinCoeffs& L, int a, int s, bool first,
-                                              double f[3], double v[3], double& tm, double& srm) {
-  slot_force(m, s, f);
+                                              double ft[3], double v[3], double& srm) {
   const double2 mt = m.mterms[a];
-  tm = L.dt * mt.x;
+  slot_force(m, s, kForceUnit * L.dt * mt.x, ft);
   srm = mt.y;
 #pragma unroll
   for (int c = 0; c < 3; c++) {
     v[c] = m.vel[3 * a + c];
-    if (!first) v[c] += L.kick * f[c] * tm;
+    if (!first) v[c] += L.kick * ft[c];
   }
 }
 __device__ __forceinline__ void langevin_move(const MDView& m, const LangevinCoeffs& L, int a, unsigned long long step,
-                                              const double f[3], double v[3], double p[3], double tm, double srm) {
+                                              const double ft[3], double v[3], double p[3], double srm) {
   // sqrt(k_B T / m): the temperature's root in FP32 (it only scales the noise)
   const double s = (double)sqrtf((float)m.temp[m.atom_sys[a]]) * srm;
-  const double sigmav = s * L.sv;
-  const double sigmar = s * L.sr;
+  const double nr = s * L.sr, nv1 = s * L.sv1, nv2 = s * L.sv2;
   // six normals, in PD's draw order n1x n2y | n2x n1z | n1y n2z (md.cpp:1017-1019)
   uint2 key = make_uint2((unsigned)m.seed, (unsigned)(m.seed >> 32));
   uint4 r0 = philox4x32(make_uint4((unsigned)step, (unsigned)(step >> 32), (unsigned)a, 0u), key);
@@ -182,13 +177,9 @@ __device__ __forceinline__ void langevin_move(const MDView& m, const LangevinCoe
   const double n1[3] = {n1x, n1y, n1z}, n2[3] = {n2x, n2y, n2z};
 #pragma unroll
   for (int c = 0; c < 3; c++) {
-    double dvr = sigmav * (L.crv * n1[c] + L.sq1mcrv2 * n2[c]);
-    double drr = sigmar * n1[c];
-    double dr = L.dt * (L.c1 * v[c] + L.c2 * f[c] * tm) + drr;
-    double dv = L.drift_f * f[c] * tm + dvr;
-    p[c] = m.pos[3 * a + c] + dr * (1.0 / kAngstrom);
+    p[c] = m.pos[3 * a + c] + nr * n1[c] + L.drift_p * ft[c] + L.drift_v * v[c];
     m.pos[3 * a + c] = p[c];
-    v[c] = v[c] * L.c0 + dv;
+    v[c] = L.c0 * v[c] + L.drift_f * ft[c] + nv1 * n1[c] + nv2 * n2[c];
   }
 }
 
@@ -196,11 +187,11 @@ __global__ void k_langevin(MDView m, LangevinCoeffs L, int first_step, int last_
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
   const bool valid = a < m.natom;
   const unsigned long long step = *m.stepc;
-  double f[3] = {0.0, 0.0, 0.0}, v[3] = {0.0, 0.0, 0.0}, p[3];
-  double tm = 0.0, srm = 0.0;
-  if (valid) langevin_kick(m, L, a, m.slot_of[a], first_step, f, v, tm, srm);
+  double ft[3] = {0.0, 0.0, 0.0}, v[3] = {0.0, 0.0, 0.0}, p[3];
+  double srm = 0.0;
+  if (valid) langevin_kick(m, L, a, m.slot_of[a], first_step, ft, v, srm);
   add_ke(m, a, valid, v);
-  if (valid && !last_step) langevin_move(m, L, a, step, f, v, p, tm, srm);
+  if (valid && !last_step) langevin_move(m, L, a, step, ft, v, p, srm);
   if (valid) {
 #pragma unroll
     for (int c = 0; c < 3; c++) m.vel[3 * a + c] = v[c];
@@ -215,9 +206,9 @@ __global__ void k_langevin_pack(MDView m, LangevinCoeffs L, DevView d, PackArgs 
     const int a = d.sorted_atom[s];
     double p[3] = {0.0, 0.0, 0.0};
     if (a >= 0) {
-      double f[3], v[3], tm, srm;
-      langevin_kick(m, L, a, s, false, f, v, tm, srm);
-      langevin_move(m, L, a, step, f, v, p, tm, srm);
+      double ft[3], v[3], srm;
+      langevin_kick(m, L, a, s, false, ft, v, srm);
+      langevin_move(m, L, a, step, ft, v, p, srm);
 #pragma unroll
       for (int c = 0; c < 3; c++) m.vel[3 * a + c] = v[c];
     }

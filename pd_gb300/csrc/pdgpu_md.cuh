@@ -9,7 +9,10 @@ namespace pdgpu {
 // Langevin coefficients (md.cpp:941-1003), FP64
 struct LangevinCoeffs {
   double dt, gamma, gt, c0, c1, c2, varv, varr, crv, sq1mcrv2;
-  double kick, drift_f, sv, sr;   // (1 - c0/c1)/gt, c0 c2 / c1, sqrt(varv), sqrt(varr)/gamma
+  // products of these: (1 - c0/c1)/gt, c0 c2 / c1; drift in A per velocity and per force x
+  // dt / m: c1 dt, c2 dt; noise per sqrt(k_B T / m): sqrt(varr)/gamma (A), crv sqrt(varv),
+  // sqrt(1 - crv^2) sqrt(varv)
+  double kick, drift_f, drift_v, drift_p, sr, sv1, sv2;
 };
 
 struct MDState {

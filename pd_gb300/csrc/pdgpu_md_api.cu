@@ -192,8 +192,11 @@ LangevinCoeffs coeffs(double gamma, double t) {
   L.sq1mcrv2 = std::sqrt(1.0 - L.crv * L.crv);
   L.kick = (1.0 - L.c0 / L.c1) / L.gt;
   L.drift_f = L.c0 * L.c2 / L.c1;
-  L.sv = std::sqrt(L.varv);
-  L.sr = std::sqrt(L.varr) / L.gamma;
+  L.drift_v = L.dt * L.c1 / kAngstrom;
+  L.drift_p = L.dt * L.c2 / kAngstrom;
+  L.sr = std::sqrt(L.varr) / L.gamma / kAngstrom;
+  L.sv1 = L.crv * std::sqrt(L.varv);
+  L.sv2 = L.sq1mcrv2 * std::sqrt(L.varv);
   return L;
 }
 
