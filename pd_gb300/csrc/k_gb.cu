@@ -95,7 +95,7 @@ constexpr int kBornWarps = kBornThreads / 32;
 // rows of the rotating block in the warp's shared memory, twice over, so that a
 // lane's row at step kk lies at a fixed offset from its first (no wrap-around)
 struct BornRows {
-  float4 xy[64], zv[64];   // (x, x', y, y'), (z, z', P4 V, P4 V')
+  float4 xy[64], zv[64];   // (x, x', y, y'), (z, z', P4 V, P4 V'); with the base law (x, y, z, q), (LJ R, sqrt(12 eps), P4 V, -)
   float2 r[64];            // (R, R'), single tiles only
 };
 
@@ -217,6 +217,99 @@ __device__ __forceinline__ void born_full2(const DevView& v, const GBConst& k, c
   atomic_add_ll(&gpol[r0 + lane], fx32(gr));
 }
 
+// ---------------------------------------------------------------------------
+// pass 2: GB cross term fused with vacuum LJ + Coulomb, i > j pairs within Cutoff
+// (forces, dE/da and, with ENERGY, the pair energies).
+// ---------------------------------------------------------------------------
+struct PairAcc {
+  float fx, fy, fz, da;
+};
+
+// per-tile FP32 sums enter 64-bit fixed point before they are combined, so a
+// slot's total does not depend on how its tiles were grouped into work items
+__device__ __forceinline__ void flush_pair(const DevView& v, long long* deda, int s, const PairAcc& a) {
+  fix_range(v.status, fabsf(a.fx) + fabsf(a.fy) + fabsf(a.fz) + fabsf(a.da));
+  atomic_add_ll(&v.facc[force_at(s, 0)], fx32(a.fx));
+  atomic_add_ll(&v.facc[force_at(s, 1)], fx32(a.fy));
+  atomic_add_ll(&v.facc[force_at(s, 2)], fx32(a.fz));
+  if (deda) atomic_add_ll(&deda[s], fx32(a.da));
+}
+
+// Born sums and the base law of an all-inside tile pair in one pass (the dynamics
+// step's body): LJ and Coulomb at eps_out, which hold for every pair but those above the
+// exp threshold (k_gb_pair adds what these differ by, once the radii are known).  Two
+// passes used to walk every pair and form its distance; now the second walks a tenth of
+// the items.  Each lane holds one atom of either j block (.x, .y), the i block's atoms
+// come from the warp's rows.  Bound by the FMA pipe (56 of its cycles a step of two
+// pairs a lane).  64 peptides (523 M pairs): Born 271 + pair 663 us -> 638 + 215 (half
+// of it single tiles); one of 4,224 atoms 14.3 + 23.4 -> 20.7 + 18.0.  FAR: no pair of
+// the item in close contact.
+template <bool FAR>
+__device__ __forceinline__ void born_base_loop2(const DevView& v, const GBConst& k, int lane, int r0, const BornRows& rs,
+                                                const float4& xa, const float4& xb, const float4& pa, const float4& pb,
+                                                float c2, float2& G, float2& FX, float2& FY, float2& FZ, float& gr,
+                                                float3& R) {
+  const float2 nx = make_float2(-xa.x, -xb.x), ny = make_float2(-xa.y, -xb.y), nz = make_float2(-xa.z, -xb.z);
+  const float2 QN = make_float2(k.neg_sq_eout * xa.w, k.neg_sq_eout * xb.w), S = make_float2(pa.x, pb.x);
+  const float2 EN = make_float2(-k.sqrt12 * pa.y, -k.sqrt12 * pb.y), V = make_float2(k.P4 * pa.w, k.P4 * pb.w);
+  const float4 *x2 = rs.xy + lane, *p2 = rs.zv + lane;
+#pragma unroll 2
+  for (int kk = 0; kk < 32; kk++) {
+    const float4 xr = x2[kk], pr = p2[kk];
+    const float2 dx = __fadd2_rn(f2(xr.x), nx), dy = __fadd2_rn(f2(xr.y), ny), dz = __fadd2_rn(f2(xr.z), nz);
+    const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
+    const float2 QQ = __fmul2_rn(QN, f2(xr.w)), SS = __fadd2_rn(S, f2(pr.x)), EE = __fmul2_rn(EN, f2(pr.y));
+    const float2 ir = make_float2(rsqrtf(r2.x), rsqrtf(r2.y)), i2 = make_float2(rcp_ftz(r2.x), rcp_ftz(r2.y));
+    const float2 ir2 = __fmul2_rn(ir, ir);
+    float2 w = __fmul2_rn(i2, i2);
+    if (!FAR) {
+      if (__any_sync(0xffffffffu, fminf(r2.x, r2.y) <= c2)) {
+        const float R0 = v.par[r0 + ((lane + kk) & 31)].z;   // (rare: the radii are read here, not staged)
+        w.x *= born_ccf(k, r2.x, pa.z + R0);
+        w.y *= born_ccf(k, r2.y, pb.z + R0);
+      }
+    }
+    G = __ffma2_rn(w, f2(pr.z), G);
+    gr = fmaf(w.x, V.x, gr);
+    gr = fmaf(w.y, V.y, gr);
+    const float2 t2 = __fmul2_rn(__fmul2_rn(SS, SS), ir2);
+    const float2 b6 = __fmul2_rn(__fmul2_rn(t2, t2), t2);
+    const float2 amb = __fmul2_rn(b6, __fadd2_rn(b6, f2(-1.f)));
+    const float2 g = __fmul2_rn(__ffma2_rn(EE, amb, __fmul2_rn(QQ, ir)), ir2);
+    FX = __ffma2_rn(g, dx, FX);
+    FY = __ffma2_rn(g, dy, FY);
+    FZ = __ffma2_rn(g, dz, FZ);
+    R.x = fmaf(g.x, dx.x, R.x); R.x = fmaf(g.y, dx.y, R.x);
+    R.y = fmaf(g.x, dy.x, R.y); R.y = fmaf(g.y, dy.y, R.y);
+    R.z = fmaf(g.x, dz.x, R.z); R.z = fmaf(g.y, dz.y, R.z);
+    ROT(gr); ROT(R.x); ROT(R.y); ROT(R.z);
+  }
+}
+
+__device__ __forceinline__ void born_base_full2(const DevView& v, const GBConst& k, const Tile& A, const Tile& B, int lane,
+                                                long long* gpol, BornRows& rs) {
+  const int sa = A.bj * 32 + lane, sb = B.bj * 32 + lane, r0 = A.bi * 32;
+  const float4 xa = j_in_i_frame(v, A, lane), xb = j_in_i_frame(v, B, lane);
+  const float4 pa = v.par[sa], pb = v.par[sb], x0 = v.xq[r0 + lane], p0 = v.par[r0 + lane];
+  __syncwarp();
+  rs.xy[lane] = rs.xy[lane + 32] = make_float4(x0.x, x0.y, x0.z, k.sq_eout * x0.w);
+  rs.zv[lane] = rs.zv[lane + 32] = make_float4(p0.x, k.sqrt12 * p0.y, k.P4 * p0.w, 0.f);
+  __syncwarp();
+  const float c2 = pair_contact2(k, make_float2(pa.z, pb.z), p0.z);
+  float2 G = f2(0.f), FX = f2(0.f), FY = f2(0.f), FZ = f2(0.f);
+  float gr = 0.f;
+  float3 R = make_float3(0.f, 0.f, 0.f);   // minus the rotating atom's force
+  if (item_far(xa, xb, x0, c2, c2)) born_base_loop2<true>(v, k, lane, r0, rs, xa, xb, pa, pb, c2, G, FX, FY, FZ, gr, R);
+  else born_base_loop2<false>(v, k, lane, r0, rs, xa, xb, pa, pb, c2, G, FX, FY, FZ, gr, R);
+  fix_range(v.status, fabsf(G.x) + fabsf(G.y) + fabsf(gr));
+  atomic_add_ll(&gpol[sa], fx32(G.x));
+  atomic_add_ll(&gpol[sb], fx32(G.y));
+  atomic_add_ll(&gpol[r0 + lane], fx32(gr));
+  flush_pair(v, nullptr, sa, PairAcc{FX.x, FY.x, FZ.x, 0.f});
+  flush_pair(v, nullptr, sb, PairAcc{FX.y, FY.y, FZ.y, 0.f});
+  flush_pair(v, nullptr, r0 + lane, PairAcc{-R.x, -R.y, -R.z, 0.f});
+}
+
 // whether both tiles of a work item are all inside, by their flags or (gradient
 // calls, whose lists carry none) at run time
 __device__ __forceinline__ bool pair_full_now(const DevView& v, const GBConst& k, const Tile& T, const Tile& U,
@@ -243,9 +336,14 @@ __device__ __forceinline__ void born_single(const DevView& v, const GBConst& k, 
   }
 }
 
-__global__ void __launch_bounds__(kBornThreads, 5) k_gb_born(const __grid_constant__ DevView v, const __grid_constant__ GBConst k, long long* gpol) {
+// BASE: with the base law's forces of all-inside tile pairs (force-only FastMode passes);
+// six CTAs of 128 threads an SM (five: 657 us on the 64 peptides)
+constexpr int kBaseThreads = 128;
+template <bool BASE>
+__global__ void __launch_bounds__(BASE ? kBaseThreads : kBornThreads, BASE ? 6 : 5)
+    k_gb_born(const __grid_constant__ DevView v, const __grid_constant__ GBConst k, long long* gpol) {
   pdl_sync();
-  __shared__ BornRows rows[kBornWarps];
+  __shared__ BornRows rows[(BASE ? kBaseThreads : kBornThreads) / 32];
   BornRows& rs = rows[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -255,6 +353,10 @@ __global__ void __launch_bounds__(kBornThreads, 5) k_gb_born(const __grid_consta
     const Tile T = v.tiles[t.x];
     if (t.y >= 0) {
       const Tile U = v.tiles[t.y];
+      if (BASE && tile_full(T) && tile_full(U)) {
+        born_base_full2(v, k, T, U, lane, gpol, rs);
+        continue;
+      }
       if (pair_full_now(v, k, T, U, lane)) {
         born_full2(v, k, T, U, lane, gpol, rs);
         continue;
@@ -267,37 +369,23 @@ __global__ void __launch_bounds__(kBornThreads, 5) k_gb_born(const __grid_consta
 
 // Born radii a = -halfeconv / (terms123 + sum) + BornRadiusOffset  (FP64)
 __global__ void k_gb_radii(DevView v, const double* terms123, const long long* gpol, double halfeconv,
-                           double offset, float* born_f, double* born_d) {
+                           double offset, float* born_f, double* born_d, float* bborn) {
   pdl_sync();
   int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= v.nslots) return;
+  if (s >= v.nslots) return;   // (whole warps)
   int a = v.sorted_atom[s];
-  if (a < 0) {
-    born_f[s] = 1.f;
-    return;
+  float f = 1.f;
+  if (a >= 0) {
+    double G = terms123[a] + (double)gpol[s] * (1.0 / kSumScale);
+    double r = -halfeconv / G + offset;
+    f = (float)r;
+    born_d[a] = r;
   }
-  double G = terms123[a] + (double)gpol[s] * (1.0 / kSumScale);
-  double r = -halfeconv / G + offset;
-  born_f[s] = (float)r;
-  born_d[a] = r;
-}
-
-// ---------------------------------------------------------------------------
-// pass 2: GB cross term fused with vacuum LJ + Coulomb, i > j pairs within Cutoff
-// (forces, dE/da and, with ENERGY, the pair energies).
-// ---------------------------------------------------------------------------
-struct PairAcc {
-  float fx, fy, fz, da;
-};
-
-// per-tile FP32 sums enter 64-bit fixed point before they are combined, so a
-// slot's total does not depend on how its tiles were grouped into work items
-__device__ __forceinline__ void flush_pair(const DevView& v, long long* deda, int s, const PairAcc& a) {
-  fix_range(v.status, fabsf(a.fx) + fabsf(a.fy) + fabsf(a.fz) + fabsf(a.da));
-  atomic_add_ll(&v.facc[force_at(s, 0)], fx32(a.fx));
-  atomic_add_ll(&v.facc[force_at(s, 1)], fx32(a.fy));
-  atomic_add_ll(&v.facc[force_at(s, 2)], fx32(a.fz));
-  if (deda) atomic_add_ll(&deda[s], fx32(a.da));
+  born_f[s] = f;
+  f = fabsf(f);   // (a non-finite radius leaves no bound: every item is looked at)
+  if (!(f < 3.0e38f)) f = 3.0e38f;
+  f = warp_max(f);
+  if ((s & 31) == 0) bborn[s >> 5] = f;
 }
 
 // Two pairs of the fused law on packed FP32x2 arithmetic.  In: r^2, the scaled
@@ -650,86 +738,82 @@ __device__ __forceinline__ void gb_pair_tile(const DevView& v, const GBConst& k,
   }
 }
 
-// Force-only pass of an all-inside tile pair (the dynamics step's body): each
-// lane holds one atom of either j block (.x: bj, .y: bj + 1), the shared bi
-// block's atoms come from the warp's rows, their sums rotate by shuffles.  FAR:
-// no pair of the item may lie above the exp threshold (no GB term, no dE/da).
-template <bool FAR>
-__device__ __forceinline__ void gb_pair_loop2(const DevView& v, const GBConst& k, int lane, int sa, int sb, int r0,
-                                              const PairRows& rs, const float4& xa, const float4& xb,
-                                              const float4& pa, const float4& pb, float2 AK, float2& FX, float2& FY,
-                                              float2& FZ, float2& DA, PairAcc& R) {
-  const float2 nx = make_float2(-xa.x, -xb.x), ny = make_float2(-xa.y, -xb.y), nz = make_float2(-xa.z, -xb.z);
-  const float2 QN = make_float2(k.neg_sq_eout * xa.w, k.neg_sq_eout * xb.w);
-  const float2 S = make_float2(pa.x, pb.x);
-  const float2 EN = make_float2(-k.sqrt12 * pa.y, -k.sqrt12 * pb.y);
-  const Mask2 m = {true, true, false, false, false, false};
-  const float4 *x2 = rs.x2 + lane, *p2 = rs.p2 + lane;
-#pragma unroll 2
-  for (int kk = 0; kk < 32; kk++) {
-    const float4 xr = x2[kk];
-    const float4 pr = p2[kk];
-    const float2 dx = __fadd2_rn(f2(xr.x), nx), dy = __fadd2_rn(f2(xr.y), ny), dz = __fadd2_rn(f2(xr.z), nz);
-    const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
-    const float2 QQ = __fmul2_rn(QN, f2(xr.w)), SS = __fadd2_rn(S, f2(pr.x)), EE = __fmul2_rn(EN, f2(pr.y));
-    float2 g;
-    if (FAR) {
-      const float2 ir = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
-      const float2 ir2 = __fmul2_rn(ir, ir);
-      const float2 t2 = __fmul2_rn(__fmul2_rn(SS, SS), ir2);
-      const float2 b6 = __fmul2_rn(__fmul2_rn(t2, t2), t2);
-      const float2 amb = __fmul2_rn(b6, __fadd2_rn(b6, f2(-1.f)));
-      g = __fmul2_rn(__ffma2_rn(EE, amb, __fmul2_rn(QQ, ir)), ir2);
-    } else {
-      const int sr = r0 + ((lane + kk) & 31);
-      const Pair2 o = gb_pair2<false, true, true, false>(v, k, r2, QQ, SS, EE, __fmul2_rn(AK, f2(pr.z)), m, sa, sb,
-                                                         sr, sr);
-      g = o.g;
-      if (o.any) {
-        DA = __ffma2_rn(o.W, f2(pr.z), DA);
-        R.da = fmaf(o.W.x, AK.x, R.da);
-        R.da = fmaf(o.W.y, AK.y, R.da);
-      }
-    }
-    FX = __ffma2_rn(g, dx, FX);
-    FY = __ffma2_rn(g, dy, FY);
-    FZ = __ffma2_rn(g, dz, FZ);
-    R.fx = fmaf(g.x, dx.x, R.fx); R.fx = fmaf(g.y, dx.y, R.fx);
-    R.fy = fmaf(g.x, dy.x, R.fy); R.fy = fmaf(g.y, dy.y, R.fy);
-    R.fz = fmaf(g.x, dz.x, R.fz); R.fz = fmaf(g.y, dz.y, R.fz);
-    ROT(R.fx); ROT(R.fy); ROT(R.fz);
-    if (!FAR) ROT(R.da);
-  }
+// What pairs above the exp threshold have beyond the base law (k_gb_born): Coulomb at
+// eps_in for eps_out, the GB term and its dE/da (QQ, AA as gb_pair2).  Zero, and any
+// false, where no lane has such a pair.
+__device__ __forceinline__ float2 gb_near2(const DevView& v, const GBConst& k, float2 r2, float2 QQ, float2 AA, int ha,
+                                           int hb, int r, float2& W, bool& any) {
+  const bool na = r2.x <= AA.x, nb = r2.y <= AA.y;
+  any = __any_sync(0xffffffffu, na || nb);
+  if (!any) return f2(0.f);
+  const float2 ir = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
+  const float2 rc = make_float2(rcp_ftz(AA.x), rcp_ftz(AA.y));
+  const float2 u = __fmul2_rn(__fmul2_rn(r2, rc), f2(k.kU));
+  const float tie = 2e-6f * fabsf(k.thresh);
+  bool ona = na && u.x > k.thresh, onb = nb && u.y > k.thresh;
+  if (na && fabsf(u.x - k.thresh) <= tie) ona = gb_on_fp64(v, ha, r, k.thresh_d);
+  if (nb && fabsf(u.y - k.thresh) <= tie) onb = gb_on_fp64(v, hb, r, k.thresh_d);
+  QQ = make_float2(ona ? QQ.x : 0.f, onb ? QQ.y : 0.f);
+  const float2 tg = make_float2(__expf(u.x), __expf(u.y));
+  const float2 D = __ffma2_rn(tg, __fmul2_rn(AA, f2(k.invK)), r2);
+  const float2 fgb = make_float2(rsqrtf(D.x), rsqrtf(D.y));
+  const float2 w = __fmul2_rn(__fmul2_rn(__fmul2_rn(QQ, f2(k.gb_ep)), fgb), __fmul2_rn(fgb, fgb));
+  const float2 gg = __fmul2_rn(w, __ffma2_rn(tg, f2(0.5f), f2(-2.f)));
+  W = __fmul2_rn(__fmul2_rn(w, tg), __fadd2_rn(u, f2(-1.f)));
+  const float2 e1 = __fmul2_rn(__fmul2_rn(QQ, ir), f2(k.in_over_out - 1.f));
+  return __ffma2_rn(e1, __fmul2_rn(ir, ir), gg);
 }
 
-__device__ __forceinline__ void gb_pair_full2(const DevView& v, const GBConst& k, const Tile& A, const Tile& B,
-                                              int lane, const float* born, long long* deda, PairRows& rs) {
+// those of an all-inside tile pair: the shape of born_base_full2
+__device__ __forceinline__ void gb_near_full2(const DevView& v, const GBConst& k, const Tile& A, const Tile& B, int lane,
+                                              const float* born, long long* deda, PairRows& rs) {
   const int sa = A.bj * 32 + lane, sb = B.bj * 32 + lane, r0 = A.bi * 32;
-  const float4 xa = j_in_i_frame(v, A, lane), xb = j_in_i_frame(v, B, lane);
-  const float4 pa = v.par[sa], pb = v.par[sb];
+  const float4 xa = j_in_i_frame(v, A, lane), xb = j_in_i_frame(v, B, lane), x0 = v.xq[r0 + lane];
   const float2 AK = make_float2(k.sqrtK * born[sa], k.sqrtK * born[sb]);
-  float akm;
-  const float4 x0 = v.xq[r0 + lane];
-  {
-    const float4 p0 = v.par[r0 + lane];
-    const float a0 = k.sqrtK * born[r0 + lane];
-    __syncwarp();
-    rs.x2[lane] = rs.x2[lane + 32] = make_float4(x0.x, x0.y, x0.z, k.sq_eout * x0.w);
-    rs.p2[lane] = rs.p2[lane + 32] = make_float4(p0.x, k.sqrt12 * p0.y, a0, 0.f);
-    __syncwarp();
-    akm = warp_max(a0) * 1.00001f;
-  }
+  const float a0 = k.sqrtK * born[r0 + lane], akm = warp_max(a0) * 1.00001f;
+  if (item_far(xa, xb, x0, AK.x * akm, AK.y * akm)) return;
+  float* ar = reinterpret_cast<float*>(rs.p2);
+  __syncwarp();
+  rs.x2[lane] = rs.x2[lane + 32] = make_float4(x0.x, x0.y, x0.z, k.sq_eout * x0.w);
+  ar[lane] = ar[lane + 32] = a0;
+  __syncwarp();
+  const float2 nx = make_float2(-xa.x, -xb.x), ny = make_float2(-xa.y, -xb.y), nz = make_float2(-xa.z, -xb.z);
+  const float2 QN = make_float2(k.neg_sq_eout * xa.w, k.neg_sq_eout * xb.w);
   float2 FX = f2(0.f), FY = f2(0.f), FZ = f2(0.f), DA = f2(0.f);
   PairAcc R = {0.f, 0.f, 0.f, 0.f};   // minus the rotating atom's force; its dE/da
-  if (item_far(xa, xb, x0, AK.x * akm, AK.y * akm)) {
-    gb_pair_loop2<true>(v, k, lane, sa, sb, r0, rs, xa, xb, pa, pb, AK, FX, FY, FZ, DA, R);
-    deda = nullptr;
-  } else {
-    gb_pair_loop2<false>(v, k, lane, sa, sb, r0, rs, xa, xb, pa, pb, AK, FX, FY, FZ, DA, R);
+#pragma unroll 2
+  for (int kk = 0; kk < 32; kk++) {
+    const float4 xr = rs.x2[lane + kk];
+    const float ak = ar[lane + kk];
+    const float2 dx = __fadd2_rn(f2(xr.x), nx), dy = __fadd2_rn(f2(xr.y), ny), dz = __fadd2_rn(f2(xr.z), nz);
+    const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
+    float2 W;
+    bool any;
+    const float2 g = gb_near2(v, k, r2, __fmul2_rn(QN, f2(xr.w)), __fmul2_rn(AK, f2(ak)), sa, sb,
+                              r0 + ((lane + kk) & 31), W, any);
+    if (any) {
+      FX = __ffma2_rn(g, dx, FX);
+      FY = __ffma2_rn(g, dy, FY);
+      FZ = __ffma2_rn(g, dz, FZ);
+      DA = __ffma2_rn(W, f2(ak), DA);
+      R.fx = fmaf(g.x, dx.x, R.fx); R.fx = fmaf(g.y, dx.y, R.fx);
+      R.fy = fmaf(g.x, dy.x, R.fy); R.fy = fmaf(g.y, dy.y, R.fy);
+      R.fz = fmaf(g.x, dz.x, R.fz); R.fz = fmaf(g.y, dz.y, R.fz);
+      R.da = fmaf(W.x, AK.x, R.da);
+      R.da = fmaf(W.y, AK.y, R.da);
+    }
+    ROT(R.fx); ROT(R.fy); ROT(R.fz); ROT(R.da);
   }
   flush_pair(v, deda, sa, PairAcc{FX.x, FY.x, FZ.x, DA.x * k.inv_sqrtK});
   flush_pair(v, deda, sb, PairAcc{FX.y, FY.y, FZ.y, DA.y * k.inv_sqrtK});
   flush_pair(v, deda, r0 + lane, PairAcc{-R.fx, -R.fy, -R.fz, R.da * k.inv_sqrtK});
+}
+
+// whether no pair of the tile may lie above the exp threshold, from its blocks' radii
+// and largest Born radii
+__device__ __forceinline__ bool blocks_far(const DevView& v, const GBConst& k, const Tile& T) {
+  const float d = sqrtf(T.ox * T.ox + T.oy * T.oy + T.oz * T.oz) * 0.9999f - v.brad[T.bi] - v.brad[T.bj];
+  return d > 0.f && d * d > k.sqrtK * v.bborn[T.bi] * 1.0001f * (k.sqrtK * v.bborn[T.bj]);
 }
 
 template <bool FAST, bool ENERGY>
@@ -751,30 +835,43 @@ __device__ __forceinline__ void gb_pair_single(const DevView& v, const GBConst& 
   }
 }
 
-// the force-only pass (every dynamics step) runs in CTAs of 128 threads, five
-// per SM (20 warps at 96 registers; seven at 72 spill and were 5 % slower); FAST off: calcBornForces (gbff.cpp:1189-1340),
-// LJ and Coulomb come from the NB kernel with the GB object's own settings
+// The force-only pass (every dynamics step).  FAST: of an all-inside tile pair only what
+// the base law lacks, and nothing where no pair of it may lie above the exp threshold
+// (most items of a large peptide): each lane asks that of one item of the warp's, by
+// block bounds.  FAST off: calcBornForces (gbff.cpp:1189-1340), tile by tile; LJ and
+// Coulomb come from the NB kernel with the GB object's own settings.
 constexpr int kPairThreads = 128, kPairEThreads = 128;
 template <bool FAST>
-__global__ void __launch_bounds__(kPairThreads, 5) k_gb_pair(const __grid_constant__ DevView v, const __grid_constant__ GBConst k, const float* born, long long* deda) {
+__global__ void __launch_bounds__(kPairThreads, 6) k_gb_pair(const __grid_constant__ DevView v, const __grid_constant__ GBConst k, const float* born, long long* deda) {
   pdl_sync();
   __shared__ PairRows rows[kPairThreads / 32];
   PairRows& rs = rows[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   const int ni = *v.nitems;
-  for (int it = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; it < ni; it += nwarps) {
-    const int2 t = v.items[it];
-    const Tile T = v.tiles[t.x];
-    if (t.y >= 0) {
-      const Tile U = v.tiles[t.y];
-      if (FAST && tile_full(T) && tile_full(U)) {
-        gb_pair_full2(v, k, T, U, lane, born, deda, rs);
-        continue;
+  for (int first = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; first < ni; first += 32 * nwarps) {
+    const int mine = first + lane * nwarps;
+    bool work = mine < ni;
+    if (FAST && work) {
+      const int2 t = v.items[mine];
+      if (t.y >= 0) {
+        const Tile T = v.tiles[t.x], U = v.tiles[t.y];
+        work = !(tile_full(T) && tile_full(U) && blocks_far(v, k, T) && blocks_far(v, k, U));
       }
-      gb_pair_single<FAST, false>(v, k, U, lane, born, deda, rs, nullptr);
     }
-    gb_pair_single<FAST, false>(v, k, T, lane, born, deda, rs, nullptr);
+    for (unsigned m = __ballot_sync(0xffffffffu, work); m; m &= m - 1u) {
+      const int2 t = v.items[first + (__ffs(m) - 1) * nwarps];
+      const Tile T = v.tiles[t.x];
+      if (t.y >= 0) {
+        const Tile U = v.tiles[t.y];
+        if (FAST && tile_full(T) && tile_full(U)) {
+          gb_near_full2(v, k, T, U, lane, born, deda, rs);
+          continue;
+        }
+        gb_pair_single<FAST, false>(v, k, U, lane, born, deda, rs, nullptr);
+      }
+      gb_pair_single<FAST, false>(v, k, T, lane, born, deda, rs, nullptr);
+    }
   }
 }
 
@@ -1041,9 +1138,10 @@ int launch_gb(Context& c, const GBConst& k, double halfeconv, double born_offset
   cudaStream_t st = c.stream;
   int g = tile_grid(c);
   const Spread sp = spread(c.nslots);
-  launch_pdl(st, g, kBornThreads, 0, k_gb_born, v, k, c.d_gpol.p);
-  launch_pdl(st, sp.grid, sp.threads, 0, k_gb_radii, v, c.d_gbT.p, c.d_gpol.p, halfeconv, born_offset, c.d_born_f.p, c.d_born_d.p);
   const int gp = g * (256 / kPairThreads), ge = g * (256 / kPairEThreads);
+  if (k.fast && !energy && !c.gb_no_chain) launch_pdl(st, g * (256 / kBaseThreads), kBaseThreads, 0, k_gb_born<true>, v, k, c.d_gpol.p);
+  else launch_pdl(st, g, kBornThreads, 0, k_gb_born<false>, v, k, c.d_gpol.p);
+  launch_pdl(st, sp.grid, sp.threads, 0, k_gb_radii, v, c.d_gbT.p, c.d_gpol.p, halfeconv, born_offset, c.d_born_f.p, c.d_born_d.p, c.d_bborn.p);
   if (c.gb_no_chain) {
     // a gradient call: energies (FP32 pair terms: they weight a loss), dE/da and the
     // pair terms' gradients in one pass, no forces
@@ -1055,7 +1153,7 @@ int launch_gb(Context& c, const GBConst& k, double halfeconv, double born_offset
   } else if (!k.fast) {
     launch_pdl(st, gp, kPairThreads, 0, k_gb_pair<false>, v, k, c.d_born_f.p, c.d_deda.p);
   } else {
-    launch_pdl(st, gp, kPairThreads, 0, k_gb_pair<true>, v, k, c.d_born_f.p, c.d_deda.p);
+    launch_pdl(st, 2 * gp, kPairThreads, 0, k_gb_pair<true>, v, k, c.d_born_f.p, c.d_deda.p);   // (unequal items: 222 -> 215 us)
   }
   launch_pdl(st, sp.grid, sp.threads, 0, k_gb_self, v, c.d_charge.p, k, premul, c.d_deda.p, c.d_born_d.p, c.d_chain_f.p,
                                 energy ? 1 : 0);
@@ -1069,8 +1167,8 @@ int launch_gb_stage(Context& c, const GBConst& k, int stage) {
   DevView v = c.view();
   int g = tile_grid(c);
   c.kernel_launches += 1;
-  if (stage == 1) launch_pdl(c.stream, g, kBornThreads, 0, k_gb_born, v, k, c.d_gpol.p);
-  else if (stage == 2) launch_pdl(c.stream, g * (256 / kPairThreads), kPairThreads, 0, k_gb_pair<true>, v, k, c.d_born_f.p, c.d_deda.p);
+  if (stage == 1) launch_pdl(c.stream, g * (256 / kBaseThreads), kBaseThreads, 0, k_gb_born<true>, v, k, c.d_gpol.p);
+  else if (stage == 2) launch_pdl(c.stream, 2 * g * (256 / kPairThreads), kPairThreads, 0, k_gb_pair<true>, v, k, c.d_born_f.p, c.d_deda.p);
   else launch_pdl(c.stream, 2 * g, kChainThreads, 0, k_gb_chain, v, k, c.d_chain_f.p);
   return cudaGetLastError() == cudaSuccess ? PDGPU_OK : PDGPU_ERR_CUDA;
 }

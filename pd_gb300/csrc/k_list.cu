@@ -393,6 +393,7 @@ __global__ void __launch_bounds__(128) k_blocks(DevView v, SlotParams P, StepCle
   v.xq[slot] = o;
   v.rel0[slot] = o;
   if (sub) write_sub(v, slot, o);
+  if (P.gbR) write_radius(v, slot, a, o);
   if (lane == 0) {
     v.half[b] = make_float4(hf[0], hf[1], hf[2], 0.f);
     v.cenf[b] = make_float4(cf[0], cf[1], cf[2], 0.f);
@@ -1181,6 +1182,7 @@ PackArgs pack_args(const Context& c, float check_disp) {
   }
   P.npairs_all = c.npairs_all;
   P.cull = c.cull_built ? 1 : 0;
+  P.gb = c.has_gb ? 1 : 0;
   return P;
 }
 

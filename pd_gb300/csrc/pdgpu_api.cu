@@ -545,6 +545,8 @@ pdgpu_ctx* pdgpu_create(int device, const pdgpu_system_desc* d, int* status) {
     if (e == cudaSuccess) e = c.d_gpol.alloc(c.nslots);
     if (e == cudaSuccess) e = c.d_deda.alloc(c.nslots);
     if (e == cudaSuccess) e = c.d_born_f.alloc(c.nslots);
+    if (e == cudaSuccess) e = c.d_brad.alloc(c.nblocks);
+    if (e == cudaSuccess) e = c.d_bborn.alloc(c.nblocks);
     if (e == cudaSuccess) e = c.d_chain_f.alloc(c.nslots);
     if (e == cudaSuccess) e = c.d_born_d.alloc(N);
   }

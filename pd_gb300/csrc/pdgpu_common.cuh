@@ -162,6 +162,8 @@ struct DevView {
   double* center;            // [nblocks*3]
   float4* half;              // [nblocks] half extents
   float4* sub;               // [nblocks*8] box (lo, hi) of each 8 slots at the packed positions, in the block's frame
+  float* brad;               // [nblocks] (GB) radius about the centre at the packed positions, rounded up
+  const float* bborn;        // [nblocks] largest Born radius of the last GB pass
   float4* cenf;              // [nblocks] centre in FP32 (exact: centres are FP32 numbers)
   // (energy evaluations) what FP32 rounding takes off the packed slots:
   // (x, y, z, charge) - xq and (LJ radius, sqrt(eps)) - par, written before the energy pass

@@ -134,6 +134,7 @@ struct Context {
   DBuf<double> d_center;       // [nblocks*3]
   DBuf<float4> d_half;         // [nblocks]
   DBuf<float4> d_cenf;         // [nblocks]
+  DBuf<float> d_brad, d_bborn; // [nblocks] (with GB only)
   DBuf<float4> d_sub;          // [nblocks*8]
   DBuf<float> d_sys_hmax;      // [nsys*3] largest block half-extent (ordered ints)
   DBuf<BlockGrid> d_bgrid;     // [nsys]
@@ -231,6 +232,8 @@ struct Context {
     v.half = d_half.p;
     v.cenf = d_cenf.p;
     v.sub = d_sub.p;
+    v.brad = d_brad.p;
+    v.bborn = d_bborn.p;
     v.rlo = d_rlo.p;
     v.plo = d_plo.p;
     v.band_excl = d_band_excl.p;

@@ -23,6 +23,14 @@ __device__ __forceinline__ void write_sub(const DevView& v, int s, const float4&
   }
 }
 
+// the block's radius about its centre (padding apart); every lane of the warp calls this
+__device__ __forceinline__ void write_radius(const DevView& v, int s, int a, const float4& o) {
+  float r2 = a >= 0 ? o.x * o.x + o.y * o.y + o.z * o.z : 0.f;
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) r2 = fmaxf(r2, __shfl_xor_sync(0xffffffffu, r2, d));
+  if ((s & 31) == 0) v.brad[s >> 5] = sqrtf(r2) * 1.00001f;
+}
+
 // slot s of atom a (-1: padding) at FP64 position x -> FP32 offset from the block centre
 __device__ __forceinline__ float4 packed_slot(const DevView& v, const SystemInfo& S, const double* charge, int s, int a,
                                               const double* x, const double c[3]) {
@@ -47,6 +55,7 @@ struct PackArgs {
   float check2, full2;
   long long npairs_all;
   int cull;
+  int gb;   // the GB passes need the blocks' radii
 };
 PackArgs pack_args(const Context& c, float check_disp);
 inline float skin_disp(const Context& c) { return c.lp.check_skin ? (float)(0.5 * c.lp.Padding) : 0.f; }
@@ -70,6 +79,7 @@ __device__ __forceinline__ void pack_slot(const DevView& v, const PackArgs& P, i
   }
   v.xq[s] = o;
   if (P.cull) write_sub(v, s, o);
+  if (P.gb) write_radius(v, s, a, o);
   step_clear(P.clear, v, s);
 }
 
