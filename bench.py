@@ -39,21 +39,20 @@ METRIC = "atom-steps/s batched vs plain GPU at force rel err <=1e-5 vs FP64; % H
 # FP32 flops per pair of the pair kernels by the branch the pair takes (FMA =
 # 2 flops, each MUFU operation = 1), counted from the pair law each kernel
 # evaluates; pairs per branch come from pdgpu_pair_census at the final state.
-#   GB fused pair (k_gb_pair), every pair inside the GB cutoff: d (3), r^2 (5),
-#     u = -r^2/(4 a_i a_j) for the threshold test (4), 1/r (1), q_i q_j (1),
-#     Coulomb energy and dE/dr (3), LJ 12-6 (12), dE/dr / r (3), forces on both
-#     atoms (12): 44.  Above ExpApproxThreshold the GB cross term adds exp,
-#     f_GB = 1/sqrt(r^2 + a_i a_j e^u), E, dE/dr, dE/da for both atoms: +23.
-#   FF_NonBonded pair inside the cutoff (k_nb_tiles, energy-switched LJ and
+#   GB base pass (k_gb_born in dynamics: Born sums and the base pair law of every
+#     pair inside the GB cutoff): d (3), r^2 (5); Born: R_i + R_j and the contact
+#     test (3), 1/r^2 (1), P4 / r^4 (3), two sums (4); base law: 1/r (1), q_i q_j
+#     (1), threshold bound (4), Coulomb energy and dE/dr (3), LJ 12-6 (12), dE/dr / r
+#     (3), forces on both atoms (12): 55; in close contact the CCF adds 7.
+#   GB term (k_gb_pair), pairs above ExpApproxThreshold: exp, f_GB = 1/sqrt(r^2 +
+#     a_i a_j e^u), E, dE/dr, dE/da for both atoms: 23.
+#   FF_NonBonded pair inside the cutoff (k_nb_force, energy-switched LJ and
 #     Coulomb): d (3), r^2 (5), 1/r and r (2), LJ (12), both switches (22),
 #     sum and 1/r (2), forces (12): 58.
-#   Born-radius pair (k_gb_born, both directions): d, r^2 (8), R_i + R_j and
-#     the contact test (3), 1/r^2 (1), P4 / r^4 (3), two sums (4): 19; in close
-#     contact the CCF adds 7.
 #   Chain-rule pair (k_gb_chain, both directions): d, r^2 (8), contact test
 #     (3), 1/r^2 (1), c_i V_j + c_j V_i (3), the factor over r^6 (4), forces
 #     (12): 31; in close contact the CCF and its derivative add 13.
-FLOPS = {"gb_pair": 44, "gb_term": 23, "nb": 58, "born": 19, "born_contact": 7, "chain": 31, "chain_contact": 13}
+FLOPS = {"gb_base": 55, "gb_term": 23, "nb": 58, "born_contact": 7, "chain": 31, "chain_contact": 13}
 # bytes per atom-step of the integrator: read p, v, f (24 B each) + mass (8 B), write p, v
 INTEGRATOR_BYTES = 80 + 48
 
@@ -180,10 +179,10 @@ NB_CUTOFF = 12.0   # FF_NonBonded Cutoff and VdwCutoff of the C1/C2 workloads (A
 # DRAM bytes (read + write) per launch of the roofline kernels, from one ncu
 # capture of each workload (the DRAM traffic summary under profiles/)
 NCU_TRAFFIC = {
-    "c4": {"k_gb_pair": 41.33e6, "k_langevin": 23.55e6},
-    "c3": {"k_gb_pair": 0.85e6, "k_langevin": 0.50e6},
-    "c2": {"k_nb_tiles": 17.47e6, "k_langevin": 2.00e6},
-    "c1": {"k_nb_tiles": 0.30e6},
+    "c4": {"k_gb_born": 41.51e6, "k_langevin": 26.92e6},
+    "c3": {"k_gb_born": 0.87e6, "k_langevin": 0.56e6},
+    "c2": {"k_nb_force": 17.73e6, "k_langevin": 2.36e6},
+    "c1": {"k_nb_force": 0.31e6},
 }
 
 
@@ -507,8 +506,8 @@ def cpu_model():
 def roofline_flops(census, dom):
     """Algorithmic FP32 flops of one launch of the dominant pair kernel, from the
     pair census (counts of each branch) and FLOPS."""
-    if dom == "gb_pair":
-        return FLOPS["gb_pair"] * census["gb"] + FLOPS["gb_term"] * census["gb_term"]
+    if dom == "gb_born":
+        return FLOPS["gb_base"] * census["gb"] + FLOPS["born_contact"] * census["born_contact"]
     return FLOPS["nb"] * census["nb"]
 
 
@@ -648,7 +647,7 @@ def run_ours(args, key, wl, image):
     value = units / t_max
 
     # kernel rooflines (measured on the live state, L2 flushed before each launch)
-    dom = "gb_pair" if "GB" in wl["what"] else "nb"
+    dom = "gb_born" if "GB" in wl["what"] else "nb"
     ms_dom = ctx.time_kernel(dom, reps=10)
     census = ctx.pair_census()
     ms_int = ctx.time_kernel("integrate", reps=10)
@@ -667,7 +666,7 @@ def run_ours(args, key, wl, image):
             peaks = json.load(open(pk))
         hbm = peaks.get("hbm_gbs", 6800.0)
         int_gbs = INTEGRATOR_BYTES * natom / (ms_int / 1e3) / 1e9
-        kdom = "k_gb_pair" if dom == "gb_pair" else "k_nb_tiles"
+        kdom = "k_gb_born" if dom == "gb_born" else "k_nb_force"
         kint = "k_langevin" if wl["integrator"] else "k_vv"
         traffic = NCU_TRAFFIC.get(key, {})
         roof = {"bound": "fp32", "kernel": kdom, "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
@@ -676,9 +675,9 @@ def run_ours(args, key, wl, image):
                                "FFMA2 %.1f TFLOP/s; SM clock in `clocks`)" % (fp32["ffma_tflops"],
                                                                               fp32["ffma2_tflops"]),
                 "flops_per_launch": flops, "ms_per_launch": ms_dom, "census": census}
-        if dom == "gb_pair":
-            roof["flops"] = ("%d per pair inside the GB cutoff + %d per pair above ExpApproxThreshold "
-                             "(GB cross term)" % (FLOPS["gb_pair"], FLOPS["gb_term"]))
+        if dom == "gb_born":
+            roof["flops"] = ("%d per pair inside the GB cutoff (Born sums and base pair law) + %d per pair in close "
+                             "contact" % (FLOPS["gb_base"], FLOPS["born_contact"]))
         else:
             visited = 1024 * (max(groups[1], 0) + (groups[2] if groups[2] >= 0 else list_stats["tiles"]))
             roof["flops"] = "%d per pair inside the cutoff" % FLOPS["nb"]

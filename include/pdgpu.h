@@ -181,9 +181,10 @@ int pdgpu_compute(pdgpu_ctx *ctx, unsigned what, pdgpu_energies *out, double *f,
  * memory) without any host synchronisation.  Energies are formed only when
  * `what` includes PDGPU_ENERGY and stay on the device until pdgpu_get_energies().
  * Forces are FP32 pair math with 64-bit fixed-point sums.  Energies, when
- * requested: GB pair energies in FP64 from FP64 positions and parameters for
- * pairs closer than 4.5 A, from FP32 terms beyond, summed in FP64 and fixed
- * point; FF_NonBonded pair energies in FP64. */
+ * requested: GB pair energies in double-float arithmetic (~45 bits) for pairs
+ * closer than 4.5 A, from FP32 terms beyond; FF_NonBonded pair energies in
+ * double-float arithmetic; summed in double-float and fixed point.  A call that
+ * reads no forces leaves out the passes that only form them. */
 int pdgpu_compute_device(pdgpu_ctx *ctx, unsigned what, double *d_f);
 int pdgpu_get_energies(pdgpu_ctx *ctx, pdgpu_energies *out);
 /* Born radii (Angstrom, original atom order) and LCPO per-atom SASA (A^2) from
@@ -198,7 +199,7 @@ int pdgpu_get_sasa(pdgpu_ctx *ctx, double *sasa);
  * nonbonded.cpp:76-386) then returns the energies after the atoms whose
  * positions differ from the reference moved: the reference minus every pair
  * touching a moved atom at its reference position plus the same pairs now
- * (FP64 pair energies, all pairs of the system inside Cutoff), and makes the
+ * (double-float pair energies, all pairs of the system inside Cutoff), and makes the
  * current positions the reference.  nmoved (may be NULL) counts the moved
  * atoms.  Call pdgpu_nb_energy_full again after a list-changing event, as PD
  * does after a full list update. */
@@ -209,7 +210,7 @@ int pdgpu_nb_energy_update(pdgpu_ctx *ctx, pdgpu_energies *out, int *nmoved);
  * PD has no counterpart: its parameter derivatives are finite differences of
  * Forcefield::calcEnergies with setup() re-run after each edit
  * (src/mmlib/forcefields/nonbonded.cpp:1078-1084).  One call evaluates the
- * energies (GB pairs from FP32 terms summed in FP64, |dE|/|E| ~ 1e-6: they
+ * energies (GB pairs from FP32 terms summed in double-float, |dE|/|E| ~ 1e-6: they
  * weight a loss; pdgpu_compute gives the closer ones) and dE/dp for every
  * per-atom parameter array of
  * pdgpu_system_desc, in original atom order, J per unit of the parameter as

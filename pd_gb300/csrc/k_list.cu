@@ -3,9 +3,9 @@
 // (PD src/mmlib/workspace/neighbourlist.cpp:222-439): PD scans all j < i at
 // minimum image; here atoms are binned on a 32^3 grid ordered along a Hilbert
 // curve, grouped into 32-atom blocks, and block pairs whose bounding boxes come
-// within max(cutoffs)+Padding form the tile list, found through a grid over the
-// block centres (work and memory follow the tiles, not the square of the block
-// count).  The bond order PD packs into
+// within max(cutoffs)+Padding form the tile list: each row tests every column in
+// systems of up to kDirectBlocks blocks, those within reach on a grid over the block
+// centres in larger ones.  The bond order PD packs into
 // each list entry (neighbourlist.cpp:398-422, 179-220) becomes a per-tile
 // exclusion / 1-4 bit mask.
 #include <algorithm>

@@ -128,8 +128,8 @@ __device__ __forceinline__ void nb_rot(const DevView& v, const NBConst& k, const
 // Bound by the FMA pipe and, in small systems, by the latency of its chains: two pairs
 // a lane in packed arithmetic.  FP64 pair energies on the rotation, with the forces:
 // 5.85 ms on the solvated 22,489 atoms at 15 A (force switch), 0.331 ms on 667 waters
-// at 12 A; scalar double-float on a list kept by
-// the force rotation: 0.461, 0.046, 0.119 ms; this pass 0.334, 0.031, 0.097 ms beside
+// at 12 A; scalar double-float on a list kept by the force rotation: 0.461 and 0.046
+// ms, 0.119 ms on 4,235 atoms without cutoff; this pass 0.334, 0.031 and 0.097 ms beside
 // force passes of 0.060, 0.011 and 0.019 ms (left out of calls that read no forces).
 // ---------------------------------------------------------------------------
 
