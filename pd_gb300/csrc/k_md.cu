@@ -217,7 +217,9 @@ __global__ void k_langevin_pack(MDView m, LangevinCoeffs L, DevView d, PackArgs 
   advance_step(m);
 }
 
-// REMD: one thread walks the temperature ladder (remd.cpp:178-215, 349-356).
+// REMD (remd.cpp:178-215, 349-356): one CTA, a thread per pair of neighbouring rungs (the
+// pairs of one parity share no rung and no system; one thread for all took 88 us for 64
+// rungs).
 // temp_sys[r] = system holding temperature rung r; ladder[r] = temperature (K).
 // Exchange sweep over rung pairs (r, r+1) of one parity (remd.cpp:178-215).
 // mode[r] is the lower rung's REX_Replica::ExchangeMode (remd.h:49):
@@ -231,13 +233,13 @@ __global__ void k_langevin_pack(MDView m, LangevinCoeffs L, DevView d, PackArgs 
 __global__ void k_remd_exchange(const long long* eacc, int nsys, int parity, const double* ladder, int* temp_sys,
                                 double* temp, double* vscale, int* accepted, unsigned long long seed,
                                 unsigned long long round, const int* mode, int* copy_src, double* copy_scale) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  for (int s = 0; s < nsys; s++) {
+  for (int s = threadIdx.x; s < nsys; s += blockDim.x) {
     vscale[s] = 1.0;
     copy_src[s] = -1;
     copy_scale[s] = 1.0;
   }
-  for (int r = parity; r < nsys - 1; r += 2) {
+  __syncthreads();
+  for (int r = parity + 2 * threadIdx.x; r < nsys - 1; r += 2 * blockDim.x) {
     int lo = temp_sys[r], hi = temp_sys[r + 1];
     double Tlo = ladder[r], Thi = ladder[r + 1];
     double Elo = 0, Ehi = 0;
@@ -384,7 +386,7 @@ int launch_remd(Context& c, MDState& md, int parity, unsigned long long round) {
   c.kernel_launches += 3;
   MDView m = md_view(c, md);
   const int nb = (c.natom + 255) / 256;
-  k_remd_exchange<<<1, 32, 0, c.stream>>>(c.d_eacc.p, c.nsys, parity, md.d_ladder.p, md.d_temp_sys.p, md.d_temp.p,
+  k_remd_exchange<<<1, 256, 0, c.stream>>>(c.d_eacc.p, c.nsys, parity, md.d_ladder.p, md.d_temp_sys.p, md.d_temp.p,
                                           md.d_vscale.p, md.d_accepted.p, md.p.seed, round, md.d_mode.p,
                                           md.d_copy_src.p, md.d_copy_scale.p);
   k_remd_copy<<<nb, 256, 0, c.stream>>>(m, c.d_sys.p, md.d_copy_src.p, md.d_copy_scale.p);
