@@ -849,8 +849,8 @@ __global__ void __launch_bounds__(kPairThreads, 6) k_gb_pair(const __grid_consta
   const int lane = threadIdx.x & 31;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   const int ni = *v.nitems;
-  for (int first = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; first < ni; first += 32 * nwarps) {
-    const int mine = first + lane * nwarps;
+  for (long long first = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; first < ni; first += 32LL * nwarps) {
+    const long long mine = first + (long long)lane * nwarps;
     bool work = mine < ni;
     if (FAST && work) {
       const int2 t = v.items[mine];
@@ -860,7 +860,7 @@ __global__ void __launch_bounds__(kPairThreads, 6) k_gb_pair(const __grid_consta
       }
     }
     for (unsigned m = __ballot_sync(0xffffffffu, work); m; m &= m - 1u) {
-      const int2 t = v.items[first + (__ffs(m) - 1) * nwarps];
+      const int2 t = v.items[first + (long long)(__ffs(m) - 1) * nwarps];
       const Tile T = v.tiles[t.x];
       if (t.y >= 0) {
         const Tile U = v.tiles[t.y];
