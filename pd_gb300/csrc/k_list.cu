@@ -72,9 +72,10 @@ struct ListState {
   int *bcell_count, *bcell_cursor; // per block cell
   int* counters;
   int ncells, nbcells, nsys3;
+  int groups;                      // this build makes NB groups
 };
 __device__ __forceinline__ void reset_counter(const ListState& I, int t) {
-  if (t < 8) I.counters[t] = t == 5 ? 1 : 0;   // [5]: the NB groups fit until a row finds they do not
+  if (t < 8) I.counters[t] = t == 5 ? I.groups : 0;   // [5]: the NB groups fit until a row finds they do not
 }
 __global__ void k_list_init(ListState I, int* sorted_atom, int nslots) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x, n = gridDim.x * blockDim.x;
@@ -1030,6 +1031,11 @@ static bool groups_serve(const Context& c, float R) {
   return false;
 }
 
+// NB j-atom groups: only where the per-step displacement check runs
+static bool makes_groups(const Context& c, float list_radius) {
+  return c.nb_set && c.nb_cull && c.lp.check_skin && c.cull_cap > 0 && groups_serve(c, list_radius);
+}
+
 static void launch_cull(Context& c, float list_radius) {
   c.kernel_launches += 1;
   const float R = list_radius + 1e-3f, Rc = fmaxf(list_radius - (float)c.lp.Padding, 0.f);
@@ -1083,12 +1089,11 @@ static void launch_list_tail(Context& c, float list_radius) {
     launch_pdl(st, nblk(c.nblocks, 4), 128, 0, k_items, c.view(), c.gb_item_tiles == 2 ? 1 : 0, far, c.d_row_start.p,
                                                 c.d_row_cnt.p);
   }
-  // NB j-atom groups: only where the per-step displacement check runs
-  c.cull_built = c.nb_set && c.nb_cull && c.lp.check_skin && c.cull_cap > 0 && groups_serve(c, list_radius);
+  c.cull_built = makes_groups(c, list_radius);
   if (c.cull_built) launch_cull(c, list_radius);
 }
 
-static ListState list_state(Context& c, bool grid) {
+static ListState list_state(Context& c, bool grid, bool groups) {
   ListState I;
   I.count = c.d_count.p;
   I.head = c.d_head.p;
@@ -1101,13 +1106,14 @@ static ListState list_state(Context& c, bool grid) {
   I.ncells = c.nsys * kCellsPerSystem;
   I.nbcells = grid ? c.nblocks : 0;
   I.nsys3 = 3 * c.nsys;
+  I.groups = groups ? 1 : 0;
   return I;
 }
 
 // (once, before a context's first build)
 int launch_list_init(Context& c) {
   k_list_init<<<std::min(nblk(std::max(c.nsys * kCellsPerSystem, c.nslots), 256), 1216), 256, 0, c.stream>>>(
-      list_state(c, false), c.d_sorted_atom.p, c.nslots);
+      list_state(c, false, false), c.d_sorted_atom.p, c.nslots);
   return cudaGetLastError() == cudaSuccess ? PDGPU_OK : PDGPU_ERR_CUDA;
 }
 
@@ -1116,7 +1122,7 @@ int launch_list_build(Context& c, float list_radius, float full_radius, ListSizi
   DevView v = c.view();
   cudaStream_t st = c.stream;
   const bool grid = c.max_sys_blocks > kDirectBlocks;
-  const ListState I = list_state(c, grid);
+  ListState I = list_state(c, grid, makes_groups(c, list_radius));
   if (!c.all_periodic) {
     c.kernel_launches += 1;
     launch_pdl(st, nblk(c.natom, 256), 256, 0, k_bbox, v, c.d_atom_sys.p, I.lo, I.hi);
@@ -1155,6 +1161,7 @@ int launch_list_build(Context& c, float list_radius, float full_radius, ListSizi
       const int e = alloc_tiles(c, total);
       if (e != PDGPU_OK) return e;
       c.kernel_launches += 1;
+      I.groups = makes_groups(c, list_radius) ? 1 : 0;
       launch_pdl(st, 1, 32, 0, k_reset_counters, I);
       launch_rows(c, list_radius, full_radius);
       launch_list_tail(c, list_radius);

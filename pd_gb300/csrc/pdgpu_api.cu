@@ -663,6 +663,13 @@ int pdgpu::alloc_tiles(Context& c, long long tiles) {
   return alloc_cull_tiles(c);
 }
 
+// captured steps hold the settings they were captured with (pair constants, list
+// radius, skin limit, whether the list has j-atom groups): dropped where these change
+template <typename T>
+static void new_settings(Context& c, bool had, const T& before, const T& now) {
+  if (!had || std::memcmp(&before, &now, sizeof(T)) != 0) drop_step_graphs(c);
+}
+
 extern "C" {
 
 int pdgpu_set_nb_params(pdgpu_ctx* h, const pdgpu_nb_params* p) {
@@ -671,6 +678,7 @@ int pdgpu_set_nb_params(pdgpu_ctx* h, const pdgpu_nb_params* p) {
     return PDGPU_ERR_ARG;
   const int st = alloc_cull(h->c);
   if (st != PDGPU_OK) return st;
+  new_settings(h->c, h->c.nb_set, h->c.nb, *p);
   h->c.nb = *p;
   h->c.nb_set = true;
   h->c.list_built = false;
@@ -681,6 +689,7 @@ int pdgpu_set_gb_params(pdgpu_ctx* h, const pdgpu_gb_params* p) {
   if (!h || !p || p->Cutoff <= 0 || p->InnerCutoff > p->Cutoff || p->DielectricSolute == 0 ||
       p->DielectricSolvent == 0 || p->P5 == 0)
     return PDGPU_ERR_ARG;
+  new_settings(h->c, h->c.gb_set, h->c.gb, *p);
   h->c.gb = *p;
   h->c.gb_set = true;
   h->c.list_built = false;
@@ -704,6 +713,7 @@ int pdgpu_set_gb_mode(pdgpu_ctx* h, int fast_mode, const pdgpu_nb_params* vacuum
 
 int pdgpu_set_list_params(pdgpu_ctx* h, const pdgpu_list_params* p) {
   if (!h || !p || p->Padding < 0) return PDGPU_ERR_ARG;
+  new_settings(h->c, true, h->c.lp, *p);
   h->c.lp = *p;
   h->c.list_built = false;
   return PDGPU_OK;
