@@ -199,10 +199,13 @@ int pdgpu_get_sasa(pdgpu_ctx *ctx, double *sasa);
  * nonbonded.cpp:76-386) then returns the energies after the atoms whose
  * positions differ from the reference moved: the reference minus every pair
  * touching a moved atom at its reference position plus the same pairs now
- * (double-float pair energies, all pairs of the system inside Cutoff), and makes the
+ * (FP64 pair energies, all pairs of the system inside Cutoff), and makes the
  * current positions the reference.  nmoved (may be NULL) counts the moved
- * atoms.  Call pdgpu_nb_energy_full again after a list-changing event, as PD
- * does after a full list update. */
+ * atoms.  A move whose new pairs leave the range of the sums (an atom put onto
+ * another) returns the status a full evaluation returns, PDGPU_ERR_FIXED_OVERFLOW
+ * or PDGPU_ERR_NAN, and leaves the reference as it was.  Call pdgpu_nb_energy_full
+ * again after a list-changing event, as PD does after a full list update, and after
+ * new parameters. */
 int pdgpu_nb_energy_full(pdgpu_ctx *ctx, pdgpu_energies *out);
 int pdgpu_nb_energy_update(pdgpu_ctx *ctx, pdgpu_energies *out, int *nmoved);
 

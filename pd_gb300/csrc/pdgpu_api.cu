@@ -805,11 +805,11 @@ static int param_grad_check(const Context& c, unsigned what) {
 }
 
 static int mc_alloc(Context& c) {
-  if (c.d_mc_ref.p) return PDGPU_OK;
+  if (c.d_mc_count.p) return PDGPU_OK;   // (the last of them)
   const size_t N = c.natom;
   if (c.d_mc_ref.alloc(3 * N) != cudaSuccess || c.d_mc_eref.alloc(2 * (size_t)c.nsys) != cudaSuccess ||
-      c.d_mc_moved.alloc(N) != cudaSuccess || c.d_mc_list.alloc(N) != cudaSuccess ||
-      c.d_mc_count.alloc(1) != cudaSuccess)
+      c.d_mc_delta.alloc(3 * (size_t)c.nsys) != cudaSuccess || c.d_mc_moved.alloc(N) != cudaSuccess ||
+      c.d_mc_list.alloc(N) != cudaSuccess || c.d_mc_count.alloc(1) != cudaSuccess)
     return PDGPU_ERR_CUDA;
   return PDGPU_OK;
 }
@@ -831,6 +831,7 @@ int pdgpu_nb_energy_full(pdgpu_ctx* h, pdgpu_energies* out) {
   CK(cudaSetDevice(c.device));
   int st = mc_alloc(c);
   if (st != PDGPU_OK) return st;
+  c.mc_ready = false;   // (the reference is overwritten before the status is known)
   st = enqueue_compute(c, PDGPU_NB, true, false);
   if (st != PDGPU_OK) return st;
   st = launch_mc_reference(c);
@@ -855,7 +856,8 @@ int pdgpu_nb_energy_update(pdgpu_ctx* h, pdgpu_energies* out, int* nmoved) {
   int n = 0;
   CK(cudaMemcpyAsync(e.data(), c.d_mc_eref.p, sizeof(long long) * e.size(), cudaMemcpyDeviceToHost, c.stream));
   CK(cudaMemcpyAsync(&n, c.d_mc_count.p, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
-  CK(cudaStreamSynchronize(c.stream));
+  st = read_status(c);
+  if (st != PDGPU_OK) return st;   // (the reference is as it was)
   if (nmoved) *nmoved = n;
   mc_energies(c, e, out);
   return PDGPU_OK;

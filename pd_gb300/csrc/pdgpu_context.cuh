@@ -175,6 +175,7 @@ struct Context {
   // Monte Carlo partial energy updates (allocated on first use)
   DBuf<double> d_mc_ref;            // [natom*3] positions of the reference evaluation
   DBuf<long long> d_mc_eref;        // [nsys*2] reference vdw, elec (fixed point, energy scale)
+  DBuf<long long> d_mc_delta;       // [nsys*3] an update's changes of them; then (as doubles) the sums of their magnitudes
   DBuf<unsigned char> d_mc_moved;   // [natom]
   DBuf<int> d_mc_list, d_mc_count;  // [natom], [1]
   bool mc_ready = false;
