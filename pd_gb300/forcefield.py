@@ -16,6 +16,22 @@ from . import ffi
 _J2KCALMOL = 6.0221418E23 / 4184.0
 
 
+_PLAIN = frozenset((int, float, bool, str, type(None)))
+_NO_SETTING = frozenset(("needsetup", "totalSASA", "wspace"))
+
+
+def _plain(v):
+    """A setting as it compares with an earlier value of itself: NumPy scalars and
+    containers by value (a copy, so that changes in place show)."""
+    if isinstance(v, (np.generic, np.ndarray)):
+        return v.item() if v.ndim == 0 else (v.shape, v.dtype.str, v.tobytes())
+    if isinstance(v, (list, tuple)):
+        return tuple(_plain(x) for x in v)
+    if isinstance(v, dict):
+        return tuple((k, _plain(x)) for k, x in v.items())
+    return v
+
+
 class ForcefieldBase:
     name = "ForcefieldBase"
     flag = 0
@@ -29,11 +45,15 @@ class ForcefieldBase:
     def getWSpace(self):
         return self.wspace
 
+    def _settings(self):
+        """Every attribute that is not a result (the epot fields, totalSASA), by value."""
+        return {k: v if type(v) in _PLAIN else _plain(v) for k, v in vars(self).items()
+                if k[0] != "_" and k[:4] != "epot" and k not in _NO_SETTING}
+
     def calcCheckSum(self):
-        """Changes with any setting; results (the epot fields, totalSASA) do not count."""
-        return hash(tuple(sorted((k, v) for k, v in vars(self).items()
-                                 if isinstance(v, (int, float, bool, str)) and
-                                 not k.startswith(("epot", "_")) and k not in ("needsetup", "totalSASA"))))
+        """A hash of the scalar settings (values such as -1.0 and -2.0 share one: whether
+        the settings changed is decided by the settings themselves, ensuresetup)."""
+        return hash(tuple(sorted((k, v) for k, v in self._settings().items() if isinstance(v, (int, float, bool, str)))))
 
     def setup(self):
         self.needsetup = False
@@ -41,9 +61,9 @@ class ForcefieldBase:
     def ensuresetup(self):
         im = self.wspace.image
         tables = (tuple(im.scaling14), tuple(im.gb_P))   # what setup() takes from the parameter set
-        if self.needsetup or (self.calcCheckSum(), tables) != getattr(self, "_checksum", None):
+        if self.needsetup or (self._settings(), tables) != getattr(self, "_configured", None):
             self.setup()
-            self._checksum = (self.calcCheckSum(), tables)   # (setup may settle some of the settings)
+            self._configured = (self._settings(), tables)   # (setup may settle some of the settings)
             self.wspace._ctx_params = None
 
     def configure(self, ctx):
@@ -310,7 +330,7 @@ class Forcefield:
         ws = self.wspace
         self.ensuresetup()
         ctx = ws.context()
-        key = tuple((type(c).__name__, c._checksum) for c in self.components) + (ws.Padding,)
+        key = tuple((type(c).__name__, c._configured) for c in self.components) + (ws.Padding,)
         if ws._ctx_params != (key, ctx.settings):
             for c in self.components:
                 c.configure(ctx)
