@@ -68,6 +68,7 @@ class DeviceContext:
         self.natom = im.natom
         self.nsystems = im.nsystems
         self.settings = 0      # counts the calls that set parameters
+        self.updates = 0       # counts the updates of per-atom parameters
 
     def close(self):
         if getattr(self, "h", None):
@@ -106,11 +107,13 @@ class DeviceContext:
     def update_params(self, charge=None, radius=None, epsilon=None, gb_radius=None, gb_vj=None, gb_terms123=None):
         arrs = [None if a is None else np.ascontiguousarray(a, np.float64) for a in
                 (charge, radius, epsilon, gb_radius, gb_vj, gb_terms123)]
+        self.updates += 1
         ffi.check(self.lib.pdgpu_update_params(self.h, *[_pd(a) for a in arrs]), "pdgpu_update_params")
 
     def update_params_device(self, charge=0, radius=0, epsilon=0, gb_radius=0, gb_vj=0, gb_terms123=0):
         """Device pointers (int addresses, 0 = keep) of per-atom FP64 parameter arrays."""
         ptrs = [ctypes.c_void_p(p or None) for p in (charge, radius, epsilon, gb_radius, gb_vj, gb_terms123)]
+        self.updates += 1
         ffi.check(self.lib.pdgpu_update_params_device(self.h, *ptrs), "pdgpu_update_params_device")
 
     def nb_energy_full(self):

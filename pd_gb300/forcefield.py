@@ -410,11 +410,13 @@ class Forcefield:
             ws = self.wspace
             ctx = self._prepare()
             ctx.set_positions(ws.cur.p)
-            # (the reference belongs to the settings it was taken with, whichever container took it)
-            if ws._mc_key != ws._ctx_params:
+            # (the reference belongs to the settings and per-atom parameters it was taken
+            # with, whichever container took it)
+            key = (ws._ctx_params, ctx.updates)
+            if ws._mc_key != key:
                 ws._mc_key = None
                 energies = self._evaluate(ctx, ctx.nb_energy_full)
-                ws._mc_key = ws._ctx_params
+                ws._mc_key = key
             else:
                 energies, _ = ctx.nb_energy_update()
             ws.zeroForces()

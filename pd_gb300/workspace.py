@@ -249,7 +249,7 @@ class WorkSpace:
         self.Padding = 0.5          # NeighbourListBase::Padding default (neighbourlist.cpp:35)
         self._ctx = None
         self._ctx_params = None     # (components' settings, the context's settings count) last configured
-        self._mc_key = None         # the same when the Monte Carlo reference was taken
+        self._mc_key = None         # the same, and the parameter updates, when the Monte Carlo reference was taken
         self._moved_from = None     # positions of the last call, after one that found the list stale
         self.per_system_energies = None
 

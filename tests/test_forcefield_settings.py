@@ -9,7 +9,7 @@ from pd_gb300 import ffi
 
 class _Context:
     def __init__(self, nsystems):
-        self.settings = 0
+        self.settings = self.updates = 0
         self.nsystems = nsystems
         self.nb, self.gb, self.lists, self.calls = [], [], [], []
 
@@ -138,3 +138,7 @@ def test_partial_recalculation_starts_anew_with_its_settings(workspace):
         ff.calcEnergies()
         ff.calcEnergies()
     assert [c for c in ctx.calls if c != "compute"] == ["full", "update", "update", "full", "update", "full", "update"]
+    ctx.updates += 1                                        # (new per-atom parameters)
+    ff.calcEnergies()
+    ff.calcEnergies()
+    assert [c for c in ctx.calls if c != "compute"][-2:] == ["full", "update"]

@@ -97,3 +97,29 @@ def test_container_energies_after_an_overlapping_move(goldens):
     ff.calcEnergies()
     assert ws.ene.epot == e0
     ws.close()
+
+
+def test_container_energies_after_new_parameters(goldens):
+    """Per-atom parameters changed between two partial recalculations: the next energy is
+    of the new ones (1e-9: both are sums of the same pairs)."""
+    import pd_gb300 as pdg
+    d = goldens["peptide30"]
+    ws = pdg.WorkSpace(pdg.SystemImage._from_fixture(d))
+    ws.Padding = 2.0
+    ff = pdg.Forcefield(ws)
+    nb = pdg.FF_NonBonded_GPU(ws)
+    for k, v in nb_kwargs(d, "nb").items():
+        setattr(nb, k, v)
+    nb.AutoScaling14 = False
+    nb.UsePartialRecalc = True
+    ff.add(nb)
+    ff.calcEnergies()
+    e0 = ws.ene.epot
+    ws.context().update_params(charge=0.9 * d["charge"])
+    ws.cur.p[3] += 0.02
+    ff.calcEnergies()
+    e1 = ws.ene.epot
+    nb.UsePartialRecalc = False
+    ff.calcEnergies()
+    assert e1 != e0 and rel_err(e1, ws.ene.epot) <= 1e-9
+    ws.close()
