@@ -90,7 +90,7 @@ int read_status(Context& c) {
   cudaError_t e = cudaMemcpyAsync(c.h_status.p, c.d_status.p, sizeof(unsigned), cudaMemcpyDeviceToHost, c.stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c.stream);
   if (e != cudaSuccess) return cuda_status(e, &c, "status");
-  return status_code(*c.h_status.p);
+  return note_status(c, *c.h_status.p);
 }
 
 }  // namespace
@@ -995,6 +995,7 @@ int pdgpu::rebuild_list_impl(Context& c) {
   c.list_radius_built = R;
   c.full_radius_built = F;
   c.list_built = true;
+  if (sizing != kListDevice) c.list_short = false;
   return PDGPU_OK;
 }
 
@@ -1036,9 +1037,9 @@ int pdgpu::enqueue_forces(Context& c, unsigned what, bool energy, bool rebuild, 
   c.clear.gpol = (what & PDGPU_GB) ? c.d_gpol.p : nullptr;
   c.clear.deda = (what & PDGPU_GB) ? c.d_deda.p : nullptr;
   c.clear.eacc = energy ? c.d_eacc.p : nullptr;
-  int st = packed                     ? PDGPU_OK
-           : rebuild || !c.list_built ? rebuild_list_impl(c)
-                                      : launch_pack(c, skin_disp(c));
+  int st = packed                                     ? PDGPU_OK
+           : rebuild || !c.list_built || c.list_short ? rebuild_list_impl(c)
+                                                      : launch_pack(c, skin_disp(c));
   c.clear = StepClear{};
   if (st != PDGPU_OK) return st;
   // the LCPO recalculation (positions, packed slots and tile list) and the bonded

@@ -80,6 +80,7 @@ struct Context {
   bool any_periodic = false, all_periodic = true;
   bool has_gb = false, has_sa = false, has_bonded = false, has_mass = false;
   bool positions_set = false, list_built = false;
+  bool list_short = false;     // a build that could not grow its arrays left the list short: the next evaluation rebuilds
   std::vector<SystemInfo> sys;
   std::vector<int> h_atom_sys;
 
@@ -284,6 +285,12 @@ constexpr double kForceToN = kKcalMolToJ / kAngstrom;           // kcal/mol/A ->
 inline double econv_kcal() {
   const double e = 1.60217645E-19, e0 = 8.854187817E-12, pi = 3.14159265358979323846;
   return ((1.0 / kKcal2J) * kNa * e * e) / (4.0 * pi * e0 * kAngstrom);
+}
+
+// the status code of a device status read back
+inline int note_status(Context& c, unsigned st) {
+  if (st & ST_TILE_OVERFLOW) c.list_short = true;
+  return status_code(st);
 }
 
 // Grid and CTA size of a kernel whose threads each do FP64 work for one of n atoms,

@@ -122,6 +122,9 @@ int run_steps(Context& c, MDState& md, int flags, int n, bool first) {
     it = md.graphs.emplace(key, ex).first;
   }
   CK(cudaGraphLaunch(it->second, c.stream));
+  // (the list of a replayed rebuild: with the radius and settings of its capture, which
+  // drops with them)
+  if (flags & 1) c.list_built = true;
   c.kernel_launches += md.graph_kernels[key];
   md.replayed += n;
   return PDGPU_OK;
@@ -204,13 +207,13 @@ LangevinCoeffs coeffs(double gamma, double t) {
 int read_status_md(Context& c) {
   CK(cudaMemcpyAsync(c.h_status.p, c.d_status.p, sizeof(unsigned), cudaMemcpyDeviceToHost, c.stream));
   CK(cudaStreamSynchronize(c.stream));
-  return status_code(*c.h_status.p);
+  return note_status(c, *c.h_status.p);
 }
 
 int md_enqueue_impl(Context& c, MDState& md, int nsteps, bool energy_on_last) {
   for (int k = 0; k < nsteps;) {
     int flags = step_flags(md, md.step);
-    if (!c.list_built) flags |= 1;
+    if (!c.list_built || c.list_short) flags |= 1;
     if ((md.p.what & PDGPU_SA) && md.force_sasa) flags |= 2;
     md.force_sasa = false;
     if (energy_on_last && k == nsteps - 1) flags |= 4;
