@@ -505,6 +505,7 @@ pdgpu_ctx* pdgpu_create(int device, const pdgpu_system_desc* d, int* status) {
   if (e == cudaSuccess) e = c.d_pos.alloc(3 * (size_t)N);
   if (e == cudaSuccess) e = c.d_fout.alloc(3 * (size_t)N);
   if (e == cudaSuccess) e = c.d_next.alloc(N);
+  if (e == cudaSuccess) e = c.d_cell.alloc(N);
   if (e == cudaSuccess) e = c.d_count.alloc(ncells);
   if (e == cudaSuccess) e = c.d_offset.alloc(ncells);
   if (e == cudaSuccess) e = c.d_head.alloc(ncells);

@@ -126,6 +126,7 @@ struct Context {
 
   // list build scratch
   DBuf<int> d_next;            // [natom] the chain of each cell's atoms
+  DBuf<int> d_cell;            // [natom] each atom's cell
   DBuf<int> d_count, d_offset, d_head;        // [nsys*kCellsPerSystem]
   DBuf<int> d_scan_tmp;
   DBuf<int> d_tmp_sorted;      // [natom]
