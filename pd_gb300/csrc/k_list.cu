@@ -1143,7 +1143,7 @@ static void launch_list_tail(Context& c, float list_radius) {
   launch_pdl(st, gm < gt ? gm : gt, 256, 0, k_masks, c.view(), c.d_slot_of.p, c.d_mlist.p, cnt + 7, cnt + 6, c.tile_cap);
   if (c.has_gb) {
     c.kernel_launches += 1;
-    const int far = c.gb_set && make_gb_const(c.gb, c.list_radius_built).far_inner > 0.f ? 1 : 0;
+    const int far = c.gb_set && make_gb_const(c.gb, list_radius).far_inner > 0.f ? 1 : 0;
     launch_pdl(st, nblk(c.nblocks, 4), 128, 0, k_items, c.view(), c.gb_item_tiles == 2 ? 1 : 0, far, c.d_row_start.p,
                                                 c.d_row_cnt.p);
   }
