@@ -390,9 +390,9 @@ __global__ void k_gb_radii(DevView v, const double* terms123, const long long* g
   if ((s & 31) == 0) bborn[s >> 5] = f;
 }
 
-// Two pairs of the fused law on packed FP32x2 arithmetic.  In: r^2, the scaled
-// products QQ = -econv_out q q, EE = -12 eps, AA = K a a, and the LJ radius sums
-// SS.  Common pair: vacuum LJ + Coulomb at eps_out, dE/dr / r = -(12 eps (A - B)
+// Two pairs of the fused law on packed FP32x2 arithmetic.  In: r^2, the products
+// QQ = -econv_out q q (ENERGY: -q q), EE = -12 eps, AA = K a a, (ENERGY) aa = a a, and
+// the LJ radius sums SS.  Common pair: vacuum LJ + Coulomb at eps_out, dE/dr / r = -(12 eps (A - B)
 // + E_out) / r^2, whose bracket is one FFMA.  A pair with r^2 <= AA may lie
 // above the exp threshold; when any lane of the warp has one (a vote), the GB
 // term (gbff.cpp:1592-1678) is formed for both halves, with Coulomb at eps_in in
@@ -407,8 +407,9 @@ struct Mask2 {
   bool pa, pb, xa, xb, ma, mb;
 };
 // out: g = dE/dr / r (force on the held atom along d), W = dE/da per unit of the
-// partner's radius (zero unless `any`), and with ENERGY the pairs' energies
-// (vdW, Coulomb, GB cross term)
+// partner's radius (zero unless `any`), and with ENERGY the pairs' energies: vdW,
+// Coulomb per econv_out, GB cross term per 2 premul (a constant in FP32, or products
+// with it, would shift all of them alike: it meets their sums in double-float)
 struct Pair2 {
   float2 g, W, ev, ee, ep;
   bool any;
@@ -416,13 +417,14 @@ struct Pair2 {
 
 template <bool MASKED, bool FULL, bool FAST, bool ENERGY>
 __device__ __forceinline__ Pair2 gb_pair2(const DevView& v, const GBConst& k, float2 r2, float2 QQ, float2 SS,
-                                          float2 EE, float2 AA, const Mask2& m, int ha, int hb, int ra, int rb) {
+                                          float2 EE, float2 AA, float2 aa, const Mask2& m, int ha, int hb, int ra,
+                                          int rb) {
   Pair2 o;
   const float2 ir = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
   const float2 ir2 = __fmul2_rn(ir, ir);
   const bool ina = (FULL || r2.x <= k.cut2) && (!MASKED || m.pa);
   const bool inb = (FULL || r2.y <= k.cut2) && (!MASKED || m.pb);
-  float2 e1 = __fmul2_rn(QQ, ir);   // -E_out
+  float2 e1 = __fmul2_rn(QQ, ir);   // -E_out (ENERGY: per econv_out)
   // switching without a branch: below the inner cutoff w = 0 gives S = 1 and dS = 0 exactly
   float2 S = f2(1.f), dS = f2(0.f), r = f2(0.f);
   if (!FULL) {
@@ -457,42 +459,50 @@ __device__ __forceinline__ Pair2 gb_pair2(const DevView& v, const GBConst& k, fl
   o.any = __any_sync(0xffffffffu, na || nb);
   bool ona = false, onb = false;
   if (o.any) {
-    const float2 rc = make_float2(rcp_ftz(AA.x), rcp_ftz(AA.y));
-    const float2 u = __fmul2_rn(__fmul2_rn(r2, rc), f2(k.kU));
+    if (!ENERGY) aa = __fmul2_rn(AA, f2(k.invK));
+    const float2 rc = ENERGY ? make_float2(rcp_ftz(aa.x), rcp_ftz(aa.y)) : make_float2(rcp_ftz(AA.x), rcp_ftz(AA.y));
+    const float2 u = __fmul2_rn(__fmul2_rn(r2, rc), f2(ENERGY ? -0.25f : k.kU));
     const float tie = 2e-6f * fabsf(k.thresh);
     ona = na && u.x > k.thresh;
     onb = nb && u.y > k.thresh;
     if (na && fabsf(u.x - k.thresh) <= tie) ona = gb_on_fp64(v, ha, ra, k.thresh_d);
     if (nb && fabsf(u.y - k.thresh) <= tie) onb = gb_on_fp64(v, hb, rb, k.thresh_d);
     const float2 tg = make_float2(__expf(u.x), __expf(u.y));
-    const float2 D = __ffma2_rn(tg, __fmul2_rn(AA, f2(k.invK)), r2);
+    const float2 D = __ffma2_rn(tg, aa, r2);
     const float2 fgb = make_float2(rsqrtf(D.x), rsqrtf(D.y));
-    float2 ep = __fmul2_rn(__fmul2_rn(QQ, f2(k.gb_ep)), fgb);
+    float2 ep = ENERGY ? __fmul2_rn(QQ, fgb) : __fmul2_rn(__fmul2_rn(QQ, f2(k.gb_ep)), fgb);
     ep = make_float2(ona ? ep.x : 0.f, onb ? ep.y : 0.f);
+    if (ENERGY) {
+      o.ep = __fmul2_rn(__fmul2_rn(ep, S), f2(-1.f));
+      ep = __fmul2_rn(ep, f2(-k.premul));
+    }
     float2 w = __fmul2_rn(ep, __fmul2_rn(fgb, fgb));
     if (!FULL) w = __fmul2_rn(w, S);
     gg = __fmul2_rn(w, __ffma2_rn(tg, f2(0.5f), f2(-2.f)));                   // 2 dE/dr / r
     if (!FULL) gg = __ffma2_rn(__fmul2_rn(__fmul2_rn(ep, dS), f2(2.f)), ir, gg);
     o.W = __fmul2_rn(__fmul2_rn(w, tg), __fadd2_rn(u, f2(-1.f)));             // -ep tg (1 - u) l
-    if (ENERGY) o.ep = __fmul2_rn(__fmul2_rn(ep, f2(2.f)), S);
     if (FAST) e1 = make_float2(ona ? e1.x * k.in_over_out : e1.x, onb ? e1.y * k.in_over_out : e1.y);
   }
   if (!FAST) {
-    float2 ep = __fmul2_rn(__fmul2_rn(QQ, f2(k.gb_ep)), ir);
+    float2 ep = ENERGY ? __fmul2_rn(QQ, ir) : __fmul2_rn(__fmul2_rn(QQ, f2(k.gb_ep)), ir);
     ep = make_float2(ona || !ina ? 0.f : ep.x, onb || !inb ? 0.f : ep.y);
+    if (ENERGY) {
+      o.ep = __ffma2_rn(__fmul2_rn(ep, f2(-1.f)), S, o.ep);
+      ep = __fmul2_rn(ep, f2(-k.premul));
+    }
     gg = __ffma2_rn(__fmul2_rn(__fmul2_rn(ep, S), f2(-2.f)), ir2, gg);
     gg = __ffma2_rn(__fmul2_rn(__fmul2_rn(ep, dS), f2(2.f)), ir, gg);
-    if (ENERGY) o.ep = __ffma2_rn(__fmul2_rn(ep, f2(2.f)), S, o.ep);
     o.g = gg;
     if (MASKED || !FULL) o.g = make_float2(ina ? o.g.x : 0.f, inb ? o.g.y : 0.f);
     return o;
   }
+  if (ENERGY) {
+    o.ee = __fmul2_rn(e1, f2(-1.f));
+    e1 = __fmul2_rn(e1, f2(k.eout));
+  }
   if (FULL) {
     o.g = __ffma2_rn(__fadd2_rn(vb, e1), ir2, gg);
-    if (ENERGY) {
-      o.ev = ev;
-      o.ee = __fmul2_rn(e1, f2(-1.f));
-    }
+    if (ENERGY) o.ev = ev;
   } else {
     const float2 w = make_float2(fmaxf(r.x - k.vdwinner, 0.f), fmaxf(r.y - k.vdwinner, 0.f));
     const float2 wi = __fmul2_rn(w, f2(-k.vdwinvw2));
@@ -506,7 +516,7 @@ __device__ __forceinline__ Pair2 gb_pair2(const DevView& v, const GBConst& k, fl
     o.g = __ffma2_rn(b, ir2, __ffma2_rn(d, ir, gg));
     if (ENERGY) {
       o.ev = __fmul2_rn(ev, Sv);
-      o.ee = __fmul2_rn(__fmul2_rn(e1, f2(-1.f)), S);
+      o.ee = __fmul2_rn(o.ee, S);
     }
   }
   if (MASKED || !FULL) {   // (a select, not a product: the diagonal's own pair has r = 0)
@@ -530,12 +540,13 @@ __device__ __forceinline__ Pair2 gb_pair2(const DevView& v, const GBConst& k, fl
 // summed over 8 rotation steps and then in double-float.  A tile's sums meet over
 // the warp in double-float and enter fixed point once.  The displacements of these
 // passes are differences of double-float positions rounded once to FP32, so their
-// forces carry no rounding of the block frames (6e-7 of them, 1.2e-6 without).
+// forces carry no rounding of the block frames (6e-7 of them, 1.2e-6 without), and the
+// close pairs' r^2 are rounded once (close_r2).
 // ---------------------------------------------------------------------------
 // the rotating block in the warp's shared memory: single tiles as step pairs
-// (x, x', y, y'), (z, z', q, q'), (LJ radius, ', sqrt(12 eps), ') and (Born radius
-// x sqrtK, '); tile pairs as (x, y, z, q) and (LJ radius, sqrt(12 eps), Born radius
-// x sqrtK, -), twice over, so that a lane's row at step kk lies at a fixed offset
+// (x, x', y, y'), (z, z', q, q'), (LJ radius, ', sqrt(eps), ') and (Born radius, x
+// sqrtK in the force-only passes, '); tile pairs as (x, y, z, q sqrt(econv_out)) and
+// Born radii x sqrtK, twice over, so that a lane's row at step kk lies at a fixed offset
 struct PairRows {
   union {
     struct {
@@ -598,6 +609,22 @@ __device__ __forceinline__ void gb_close_energy(const DevView& v, const GBConst&
   }
 }
 
+// (ENERGY) r^2 of two steps' pairs rounded once, from the displacements' exact high parts
+// p + x and low parts l; the displacements rounded once into d.  The repulsion of a close
+// pair goes with r^-14: the two or three roundings of a plain sum of squares were most of
+// its force's error.
+__device__ __forceinline__ float2 close_r2(float2 px, float2 x, float2 lx, float2 py, float2 y, float2 ly, float2 pz,
+                                           float2 z, float2 lz, float2& dx, float2& dy, float2& dz) {
+  auto exact = [](float2 p, float2 x, float2 l, float2& d) {
+    DF2 s = df_two_sum(p, x);
+    s = df_fast_two_sum(s.h, __fadd2_rn(s.l, l));
+    d = s.h;
+    return s;
+  };
+  const DF2 a = exact(px, x, lx, dx), b = exact(py, y, ly, dy), c = exact(pz, z, lz, dz);
+  return df_norm2(a, b, c).h;
+}
+
 // Pair pass of a single tile, step-packed: lane l holds i atom l (its values in
 // both halves), the j block's atoms l + kk and l + kk + 1 come from the warp's
 // rows; the rotating atoms' sums move two lanes per step.
@@ -634,7 +661,7 @@ __device__ __forceinline__ void gb_pair_tile(const DevView& v, const GBConst& k,
       YL = f2(-li.y);
       ZL = f2(-li.z);
     }
-    const float q0 = k.sq_eout * x0.w, e0 = k.sqrt12 * p0.y, a0 = k.sqrtK * born[j0 + lane];
+    const float q0 = x0.w, e0 = p0.y, a0 = (ENERGY ? 1.f : k.sqrtK) * born[j0 + lane];
     const float x1 = __shfl_sync(0xffffffffu, x0.x, l1), y1 = __shfl_sync(0xffffffffu, x0.y, l1);
     const float z1 = __shfl_sync(0xffffffffu, x0.z, l1), q1 = __shfl_sync(0xffffffffu, q0, l1);
     const float s1 = __shfl_sync(0xffffffffu, p0.x, l1), e1 = __shfl_sync(0xffffffffu, e0, l1);
@@ -646,8 +673,8 @@ __device__ __forceinline__ void gb_pair_tile(const DevView& v, const GBConst& k,
     rs.ak[lane] = make_float2(a0, a1);
     __syncwarp();
   }
-  const float2 X = f2(-xi.x), Y = f2(-xi.y), Z = f2(-xi.z), Q = f2(k.neg_sq_eout * xi.w), R = f2(pi.x);
-  const float2 E = f2(-k.sqrt12 * pi.y), AK = f2(k.sqrtK * born[si]);
+  const float2 X = f2(-xi.x), Y = f2(-xi.y), Z = f2(-xi.z), Q = f2(ENERGY ? -xi.w : -k.eout * xi.w), R = f2(pi.x);
+  const float2 E = f2(-12.f * pi.y), AK = f2((ENERGY ? 1.f : k.sqrtK) * born[si]);
   float2 FX = f2(0.f), FY = f2(0.f), FZ = f2(0.f), DA = f2(0.f);
   float2 RX = f2(0.f), RY = f2(0.f), RZ = f2(0.f), RA = f2(0.f);   // minus the rotating atoms' forces; their dE/da
   float2 cv = f2(0.f), ce = f2(0.f), cp = f2(0.f);                 // (ENERGY) FP32 sums of 8 steps
@@ -660,13 +687,17 @@ __device__ __forceinline__ void gb_pair_tile(const DevView& v, const GBConst& k,
     const float2 ak = rs.ak[j];
     float2 dx = __fadd2_rn(make_float2(P.x, P.y), X), dy = __fadd2_rn(make_float2(P.z, P.w), Y);
     float2 dz = __fadd2_rn(make_float2(ZQ.x, ZQ.y), Z);
+    float2 lx, ly, lz;
     if (ENERGY) {
       const float4 L = re->lxy[j];
-      dx = __fadd2_rn(dx, __fadd2_rn(make_float2(L.x, L.y), XL));
-      dy = __fadd2_rn(dy, __fadd2_rn(make_float2(L.z, L.w), YL));
-      dz = __fadd2_rn(dz, __fadd2_rn(re->lz[j], ZL));
+      lx = __fadd2_rn(make_float2(L.x, L.y), XL);
+      ly = __fadd2_rn(make_float2(L.z, L.w), YL);
+      lz = __fadd2_rn(re->lz[j], ZL);
+      dx = __fadd2_rn(dx, lx);
+      dy = __fadd2_rn(dy, ly);
+      dz = __fadd2_rn(dz, lz);
     }
-    const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
+    float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
     Mask2 m = {true, true, false, false, false, false};
     if (MASKED) {
       m.pa = !((dm >> kk) & 1u);
@@ -676,9 +707,19 @@ __device__ __forceinline__ void gb_pair_tile(const DevView& v, const GBConst& k,
       m.ma = (m14 >> kk) & 1u;
       m.mb = (m14 >> kk) & 2u;
     }
+    bool ca = false, cb = false, close = false;
+    if (ENERGY) {
+      ca = r2.x < k.eclose2 && (FULL || r2.x <= k.cut2) && m.pa;
+      cb = r2.y < k.eclose2 && (FULL || r2.y <= k.cut2) && m.pb;
+      close = __any_sync(0xffffffffu, ca || cb);
+      if (close)
+        r2 = close_r2(make_float2(P.x, P.y), X, lx, make_float2(P.z, P.w), Y, ly, make_float2(ZQ.x, ZQ.y), Z, lz, dx, dy, dz);
+    }
+    const float2 AA = __fmul2_rn(AK, ak);
     const Pair2 o = gb_pair2<MASKED, FULL, FAST, ENERGY>(
         v, k, r2, __fmul2_rn(Q, make_float2(ZQ.z, ZQ.w)), __fadd2_rn(R, make_float2(SE.x, SE.y)),
-        __fmul2_rn(E, make_float2(SE.z, SE.w)), __fmul2_rn(AK, ak), m, si, si, j0 + j, j0 + ((j + 1) & 31));
+        __fmul2_rn(E, make_float2(SE.z, SE.w)), ENERGY ? __fmul2_rn(AA, f2(k.K)) : AA, AA, m, si, si, j0 + j,
+        j0 + ((j + 1) & 31));
     FX = __ffma2_rn(o.g, dx, FX); FY = __ffma2_rn(o.g, dy, FY); FZ = __ffma2_rn(o.g, dz, FZ);
     RX = __ffma2_rn(o.g, dx, RX); RY = __ffma2_rn(o.g, dy, RY); RZ = __ffma2_rn(o.g, dz, RZ);
     if (o.any) {
@@ -688,21 +729,17 @@ __device__ __forceinline__ void gb_pair_tile(const DevView& v, const GBConst& k,
     ROT2(RX); ROT2(RY); ROT2(RZ); ROT2(RA);
     if (ENERGY) {
       float2 f = f2(1.f);
-      {
-        const bool ca = r2.x < k.eclose2 && (FULL || r2.x <= k.cut2) && m.pa;
-        const bool cb = r2.y < k.eclose2 && (FULL || r2.y <= k.cut2) && m.pb;
-        if (__any_sync(0xffffffffu, ca || cb)) {
-          const unsigned ma = __ballot_sync(0xffffffffu, ca), mb = __ballot_sync(0xffffffffu, cb);
-          const unsigned lt = (1u << lane) - 1u;
-          if (ca)
-            re->pair[np + __popc(ma & lt)] = (unsigned short)(lane | (j << 5) | (m.xa ? 1024 : 0) | (m.ma ? 2048 : 0));
-          np += __popc(ma);
-          if (cb)
-            re->pair[np + __popc(mb & lt)] =
-                (unsigned short)(lane | (((j + 1) & 31) << 5) | (m.xb ? 1024 : 0) | (m.mb ? 2048 : 0));
-          np += __popc(mb);
-          f = make_float2(ca ? 0.f : 1.f, cb ? 0.f : 1.f);
-        }
+      if (close) {
+        const unsigned ma = __ballot_sync(0xffffffffu, ca), mb = __ballot_sync(0xffffffffu, cb);
+        const unsigned lt = (1u << lane) - 1u;
+        if (ca)
+          re->pair[np + __popc(ma & lt)] = (unsigned short)(lane | (j << 5) | (m.xa ? 1024 : 0) | (m.ma ? 2048 : 0));
+        np += __popc(ma);
+        if (cb)
+          re->pair[np + __popc(mb & lt)] =
+              (unsigned short)(lane | (((j + 1) & 31) << 5) | (m.xb ? 1024 : 0) | (m.mb ? 2048 : 0));
+        np += __popc(mb);
+        f = make_float2(ca ? 0.f : 1.f, cb ? 0.f : 1.f);
       }
       if (FAST) {
         cv = __ffma2_rn(f, o.ev, cv);
@@ -722,14 +759,15 @@ __device__ __forceinline__ void gb_pair_tile(const DevView& v, const GBConst& k,
   const int lm = (lane + 31) & 31;
   const float rx = RX.x + __shfl_sync(0xffffffffu, RX.y, lm), ry = RY.x + __shfl_sync(0xffffffffu, RY.y, lm);
   const float rz = RZ.x + __shfl_sync(0xffffffffu, RZ.y, lm), ra = RA.x + __shfl_sync(0xffffffffu, RA.y, lm);
-  flush_pair(v, deda, si, PairAcc{FX.x + FX.y, FY.x + FY.y, FZ.x + FZ.y, (DA.x + DA.y) * k.inv_sqrtK});
-  flush_pair(v, deda, j0 + lane, PairAcc{-rx, -ry, -rz, ra * k.inv_sqrtK});
+  const float ia = ENERGY ? 1.f : k.inv_sqrtK;
+  flush_pair(v, deda, si, PairAcc{FX.x + FX.y, FY.x + FY.y, FZ.x + FZ.y, (DA.x + DA.y) * ia});
+  flush_pair(v, deda, j0 + lane, PairAcc{-rx, -ry, -rz, ra * ia});
   if (ENERGY) {
-    if (ENERGY) {
-      __syncwarp();
-      for (int p = lane; p < np; p += 32) gb_close_energy<FAST>(v, k, T, O, re->pair[p], born, sum);
-      __syncwarp();
-    }
+    if (FAST) sum.e = df_norm(df_mul(sum.e, k.eout_f));
+    sum.p = df_norm(df_mul(sum.p, k.premul2_f));
+    __syncwarp();
+    for (int p = lane; p < np; p += 32) gb_close_energy<FAST>(v, k, T, O, re->pair[p], born, sum);
+    __syncwarp();
     const DF e0 = df_warp_sum(sum.v), e1 = df_warp_sum(sum.e), e2 = df_warp_sum(sum.p);
     const DF x = lane == 0 ? e0 : (lane == 1 ? e1 : e2);
     if (lane < 3) {

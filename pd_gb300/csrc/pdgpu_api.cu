@@ -178,6 +178,7 @@ void pdgpu::set_gb_threshold(GBConst& k, double thresh) {
   k.sqrtK = K > 0 ? (float)std::sqrt(K) : 0.f;
   k.inv_sqrtK = K > 0 ? (float)(1.0 / std::sqrt(K)) : 0.f;
   k.invK = K > 0 ? (float)(1.0 / K) : 0.f;
+  k.K = (float)K;
   k.kU = (float)(-0.25 * K);   // u = -r^2 / (4 a a) = kU r^2 / (K a a)
 }
 
@@ -218,6 +219,8 @@ GBConst pdgpu::make_gb_const(const pdgpu_gb_params& p, double listR) {
   if (!(std::fabs(eout) > 1e-12)) eout = 1e-12;
   k.sq_eout = (float)std::sqrt(std::fabs(eout));
   k.neg_sq_eout = eout > 0 ? -k.sq_eout : k.sq_eout;
+  k.eout = (float)eout;
+  k.eout_f = df_split(eout);
   k.gb_ep = (float)(-premul / eout);
   k.in_over_out = (float)(ec / p.DielectricSolute / eout);
   k.sqrt12 = (float)std::sqrt(12.0);

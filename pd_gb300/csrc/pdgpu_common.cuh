@@ -126,16 +126,16 @@ struct GBConst {
   // energy passes: pairs closer than sqrt(eclose2) take their energies in
   // double-float from double-float positions and parameters
   float eclose2;
-  DF econv_in_f, econv_out_f, premul2_f, vdw14_f, elec14_f;   // premul2: 2 premul
-  // the packed pair bodies: Born radii scaled by sqrtK, so that
-  // a_i a_j K >= r^2 holds for every pair the threshold test may switch on
-  // (K = -4 x the threshold widened by 4e-6 relative); charges scaled by
-  // sqrt(econv_out) (the held atoms' by its negative), sqrt(eps) by sqrt(12);
-  // gb_ep: premul q q fgb per scaled charges' product -econv_out q q
+  DF econv_in_f, econv_out_f, premul2_f, vdw14_f, elec14_f, eout_f;   // premul2: 2 premul
+  // the packed pair bodies: a_i a_j K >= r^2 holds for every pair the threshold test
+  // may switch on (K = -4 x the threshold widened by 4e-6 relative); force-only passes
+  // scale the Born radii by sqrtK.  Tile pairs scale charges by sqrt(econv_out) (the
+  // held atoms' by its negative) and sqrt(eps) by sqrt(12); single tiles, which hold
+  // the close pairs, take the atoms' values as they are (eout = econv_out).  gb_ep: premul q q fgb per -econv_out q q
   // far_inner: the smallest inner cutoff where it is 64 A or more (0 otherwise):
   // tiles inside it are worth finding by their blocks' radii (tile_full_now)
   float far_inner;
-  float sqrtK, inv_sqrtK, invK, kU, sq_eout, neg_sq_eout, in_over_out, sqrt12, gb_ep;
+  float K, sqrtK, inv_sqrtK, invK, kU, sq_eout, neg_sq_eout, eout, in_over_out, sqrt12, gb_ep;
 };
 
 // Where component c of slot s lies in a force accumulator: a block's 32 x sums, its y
