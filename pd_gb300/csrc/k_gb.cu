@@ -634,6 +634,7 @@ __device__ __forceinline__ void gb_pair_tile(const DevView& v, const GBConst& k,
   const int si = T.bi * 32 + lane, j0 = T.bj * 32, l1 = (lane + 1) & 31;
   const float4 xi = v.xq[si], pi = v.par[si];
   DF O[3];                 // (ENERGY) centre of bj seen from bi
+  float O0[3];             // (open space: nothing left)
   float2 XL, YL, ZL;       // remainders of the held atom, negated
   unsigned ex = 0u, m14 = 0u, dm = 0u;
   if (MASKED) {
@@ -645,7 +646,7 @@ __device__ __forceinline__ void gb_pair_tile(const DevView& v, const GBConst& k,
     const float4 p0 = v.par[j0 + lane];
     if (ENERGY) {
       const float o[3] = {T.ox, T.oy, T.oz};
-      df_offset(v, v.sys[v.slot_sys[T.bi]], T.bi, T.bj, o, O);
+      df_offset(v, v.sys[v.slot_sys[T.bi]], T.bi, T.bj, o, O, O0);
       const float4 h = v.xq[j0 + lane], l = v.rlo[j0 + lane], li = v.rlo[si];
       const DF jx = df_norm(df_add(DF{h.x, l.x}, O[0])), jy = df_norm(df_add(DF{h.y, l.y}, O[1]));
       const DF jz = df_norm(df_add(DF{h.z, l.z}, O[2]));

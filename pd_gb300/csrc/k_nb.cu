@@ -176,6 +176,15 @@ struct NBEShared {
   DF sum[3];                       // the second warp's sums
 };
 
+// r less an inner radius, normalised: the sign of a difference below one unit of r.h is
+// in the low part (a virial off by 3e-5 where it was not looked at), and the radius's
+// rest counts
+__device__ __forceinline__ DF2 nb_beyond(DF2 r, DF inner, float rest) {
+  DF2 w = df_norm(df_sub(r, df2(inner)));
+  w.l = __fadd2_rn(w.l, f2(-rest));
+  return w;
+}
+
 // S = (1 - w^2 / width^2)^2 and r S' of an energy switch, w = r - inner > 0 for one of
 // the two pairs at least; 1 and 0 for a pair inside
 __device__ __forceinline__ void nb_switch_df(DF2 r, DF2 w, DF invw2, DF2& S, DF2& dS) {
@@ -190,7 +199,7 @@ __device__ __forceinline__ void nb_switch_df(DF2 r, DF2 w, DF invw2, DF2& S, DF2
 struct NBEBox {
   bool mi;
   DF x, y, z;
-  float ix, iy, iz;
+  float ix, iy, iz, tx, ty, tz;
 };
 __device__ __forceinline__ float2 nb_images(float2 d, float iL) {
   constexpr float kRint = 12582912.f;   // 1.5 2^23: adding and taking it off rounds to an integer
@@ -211,14 +220,23 @@ __device__ __forceinline__ void nb_energy_df2(const DevView& v, const NBConst& k
   DF2 dy = df_sub(df2(yha.y, yla.y, yhb.y, ylb.y), df2(xha.y, xla.y, xhb.y, xlb.y));
   DF2 dz = df_sub(df2(yha.z, yla.z, yhb.z, ylb.z), df2(xha.z, xla.z, xhb.z, xlb.z));
   if (box.mi) {
-    // (the image count times the box is exact in both parts)
-    auto wrap = [](DF2 d, DF L, float iL) {
+    // (the image count times the box is exact in all its parts; what the sums of low parts
+    // round off is kept for last: the same box for every pair, it would not average out)
+    auto wrap = [](DF2 d, DF L, float iL, float t) {
       const float2 n = nb_images(d.h, iL);
-      return df_add(d, DF2{__fmul2_rn(n, f2(L.h)), __fmul2_rn(n, f2(L.l))});
+      const DF2 s = df_two_sum(d.h, __fmul2_rn(n, f2(L.h))), u = df_two_sum(s.l, __fmul2_rn(n, f2(L.l)));
+      const DF2 w = df_two_sum(u.h, d.l);
+      d = df_fast_two_sum(s.h, w.h);
+      d.l = __fadd2_rn(d.l, __ffma2_rn(n, f2(t), __fadd2_rn(u.l, w.l)));
+      return d;
     };
-    dx = wrap(dx, box.x, box.ix);
-    dy = wrap(dy, box.y, box.iy);
-    dz = wrap(dz, box.z, box.iz);
+    dx = wrap(dx, box.x, box.ix, box.tx);
+    dy = wrap(dy, box.y, box.iy, box.ty);
+    dz = wrap(dz, box.z, box.iz, box.tz);
+  } else {
+    dx = df_norm(dx);
+    dy = df_norm(dy);
+    dz = df_norm(dz);
   }
   const DF2 r2 = df_norm2(dx, dy, dz);
   const DF2 ir = df_rsqrt(r2);
@@ -238,7 +256,7 @@ __device__ __forceinline__ void nb_energy_df2(const DevView& v, const NBConst& k
     Ev = df_norm(df_mul(eps, df_sub(AB, B)));
     gv = df_norm(df_mul(df_scale(eps, -12.f), df_norm(AB)));
     if (!SW) {
-      const DF2 w = df_sub(r, df2(e.vdwinner));
+      const DF2 w = nb_beyond(r, e.vdwinner, e.vdwinner_t);
       if (w.h.x > 0.f || w.h.y > 0.f) {
         DF2 Sv, dS;
         nb_switch_df(r, w, e.vdwinvw2, Sv, dS);
@@ -262,7 +280,7 @@ __device__ __forceinline__ void nb_energy_df2(const DevView& v, const NBConst& k
     if (scaled) qq = df_mul(qq, df_select(ca & 2048u, cb & 2048u, df2(e.elec14), one));
     Ee = fe = df_norm(df_mul(qq, ir));
     if (ELEC == 3) {
-      const DF2 w = df_sub(r, df2(e.inner));
+      const DF2 w = nb_beyond(r, e.inner, e.inner_t);
       if (w.h.x > 0.f || w.h.y > 0.f) {
         DF2 Se, dS;
         nb_switch_df(r, w, e.invw2, Se, dS);
@@ -278,9 +296,11 @@ __device__ __forceinline__ void nb_energy_df2(const DevView& v, const NBConst& k
       const bool oa = r.h.x > e.inner.h, ob = r.h.y > e.inner.h;
       DF2 h = df_sub(ir, df2(e.eshift));
       if (oa || ob) {
-        const DF2 c2 = df_norm(df_sub(df2(e.cut2), r2));
+        DF2 c2 = df_norm(df_sub(df2(e.cut2), r2)), c3 = df_norm(df_add(df2(e.fsw_k), df_scale2(r2, 2.f)));
+        c2.l = __fadd2_rn(c2.l, f2(e.cut2_t));
+        c3.l = __fadd2_rn(c3.l, f2(e.fsw_t));
         // qq sA / r (C^2 - r^2)^2 (C^2 - 3 I^2 + 2 r^2)
-        const DF2 f = df_mul(df_sqr(c2), df_norm(df_add(df2(e.fsw_k), df_scale2(r2, 2.f))));
+        const DF2 f = df_mul(df_sqr(c2), c3);
         fe = df_select(oa, ob, df_mul(df_norm(df_mul(df2(e.sA), f)), fe), fe);
         // -qq (sA r (sB / r^2 + sC + sD r^2 + sE r^4) - V(C))
         DF2 g = df_norm(df_add(df2(e.sD), df_mul(df2(e.sE), r2)));
@@ -305,13 +325,16 @@ __device__ __forceinline__ void nb_energy_df2(const DevView& v, const NBConst& k
 // both halves' sum
 __device__ __forceinline__ DF df_fold(DF2 x) { return df_add(DF{x.h.x, x.l.x}, DF{x.h.y, x.l.y}); }
 
-// one block's atom of this lane into the shared rows (O: frame offset)
+// one block's atom of this lane into the shared rows (O: frame offset, with its rest)
 __device__ __forceinline__ void nb_stage(float4* h, float4* l, float4* p, int row, const DevView& v, int slot,
-                                         const DF* O, const DF* qscale) {
+                                         const DF* O, const float* rest, const DF* qscale) {
   const float4 x = v.xq[slot], rl = v.rlo[slot], par = v.par[slot];
   const float2 pl = v.plo[slot];
   DF X = DF{x.x, rl.x}, Y = DF{x.y, rl.y}, Z = DF{x.z, rl.z}, Q = DF{x.w, rl.w};
   if (O) {
+    X.l += rest[0];
+    Y.l += rest[1];
+    Z.l += rest[2];
     X = df_norm(df_add(X, O[0]));
     Y = df_norm(df_add(Y, O[1]));
     Z = df_norm(df_add(Z, O[2]));
@@ -448,13 +471,15 @@ __global__ void __launch_bounds__(kNbEThreads, 8)
       if (T.flags & 2) ex |= diag_exclusion(lane);
       if (T.flags & 1) {
         const SystemInfo& S = v.sys[v.slot_sys[bi]];
-        box = NBEBox{true, S.boxf[0], S.boxf[1], S.boxf[2], 1.f / S.boxf[0].h, 1.f / S.boxf[1].h, 1.f / S.boxf[2].h};
+        box = NBEBox{true, S.boxf[0], S.boxf[1], S.boxf[2], 1.f / S.boxf[0].h, 1.f / S.boxf[1].h, 1.f / S.boxf[2].h,
+                     S.boxt[0], S.boxt[1], S.boxt[2]};
       }
       if (wp == 1) {
         const float o[3] = {T.ox, T.oy, T.oz};
         DF O[3];
-        df_offset(v, v.sys[v.slot_sys[bi]], bi, T.bj, o, O);
-        nb_stage(sh->jh, sh->jl, sh->jp, lane, v, T.bj * 32 + lane, O, nullptr);
+        float t[3];
+        df_offset(v, v.sys[v.slot_sys[bi]], bi, T.bj, o, O, t);
+        nb_stage(sh->jh, sh->jl, sh->jp, lane, v, T.bj * 32 + lane, O, t, nullptr);
         sh->js[lane] = T.bj * 32 + lane;
       }
     } else {
@@ -466,14 +491,15 @@ __global__ void __launch_bounds__(kNbEThreads, 8)
       if (sj >= 0) {
         const float o[3] = {en.x, en.y, en.z};
         DF O[3];
-        df_offset(v, v.sys[v.slot_sys[bi]], bi, sj >> 5, o, O);
-        nb_stage(sh->jh, sh->jl, sh->jp, row, v, sj, O, nullptr);
+        float t[3];
+        df_offset(v, v.sys[v.slot_sys[bi]], bi, sj >> 5, o, O, t);
+        nb_stage(sh->jh, sh->jl, sh->jp, row, v, sj, O, t, nullptr);
       } else {
         sh->jh[row] = make_float4(1.0e15f, 1.0e15f, 1.0e15f, 0.f);   // (empty lanes: far away)
       }
     }
     const SystemInfo& S = v.sys[v.slot_sys[bi]];
-    if (wp == 0) nb_stage(sh->ih, sh->il, sh->ip, lane, v, bi * 32 + lane, nullptr, &e.econv);
+    if (wp == 0) nb_stage(sh->ih, sh->il, sh->ip, lane, v, bi * 32 + lane, nullptr, nullptr, &e.econv);
     __syncthreads();
     // a tile's i atom of this lane; minus its two j atoms of a group pair
     const float4 xi = sh->ih[lane], ja = sh->jh[lane], jb = sh->jh[tile ? lane : 32 + lane];

@@ -166,6 +166,10 @@ NBEConst pdgpu::make_nbe_const(const NBConst& k) {
   e.eshift = df_split(k.eshift);
   e.cut2 = df_split(k.cut2_d);
   e.fsw_k = df_split(k.cut2_d - 3.0 * k.inner2_d);
+  e.vdwinner_t = df_rest(k.vdwinner_d);
+  e.inner_t = df_rest(k.inner_d);
+  e.cut2_t = df_rest(k.cut2_d);
+  e.fsw_t = df_rest(k.cut2_d - 3.0 * k.inner2_d);
   e.dovdw = k.dovdw;
   e.vdw_hard = k.vdwinvw2_d == 0.0 ? 1 : 0;
   return e;
@@ -300,6 +304,7 @@ pdgpu_ctx* pdgpu_create(int device, const pdgpu_system_desc* d, int* status) {
       S.box[k] = d->box[3 * s + k];
       S.ibox[k] = S.box[k] > 0 ? 1.0 / S.box[k] : 0.0;
       S.boxf[k] = df_split(S.box[k]);
+      S.boxt[k] = df_rest(S.box[k]);
       if (S.box[k] > 0) per++;
     }
     if (per != 0 && per != 3) return bad(PDGPU_ERR_ARG);

@@ -62,6 +62,7 @@ struct SystemInfo {
   double box[3];
   double ibox[3];   // 1 / box (periodic systems)
   DF boxf[3];       // box as double-floats
+  float boxt[3];    // and what these leave of it
 };
 
 struct __align__(16) Tile {
@@ -109,6 +110,7 @@ struct NBEConst {
   DF econv, vdw14, elec14;
   DF vdwcut, vdwinner, vdwinvw2, inner, invw2;
   DF sA, sB, sC, sD, sE, cutV, eshift, cut2, fsw_k;   // fsw_k = cut2 - 3 inner2
+  float vdwinner_t, inner_t, cut2_t, fsw_t;           // what the double-floats leave of these radii
   int dovdw, vdw_hard;   // vdw_hard: LJ ends at VdwCutoff without a switch
 };
 

@@ -18,6 +18,13 @@ inline DF df_split(double x) {
   return DF{h, (float)(x - (double)h)};
 }
 
+// what df_split leaves of x (a constant of all pairs of an energy: its error would not
+// average out)
+inline float df_rest(double x) {
+  const DF s = df_split(x);
+  return (float)(x - (double)s.h - (double)s.l);
+}
+
 __device__ __forceinline__ DF df_two_sum(float a, float b) {
   const float s = __fadd_rn(a, b);
   const float bb = __fsub_rn(s, a);

@@ -54,17 +54,21 @@ __device__ __forceinline__ void tile_masks(const DevView& v, const Tile& T, int 
 }
 
 // centre of block bj seen from block bi, as double-floats, in the image the
-// FP32 offset o was taken in
+// FP32 offset o was taken in, and what these leave of it (zero in open space): every pair
+// of the tile takes the same offset, so its rounding would not average out
 __device__ __forceinline__ void df_offset(const DevView& v, const SystemInfo& S, int bi, int bj, const float o[3],
-                                          DF O[3]) {
+                                          DF O[3], float rest[3]) {
   const float4 ci = v.cenf[bi], cj = v.cenf[bj];
   const float a[3] = {ci.x, ci.y, ci.z}, b[3] = {cj.x, cj.y, cj.z};
 #pragma unroll
   for (int c = 0; c < 3; c++) {
     O[c] = df_two_sum(b[c], -a[c]);
-    if (S.periodic) {
+    rest[c] = 0.f;
+    if (S.periodic) {   // (n = 0, 1 or -1: times the box exact)
       const float n = -rintf((O[c].h - o[c]) / S.boxf[c].h);
-      O[c] = df_norm(df_add(O[c], df_scale(S.boxf[c], n)));
+      const DF s = df_two_sum(O[c].h, n * S.boxf[c].h), u = df_two_sum(O[c].l, s.l), w = df_two_sum(u.h, n * S.boxf[c].l);
+      O[c] = df_fast_two_sum(s.h, w.h);
+      rest[c] = __fadd_rn(__fadd_rn(u.l, w.l), n * S.boxt[c]);
     }
   }
 }

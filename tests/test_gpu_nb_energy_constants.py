@@ -1,0 +1,106 @@
+"""FF_NonBonded energies and virial where an error of a constant, or a decision below
+FP32 spacing, would be the same for every pair: isolated charged pairs, all at about
+one distance, against the same law in 64 bits, summed exactly (math.fsum).
+
+Allowed per evaluation: six standard deviations of the sum of N independent errors, each
+of one rounding to 2^-32 kcal/mol (a work item's; at most one item a pair), 2^-44 of the
+pair's terms and what a rounding of its distance (2^-47 r) makes of them.  Each case states what the planted difference amounts to, well above that."""
+import math
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+KCAL = 4184.0 / 6.0221418e23
+ECONV = (6.0221418e23 / 4184.0) * 1.60217645e-19 ** 2 / (4.0 * math.pi * 8.854187817e-12 * 1e-10)
+F = np.float32
+
+
+def _rest(x):
+    """what two FP32 numbers leave of x"""
+    h = F(x)
+    return x - float(h) - float(F(x - float(h)))
+
+
+def _law(r, qq, inner, cut):
+    """Coulomb with the energy switch: energy and r dE/dr of pairs"""
+    E = qq / r
+    w = np.maximum(r - inner, 0.0)
+    iw = 1.0 / (cut - inner) ** 2
+    s = 1.0 - w * w * iw
+    return E * s * s, -(s * s * E) + E * (-4.0 * w * iw * s) * r
+
+
+def _evaluate(pos, box, q, inner, cut, far=None, lj=(0.0, 0.0)):
+    from pd_gb300 import ffi
+    from pd_gb300.engine import DeviceContext
+    from pd_gb300.workspace import SystemImage
+    n = len(pos)
+    im = SystemImage([n], box, q, np.full(n, lj[0]), np.full(n, lj[1]), np.full(n, 2e-26), np.zeros((0, 3), np.int32), pos=pos)
+    ctx = DeviceContext(im)
+    ctx.set_list(1.0)
+    ctx.set_nb(Cutoff=cut, InnerCutoff=inner, VdwCutoff=cut, VdwInnerCutoff=inner, Vdw14Scaling=1.0, Elec14Scaling=1.0,
+               Dielectric=1.0, EnergySwitch=1, ForceSwitch=0, DoVdw=1, DoElec=1)
+    ctx.set_positions(pos)
+    e = ctx.compute(ffi.NB)[0]
+    ctx.close()
+    return {k: e[k] / KCAL for k in ("vdw", "elec", "virial")}
+
+
+def _allowed(n, terms, slope):
+    return 6.0 * math.sqrt(n) * (0.29 * 2.0 ** -32 + 2.0 ** -44 * terms + 2.0 ** -47 * slope)
+
+
+def test_virial_of_pairs_a_hair_beyond_the_inner_radius():
+    """r - InnerCutoff = 2e-7 to 4.7e-7 A, below the spacing of FP32 numbers there: the
+    switch's slope, 4 u / w^2 of the energy times r, counts."""
+    cut, inner, N = 12.0, 10.0, 400
+    rng = np.random.default_rng(3)
+    site = 40.0 * np.stack(np.unravel_index(np.arange(N), (8, 8, 8)), 1)
+    pos = np.repeat(site, 2, axis=0)
+    pos[1::2, 0] += inner + rng.uniform(2e-7, 4.7e-7, N)
+    r = pos[1::2, 0] - pos[0::2, 0]
+    q = np.ones(2 * N)
+    e = _evaluate(pos, np.zeros(3), q, inner, cut)
+    E, vir = _law(r, ECONV, inner, cut)
+    tol = _allowed(N, ECONV / inner, 4.0 * ECONV / (cut - inner) ** 2 * inner)
+    assert abs(math.fsum(vir) + math.fsum(E)) > 100 * tol           # (without the slope the virial is -E)
+    assert abs(e["virial"] - math.fsum(vir)) <= tol and abs(e["elec"] - math.fsum(E)) <= tol
+
+
+@pytest.mark.parametrize("periodic", [0, 1])
+def test_sums_of_many_pairs_at_one_distance(periodic):
+    """20,000 pairs whose inner radius, or 1,600 across the faces of a box whose edge,
+    is not the sum of two FP32 numbers."""
+    rng = np.random.default_rng(periodic)
+    if periodic:
+        cand = 1203.0 + 0.01 * np.arange(400)
+        L = float(max(cand, key=lambda x: abs(_rest(x))))
+        inner, cut, m = 10.0, 12.0, 40
+        N = m * m
+        site = np.stack([np.zeros(N), *(30.0 * np.stack(np.unravel_index(np.arange(N), (m, m))))], 1)
+        pos = np.repeat(site, 2, axis=0)
+        pos[0::2, 0] = L - 4.0
+        pos[1::2, 0] = rng.uniform(6.65, 6.75, N)
+        r = pos[1::2, 0] - pos[0::2, 0] + L
+        box = np.full(3, L)
+    else:
+        cand = 10.0 + 0.01 * np.arange(200)
+        inner = float(max(cand, key=lambda x: abs(_rest(x))))
+        cut, m, L = inner + 2.0, 28, 0.0
+        N = 20_000
+        pos = np.repeat(35.0 * np.stack(np.unravel_index(np.arange(N), (m, m, m)), 1), 2, axis=0)
+        pos[1::2, 0] += inner + rng.uniform(0.15, 0.25, N)
+        r = pos[1::2, 0] - pos[0::2, 0]
+        box = np.zeros(3)
+    e = _evaluate(pos, box, np.full(2 * N, 3.0), inner, cut)
+    law = lambda r, inner: _law(r, 9.0 * ECONV, inner, cut)
+    E, vir = law(r, inner)
+    h = 1e-5
+    slope = abs(law(r + h, inner)[1] - law(r - h, inner)[1]).mean() / (2 * h)
+    tol = _allowed(N, float(np.abs(vir).max()), slope * r[0])
+    planted = N * slope * abs(_rest(L if periodic else inner))   # (the switch's width is a constant of its own)
+    assert planted > 2.5 * tol, (planted, tol)
+    assert abs(e["virial"] - math.fsum(vir)) <= tol, (e["virial"] - math.fsum(vir), tol, planted)
+    assert abs(e["elec"] - math.fsum(E)) <= tol
