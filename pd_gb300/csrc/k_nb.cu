@@ -206,6 +206,25 @@ __device__ __forceinline__ float2 nb_images(float2 d, float iL) {
   return __fadd2_rn(__ffma2_rn(d, f2(-iL), f2(kRint)), f2(-kRint));
 }
 
+// A pair whose terms exceed kNbLarge (atoms nearly on one another): 2^-45 of them is
+// beyond the fixed point's resolution, in its sums too, so it goes in FP64 straight into
+// these.
+constexpr float kNbLarge = 4096.f;   // kcal/mol: 2^-44 of it is 2^-32
+template <int ELEC>
+__device__ __noinline__ void nb_energy_large(const DevView& v, const NBConst& k, const SystemInfo& S, int si, int sj,
+                                             bool is14) {
+  const int a = v.sorted_atom[si], b = v.sorted_atom[sj];
+  if (a < 0 || b < 0) return;
+  const double eps = v.sqeps[a] * v.sqeps[b] * (is14 ? k.vdw14_d : 1.0);
+  const double qq = v.charge[a] * v.charge[b] * k.econv_diel_d * (is14 ? k.elec14_d : 1.0);
+  double ev = 0.0, ee = 0.0, f, vir;
+  nb_pair<double, ELEC>(k, nb_r2_fp64(v, S, si, sj), v.radius[a] + v.radius[b], eps, qq, ev, ee, f, vir);
+  long long* E = v.eacc + (size_t)v.slot_sys[si >> 5] * E_NSLOTS;
+  atomic_add_ll(&E[E_VDW], fix_energy_d(ev));
+  atomic_add_ll(&E[E_ELEC], fix_energy_d(ee));
+  atomic_add_ll(&E[E_VIRIAL], fix_energy_d(vir));
+}
+
 // energies of two listed pairs into the sums (same law as the force bodies; pair b
 // counts only if two).  Products of products stay unnormalised where their l holds a
 // few roundings of h: what df_mul leaves out is then below 1e-13.
@@ -312,14 +331,19 @@ __device__ __forceinline__ void nb_energy_df2(const DevView& v, const NBConst& k
     }
   }
   DF2 vir = df_sub(gv, fe);
-  Ev = df_select(true, two, Ev, zero);
-  Ee = df_select(true, two, Ee, zero);
-  vir = df_select(true, two, vir, zero);
+  const float2 f = __fmul2_rn(vir.h, ir.h);
+  sum.f = __fadd2_rn(sum.f, make_float2(fabsf(f.x), two ? fabsf(f.y) : 0.f));
+  const bool la = fmaxf(fabsf(vir.h.x), fmaxf(fabsf(Ev.h.x), fabsf(Ee.h.x))) > kNbLarge;
+  const bool lb = two && fmaxf(fabsf(vir.h.y), fmaxf(fabsf(Ev.h.y), fabsf(Ee.h.y))) > kNbLarge;
+  if (la) nb_energy_large<ELEC>(v, k, S, ibase + ia, sh->js[ja], ca & 2048u);
+  if (lb) nb_energy_large<ELEC>(v, k, S, ibase + ib, sh->js[jb], cb & 2048u);
+  const bool ka = !la, kb = two && !lb;
+  Ev = df_select(ka, kb, Ev, zero);
+  Ee = df_select(ka, kb, Ee, zero);
+  vir = df_select(ka, kb, vir, zero);
   df_acc(sum.vdw, Ev);
   df_acc(sum.elec, Ee);
   df_acc(sum.vir, vir);
-  const float2 f = __fmul2_rn(vir.h, ir.h);
-  sum.f = __fadd2_rn(sum.f, make_float2(fabsf(f.x), fabsf(f.y)));
 }
 
 // both halves' sum

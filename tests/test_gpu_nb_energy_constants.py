@@ -104,3 +104,24 @@ def test_sums_of_many_pairs_at_one_distance(periodic):
     assert planted > 2.5 * tol, (planted, tol)
     assert abs(e["virial"] - math.fsum(vir)) <= tol, (e["virial"] - math.fsum(vir), tol, planted)
     assert abs(e["elec"] - math.fsum(E)) <= tol
+
+
+def test_energies_of_overlapping_atoms_are_fp64():
+    """Two atoms 0.9 to 1.4 A apart: LJ energies of 1e4 to 1e6 kcal/mol to 2^-50 of
+    themselves (their law in FP64: some ten roundings of 2^-53) and 2^-31 kcal/mol."""
+    radius, eps = 1.6, 1.0e-11
+    se2 = (eps * math.sqrt(6.0221418e23 / 4184.0)) ** 2
+    for k, r in enumerate((0.9, 1.05, 1.23, 1.4)):
+        for image in (0, 1):
+            L = 25.3
+            pos = np.array([[0.3, 0.2, 0.1], [0.3 + r, 0.2, 0.1]])
+            box = np.full(3, L if image else 0.0)
+            if image:
+                pos[0, 0] += L
+            e = _evaluate(pos, box, np.array([0.7, 0.4]), 10.0, 12.0, lj=(radius, eps))
+            d = pos[1, 0] - pos[0, 0]
+            d -= box[0] * np.rint(d / box[0]) if image else 0.0
+            B = (2.0 * radius / abs(d)) ** 6
+            for key, ref in (("vdw", se2 * (B * B - 2.0 * B)), ("elec", ECONV * 0.7 * 0.4 / abs(d)),
+                             ("virial", -12.0 * se2 * (B * B - B) - ECONV * 0.7 * 0.4 / abs(d))):
+                assert abs(e[key] - ref) <= 2.0 ** -49 * abs(ref) + 2.0 ** -31, (r, image, key, e[key] - ref, ref)
