@@ -20,9 +20,10 @@
 // FP32 sums do not resolve to the 1e-4 a parameter fit checks against.  The
 // kernels therefore sum per tile in compensated FP32 (value plus running
 // rounding error, about 48 significant bits, on the FP32 pipe: GB300's FP64 rate
-// is a small fraction of its FP32 rate), fed by plain FP32 sums over 8 rotation
-// steps (FF_NonBonded's charge gradients: by every term).  Per-tile sums enter 64-bit fixed point (2^32
-// per kcal/mol per parameter unit), so the result does not depend on scheduling.
+// is a small fraction of its FP32 rate), fed by every term of FF_NonBonded and by
+// plain FP32 sums over 8 rotation steps of GB.  Per-tile sums enter 64-bit fixed
+// point (2^32 per kcal/mol per parameter unit), so the result does not depend on
+// scheduling.
 #include "pdgpu_tile.cuh"
 
 namespace pdgpu {
@@ -424,8 +425,8 @@ __global__ void k_adj_w(DevView v, const double* terms123, const long long* gpol
 // ---------------------------------------------------------------------------
 // NB (FF_NonBonded) pair terms: dE/dq, dE/dRmin, dE/dsqrt(eps).  The Coulomb
 // energy per unit charge product is formed in double-float from the FP32 distance
-// and its sums are double-float; the LJ terms are FP32, summed over 8 steps and
-// then compensated.  (In FP64, with FP64 sums on the rotation, the pass took
+// and its sums are double-float; the LJ terms are FP32, each entered into a
+// compensated sum.  (In FP64, with FP64 sums on the rotation, the pass took
 // 751 us on 4 frames of 1,094 waters, bound by the FP64 pipe; 120 us so.)
 // ---------------------------------------------------------------------------
 // Coulomb energy of a pair per unit q q econv (elec14 aside): nb_pair's law
@@ -452,7 +453,6 @@ template <int ELEC, bool MASKED>
 __device__ __forceinline__ void adj_nb_tile(const DevView& v, const NBConst& k, const Tile& T, const NBEConst& e,
                                             const SystemInfo& S, int lane, int si, const float4& xi, const float4& pi,
                                             unsigned ex, unsigned m14, CAcc3& I, CAcc3& J) {
-  float ib = 0.f, ic = 0.f, jb = 0.f, jc = 0.f;   // LJ sums of 8 steps (the j atom's rotate with it)
   float4 xj = v.xq[T.bj * 32 + lane];
   float4 pj = v.par[T.bj * 32 + lane];
   float Lx = 1.f, Ly = 1.f, Lz = 1.f;
@@ -504,22 +504,14 @@ __device__ __forceinline__ void adj_nb_tile(const DevView& v, const NBConst& k, 
         const float R = pi.x + pj.x, t2 = R * R * invr * invr, B = t2 * t2 * t2;
         const float dR = lj_dR(R, invr) * Sv * pi.y * pj.y;
         const float e1 = (B * B - 2.f * B) * Sv;   // energy per unit sqrt(eps_i) sqrt(eps_j)
-        ib += dR;
-        jb += dR;
-        ic += e1 * pj.y;
-        jc += e1 * pi.y;
+        csum_add(I.b, dR);
+        csum_add(J.b, dR);
+        csum_add(I.c, e1 * pj.y);
+        csum_add(J.c, e1 * pi.y);
       }
     }
     ROT(xj.x); ROT(xj.y); ROT(xj.z); ROT(xj.w); ROT(pj.x); ROT(pj.y);
-    ROT(J.a.hi); ROT(J.a.lo); ROT(jb); ROT(jc);
-    if ((kk & 7) == 7) {
-      csum_add(I.b, ib);
-      csum_add(I.c, ic);
-      // the j atom now at this lane lives in lane + kk + 1: its sums go home
-      csum_add(J.b, __shfl_sync(0xffffffffu, jb, (lane - kk - 1) & 31));
-      csum_add(J.c, __shfl_sync(0xffffffffu, jc, (lane - kk - 1) & 31));
-      ib = ic = jb = jc = 0.f;
-    }
+    ROT(J.a.hi); ROT(J.a.lo); ROT(J.b.hi); ROT(J.b.lo); ROT(J.c.hi); ROT(J.c.lo);
   }
 }
 
