@@ -407,19 +407,20 @@ __global__ void __launch_bounds__(kAdjThreads, 6) k_adj_born(const __grid_consta
 
 // dE/dGpol per slot: (dE/da from the pair pass - E_self / a) * halfeconv / Gpol^2
 __device__ __forceinline__ double dE_dGpol(const DevView& v, const double* terms123, const long long* gpol,
-                                           const long long* deda, double premul, double halfeconv, int s, int a) {
-  const double G = terms123[a] + (double)gpol[s] * (1.0 / kSumScale);
+                                           const long long* deda, double gscale, double premul, double halfeconv,
+                                           int s, int a) {
+  const double G = terms123[a] + (double)gpol[s] * gscale;
   const double ai = v.born[a], q = v.charge[a];
   const double da = (double)deda[s] * (1.0 / kSumScale) - premul * q * q / (ai * ai);
   return da * halfeconv / (G * G);
 }
 
 __global__ void k_adj_w(DevView v, const double* terms123, const long long* gpol, const long long* deda,
-                        double premul, double halfeconv, float* w) {
+                        double gscale, double premul, double halfeconv, float* w) {
   int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= v.nslots) return;
   int a = v.sorted_atom[s];
-  w[s] = a < 0 ? 0.f : (float)dE_dGpol(v, terms123, gpol, deda, premul, halfeconv, s, a);
+  w[s] = a < 0 ? 0.f : (float)dE_dGpol(v, terms123, gpol, deda, gscale, premul, halfeconv, s, a);
 }
 
 // ---------------------------------------------------------------------------
@@ -548,8 +549,8 @@ struct AdjOut {
 };
 
 __global__ void k_adj_out(DevView v, const long long* g, int nslots, bool gb, const double* terms123,
-                          const long long* gpol, const long long* deda, double premul, double halfeconv,
-                          double eps_unit, AdjOut o) {
+                          const long long* gpol, const long long* deda, double gscale, double premul,
+                          double halfeconv, double eps_unit, AdjOut o) {
   int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= v.nslots) return;
   int a = v.sorted_atom[s];
@@ -565,7 +566,7 @@ __global__ void k_adj_out(DevView v, const long long* g, int nslots, bool gb, co
   if (o.e) o.e[a] = (double)g[G_EPS * (size_t)nslots + s] * f * eps_unit * kKcalMolToJ;
   if (o.R) o.R[a] = gb ? (double)g[G_GBR * (size_t)nslots + s] * f * kKcalMolToJ : 0.0;
   if (o.V) o.V[a] = gb ? (double)g[G_VJ * (size_t)nslots + s] * f * kKcalMolToJ : 0.0;
-  if (o.T) o.T[a] = gb ? dE_dGpol(v, terms123, gpol, deda, premul, halfeconv, s, a) * kKcalMolToJ : 0.0;
+  if (o.T) o.T[a] = gb ? dE_dGpol(v, terms123, gpol, deda, gscale, premul, halfeconv, s, a) * kKcalMolToJ : 0.0;
 }
 
 
@@ -583,11 +584,12 @@ int launch_adjoint(Context& c, unsigned what, const AdjScratch& a, double* d_q, 
   const double ec = econv_kcal();
   const double halfeconv = 0.5 * ec;
   const double premul = gb ? -0.5 * ec * (1.0 / c.gb.DielectricSolute - 1.0 / c.gb.DielectricSolvent) : 0.0;
+  const double gscale = gb ? born_sum_unit(c.gb) : 0.0;
   long long* g = a.g;
   if (gb) {
     GBConst k = make_gb_const(c.gb, c.list_radius_built);
     c.kernel_launches += 2;
-    k_adj_w<<<nb, 256, 0, st>>>(v, c.d_gbT.p, c.d_gpol.p, c.d_deda.p, premul, halfeconv, a.w);
+    k_adj_w<<<nb, 256, 0, st>>>(v, c.d_gbT.p, c.d_gpol.p, c.d_deda.p, gscale, premul, halfeconv, a.w);
     k_adj_born<<<2 * grid, kAdjThreads, 0, st>>>(v, k, a.w, g + G_GBR * (size_t)ns, g + G_VJ * (size_t)ns);
   } else {
     long long *gq = g + G_Q * (size_t)ns, *gr = g + G_R * (size_t)ns, *ge = g + G_EPS * (size_t)ns;
@@ -603,7 +605,7 @@ int launch_adjoint(Context& c, unsigned what, const AdjScratch& a, double* d_q, 
   }
   AdjOut o = {d_q, d_r, d_e, d_R, d_V, d_T};
   c.kernel_launches += 1;
-  k_adj_out<<<nb, 256, 0, st>>>(v, g, ns, gb, c.d_gbT.p, c.d_gpol.p, c.d_deda.p, premul, halfeconv,
+  k_adj_out<<<nb, 256, 0, st>>>(v, g, ns, gb, c.d_gbT.p, c.d_gpol.p, c.d_deda.p, gscale, premul, halfeconv,
                                 std::sqrt(kNa / kKcal2J), o);
   return cudaGetLastError() == cudaSuccess ? PDGPU_OK : PDGPU_ERR_CUDA;
 }

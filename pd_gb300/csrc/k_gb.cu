@@ -22,7 +22,10 @@
 namespace pdgpu {
 
 // ---------------------------------------------------------------------------
-// pass 1: Born-radius pair sums  Gpol_i += P4 Vj CCF / r^4  (bond order > 2)
+// pass 1: Born-radius pair sums  Gpol_i += P4 Vj CCF / r^4  (bond order > 2).  The sums
+// carry the power of two next to P4 (GBConst::born2, exact in every volume); the rest of
+// P4 meets them in FP64 (k_gb_radii): rounded with P4 in it, a volume would shift the sums
+// of all its partners alike.
 // ---------------------------------------------------------------------------
 // inside GbsaStillCutoff (FULL: the whole tile is); pairs within FP32 rounding of
 // the cutoff are decided in FP64
@@ -95,7 +98,7 @@ constexpr int kBornWarps = kBornThreads / 32;
 // rows of the rotating block in the warp's shared memory, twice over, so that a
 // lane's row at step kk lies at a fixed offset from its first (no wrap-around)
 struct BornRows {
-  float4 xy[64], zv[64];   // (x, x', y, y'), (z, z', V, V'); with the base law (x, y, z, q), (LJ R, sqrt(12 eps), V, -)
+  float4 xy[64], zv[64];   // (x, x', y, y'), (z, z', V, V'); with the base law (x, y, z, q), (LJ R, sqrt(12 eps), V, -) (V: times born2)
   float2 r[64];            // (R, R'), single tiles only
 };
 
@@ -108,7 +111,7 @@ __device__ __forceinline__ void born_tile(const DevView& v, const GBConst& k, co
   const float4 xi = v.xq[si], pi = v.par[si];
   {
     const float4 x0 = j_in_i_frame(v, T, lane), p0 = v.par[j0 + lane];
-    const float v0 = p0.w;
+    const float v0 = k.born2 * p0.w;
     const float x1 = __shfl_sync(0xffffffffu, x0.x, l1), y1 = __shfl_sync(0xffffffffu, x0.y, l1);
     const float z1 = __shfl_sync(0xffffffffu, x0.z, l1), v1 = __shfl_sync(0xffffffffu, v0, l1);
     const float r1 = __shfl_sync(0xffffffffu, p0.z, l1);
@@ -118,7 +121,7 @@ __device__ __forceinline__ void born_tile(const DevView& v, const GBConst& k, co
     rs.r[lane] = rs.r[lane + 32] = make_float2(p0.z, r1);
     __syncwarp();
   }
-  const float2 AX = f2(-xi.x), AY = f2(-xi.y), AZ = f2(-xi.z), RA = f2(pi.z), VA = f2(pi.w);
+  const float2 AX = f2(-xi.x), AY = f2(-xi.y), AZ = f2(-xi.z), RA = f2(pi.z), VA = f2(k.born2 * pi.w);
   float2 GA = f2(0.f), GR = f2(0.f);
 #pragma unroll 4
   for (int kk = 0; kk < 32; kk += 2) {
@@ -148,7 +151,7 @@ __device__ __forceinline__ void born_tile(const DevView& v, const GBConst& k, co
     GR = __ffma2_rn(w, VA, GR);
     ROT2(GR);
   }
-  const float gr = k.P4 * (GR.x + __shfl_sync(0xffffffffu, GR.y, (lane + 31) & 31)), ga = k.P4 * (GA.x + GA.y);
+  const float gr = GR.x + __shfl_sync(0xffffffffu, GR.y, (lane + 31) & 31), ga = GA.x + GA.y;
   fix_range(v.status, fabsf(ga) + fabsf(gr));
   atomic_add_ll(&gpol[si], fx32(ga));
   atomic_add_ll(&gpol[j0 + lane], fx32(gr));
@@ -160,7 +163,7 @@ __device__ __forceinline__ void born_loop2(const DevView& v, const GBConst& k, i
                                            const float4& xa, const float4& xb, const float4& pa, const float4& pb,
                                            float c2, float2& GA, float2& GB, float2& GR) {
   const float2 AX = f2(-xa.x), AY = f2(-xa.y), AZ = f2(-xa.z), BX = f2(-xb.x), BY = f2(-xb.y), BZ = f2(-xb.z);
-  const float2 VA = f2(pa.w), VB = f2(pb.w);
+  const float2 VA = f2(k.born2 * pa.w), VB = f2(k.born2 * pb.w);
   const float4 *xy = rs.xy + lane, *zv = rs.zv + lane;
 #pragma unroll 4
   for (int kk = 0; kk < 32; kk += 2) {
@@ -202,15 +205,15 @@ __device__ __forceinline__ void born_full2(const DevView& v, const GBConst& k, c
   const float4 p0 = v.par[r0 + lane], p1 = v.par[r0 + l1];
   __syncwarp();
   rs.xy[lane] = rs.xy[lane + 32] = make_float4(x0.x, x1.x, x0.y, x1.y);
-  rs.zv[lane] = rs.zv[lane + 32] = make_float4(x0.z, x1.z, p0.w, p1.w);
+  rs.zv[lane] = rs.zv[lane + 32] = make_float4(x0.z, x1.z, k.born2 * p0.w, k.born2 * p1.w);
   __syncwarp();
   const float c2 = pair_contact2(k, make_float2(pa.z, pb.z), p0.z);
   float2 GA = f2(0.f), GB = f2(0.f), GR = f2(0.f);
   if (item_far(xa, xb, x0, c2, c2)) born_loop2<true>(v, k, lane, r0, rs, xa, xb, pa, pb, c2, GA, GB, GR);
   else born_loop2<false>(v, k, lane, r0, rs, xa, xb, pa, pb, c2, GA, GB, GR);
   // GR.x holds the sum of the rotating atom of this lane, GR.y that of lane + 1
-  const float gr = k.P4 * (GR.x + __shfl_sync(0xffffffffu, GR.y, (lane + 31) & 31));
-  const float ga = k.P4 * (GA.x + GA.y), gb = k.P4 * (GB.x + GB.y);
+  const float gr = GR.x + __shfl_sync(0xffffffffu, GR.y, (lane + 31) & 31);
+  const float ga = GA.x + GA.y, gb = GB.x + GB.y;
   fix_range(v.status, fabsf(ga) + fabsf(gb) + fabsf(gr));
   atomic_add_ll(&gpol[sa], fx32(ga));
   atomic_add_ll(&gpol[sb], fx32(gb));
@@ -251,7 +254,7 @@ __device__ __forceinline__ void born_base_loop2(const DevView& v, const GBConst&
                                                 float3& R) {
   const float2 nx = make_float2(-xa.x, -xb.x), ny = make_float2(-xa.y, -xb.y), nz = make_float2(-xa.z, -xb.z);
   const float2 QN = make_float2(k.neg_sq_eout * xa.w, k.neg_sq_eout * xb.w), S = make_float2(pa.x, pb.x);
-  const float2 EN = make_float2(-k.sqrt12 * pa.y, -k.sqrt12 * pb.y), V = make_float2(pa.w, pb.w);
+  const float2 EN = make_float2(-k.sqrt12 * pa.y, -k.sqrt12 * pb.y), V = make_float2(k.born2 * pa.w, k.born2 * pb.w);
   const float4 *x2 = rs.xy + lane, *p2 = rs.zv + lane;
 #pragma unroll 2
   for (int kk = 0; kk < 32; kk++) {
@@ -293,7 +296,7 @@ __device__ __forceinline__ void born_base_full2(const DevView& v, const GBConst&
   const float4 pa = v.par[sa], pb = v.par[sb], x0 = v.xq[r0 + lane], p0 = v.par[r0 + lane];
   __syncwarp();
   rs.xy[lane] = rs.xy[lane + 32] = make_float4(x0.x, x0.y, x0.z, k.sq_eout * x0.w);
-  rs.zv[lane] = rs.zv[lane + 32] = make_float4(p0.x, k.sqrt12 * p0.y, p0.w, 0.f);
+  rs.zv[lane] = rs.zv[lane + 32] = make_float4(p0.x, k.sqrt12 * p0.y, k.born2 * p0.w, 0.f);
   __syncwarp();
   const float c2 = pair_contact2(k, make_float2(pa.z, pb.z), p0.z);
   float2 G = f2(0.f), FX = f2(0.f), FY = f2(0.f), FZ = f2(0.f);
@@ -301,8 +304,6 @@ __device__ __forceinline__ void born_base_full2(const DevView& v, const GBConst&
   float3 R = make_float3(0.f, 0.f, 0.f);   // minus the rotating atom's force
   if (item_far(xa, xb, x0, c2, c2)) born_base_loop2<true>(v, k, lane, r0, rs, xa, xb, pa, pb, c2, G, FX, FY, FZ, gr, R);
   else born_base_loop2<false>(v, k, lane, r0, rs, xa, xb, pa, pb, c2, G, FX, FY, FZ, gr, R);
-  G = __fmul2_rn(G, f2(k.P4));
-  gr *= k.P4;
   fix_range(v.status, fabsf(G.x) + fabsf(G.y) + fabsf(gr));
   atomic_add_ll(&gpol[sa], fx32(G.x));
   atomic_add_ll(&gpol[sb], fx32(G.y));
@@ -370,7 +371,7 @@ __global__ void __launch_bounds__(BASE ? kBaseThreads : kBornThreads, BASE ? 6 :
 }
 
 // Born radii a = -halfeconv / (terms123 + sum) + BornRadiusOffset  (FP64)
-__global__ void k_gb_radii(DevView v, const double* terms123, const long long* gpol, double halfeconv,
+__global__ void k_gb_radii(DevView v, const double* terms123, const long long* gpol, double gscale, double halfeconv,
                            double offset, float* born_f, double* born_d, float* bborn) {
   pdl_sync();
   int s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -378,7 +379,7 @@ __global__ void k_gb_radii(DevView v, const double* terms123, const long long* g
   int a = v.sorted_atom[s];
   float f = 1.f;
   if (a >= 0) {
-    double G = terms123[a] + (double)gpol[s] * (1.0 / kSumScale);
+    double G = terms123[a] + (double)gpol[s] * gscale;
     double r = -halfeconv / G + offset;
     f = (float)r;
     born_d[a] = r;
@@ -1182,7 +1183,8 @@ int launch_gb(Context& c, const GBConst& k, double halfeconv, double born_offset
   const int gp = g * (256 / kPairThreads), ge = g * (256 / kPairEThreads);
   if (k.fast && !energy && !c.gb_no_chain) launch_pdl(st, g * (256 / kBaseThreads), kBaseThreads, 0, k_gb_born<true>, v, k, c.d_gpol.p);
   else launch_pdl(st, g, kBornThreads, 0, k_gb_born<false>, v, k, c.d_gpol.p);
-  launch_pdl(st, sp.grid, sp.threads, 0, k_gb_radii, v, c.d_gbT.p, c.d_gpol.p, halfeconv, born_offset, c.d_born_f.p, c.d_born_d.p, c.d_bborn.p);
+  launch_pdl(st, sp.grid, sp.threads, 0, k_gb_radii, v, c.d_gbT.p, c.d_gpol.p, born_sum_unit(c.gb), halfeconv, born_offset,
+             c.d_born_f.p, c.d_born_d.p, c.d_bborn.p);
   if (c.gb_no_chain) {
     // a gradient call: energies (FP32 pair terms: they weight a loss), dE/da and the
     // pair terms' gradients in one pass, no forces

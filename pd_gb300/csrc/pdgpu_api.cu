@@ -175,6 +175,10 @@ NBEConst pdgpu::make_nbe_const(const NBConst& k) {
   return e;
 }
 
+// the power of two next to |P4|
+static double born_power(double P4) { return P4 == 0.0 ? 1.0 : std::exp2(std::round(std::log2(std::fabs(P4)))); }
+double pdgpu::born_sum_unit(const pdgpu_gb_params& p) { return p.P4 / born_power(p.P4) / kSumScale; }
+
 void pdgpu::set_gb_threshold(GBConst& k, double thresh) {
   k.thresh = (float)thresh;
   k.thresh_d = thresh;
@@ -207,6 +211,7 @@ GBConst pdgpu::make_gb_const(const pdgpu_gb_params& p, double listR) {
   k.P4 = (float)p.P4;
   k.P5 = (float)p.P5;
   k.invP5 = (float)(1.0 / p.P5);
+  k.born2 = (float)born_power(p.P4);
   k.still2_d = still * still;
   k.thresh_d = p.ExpApproxThreshold;
   k.fast = 1;

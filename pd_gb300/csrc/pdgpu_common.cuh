@@ -121,6 +121,7 @@ struct GBConst {
   float econv_in, econv_out, premul;  // kcal units
   float vdw14, elec14, thresh;
   float P4, P5, invP5;
+  float born2;             // the power of two next to P4: what the Born sums carry of it
   double still2_d, thresh_d;
   // 1: FastMode (GB fused with LJ + Coulomb, eps_out Coulomb below the threshold);
   // 0: calcBornForces (GB term alone for every pair, premul q q / r below it)
@@ -351,6 +352,7 @@ int launch_census(Context& c, const NBConst& nk, const GBConst& gk, bool do_nb, 
 int measure_fp32_peak(int device, double* tflops_ffma, double* tflops_ffma2);
 NBConst make_nb_const(const pdgpu_nb_params& p);
 NBEConst make_nbe_const(const NBConst& k);
+double born_sum_unit(const pdgpu_gb_params& p);     // Gpol per unit of the Born sums' fixed point
 void set_gb_threshold(GBConst& k, double thresh);   // ExpApproxThreshold and what the bodies derive from it
 GBConst make_gb_const(const pdgpu_gb_params& p, double listR);
 int launch_bonded(Context& c, bool energy);
