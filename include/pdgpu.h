@@ -181,10 +181,12 @@ int pdgpu_compute(pdgpu_ctx *ctx, unsigned what, pdgpu_energies *out, double *f,
  * memory) without any host synchronisation.  Energies are formed only when
  * `what` includes PDGPU_ENERGY and stay on the device until pdgpu_get_energies().
  * Forces are FP32 pair math with 64-bit fixed-point sums.  Energies, when
- * requested: GB pair energies in double-float arithmetic (~45 bits) for pairs
- * closer than 4.5 A, from FP32 terms beyond; FF_NonBonded pair energies in
- * double-float arithmetic; summed in double-float and fixed point.  A call that
- * reads no forces leaves out the passes that only form them. */
+ * requested: FF_NonBonded's in double-float arithmetic (two FP32 numbers, ~45
+ * bits; pairs with terms above 4096 kcal/mol in FP64), summed in double-float and
+ * fixed point.  GB's with its vacuum LJ and Coulomb: pairs closer than 4.5 A in
+ * double-float, but for the GB function and the switches, which are FP32; beyond,
+ * FP32 terms in FP32 sums of 8, these in double-float and fixed point.  A call
+ * that reads no forces leaves out the passes that only form them. */
 int pdgpu_compute_device(pdgpu_ctx *ctx, unsigned what, double *d_f);
 int pdgpu_get_energies(pdgpu_ctx *ctx, pdgpu_energies *out);
 /* Born radii (Angstrom, original atom order) and LCPO per-atom SASA (A^2) from

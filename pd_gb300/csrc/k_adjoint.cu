@@ -444,10 +444,12 @@ __device__ __forceinline__ DF nb_phi_df(const NBEConst& e, float r2f) {
   }
   // Steinbach & Brooks force switch, nonbonded.cpp:798-819
   if (w.h <= 0.f) return df_norm(df_sub(ir, e.eshift));
-  DF h = df_norm(df_add(e.sD, df_mul(e.sE, r2)));
-  h = df_norm(df_add(e.sC, df_mul(h, r2)));
-  h = df_norm(df_add(df_mul(h, r), df_mul(e.sB, ir)));
-  return df_norm(df_sub(e.cutV, df_mul(e.sA, h)));
+  const DF c = df_norm(df_sub(e.cut, r));
+  DF h = df_norm(df_add(e.q2, df_mul(e.q3, r)));
+  h = df_norm(df_add(e.q1, df_mul(h, r)));
+  h = df_norm(df_add(e.q0, df_mul(h, r)));
+  h = df_norm(df_mul(df_norm(df_mul(h, ir)), df_norm(df_mul(df_norm(df_mul(c, c)), c))));
+  return df_norm(df_mul(e.sA, h));
 }
 
 template <int ELEC, bool MASKED>

@@ -50,10 +50,11 @@ __device__ __forceinline__ int hilbert3(unsigned x0, unsigned x1, unsigned x2) {
   return h;
 }
 
-// rows of systems of up to this many blocks (262,144 atoms) test every column: at
-// 5,623 blocks a build takes 334 us so, 430 us through the block grid (703 blocks:
-// 122 and 152 us); the tests grow with the square of the blocks, so larger systems
-// take the grid
+// rows of systems of up to this many blocks (262,144 atoms) test every column; the tests
+// grow with the square of the blocks, so larger systems take the grid.  A build of a dense
+// box at R = 14 A, all columns and grid: 703 blocks 65 and 93 us, 5,623 290 and 388, 8,192
+// 464 and 562, 12,288 747 and 804, 16,384 1,116 and 1,094, 24,576 1,950 and 1,586.  The two
+// meet near 16,000; the line stays below, where the grid gives up 20 % at most.
 constexpr int kDirectBlocks = 8192;
 
 // order-preserving float <-> int for atomic min / max

@@ -56,16 +56,16 @@ __global__ void k_mc_delta(const __grid_constant__ DevView v, const __grid_const
       const double eps = v.sqeps[i] * v.sqeps[j] * (is14 ? k.vdw14_d : 1.0);
       const double qq = v.charge[i] * v.charge[j] * k.econv_diel_d * (is14 ? k.elec14_d : 1.0);
       const double rs = v.radius[i] + v.radius[j];
-      double f, rd, evn = 0.0, een = 0.0, evo = 0.0, eeo = 0.0;
+      double rd, evn = 0.0, een = 0.0, evo = 0.0, eeo = 0.0;
       const double r2n = mc_r2(v.pos, S, i, j);
       if (r2n <= k.cut2_dd) {
-        nb_pair<double, ELEC>(k, r2n, rs, eps, qq, evn, een, f, rd);
+        nb_pair<ELEC>(k, r2n, rs, eps, qq, evn, een, rd);
         fsum += (float)fabs(rd / sqrt(r2n));
       } else if (r2n != r2n) {   // (a non-finite position)
         fsum += (float)r2n;
       }
       const double r2o = mc_r2(ref, S, i, j);
-      if (r2o <= k.cut2_dd) nb_pair<double, ELEC>(k, r2o, rs, eps, qq, evo, eeo, f, rd);
+      if (r2o <= k.cut2_dd) nb_pair<ELEC>(k, r2o, rs, eps, qq, evo, eeo, rd);
       ev += evn - evo;
       ee += een - eeo;
     }

@@ -354,13 +354,6 @@ __global__ void k_scale_vel(MDView m, const double* vscale) {
     for (int c = 0; c < 3; c++) m.vel[3 * a + c] *= s;
 }
 
-// zero a fixed-point buffer (kernel form so it can sit inside a captured graph
-// and be skipped on steps that keep the cached LCPO forces)
-__global__ void k_zero_ll(long long* p, size_t n) {
-  size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) p[i] = 0;
-}
-
 // (the kinetic sums were cleared with the step's other accumulators)
 int launch_integrate(Context& c, MDState& md, bool first, bool last) {
   c.kernel_launches += 1;
@@ -410,12 +403,6 @@ int launch_rescue(Context& c, MDState& md, unsigned long long seed, int* bad_hos
   if (cudaMemsetAsync(md.d_ke.p, 0, sizeof(long long) * c.nsys, c.stream) != cudaSuccess) return PDGPU_ERR_CUDA;
   k_rescue<<<nb, 256, 0, c.stream>>>(m, md.d_bad.p, md.d_ckpt_pos.p, seed, md.d_ke.p);
   k_rescale_ke<<<nb, 256, 0, c.stream>>>(m, md.d_bad.p, c.d_sys.p, md.d_ke.p);
-  return cudaGetLastError() == cudaSuccess ? PDGPU_OK : PDGPU_ERR_CUDA;
-}
-
-int launch_zero_ll(Context& c, long long* p, size_t n) {
-  if (n == 0) return PDGPU_OK;
-  k_zero_ll<<<(unsigned)((n + 255) / 256), 256, 0, c.stream>>>(p, n);
   return cudaGetLastError() == cudaSuccess ? PDGPU_OK : PDGPU_ERR_CUDA;
 }
 

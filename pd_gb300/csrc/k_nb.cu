@@ -217,8 +217,8 @@ __device__ __noinline__ void nb_energy_large(const DevView& v, const NBConst& k,
   if (a < 0 || b < 0) return;
   const double eps = v.sqeps[a] * v.sqeps[b] * (is14 ? k.vdw14_d : 1.0);
   const double qq = v.charge[a] * v.charge[b] * k.econv_diel_d * (is14 ? k.elec14_d : 1.0);
-  double ev = 0.0, ee = 0.0, f, vir;
-  nb_pair<double, ELEC>(k, nb_r2_fp64(v, S, si, sj), v.radius[a] + v.radius[b], eps, qq, ev, ee, f, vir);
+  double ev = 0.0, ee = 0.0, vir;
+  nb_pair<ELEC>(k, nb_r2_fp64(v, S, si, sj), v.radius[a] + v.radius[b], eps, qq, ev, ee, vir);
   long long* E = v.eacc + (size_t)v.slot_sys[si >> 5] * E_NSLOTS;
   atomic_add_ll(&E[E_VDW], fix_energy_d(ev));
   atomic_add_ll(&E[E_ELEC], fix_energy_d(ee));
@@ -313,7 +313,8 @@ __device__ __forceinline__ void nb_energy_df2(const DevView& v, const NBConst& k
     } else if (ELEC == 4) {
       // Steinbach & Brooks force switch, nonbonded.cpp:798-819
       const bool oa = r.h.x > e.inner.h, ob = r.h.y > e.inner.h;
-      DF2 h = df_sub(ir, df2(e.eshift));
+      DF2 h = df_norm(df_sub(ir, df2(e.eshift)));
+      h.l = __fadd2_rn(h.l, f2(-e.eshift_t));
       if (oa || ob) {
         DF2 c2 = df_norm(df_sub(df2(e.cut2), r2)), c3 = df_norm(df_add(df2(e.fsw_k), df_scale2(r2, 2.f)));
         c2.l = __fadd2_rn(c2.l, f2(e.cut2_t));
@@ -321,11 +322,14 @@ __device__ __forceinline__ void nb_energy_df2(const DevView& v, const NBConst& k
         // qq sA / r (C^2 - r^2)^2 (C^2 - 3 I^2 + 2 r^2)
         const DF2 f = df_mul(df_sqr(c2), c3);
         fe = df_select(oa, ob, df_mul(df_norm(df_mul(df2(e.sA), f)), fe), fe);
-        // -qq (sA r (sB / r^2 + sC + sD r^2 + sE r^4) - V(C))
-        DF2 g = df_norm(df_add(df2(e.sD), df_mul(df2(e.sE), r2)));
-        g = df_norm(df_add(df2(e.sC), df_mul(g, r2)));
-        g = df_norm(df_add(df_mul(g, r), df_mul(df2(e.sB), ir)));
-        h = df_select(oa, ob, df_sub(df2(e.cutV), df_mul(df2(e.sA), g)), h);
+        // qq sA (C - r)^3 Q(r) / r
+        DF2 c = df_norm(df_sub(df2(e.cut), r));
+        c.l = __fadd2_rn(c.l, f2(e.cut_t));
+        DF2 g = df_norm(df_add(df2(e.q2), df_mul(df2(e.q3), r)));
+        g = df_norm(df_add(df2(e.q1), df_mul(g, r)));
+        g = df_norm(df_add(df2(e.q0), df_mul(g, r)));
+        g = df_mul(df_norm(df_mul(g, ir)), df_norm(df_mul(df_sqr(c), c)));
+        h = df_select(oa, ob, df_mul(df2(e.sA), df_norm(g)), h);
       }
       Ee = df_mul(qq, df_norm(h));
     }

@@ -158,12 +158,15 @@ NBEConst pdgpu::make_nbe_const(const NBConst& k) {
   e.inner = df_split(k.inner_d);
   e.invw2 = df_split(k.invw2_d);
   e.sA = df_split(k.sA);
-  e.sB = df_split(k.sB);
-  e.sC = df_split(k.sC);
-  e.sD = df_split(k.sD);
-  e.sE = df_split(k.sE);
-  e.cutV = df_split(k.fsw_cutV);
+  const double C = std::sqrt(k.cut2_d);
+  e.cut = df_split(C);
+  e.cut_t = df_rest(C);
+  e.q0 = df_split(C * (k.cut2_d - 3.0 * k.inner2_d));
+  e.q1 = df_split(1.4 * k.cut2_d - k.inner2_d);
+  e.q2 = df_split(1.2 * C);
+  e.q3 = df_split(0.4);
   e.eshift = df_split(k.eshift);
+  e.eshift_t = df_rest(k.eshift);
   e.cut2 = df_split(k.cut2_d);
   e.fsw_k = df_split(k.cut2_d - 3.0 * k.inner2_d);
   e.vdwinner_t = df_rest(k.vdwinner_d);
@@ -1025,11 +1028,6 @@ int pdgpu_rebuild_list(pdgpu_ctx* h) {
 
 }  // extern "C"
 
-// One force evaluation on the context stream (no host synchronisation).
-// rebuild: rebuild the list first (else pack the positions and check the skin).
-// LCPO forces go to lcpo_f and its energy to lcpo_e (stride lcpo_e_stride) when
-// run_lcpo; dynamics points them at the cached-LCPO buffers.  packed: the last
-// integrator packed the positions and cleared the accumulators already.
 // (set-up failure) the context's streams and events
 void pdgpu::release_streams(Context& c) {
   if (c.ev_fork) cudaEventDestroy(c.ev_fork);
@@ -1045,6 +1043,11 @@ void pdgpu::release_streams(Context& c) {
   c.side = c.side2 = c.stream = nullptr;
 }
 
+// One force evaluation on the context stream (no host synchronisation).
+// rebuild: rebuild the list first (else pack the positions and check the skin).
+// LCPO forces go to lcpo_f and its energy to lcpo_e (stride lcpo_e_stride) when
+// run_lcpo; dynamics points them at the cached-LCPO buffers.  packed: the last
+// integrator packed the positions and cleared the accumulators already.
 int pdgpu::enqueue_forces(Context& c, unsigned what, bool energy, bool rebuild, long long* lcpo_f,
                           long long* lcpo_e, int lcpo_e_stride, bool run_lcpo, bool packed) {
   c.clear.facc = c.d_facc.p;

@@ -109,8 +109,12 @@ struct NBConst {
 struct NBEConst {
   DF econv, vdw14, elec14;
   DF vdwcut, vdwinner, vdwinvw2, inner, invw2;
-  DF sA, sB, sC, sD, sE, cutV, eshift, cut2, fsw_k;   // fsw_k = cut2 - 3 inner2
-  float vdwinner_t, inner_t, cut2_t, fsw_t;           // what the double-floats leave of these radii
+  DF sA, eshift, cut, cut2, fsw_k;                    // fsw_k = cut2 - 3 inner2
+  // the force switch's energy is qq sA (C - r)^3 Q(r) / r with Q = q0 + q1 r + q2 r^2 + q3 r^3:
+  // PD's sum of powers and its value at C, of which little is left at r near C, divided by
+  // their triple root
+  DF q0, q1, q2, q3;
+  float vdwinner_t, inner_t, cut_t, cut2_t, fsw_t, eshift_t;   // what the double-floats leave of these
   int dovdw, vdw_hard;   // vdw_hard: LJ ends at VdwCutoff without a switch
 };
 

@@ -94,7 +94,6 @@ inline MDView md_view(Context& c, MDState& md) {
 int launch_integrate(Context& c, MDState& md, bool first, bool last);
 int launch_integrate_pack(Context& c, MDState& md);
 int launch_remd(Context& c, MDState& md, int parity, unsigned long long round);
-int launch_zero_ll(Context& c, long long* p, size_t n);
 // crash rescue: flags non-finite systems into bad_host (nsys ints, synchronous)
 // and restores them from the checkpoint with fresh velocities
 int launch_rescue(Context& c, MDState& md, unsigned long long seed, int* bad_host);

@@ -122,32 +122,19 @@ __device__ __forceinline__ int pair_bondorder(const DevView& v, int a, int b) {
   return best;
 }
 
-// Pair law in arithmetic type T (float for forces, double for energies).
-template <typename T, int ELEC>
-__device__ __forceinline__ void nb_pair(const NBConst& k, T r2, T rsum, T eps, T qq, T& ev, T& ee, T& dEdr_over_r,
-                                        T& r_dEdr) {
-  T invr, r;
-  if (sizeof(T) == 4) {
-    invr = rsqrtf((float)r2);
-    r = r2 * invr;
-  } else {
-    r = sqrt((double)r2);
-    invr = (T)1 / r;
-  }
-  T dv = 0, de = 0, Ev = 0, Ee = 0;
-  if (k.dovdw && r < (T)k.vdwcut_d) {
-    T t = rsum * invr;
-    T B = t * t;
-    B = B * B * B;
-    T A = B * B;
-    Ev = eps * (A - (T)2 * B);
-    dv = (T)-12 * eps * invr * (A - B);
-    if (r > (T)k.vdwinner_d) {
-      T u = r - (T)k.vdwinner_d;
-      T sw = (T)1 - u * u * (T)k.vdwinvw2_d;
-      T dS = (T)-4 * (T)k.vdwinvw2_d * u * sw;
-      T S = sw * sw;
-      dv = S * dv + Ev * dS;
+// FF_NonBonded's pair law in FP64 (Monte Carlo updates, energies of overlapping pairs)
+template <int ELEC>
+__device__ __forceinline__ void nb_pair(const NBConst& k, double r2, double rsum, double eps, double qq, double& ev,
+                                        double& ee, double& r_dEdr) {
+  const double r = sqrt(r2), invr = 1.0 / r;
+  double dv = 0.0, de = 0.0, Ev = 0.0, Ee = 0.0;
+  if (k.dovdw && r < k.vdwcut_d) {
+    const double t = rsum * invr, t2 = t * t, B = t2 * t2 * t2, A = B * B;
+    Ev = eps * (A - 2.0 * B);
+    dv = -12.0 * eps * invr * (A - B);
+    if (r > k.vdwinner_d) {
+      const double u = r - k.vdwinner_d, sw = 1.0 - u * u * k.vdwinvw2_d, S = sw * sw;
+      dv = S * dv + Ev * (-4.0 * k.vdwinvw2_d * u * sw);
       Ev *= S;
     }
   }
@@ -157,35 +144,30 @@ __device__ __forceinline__ void nb_pair(const NBConst& k, T r2, T rsum, T eps, T
   } else if (ELEC == 3) {
     Ee = qq * invr;
     de = -Ee * invr;
-    if (r > (T)k.inner_d) {
-      T u = r - (T)k.inner_d;
-      T sw = (T)1 - u * u * (T)k.invw2_d;
-      T dS = (T)-4 * (T)k.invw2_d * u * sw;
-      T S = sw * sw;
-      de = S * de + Ee * dS;
+    if (r > k.inner_d) {
+      const double u = r - k.inner_d, sw = 1.0 - u * u * k.invw2_d, S = sw * sw;
+      de = S * de + Ee * (-4.0 * k.invw2_d * u * sw);
       Ee *= S;
     }
   } else if (ELEC == 4) {
     // Steinbach & Brooks force switch, nonbonded.cpp:798-819
-    if (r > (T)k.inner_d) {
-      T c2mr2 = (T)k.cut2_d - r2;
-      de = -qq * (T)k.sA * invr * invr * c2mr2 * c2mr2 * ((T)k.cut2_d - (T)3 * (T)k.inner2_d + (T)2 * r2);
-      Ee = -qq * ((T)k.sA * r * ((T)k.sB * invr * invr + (T)k.sC + (T)k.sD * r2 + (T)k.sE * r2 * r2) - (T)k.fsw_cutV);
+    if (r > k.inner_d) {
+      const double c2mr2 = k.cut2_d - r2;
+      de = -qq * k.sA * invr * invr * c2mr2 * c2mr2 * (k.cut2_d - 3.0 * k.inner2_d + 2.0 * r2);
+      Ee = -qq * (k.sA * r * (k.sB * invr * invr + k.sC + k.sD * r2 + k.sE * r2 * r2) - k.fsw_cutV);
     } else {
       de = -qq * invr * invr;
-      Ee = qq * (invr - (T)k.eshift);
+      Ee = qq * (invr - k.eshift);
     }
   }
   ev += Ev;
   ee += Ee;
-  T d = dv + de;
-  dEdr_over_r = d * invr;
-  r_dEdr = r * d;
+  r_dEdr = r * (dv + de);
 }
 
 // FP64 squared distance of two sorted slots from the original positions
-// (minimum image in a periodic box); used for energies and for pairs whose
-// FP32 distance lies within 2e-6 of a hard cutoff.
+// (minimum image in a periodic box): pairs whose FP32 distance lies within 2e-6
+// of a hard cutoff, and overlapping pairs' energies.
 __device__ __forceinline__ double r2_fp64(const DevView& v, const SystemInfo& S, int sa, int sb) {
   int a = v.sorted_atom[sa], b = v.sorted_atom[sb];
   if (a < 0 || b < 0) return 1e300;
