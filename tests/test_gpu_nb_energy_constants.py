@@ -125,3 +125,38 @@ def test_energies_of_overlapping_atoms_are_fp64():
             for key, ref in (("vdw", se2 * (B * B - 2.0 * B)), ("elec", ECONV * 0.7 * 0.4 / abs(d)),
                              ("virial", -12.0 * se2 * (B * B - B) - ECONV * 0.7 * 0.4 / abs(d))):
                 assert abs(e[key] - ref) <= 2.0 ** -49 * abs(ref) + 2.0 ** -31, (r, image, key, e[key] - ref, ref)
+
+
+def test_sum_of_force_switched_pairs():
+    """Coulomb with the force switch, 10,000 pairs across its shell: PD's powers of r
+    (nonbonded.cpp:798-819) in extended precision.  Held as pairs of FP32 numbers, their
+    constants are off by 2^-49, some 1e-14 of qq in the difference of powers, alike for every
+    pair: 5e-7 kcal/mol in all."""
+    cut, inner, N, m = 10.39, 9.04, 10_000, 22
+    ld = np.longdouble
+    if np.finfo(ld).eps > 1e-18:
+        pytest.skip("no extended precision on this host")
+    rng = np.random.default_rng(7)
+    pos = np.repeat(30.0 * np.stack(np.unravel_index(np.arange(N), (m, m, m)), 1), 2, axis=0)
+    pos[1::2, 0] += rng.uniform(inner + 0.1, cut - 0.1, N)
+    r = (pos[1::2, 0] - pos[0::2, 0]).astype(ld)
+    from pd_gb300 import ffi
+    from pd_gb300.engine import DeviceContext
+    from pd_gb300.workspace import SystemImage
+    im = SystemImage([2 * N], np.zeros(3), np.full(2 * N, 3.0), np.zeros(2 * N), np.zeros(2 * N), np.full(2 * N, 2e-26),
+                     np.zeros((0, 3), np.int32), pos=pos)
+    ctx = DeviceContext(im)
+    ctx.set_list(1.0)
+    ctx.set_nb(Cutoff=cut, InnerCutoff=inner, VdwCutoff=cut, VdwInnerCutoff=inner, Vdw14Scaling=1.0, Elec14Scaling=1.0,
+               Dielectric=1.0, EnergySwitch=0, ForceSwitch=1, DoVdw=1, DoElec=1)
+    ctx.set_positions(pos)
+    e = ctx.compute(ffi.NB)[0]["elec"] / KCAL
+    ctx.close()
+    C, I = ld(cut), ld(inner)
+    V = lambda x: (-(C ** 6 - 3 * C ** 4 * I ** 2) / x + 6 * C * C * I * I * x - (C * C + I * I) * x ** 3 + ld(2) / 5 * x ** 5) / (
+        C * C - I * I) ** 3
+    qq = 9.0 * ECONV
+    E = (-ld(qq) * (V(r) - V(C))).astype(np.float64)
+    tol = _allowed(N, float(np.abs(E).max()), qq / inner ** 2 * cut)
+    assert 5e-7 > 2.5 * tol
+    assert abs(e - math.fsum(E)) <= tol, (e - math.fsum(E), tol)
