@@ -633,7 +633,8 @@ __global__ void __launch_bounds__(kNbEThreads, 8)
 enum NBLaw { kLawSame = 0, kLawSplit = 1, kLawForce = 2, kLawVdw = 3 };
 
 // dE/dr / r of two pairs; QQ = -econv q q, SS the radius sums, EE = eps.
-// Switch S = s^2, s = 1 - u^2 clamped at 0, u = (r - inner) / w clamped at 0.
+// Switch S = s^2, s = 1 - u^2 / w^2 clamped at 0, u = r - inner clamped at 0 (that difference
+// is exact; r and the inner radius over a width rounded in FP32 move the shell by 7e-7 of it).
 template <int LAW>
 __device__ __forceinline__ float2 nb_law2(const NBConst& k, float2 r2, float2 QQ, float2 SS, float2 EE) {
   const float2 M1 = f2(-1.f);
@@ -643,23 +644,23 @@ __device__ __forceinline__ float2 nb_law2(const NBConst& k, float2 r2, float2 QQ
   const float2 b6 = __fmul2_rn(__fmul2_rn(t2, t2), t2);
   const float2 eb = __fmul2_rn(EE, b6), ea = __fmul2_rn(eb, b6);      // eps B, eps A
   const float2 t = __ffma2_rn(eb, M1, ea), ev = __ffma2_rn(eb, M1, t);   // eps (A - B), eps (A - 2B)
-  float2 u = __ffma2_rn(r, f2(k.vdwiw_f), f2(-k.vdwinner_iw_f));
+  float2 u = __fadd2_rn(r, f2(-k.vdwinner_f));
   u = make_float2(fmaxf(u.x, 0.f), fmaxf(u.y, 0.f));
-  float2 s = __ffma2_rn(__fmul2_rn(u, u), M1, f2(1.f));
+  float2 s = __ffma2_rn(__fmul2_rn(u, u), f2(-k.vdwinvw2_f), f2(1.f));
   s = make_float2(fmaxf(s.x, 0.f), fmaxf(s.y, 0.f));
   const float2 Sv = __fmul2_rn(__fmul2_rn(s, s), ir2);                                 // S / r^2
-  const float2 nv = __fmul2_rn(__fmul2_rn(u, s), __fmul2_rn(ir, f2(-4.f * k.vdwiw_f)));   // S' / r
+  const float2 nv = __fmul2_rn(__fmul2_rn(u, s), __fmul2_rn(ir, f2(-4.f * k.vdwinvw2_f)));   // S' / r
   if (LAW == kLawVdw) return __ffma2_rn(__fmul2_rn(t, f2(-12.f)), Sv, __fmul2_rn(ev, nv));
   const float2 e1 = __fmul2_rn(QQ, ir);   // -E_coulomb
   if (LAW == kLawSame) return __ffma2_rn(__ffma2_rn(t, f2(-12.f), e1), Sv, __fmul2_rn(__ffma2_rn(e1, M1, ev), nv));
   const float2 gv = __ffma2_rn(__fmul2_rn(t, f2(-12.f)), Sv, __fmul2_rn(ev, nv));
   if (LAW == kLawSplit) {
-    u = __ffma2_rn(r, f2(k.iw_f), f2(-k.inner_iw_f));
+    u = __fadd2_rn(r, f2(-k.inner_f));
     u = make_float2(fmaxf(u.x, 0.f), fmaxf(u.y, 0.f));
-    s = __ffma2_rn(__fmul2_rn(u, u), M1, f2(1.f));
+    s = __ffma2_rn(__fmul2_rn(u, u), f2(-k.invw2_f), f2(1.f));
     s = make_float2(fmaxf(s.x, 0.f), fmaxf(s.y, 0.f));
     const float2 Se = __fmul2_rn(__fmul2_rn(s, s), ir2);
-    const float2 ne = __fmul2_rn(__fmul2_rn(u, s), __fmul2_rn(ir, f2(4.f * k.iw_f)));
+    const float2 ne = __fmul2_rn(__fmul2_rn(u, s), __fmul2_rn(ir, f2(4.f * k.invw2_f)));
     return __ffma2_rn(e1, Se, __ffma2_rn(e1, ne, gv));
   }
   // Steinbach & Brooks force switch, nonbonded.cpp:798-819

@@ -140,10 +140,6 @@ NBConst pdgpu::make_nb_const(const pdgpu_nb_params& p) {
   k.dovdw = p.DoVdw ? 1 : 0;
   k.samesw = (k.elecmode == 3 && k.dovdw && p.VdwCutoff == p.Cutoff && p.VdwInnerCutoff == p.InnerCutoff) ? 1 : 0;
   k.smooth = k.dovdw && vw > 0 && p.VdwCutoff <= p.Cutoff && (k.elecmode == 0 || (k.elecmode >= 3 && w > 0)) ? 1 : 0;
-  k.vdwiw_f = vw > 0 ? (float)(1.0 / vw) : 0.f;
-  k.vdwinner_iw_f = vw > 0 ? (float)(p.VdwInnerCutoff / vw) : 0.f;
-  k.iw_f = w > 0 ? (float)(1.0 / w) : 0.f;
-  k.inner_iw_f = w > 0 ? (float)(I / w) : 0.f;
   return k;
 }
 

@@ -102,7 +102,6 @@ struct NBConst {
   // 1: LJ and Coulomb (if any) both end by a switch, LJ not beyond Cutoff, so the
   // law is continuous at every cutoff (the packed force pass)
   int smooth;
-  float vdwiw_f, vdwinner_iw_f, iw_f, inner_iw_f;   // 1 / switch width, inner radius / width
 };
 
 // The same constants as double-floats, for the pair energies (FF_NonBonded)
