@@ -355,9 +355,12 @@ class Forcefield:
         left its skin: PD's callers may move atoms at will between two calls.  A list
         that proves stale (a non-finite or overflowing result may come of one as well)
         is rebuilt and the call repeated; while every call comes with new coordinates
-        like that, the list is rebuilt before the call instead."""
+        like that, the list is rebuilt before the call instead.  Without padding there
+        is no skin to leave, and every call gets a list of its own."""
         ws = self.wspace
-        if ws._moved_from is not None:
+        if ws.Padding <= 0:
+            ctx.rebuild_list()
+        elif ws._moved_from is not None:
             if 2.0 * np.abs(ws.cur.p - ws._moved_from).max() > ws.Padding:
                 ctx.rebuild_list()
                 ws._moved_from = ws.cur.p.copy()
