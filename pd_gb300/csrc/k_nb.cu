@@ -124,13 +124,14 @@ __device__ __forceinline__ void nb_rot(const DevView& v, const NBConst& k, const
 // items and skipping and nothing else in the loop, and deals the list over the
 // lanes, so the ~300 instructions of a pair's energy run on full warps; an item
 // passes its odd pairs on from one eighth to the next.  Against 64-bit sums the
-// energies are within 2e-8 kcal/mol (one fixed-point rounding per item).
+// energies are within 3e-8 kcal/mol on up to 89,956 atoms (one fixed-point rounding per
+// item); the same pass with constants short of 64 bits left 1.2e-7, and 1.3e-4 in virials.
 // Bound by the FMA pipe and, in small systems, by the latency of its chains: two pairs
 // a lane in packed arithmetic.  FP64 pair energies on the rotation, with the forces:
 // 5.85 ms on the solvated 22,489 atoms at 15 A (force switch), 0.331 ms on 667 waters
 // at 12 A; scalar double-float on a list kept by the force rotation: 0.461 and 0.046
-// ms, 0.119 ms on 4,235 atoms without cutoff; this pass 0.334, 0.031 and 0.097 ms beside
-// force passes of 0.060, 0.011 and 0.019 ms (left out of calls that read no forces).
+// ms, 0.119 ms on 4,235 atoms without cutoff; this pass 0.366, 0.032 and 0.105 ms beside
+// force passes of 0.060, 0.009 and 0.019 ms (left out of calls that read no forces).
 // ---------------------------------------------------------------------------
 
 // remainders of the packed slots (before each energy pass)
@@ -227,7 +228,7 @@ __device__ __noinline__ void nb_energy_large(const DevView& v, const NBConst& k,
 
 // energies of two listed pairs into the sums (same law as the force bodies; pair b
 // counts only if two).  Products of products stay unnormalised where their l holds a
-// few roundings of h: what df_mul leaves out is then below 1e-13.
+// few roundings of h: what df_mul leaves out is then below 1e-13, of either sign.
 template <int ELEC, bool SW>
 __device__ __forceinline__ void nb_energy_df2(const DevView& v, const NBConst& k, const NBEConst& e,
                                               const SystemInfo& S, const NBEBox& box, int ibase, const NBEShared* sh,
