@@ -20,16 +20,31 @@ _PLAIN = frozenset((int, float, bool, str, type(None)))
 _NO_SETTING = frozenset(("needsetup", "totalSASA", "wspace"))
 
 
+class _Object:
+    """Stands for an attribute that has no value to compare: the same object or not."""
+
+    def __init__(self, v):
+        self.v = v
+
+    def __eq__(self, other):
+        return isinstance(other, _Object) and self.v is other.v
+
+
 def _plain(v):
-    """A setting as it compares with an earlier value of itself: NumPy scalars and
-    containers by value (a copy, so that changes in place show)."""
+    """A setting as it compares with an earlier value of itself: numbers and containers
+    by value (a copy, so that changes in place show)."""
     if isinstance(v, (np.generic, np.ndarray)):
         return v.item() if v.ndim == 0 else (v.shape, v.dtype.str, v.tobytes())
     if isinstance(v, (list, tuple)):
         return tuple(_plain(x) for x in v)
     if isinstance(v, dict):
         return tuple((k, _plain(x)) for k, x in v.items())
-    return v
+    if v is None or isinstance(v, str):
+        return v
+    try:
+        return float(v)                # (what the context gets of it: 0-d tensors, fractions)
+    except (TypeError, ValueError, RuntimeError, OverflowError):
+        return _Object(v)
 
 
 class ForcefieldBase:

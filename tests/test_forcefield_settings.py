@@ -85,6 +85,22 @@ def test_a_cutoff_scan_reaches_the_context(workspace, values):
     assert ctx.settings == 2 * len(values)                  # once a value: nb and list
 
 
+def test_settings_of_other_types(workspace):
+    torch = pytest.importorskip("torch")
+    ff, nb = _container(workspace, pdg.FF_NonBonded_GPU)
+    nb.InnerCutoff = nb.VdwInnerCutoff = 8.0
+    nb.notes = {"a": [1, np.arange(3)]}
+    nb.table, nb.callback = torch.arange(4), print          # (no settings: kept, not compared element by element)
+    cut = torch.tensor(9.0)
+    for v in (9.0, 11.5):
+        cut.fill_(v)
+        nb.Cutoff = nb.VdwCutoff = cut
+        ff.calcForces()
+        ff.calcForces()
+    ctx = workspace.context()
+    assert [k["Cutoff"] for k in ctx.nb] == [9.0, 11.5] and ctx.settings == 4
+
+
 def test_values_of_one_hash(workspace):
     ff, gb = _container(workspace, pdg.FF_GeneralizedBorn_Still_GPU)
     values = [-4.0, -1.0, -2.0, np.float32(-1), np.int64(-2)]
